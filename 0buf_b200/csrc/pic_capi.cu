@@ -141,12 +141,49 @@ int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
     return PIC_OK;
 }
 
+// CTAs per tile of the next push.  The GPU holds two push CTAs per SM; with
+// fewer tiles than that, one CTA per tile leaves SMs idle (the reference's
+// default run has 13 tiles: push 10.5 ms), so a tile's bins are shared out to
+// as many CTAs as fit at once, each of at least one 256-particle iteration.
+// Where such a share is long, twice as many even out its length.  Measured
+// push, us, by CTAs per tile:
+//   FP64 100x4x4 x 1300 (13 tiles):  1 10508, 11 1161, 22 712, 23 693, 45 680, 91 672
+//   FP32 100x4x4 x 1300 (17 tiles):  1 1441, 8 247, 17 183, 34 181, 52 183
+//   FP64 32x4x4 x 32 (4 tiles):      1 242, 4 90, 12 48, 24 40, 48 33
+//   FP32 37x13x21 x 17 (84 tiles):   1 61.7, 2 50.0, 3 48.0, 4 44.0, 5 52.1
+// From that many tiles on, sharing costs more than the idle part of the last
+// wave (each CTA stages the fields and flushes a tile current of its own):
+//   FP64 64x32x32 x 16 (256 tiles):  1 335, 2 403, 3 401
+//   FP32 64x32x32 x 16 (352 tiles):  1 133, 2 135, 3 134, 4 154
+//   FP64 128x32x32 x 32 (512 tiles): 1 1260, 2 1424, 4 1362
+int push_slices(pic_handle *h) {
+    const int64_t resident = 2 * h->sms, fit = resident / h->g.ntiles;
+    if (fit < 2) return 1;
+    int64_t cap = 0;
+    for (int s = 0; s < h->cfg.nspecies; s++) cap += h->sp[s].cap_total;
+    const int64_t blocks = std::max<int64_t>(1, cap / h->g.ntiles / kPushThreads);  // iterations of one tile
+    return (int)std::min(blocks / fit >= 64 ? 2 * fit : fit, blocks);
+}
+
+size_t split_ints(const pic_handle *h) { return (size_t)h->cfg.nspecies * h->g.ntiles * kHoleMax; }
+
+int ensure_split(pic_handle *h) {
+    if (h->split_buf) return PIC_OK;
+    const size_t n = split_ints(h) + (size_t)(h->cfg.nspecies + 1) * h->g.ntiles;
+    CK(cudaMalloc(&h->split_buf, n * sizeof(int)), "alloc hole lists");
+    return PIC_OK;
+}
+
 int ensure_outbox(pic_handle *h) {
     if (h->outbox_pinned) return PIC_OK;  // leftovers of an overflowing insert still live in it
     int64_t total = 0;
     for (int s = 0; s < h->cfg.nspecies; s++) total += h->sp[s].cap_total;
     double frac = h->cfg.outbox_fraction > 0 ? h->cfg.outbox_fraction : 0.04;
     int64_t want = (int64_t)(frac * (double)total) + 65536;
+    // the FP32 push leaves up to a chunk per warp unused: keep that out of the
+    // share of the particles when several CTAs work on a tile
+    const int slices = push_slices(h);
+    if (h->mixed && slices > 1) want += (int64_t)h->g.ntiles * slices * (kPushThreads / 32) * kOutboxChunk;
     if (want > 0x7fffffffLL) want = 0x7fffffffLL;
     if (h->outbox && (int64_t)h->out_cap >= want) return PIC_OK;
     if (h->outbox) cudaFree(h->outbox);
@@ -374,6 +411,15 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
     }
     StepParams p = make_params(h);
     p.b_half = b_half_in_push;
+    p.slices = push_slices(h);
+    if (p.slices > 1) {
+        if ((rc = ensure_split(h))) return rc;
+        const size_t nc = (size_t)h->cfg.nspecies * h->g.ntiles;
+        p.holes = h->split_buf;
+        p.hole_count = (unsigned *)(h->split_buf + split_ints(h));
+        p.ticket = p.hole_count + nc;
+        CK(cudaMemsetAsync(p.hole_count, 0, (nc + h->g.ntiles) * sizeof(unsigned), h->stream), "reset hole counts");
+    }
     cudaEventRecord(h->ev[2], h->stream);
     CK(h->mixed ? launch_push_mixed(p, h->maps, h->stream) : launch_push_plain(p, plain_lo32(h), h->stream),
        "push_deposit");
@@ -511,6 +557,8 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
     int rc = set_device(h);
     if (rc) { delete h; return rc; }
     size_t smem = h->mixed ? push_smem_total_mixed(g) : push_smem_plain(g);
+    h->sms = 148;
+    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     if (smem > (size_t)optin) { delete h; return PIC_ERR_ARG; }
@@ -571,6 +619,7 @@ int pic_destroy(pic_handle *h) {
     if (h->hred) cudaFreeHost(h->hred);
     if (h->dcounts) cudaFree(h->dcounts);
     if (h->lb_buf) cudaFree(h->lb_buf);
+    if (h->split_buf) cudaFree(h->split_buf);
     release_load_scratch(h);
 
     double *diag[3] = {h->rho, h->gauss, h->gauss0};

@@ -73,6 +73,10 @@ struct pic_handle {
     // (release_load_scratch)
     void *load_buf;
     size_t load_bytes;
+    // pushes with several CTAs per tile (StepParams::slices): hole lists and,
+    // after them, hole counts and tickets; allocated at the first such push
+    int *split_buf;
+    int sms;  // SMs of the device
 };
 
 namespace pic_host {

@@ -26,7 +26,8 @@ namespace pic {
 
 constexpr int kMaxSpecies = PIC_MAX_SPECIES;
 constexpr int kHoleMax = 1024;          // departures per tile per species handled in-kernel
-constexpr int kPushThreads = 256;
+constexpr int kPushThreads = 256;       // threads of a push CTA: particles per block of a slice
+constexpr unsigned kOutboxChunk = 16;   // outbox slots a warp of the FP32 push takes at once
 
 // status flag bits (DevStatus::flags)
 enum : unsigned {
@@ -233,7 +234,85 @@ struct StepParams {
     // push forms the B half step of its staged tile itself (pic_step); zero
     // when the sub-step call pic_b_half has already advanced H
     int b_half;
+    // a tile's bins are shared out to `slices` CTAs (1: one CTA per tile; the
+    // pointers below are then unused).  The CTAs of a tile list their leavers'
+    // slots in holes ([species][tile][kHoleMax], filled to hole_count
+    // [species][tile]) and count themselves off in ticket[tile]; the last one
+    // compacts the tile's bins.  hole_count and ticket start a push at zero.
+    int slices;
+    int *holes;
+    unsigned *hole_count, *ticket;
 };
+
+// The particles of one species that slice q of P.slices of tile t handles:
+// [jbeg, jend) of the bin.  The bins of all species, cut into blocks of
+// `threads` particles and laid end to end, are dealt out evenly, so the slices
+// of a tile cover every particle once and each is a few whole iterations.
+struct SliceRange {
+    int lo, hi;  // blocks of this slice
+};
+__device__ __forceinline__ SliceRange slice_blocks(const StepParams &P, int t, int q, int threads) {
+    long long w = 0;
+    for (int s = 0; s < P.nsp; s++) w += (P.sp[s].tile_count[t] + threads - 1) / threads;
+    SliceRange r;
+    r.lo = (int)(w * q / P.slices);
+    r.hi = (int)(w * (q + 1) / P.slices);
+    return r;
+}
+// this slice's particles of a species whose first block is block `first`
+__device__ __forceinline__ void slice_range(const SliceRange &r, int first, int count, int threads, int &jbeg, int &jend) {
+    const long long a = (long long)(r.lo - first) * threads, b = (long long)(r.hi - first) * threads;
+    jbeg = (int)(a < 0 ? 0 : (a > count ? count : a));
+    jend = (int)(b < jbeg ? jbeg : (b > count ? count : b));
+}
+
+// True in the last CTA of tile t to get here, whose threads then see what the
+// tile's other CTAs wrote (fence, ticket, fence).  No CTA waits for another.
+// Every thread calls it; flag is shared memory.
+__device__ __forceinline__ bool last_of_tile(const StepParams &P, int t, int *flag) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *flag = atomicAdd(&P.ticket[t], 1u) == (unsigned)P.slices - 1u;
+        __threadfence();
+    }
+    __syncthreads();
+    return *flag != 0;
+}
+
+// Compaction of tile t's bin of species s by one CTA, from the holes that all
+// the tile's CTAs listed: the last live particles move into the holes in front
+// of the new count.  front: kHoleMax ints and ctr: 2 ints of shared memory;
+// move(dst, src) copies one particle.  The data comes from other SMs, so it is
+// read past L1 (__ldcg).
+template <class Move>
+__device__ __forceinline__ void compact_listed(const StepParams &P, int t, int s, int *front, int *ctr, unsigned &bad,
+                                               Move move) {
+    const SpeciesView &S = P.sp[s];
+    const size_t e = (size_t)s * P.g.ntiles + t;
+    const unsigned listed = __ldcg(&P.hole_count[e]);
+    if (listed == 0u || listed > (unsigned)kHoleMax) return;
+    const int nh = (int)listed, start = S.tile_start[t], newcount = S.tile_count[t] - nh;
+    const int *holes = P.holes + e * kHoleMax;
+    if (threadIdx.x == 0) ctr[0] = ctr[1] = 0;
+    __syncthreads();
+    for (int r = threadIdx.x; r < nh; r += blockDim.x) {
+        const int h = __ldcg(holes + r);
+        if (h < newcount) front[atomicAdd(&ctr[0], 1)] = h;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < nh; r += blockDim.x) {
+        const int src = start + newcount + r;
+        if (__ldcg(&S.cell[src]) >= 0) {
+            const int m = atomicAdd(&ctr[1], 1);
+            if (m >= ctr[0]) { bad |= ST_BADCELL; continue; }
+            move(start + front[m], src);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) S.tile_count[t] = newcount;
+    __syncthreads();
+}
 
 // FP32 form: TMA descriptors of the six E/H field arrays (3D {Nz+2, Ny+2,
 // Nx+2} FP32 with the pitched z row, box = one tile + halo); a kernel

@@ -336,7 +336,8 @@ constexpr int kMixedThreads = PIC_MIXED_THREADS;  // threads per CTA of k_push_m
 constexpr int kMixedWarps = kMixedThreads / 32;
 constexpr int kJCopies = kMixedWarps / 2;         // int32 tile currents per CTA: one per two warps
 constexpr int kQueue = PIC_MIXED_QUEUE;           // queued segments per warp
-constexpr unsigned kOutChunk = 16;                // outbox slots a warp takes from the global counter at once
+constexpr unsigned kOutChunk = kOutboxChunk;      // outbox slots a warp takes from the global counter at once
+static_assert(kMixedThreads == kPushThreads, "the slices of a tile are cut in blocks of kPushThreads particles");
 static_assert(kMixedThreads % 32 == 0, "whole warps");
 static_assert(kQueue >= 64, "one iteration can queue two segments per lane");
 
@@ -376,7 +377,8 @@ __host__ __device__ inline MixedSmem mixed_smem(int tx, int ty, int tz) {
 #define PIC_MIXED_BOUNDS __launch_bounds__(kMixedThreads, PIC_MIXED_MIN_BLOCKS)
 // TX, TY, TZ: the tile's cells per axis when fixed at compile time (shared-
 // memory offsets become immediates), 0 to take them from the grid
-template <int TX, int TY, int TZ>
+// SPLIT: P.slices CTAs share a tile (see StepParams::slices)
+template <int TX, int TY, int TZ, bool SPLIT>
 __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps maps, StepParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long sBar;
@@ -394,7 +396,9 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
     __shared__ float4 sQueue[kMixedWarps][kQueue][2];
     const Grid &g = P.g;
     const int tx = TX ? TX : g.tx, ty = TY ? TY : g.ty, tz = TZ ? TZ : g.tz;
-    const int t = blockIdx.x;
+    const int t = SPLIT ? blockIdx.x / P.slices : blockIdx.x;
+    SliceRange slice = {0, 0};
+    if (SPLIT) slice = slice_blocks(P, t, blockIdx.x - t * P.slices, kMixedThreads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     const unsigned lt = (1u << lane) - 1;
@@ -420,7 +424,13 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
     if (threadIdx.x == 0) {
         // quantum of the fixed-point tile J (see fx_add): |contribution| < 1.0834 |m| per segment
         double bound = 0.0;
-        for (int s = 0; s < P.nsp; s++) bound += 2.5 * fabs(P.sp[s].m) * (double)P.sp[s].tile_count[t];
+        for (int s = 0, first = 0; s < P.nsp; s++) {
+            const int count = P.sp[s].tile_count[t];
+            int jbeg = 0, jend = count;
+            if (SPLIT) slice_range(slice, first, count, kMixedThreads, jbeg, jend);
+            first += (count + kMixedThreads - 1) / kMixedThreads;
+            bound += 2.5 * fabs(P.sp[s].m) * (double)(jend - jbeg);
+        }
         int e2;
         frexp(bound, &e2);
         sQ = ldexp(1.0, e2 - 62);
@@ -499,11 +509,18 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
     unsigned ob_base = 0, ob_used = kOutChunk;
     bool ob_any = false;
 
-    for (int s = 0; s < P.nsp; s++) {
+    for (int s = 0, first = 0; s < P.nsp; s++) {
         const SpeciesView &S = P.sp[s];
         const int sp = s % 3;  // hole-list counters of this species
         const int start = S.tile_start[t];
-        const int count = S.tile_count[t];
+        // the particles [jbeg, count) of the bin are this CTA's
+        int count = S.tile_count[t], jbeg = 0;
+        if (SPLIT) {
+            const int all = count;
+            slice_range(slice, first, all, kMixedThreads, jbeg, count);
+            first += (all + kMixedThreads - 1) / kMixedThreads;
+            if (jbeg == count) continue;
+        }
         const float tau1 = (float)(S.q_m * g.tau * 0.5);
         const double M = S.m / S.q_m;
         // per-species deposit weights a*h/tau (see pqr_mixed)
@@ -552,8 +569,8 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         const int stride = blockDim.x;
         PartM nxt;
         nxt.cell = -1;
-        if (warp * 32 + lane < count) nxt = load_part(S, start + warp * 32 + lane);
-        for (int base = warp * 32; base < count; base += stride) {
+        if (jbeg + warp * 32 + lane < count) nxt = load_part(S, start + jbeg + warp * 32 + lane);
+        for (int base = jbeg + warp * 32; base < count; base += stride) {
             const int j = base + lane;
             const int slot = start + j;
             PartM cur = nxt;
@@ -731,7 +748,9 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
             if (lm) {
                 const int nl = __popc(lm), rank = __popc(lm & lt);
                 int hbase = 0;
-                if (lane == 0) hbase = atomicAdd(&sNHoles[sp], nl);
+                if (lane == 0)
+                    hbase = SPLIT ? (int)atomicAdd(&P.hole_count[(size_t)s * g.ntiles + t], (unsigned)nl)
+                                  : atomicAdd(&sNHoles[sp], nl);
                 hbase = __shfl_sync(FULL, hbase, 0);
                 const unsigned room = kOutChunk - ob_used;
                 unsigned nb = 0;
@@ -768,7 +787,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                     }
                     S.cell[slot] = -1;
                     const int hpos = hbase + rank;
-                    if (hpos < kHoleMax) sHoles[hpos] = j;
+                    if (hpos < kHoleMax) (SPLIT ? P.holes + ((size_t)s * g.ntiles + t) * kHoleMax : sHoles)[hpos] = j;
                     else bad |= ST_HOLES;
                 }
             }
@@ -795,7 +814,8 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         }
         // compaction: the last live particles of the bin move into the holes in
         // front of the new count
-        const int nh = sNHoles[sp];
+        // (SPLIT: by the tile's last CTA, after its last species)
+        const int nh = SPLIT ? 0 : sNHoles[sp];
         if (nh > 0 && nh <= kHoleMax) {
             const int newcount = count - nh;
             for (int r = threadIdx.x; r < nh; r += blockDim.x) {
@@ -841,6 +861,16 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         double tot = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += sRed[w];
         atomicAdd(&P.st->kinetic, tot);
+    }
+    if (SPLIT && last_of_tile(P, t, &sNHoles[0])) {
+        for (int s = 0; s < P.nsp; s++) {
+            const SpeciesView &S = P.sp[s];
+            compact_listed(P, t, s, sFront, sHoles, bad, [&](int dst, int src) {
+                S.cell[dst] = __ldcg(&S.cell[src]);
+                S.ox[dst] = __ldcg(&S.ox[src]); S.oy[dst] = __ldcg(&S.oy[src]); S.oz[dst] = __ldcg(&S.oz[src]);
+                S.fx[dst] = __ldcg(&S.fx[src]); S.fy[dst] = __ldcg(&S.fy[src]); S.fz[dst] = __ldcg(&S.fz[src]);
+            });
+        }
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (moved) atomicAdd(&P.st->moved, moved);
@@ -942,27 +972,30 @@ size_t push_smem_mixed(const Grid &g) { return mixed_smem(g.tx, g.ty, g.tz).tota
 
 using PushMixedFn = void (*)(const MixedMaps, StepParams);
 // the instantiation for a grid's tile: fixed dimensions for the automatic tiles, else runtime
+template <bool SPLIT>
 static PushMixedFn push_mixed_fn(const Grid &g) {
-    if (g.tx == 6 && g.ty == 4 && g.tz == 8) return k_push_mixed<6, 4, 8>;
-    if (g.tx == 6 && g.ty == 4 && g.tz == 4) return k_push_mixed<6, 4, 4>;
-    if (g.tx == 4 && g.ty == 4 && g.tz == 12) return k_push_mixed<4, 4, 12>;
-    if (g.tx == 4 && g.ty == 4 && g.tz == 8) return k_push_mixed<4, 4, 8>;
-    if (g.tx == 4 && g.ty == 4 && g.tz == 4) return k_push_mixed<4, 4, 4>;
-    return k_push_mixed<0, 0, 0>;
+    if (g.tx == 6 && g.ty == 4 && g.tz == 8) return k_push_mixed<6, 4, 8, SPLIT>;
+    if (g.tx == 6 && g.ty == 4 && g.tz == 4) return k_push_mixed<6, 4, 4, SPLIT>;
+    if (g.tx == 4 && g.ty == 4 && g.tz == 12) return k_push_mixed<4, 4, 12, SPLIT>;
+    if (g.tx == 4 && g.ty == 4 && g.tz == 8) return k_push_mixed<4, 4, 8, SPLIT>;
+    if (g.tx == 4 && g.ty == 4 && g.tz == 4) return k_push_mixed<4, 4, 4, SPLIT>;
+    return k_push_mixed<0, 0, 0, SPLIT>;
 }
 
 size_t push_smem_total_mixed(const Grid &g) {
-    cudaFuncAttributes a;
-    if (cudaFuncGetAttributes(&a, push_mixed_fn(g)) != cudaSuccess) return (size_t)-1;
-    return push_smem_mixed(g) + a.sharedSizeBytes;
+    cudaFuncAttributes a, b;
+    if (cudaFuncGetAttributes(&a, push_mixed_fn<false>(g)) != cudaSuccess) return (size_t)-1;
+    if (cudaFuncGetAttributes(&b, push_mixed_fn<true>(g)) != cudaSuccess) return (size_t)-1;
+    return push_smem_mixed(g) + std::max(a.sharedSizeBytes, b.sharedSizeBytes);
 }
 
 cudaError_t launch_push_mixed(const StepParams &p, const MixedMaps &maps, cudaStream_t s) {
-    const PushMixedFn fn = push_mixed_fn(p.g);
+    const bool split = p.slices > 1;
+    const PushMixedFn fn = split ? push_mixed_fn<true>(p.g) : push_mixed_fn<false>(p.g);
     size_t smem = push_smem_mixed(p.g);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fn<<<p.g.ntiles, kMixedThreads, smem, s>>>(maps, p);
+    fn<<<p.g.ntiles * (split ? p.slices : 1), kMixedThreads, smem, s>>>(maps, p);
     return cudaGetLastError();
 }
 

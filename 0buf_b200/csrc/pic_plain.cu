@@ -286,12 +286,14 @@ constexpr int kPlainThreads = PIC_PLAIN_THREADS;  // threads per CTA of k_push_p
 // (at most 32 per drain), so it never holds more than 15 + 32 entries
 constexpr int kQPlain = 48;
 static_assert(kPlainThreads % 32 == 0, "whole warps");
+static_assert(kPlainThreads == kPushThreads, "the slices of a tile are cut in blocks of kPushThreads particles");
 #ifdef PIC_PLAIN_MIN_BLOCKS
 #define PIC_PLAIN_BOUNDS __launch_bounds__(kPlainThreads, PIC_PLAIN_MIN_BLOCKS)
 #else
 #define PIC_PLAIN_BOUNDS __launch_bounds__(kPlainThreads)
 #endif
-template <bool LO32>
+// SPLIT: P.slices CTAs share a tile (see StepParams::slices)
+template <bool LO32, bool SPLIT>
 __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sNHoles, sNFront, sNMove;
@@ -299,7 +301,9 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     __shared__ double sQ, sInvQ, sLoScale;
     __shared__ int sQn[kPlainThreads / 32];  // entries in each warp's segment queue
     const Grid &g = P.g;
-    const int t = blockIdx.x;
+    const int t = SPLIT ? blockIdx.x / P.slices : blockIdx.x;
+    SliceRange slice = {0, 0};
+    if (SPLIT) slice = slice_blocks(P, t, blockIdx.x - t * P.slices, kPlainThreads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tk = t % g.ntz, tl = (t / g.ntz) % g.nty, ti = t / (g.ntz * g.nty);
     const int i0 = ti * g.tx, l0 = tl * g.ty, k0 = tk * g.tz;
@@ -318,9 +322,13 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     if (threadIdx.x == 0) {
         double bound = 0.0;
         long long ntile = 0;
-        for (int s = 0; s < P.nsp; s++) {
-            bound += 2.5 * fabs(P.sp[s].m) * (double)P.sp[s].tile_count[t];
-            ntile += P.sp[s].tile_count[t];
+        for (int s = 0, first = 0; s < P.nsp; s++) {
+            const int count = P.sp[s].tile_count[t];
+            int jbeg = 0, jend = count;
+            if (SPLIT) slice_range(slice, first, count, kPlainThreads, jbeg, jend);
+            first += (count + kPlainThreads - 1) / kPlainThreads;
+            bound += 2.5 * fabs(P.sp[s].m) * (double)(jend - jbeg);
+            ntile += jend - jbeg;
         }
         int e2;
         frexp(bound, &e2);  // bound < 2^e2
@@ -357,19 +365,28 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     unsigned long long moved = 0, dropped = 0, dup = 0;
     OutPlain *outbox = (OutPlain *)P.outbox;
 
-    for (int s = 0; s < P.nsp; s++) {
+    for (int s = 0, first = 0; s < P.nsp; s++) {
         const SpeciesView &S = P.sp[s];
         const int start = S.tile_start[t];
-        const int count = S.tile_count[t];
+        // the particles [jbeg, count) of the bin are this CTA's
+        int count = S.tile_count[t], jbeg = 0;
+        if (SPLIT) {
+            const int all = count;
+            slice_range(slice, first, all, kPlainThreads, jbeg, count);
+            first += (all + kPlainThreads - 1) / kPlainThreads;
+            if (jbeg == count) continue;
+        }
         const double q_m = S.q_m, mw = S.m, M = S.m / S.q_m;
-        if (threadIdx.x == 0) { sNHoles = 0; sNFront = 0; sNMove = 0; }
-        __syncthreads();
+        if (!SPLIT) {
+            if (threadIdx.x == 0) { sNHoles = 0; sNFront = 0; sNMove = 0; }
+            __syncthreads();
+        }
         int qn = 0;  // entries in this warp's segment queue (warp-uniform)
         if (lane == 0) sQn[warp] = 0;
         __syncwarp();
         // Whole warps iterate together (the queue is drained by whole warps),
         // and past the last particle until the queue is empty.
-        for (int jw = threadIdx.x - lane;; jw += blockDim.x) {
+        for (int jw = jbeg + threadIdx.x - lane;; jw += blockDim.x) {
             const bool tail = jw >= count;
             if (tail && qn == 0) break;
             const int j = jw + lane;
@@ -567,9 +584,16 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                 }
                 if (leave) {
                     S.cell[slot] = -1;
-                    int hpos = atomicAdd(&sNHoles, 1);
-                    if (hpos < kHoleMax) sHoles[hpos] = j;
-                    else bad |= ST_HOLES;
+                    if (SPLIT) {
+                        const size_t e = (size_t)s * g.ntiles + t;
+                        const unsigned hpos = atomicAdd(&P.hole_count[e], 1u);
+                        if (hpos < (unsigned)kHoleMax) P.holes[e * kHoleMax + hpos] = j;
+                        else bad |= ST_HOLES;
+                    } else {
+                        int hpos = atomicAdd(&sNHoles, 1);
+                        if (hpos < kHoleMax) sHoles[hpos] = j;
+                        else bad |= ST_HOLES;
+                    }
                 } else {
                     S.cell[slot] = newcell;
                     S.x[slot] = x; S.y[slot] = y; S.z[slot] = z;
@@ -602,6 +626,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
             }
             __syncwarp();
         }
+        if (SPLIT) continue;  // the tile's last CTA compacts its bins
         __syncthreads();
         // ---- compaction of the tile bin (replaces GPU_MakeDepartureLists_rm, kernels.cu:219-242)
         const int L = sNHoles;
@@ -628,6 +653,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
         __syncthreads();
     }
 
+    if (SPLIT) __syncthreads();
     // ---- tile J -> global J (GPU_WriteAllCurrents, kernels.cu:83-112)
     for (int idx = threadIdx.x; idx < 3 * nn; idx += blockDim.x) {
         const long long ih = (long long)sJ[idx];
@@ -648,6 +674,17 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
         double tot = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) tot += sRed[w];
         atomicAdd(&P.st->kinetic, tot);
+    }
+    if (SPLIT && last_of_tile(P, t, &sNHoles)) {
+        int *ctr = sHoles;
+        for (int s = 0; s < P.nsp; s++) {
+            const SpeciesView &S = P.sp[s];
+            compact_listed(P, t, s, sFront, ctr, bad, [&](int dst, int src) {
+                S.cell[dst] = __ldcg(&S.cell[src]);
+                S.x[dst] = __ldcg(&S.x[src]); S.y[dst] = __ldcg(&S.y[src]); S.z[dst] = __ldcg(&S.z[src]);
+                S.px[dst] = __ldcg(&S.px[src]); S.py[dst] = __ldcg(&S.py[src]); S.pz[dst] = __ldcg(&S.pz[src]);
+            });
+        }
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (moved) atomicAdd(&P.st->moved, moved);
@@ -731,10 +768,12 @@ size_t push_smem_plain(const Grid &g) {
 
 cudaError_t launch_push_plain(const StepParams &p, bool lo32, cudaStream_t s) {
     size_t smem = push_smem_plain(p.g);
-    auto *kern = lo32 ? k_push_plain<true> : k_push_plain<false>;
+    const bool split = p.slices > 1;
+    auto *kern = lo32 ? (split ? k_push_plain<true, true> : k_push_plain<true, false>)
+                      : (split ? k_push_plain<false, true> : k_push_plain<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<p.g.ntiles, kPlainThreads, smem, s>>>(p);
+    kern<<<p.g.ntiles * (split ? p.slices : 1), kPlainThreads, smem, s>>>(p);
     return cudaGetLastError();
 }
 
