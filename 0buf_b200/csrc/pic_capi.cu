@@ -5,6 +5,7 @@
 // e.g. gpu_plasma.h:1904-1910, 1953-1958).
 #include <cuda_runtime.h>
 #include <string.h>
+#include <stddef.h>
 #include <stdio.h>
 #include <math.h>
 #include <string>
@@ -82,9 +83,8 @@ StepParams make_params(pic_handle *h) {
 
 void free_species(pic_handle *h, int s) {
     SpeciesView &v = h->sp[s].v;
-    void *ptrs[] = {v.x, v.y, v.z, v.px, v.py, v.pz, v.ox, v.oy, v.oz, v.fx, v.fy, v.fz, v.cell, v.tile_start,
-                    v.tile_count};
-    for (void *p : ptrs) dev_free(h, p);
+    dev_free(h, h->sp[s].arena);
+    h->sp[s].arena = nullptr;
     double q_m = v.q_m, m = v.m;
     memset(&v, 0, sizeof(v));
     v.q_m = q_m;
@@ -95,12 +95,12 @@ void free_species(pic_handle *h, int s) {
     h->tile_cap_valid = 0;
 }
 
-// capacity per tile from counts; allocates the species arrays and uploads the
-// tile starts.  Slots start on multiples of 32 particles.
-int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
+// tile starts from particle counts: the capacity of every tile (start has
+// ntiles + 1 entries).  Slots start on multiples of 32 particles.
+int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> &start) {
     const Grid &g = h->g;
     double slack = h->cfg.capacity_slack > 0 ? h->cfg.capacity_slack : 0.25;
-    std::vector<int> start(g.ntiles + 1);
+    start.resize(g.ntiles + 1);
     int64_t acc = 0;
     for (int t = 0; t < g.ntiles; t++) {
         start[t] = (int)acc;
@@ -117,22 +117,49 @@ int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
         if (acc > 0x7fffff00LL) return set_err(h, PIC_ERR_ARG, "species capacity exceeds 2^31 slots");
     }
     start[g.ntiles] = (int)acc;
+    return PIC_OK;
+}
+
+// a species' arrays for `slots` slots, carved from one allocation (a driver
+// call per array costs a rebin of a small run more than its copies)
+cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **arena) {
+    const size_t n = (size_t)slots, el = h->mixed ? sizeof(float) : sizeof(double);
+    size_t o = 0;
+    auto room = [&](size_t bytes) { size_t a = o; o += (bytes + 255) / 256 * 256; return a; };
+    const size_t cell = room(n * sizeof(int));
+    size_t val[6];
+    for (size_t &a : val) a = room(n * el);
+    const size_t st = room(((size_t)h->g.ntiles + 1) * sizeof(int)), ct = room((size_t)h->g.ntiles * sizeof(int));
+    const size_t sp = room(n / (kHoleSpill / 2) * sizeof(int));
+    cudaError_t e = dev_alloc(h, arena, o);
+    if (e != cudaSuccess) return e;
+    char *b = (char *)*arena;
+    v.cell = (int *)(b + cell);
+    v.tile_start = (int *)(b + st);
+    v.tile_count = (int *)(b + ct);
+    v.spill = (int *)(b + sp);
+    double **d[6] = {&v.x, &v.y, &v.z, &v.px, &v.py, &v.pz};
+    float **f[6] = {&v.ox, &v.oy, &v.oz, &v.fx, &v.fy, &v.fz};
+    for (int a = 0; a < 6; a++) {
+        if (h->mixed) *f[a] = (float *)(b + val[a]);
+        else *d[a] = (double *)(b + val[a]);
+    }
+    return cudaSuccess;
+}
+
+// replaces the species' arrays by empty bins with room for the counts
+int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
+    const Grid &g = h->g;
+    std::vector<int> start;
+    int rc = layout_bins(h, counts, start);
+    if (rc) return rc;
     free_species(h, s);
     SpeciesView &v = h->sp[s].v;
-    size_t n = (size_t)acc;
-    CK(dev_alloc_n(h, &v.cell, n), "alloc cell");
-    if (!h->mixed) {
-        double **arr[6] = {&v.x, &v.y, &v.z, &v.px, &v.py, &v.pz};
-        for (auto a : arr) CK(dev_alloc_n(h, a, n), "alloc particles");
-    } else {
-        float **arr[6] = {&v.ox, &v.oy, &v.oz, &v.fx, &v.fy, &v.fz};
-        for (auto a : arr) CK(dev_alloc_n(h, a, n), "alloc particles");
-    }
-    CK(dev_alloc_n(h, &v.tile_start, (size_t)g.ntiles + 1), "alloc tile_start");
-    CK(dev_alloc_n(h, &v.tile_count, (size_t)g.ntiles), "alloc tile_count");
+    const int64_t acc = start[g.ntiles];
+    CK(carve_species(h, acc, v, &h->sp[s].arena), "alloc particles");
     CK(cudaMemcpyAsync(v.tile_start, start.data(), (g.ntiles + 1) * sizeof(int), cudaMemcpyHostToDevice, h->stream),
        "upload tile_start");
-    CK(cudaMemsetAsync(v.cell, 0xff, n * sizeof(int), h->stream), "clear cells");
+    CK(cudaMemsetAsync(v.cell, 0xff, (size_t)acc * sizeof(int), h->stream), "clear cells");
     h->sp[s].cap_total = acc;
     h->sp[s].h_start = start;
     h->sp[s].loaded = 1;
@@ -258,8 +285,63 @@ int load_device(pic_handle *h, int s, int64_t n, const double *x, const double *
     return build_bins(h, s, n, cell, x, y, z, px, py, pz, inserted);
 }
 
+// Rebin: new bins for species s with room for its particles and for the
+// outbox entries that did not fit (n_out entries to look through), filled by a
+// copy from the old ones.  dead: the old bins may hold dead slots.  Where the
+// old and the new arrays do not fit side by side, the particles go through a
+// flat list instead (rebin_flat).
+int rebin_flat(pic_handle *h, int s, unsigned n_out);
+int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
+    const Grid &g = h->g;
+    auto &sp = h->sp[s];
+    StepParams p = make_params(h);
+    ScratchGuard guard(h);
+    int *extra = nullptr;
+    CK(guard.alloc(&extra, (size_t)g.ntiles), "rebin counts");
+    CK(cudaMemsetAsync(extra, 0, g.ntiles * sizeof(int), h->stream), "memset");
+    CK(outbox_histogram(p, s, n_out, extra, h->stream), "outbox histogram");
+    std::vector<int> counts(g.ntiles), left(g.ntiles);
+    CK(cudaMemcpyAsync(counts.data(), sp.v.tile_count, g.ntiles * sizeof(int), cudaMemcpyDeviceToHost, h->stream),
+       "counts");
+    CK(cudaMemcpyAsync(left.data(), extra, g.ntiles * sizeof(int), cudaMemcpyDeviceToHost, h->stream), "counts");
+    CK(cudaStreamSynchronize(h->stream), "sync");
+    for (int t = 0; t < g.ntiles; t++) counts[t] += left[t];
+    std::vector<int> start;
+    int rc = layout_bins(h, counts, start);
+    if (rc) return rc;
+    SpeciesView v = sp.v;
+    void *arena = nullptr;
+    const cudaError_t e = carve_species(h, start[g.ntiles], v, &arena);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return rebin_flat(h, s, n_out);
+    }
+    CK(e, "alloc particles");
+    auto fill = [&]() -> cudaError_t {
+        cudaError_t r = cudaMemcpyAsync(v.tile_start, start.data(), (g.ntiles + 1) * sizeof(int),
+                                        cudaMemcpyHostToDevice, h->stream);
+        if (r == cudaSuccess) r = cudaMemsetAsync(v.cell, 0xff, (size_t)start[g.ntiles] * sizeof(int), h->stream);
+        if (r == cudaSuccess) r = rebin_copy(g, h->mixed, dead, sp.v, v, h->stream);
+        if (r == cudaSuccess) r = insert_left(p, s, n_out, v, h->stream);
+        if (r == cudaSuccess) r = cudaStreamSynchronize(h->stream);  // the old arrays are free after this
+        return r;
+    };
+    const cudaError_t r = fill();
+    if (r != cudaSuccess) {
+        dev_free(h, arena);
+        return cuda_err(h, r, "rebin");
+    }
+    dev_free(h, sp.arena);
+    sp.arena = arena;
+    sp.v = v;
+    sp.cap_total = start[g.ntiles];
+    sp.h_start = std::move(start);
+    h->tile_cap_valid = 0;
+    return PIC_OK;
+}
+
 // gather the live particles (+ outbox leftovers) of species s and rebuild its bins
-int rebin_species(pic_handle *h, int s, unsigned n_out) {
+int rebin_flat(pic_handle *h, int s, unsigned n_out) {
     const Grid &g = h->g;
     SpeciesView &v = h->sp[s].v;
     std::vector<int> counts(g.ntiles);
@@ -313,30 +395,25 @@ int check_status(pic_handle *h) {
                  pic_error_string(code), st.flags);
         return set_err(h, code, msg);
     }
-    if (st.flags & ST_TILE_FULL) {
-        unsigned n_out = st.out_count < h->out_cap ? st.out_count : h->out_cap;
+    if (st.flags & (ST_TILE_FULL | ST_HOLES)) {
+        // arrivals that did not fit wait in the outbox, and a compaction that
+        // had too many holes left dead slots inside the bins (no telling in
+        // which species' bins): new bins for the species concerned
+        const bool holes = (st.flags & ST_HOLES) != 0;
+        const unsigned n_out = st.flags & ST_TILE_FULL ? std::min(st.out_count, h->out_cap) : 0u;
         // the outbox keeps every species' leftovers until the last species has
         // taken its own: a rebin must not resize (and so clear) it on the way
         h->outbox_pinned = 1;
         for (int s = 0; s < h->cfg.nspecies; s++) {
-            int rc = rebin_species(h, s, n_out);
+            if (!holes && !(st.full_species >> s & 1u)) continue;
+            int rc = rebin_species(h, s, n_out, holes);
             if (rc) { h->outbox_pinned = 0; return rc; }
         }
         h->outbox_pinned = 0;
         int rc = ensure_outbox(h);
         if (rc) return rc;
-        // leftovers are in the bins now
-        CK(cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream), "reset status");
-        h->kin_valid = 0;
-    }
-    if (st.flags & ST_HOLES) {
-        // dead slots remain inside the bins; a rebin compacts them
-        for (int s = 0; s < h->cfg.nspecies; s++) {
-            int rc = rebin_species(h, s, 0);
-            if (rc) return rc;
-        }
-        CK(cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream), "reset status");
-        h->kin_valid = 0;
+        // leftovers are in the bins now; the kinetic energy stays
+        CK(cudaMemsetAsync(h->st, 0, offsetof(DevStatus, moved), h->stream), "reset status");
     }
     return PIC_OK;
 }

@@ -189,8 +189,76 @@ __global__ void k_insert(StepParams P) {
         } else {
             atomicAdd(&P.st->overflow_count, 1u);
             atomicOr(&P.st->flags, (unsigned)ST_TILE_FULL);
+            atomicOr(&P.st->full_species, 1u << o.species);
         }
     }
+}
+
+// A species' bins copied to a new layout (rebin), one CTA per tile.  DEAD: the
+// bins may hold dead slots (cell < 0), which stay behind.
+template <bool MIXED, bool DEAD>
+__global__ void k_rebin_copy(SpeciesView A, SpeciesView B) {
+    __shared__ int fill;
+    const int t = blockIdx.x, a = A.tile_start[t], b = B.tile_start[t], n = A.tile_count[t];
+    if (threadIdx.x == 0) fill = 0;
+    __syncthreads();
+    for (int base = 0; base < n; base += blockDim.x) {
+        const int j = base + threadIdx.x;
+        const int c = j < n ? A.cell[a + j] : -1;
+        int d = j;
+        if (DEAD) {
+            const unsigned m = __ballot_sync(0xffffffffu, c >= 0);
+            int first = 0;
+            if ((threadIdx.x & 31) == 0) first = atomicAdd(&fill, __popc(m));
+            d = __shfl_sync(0xffffffffu, first, 0) + __popc(m & ((1u << (threadIdx.x & 31)) - 1));
+        }
+        if (DEAD ? c < 0 : j >= n) continue;
+        const int q = a + j, r = b + d;
+        B.cell[r] = c;
+        if (MIXED) {
+            B.ox[r] = A.ox[q]; B.oy[r] = A.oy[q]; B.oz[r] = A.oz[q];
+            B.fx[r] = A.fx[q]; B.fy[r] = A.fy[q]; B.fz[r] = A.fz[q];
+        } else {
+            B.x[r] = A.x[q]; B.y[r] = A.y[q]; B.z[r] = A.z[q];
+            B.px[r] = A.px[q]; B.py[r] = A.py[q]; B.pz[r] = A.pz[q];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) B.tile_count[t] = DEAD ? fill : n;
+}
+
+// per tile, the outbox entries of a species that did not fit (counts[tile] += 1 each)
+template <class Out>
+__global__ void k_outbox_hist(Grid g, const Out *ob, unsigned n, int species, int *counts) {
+    const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n || ob[e].cell < 0 || ob[e].species != species) return;
+    int i, l, k;
+    cell_ijk(g, ob[e].cell, i, l, k);
+    atomicAdd(&counts[g.tile_of_cell(i, l, k)], 1);
+}
+
+// those entries into bins that now have room for them
+template <class Out, bool MIXED>
+__global__ void k_insert_left(Grid g, Out *ob, unsigned n, int species, SpeciesView S) {
+    const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n || ob[e].cell < 0 || ob[e].species != species) return;
+    const Out o = ob[e];
+    int i, l, k;
+    cell_ijk(g, o.cell, i, l, k);
+    const int t = g.tile_of_cell(i, l, k);
+    const int slot = S.tile_start[t] + atomicAdd(&S.tile_count[t], 1);
+    if (slot >= S.tile_start[t + 1]) return;  // never: the bins were sized from the same entries
+    S.cell[slot] = o.cell;
+    if (MIXED) {
+        const OutMixed &q = *(const OutMixed *)&o;
+        S.ox[slot] = q.ox; S.oy[slot] = q.oy; S.oz[slot] = q.oz;
+        S.fx[slot] = q.px; S.fy[slot] = q.py; S.fz[slot] = q.pz;
+    } else {
+        const OutPlain &q = *(const OutPlain *)&o;
+        S.x[slot] = q.x; S.y[slot] = q.y; S.z[slot] = q.z;
+        S.px[slot] = q.px; S.py[slot] = q.py; S.pz[slot] = q.pz;
+    }
+    ob[e].cell = -1;
 }
 
 // clamp tile counts after an overflowing insert so the bins stay consistent
@@ -508,6 +576,30 @@ cudaError_t cell_particles(const Grid &g, int mixed, const SpeciesView &sv, int 
                            double *y, double *z, double *px, double *py, double *pz, int64_t *slot, unsigned *count,
                            cudaStream_t s) {
     k_cell_particles<<<64, 256, 0, s>>>(g, mixed, sv, tile, cell, cap, x, y, z, px, py, pz, slot, count);
+    return cudaGetLastError();
+}
+
+cudaError_t rebin_copy(const Grid &g, int mixed, bool dead, const SpeciesView &from, const SpeciesView &to,
+                       cudaStream_t s) {
+    auto *k = mixed ? (dead ? k_rebin_copy<true, true> : k_rebin_copy<true, false>)
+                    : (dead ? k_rebin_copy<false, true> : k_rebin_copy<false, false>);
+    k<<<g.ntiles, 512, 0, s>>>(from, to);
+    return cudaGetLastError();
+}
+
+cudaError_t outbox_histogram(const StepParams &p, int species, unsigned n_out, int *counts, cudaStream_t s) {
+    if (n_out == 0) return cudaSuccess;
+    const unsigned blocks = blocks_for(n_out, 256);
+    if (p.mixed) k_outbox_hist<<<blocks, 256, 0, s>>>(p.g, (const OutMixed *)p.outbox, n_out, species, counts);
+    else k_outbox_hist<<<blocks, 256, 0, s>>>(p.g, (const OutPlain *)p.outbox, n_out, species, counts);
+    return cudaGetLastError();
+}
+
+cudaError_t insert_left(const StepParams &p, int species, unsigned n_out, const SpeciesView &to, cudaStream_t s) {
+    if (n_out == 0) return cudaSuccess;
+    const unsigned blocks = blocks_for(n_out, 256);
+    if (p.mixed) k_insert_left<OutMixed, true><<<blocks, 256, 0, s>>>(p.g, (OutMixed *)p.outbox, n_out, species, to);
+    else k_insert_left<OutPlain, false><<<blocks, 256, 0, s>>>(p.g, (OutPlain *)p.outbox, n_out, species, to);
     return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@ struct pic_handle {
     double *dense;             // one reference-layout FP64 array (I/O staging)
     struct Sp {
         pic::SpeciesView v;
+        void *arena;  // the one allocation that holds v's arrays
         int64_t cap_total;
         int loaded;
         std::vector<int> h_start;

@@ -25,7 +25,8 @@
 namespace pic {
 
 constexpr int kMaxSpecies = PIC_MAX_SPECIES;
-constexpr int kHoleMax = 1024;          // departures per tile per species handled in-kernel
+constexpr int kHoleMax = 1024;          // departures per tile per species listed before the spill list
+constexpr int kHoleSpill = 16;          // one spill entry per this many slots of the bin
 constexpr int kPushThreads = 256;       // threads of a push CTA: particles per block of a slice
 constexpr unsigned kOutboxChunk = 16;   // outbox slots a warp of the FP32 push takes at once
 
@@ -44,7 +45,7 @@ struct DevStatus {
     unsigned flags;
     unsigned out_count;        // outbox entries this step
     unsigned overflow_count;   // outbox entries that did not fit their tile
-    unsigned pad0;
+    unsigned full_species;     // bit s: species s has such entries
     unsigned long long moved;  // particles written to the outbox
     unsigned long long dropped;
     unsigned long long duplicated;
@@ -199,8 +200,33 @@ struct SpeciesView {
     int *cell;
     int *tile_start;  // ntiles + 1
     int *tile_count;  // ntiles
+    // holes of a push past the first kHoleMax of a bin, and the compaction's
+    // front holes past theirs: slots / 8 ints (see HoleList)
+    int *spill;
     double q_m, m;
 };
+
+// The holes that a push leaves in one bin: the first kHoleMax entries in
+// `base` (shared memory, or global memory when several CTAs share the tile),
+// the rest in the bin's part of the spill list, one entry per kHoleSpill slots.
+// A second list of the same shape takes the compaction's front holes.  Dense
+// hot tiles need the spill: at 700 particles per cell and vth 0.1 about 2000
+// leave a tile per step, and a list of 1024 alone had the host rebin every
+// species after nearly every step.
+struct HoleList {
+    int *base, *spill;
+    int cap;  // spill entries
+    __device__ __forceinline__ int limit() const { return kHoleMax + cap; }
+    __device__ __forceinline__ int *at(int r) const { return r < kHoleMax ? base + r : spill + (r - kHoleMax); }
+};
+__device__ __forceinline__ HoleList hole_list(const SpeciesView &S, int t, int *base, bool front) {
+    HoleList h;
+    const int a = S.tile_start[t];
+    h.base = base;
+    h.cap = (S.tile_start[t + 1] - a) / kHoleSpill;
+    h.spill = S.spill + a / (kHoleSpill / 2) + (front ? h.cap : 0);
+    return h;
+}
 
 // one migrating particle (plain form): 56 bytes
 struct OutPlain {
@@ -266,6 +292,18 @@ __device__ __forceinline__ void slice_range(const SliceRange &r, int first, int 
     jend = (int)(b < jbeg ? jbeg : (b > count ? count : b));
 }
 
+// lists hole j as entry r of a bin's holes; false when the list is full
+__device__ __forceinline__ bool list_hole(const SpeciesView &S, int t, int *base, unsigned r, int j) {
+    if (r < (unsigned)kHoleMax) {
+        base[r] = j;
+        return true;
+    }
+    const HoleList h = hole_list(S, t, base, false);
+    if (r >= (unsigned)h.limit()) return false;
+    *h.at((int)r) = j;
+    return true;
+}
+
 // True in the last CTA of tile t to get here, whose threads then see what the
 // tile's other CTAs wrote (fence, ticket, fence).  No CTA waits for another.
 // Every thread calls it; flag is shared memory.
@@ -291,14 +329,14 @@ __device__ __forceinline__ void compact_listed(const StepParams &P, int t, int s
     const SpeciesView &S = P.sp[s];
     const size_t e = (size_t)s * P.g.ntiles + t;
     const unsigned listed = __ldcg(&P.hole_count[e]);
-    if (listed == 0u || listed > (unsigned)kHoleMax) return;
+    const HoleList holes = hole_list(S, t, P.holes + e * kHoleMax, false), fronts = hole_list(S, t, front, true);
+    if (listed == 0u || listed > (unsigned)holes.limit()) return;
     const int nh = (int)listed, start = S.tile_start[t], newcount = S.tile_count[t] - nh;
-    const int *holes = P.holes + e * kHoleMax;
     if (threadIdx.x == 0) ctr[0] = ctr[1] = 0;
     __syncthreads();
     for (int r = threadIdx.x; r < nh; r += blockDim.x) {
-        const int h = __ldcg(holes + r);
-        if (h < newcount) front[atomicAdd(&ctr[0], 1)] = h;
+        const int h = __ldcg(holes.at(r));
+        if (h < newcount) *fronts.at(atomicAdd(&ctr[0], 1)) = h;
     }
     __syncthreads();
     for (int r = threadIdx.x; r < nh; r += blockDim.x) {
@@ -306,7 +344,7 @@ __device__ __forceinline__ void compact_listed(const StepParams &P, int t, int s
         if (__ldcg(&S.cell[src]) >= 0) {
             const int m = atomicAdd(&ctr[1], 1);
             if (m >= ctr[0]) { bad |= ST_BADCELL; continue; }
-            move(start + front[m], src);
+            move(start + *fronts.at(m), src);
         }
     }
     __syncthreads();

@@ -58,6 +58,13 @@ cudaError_t gather_from_bins(const Grid &g, int mixed, SpeciesView sv, const int
 cudaError_t cell_particles(const Grid &g, int mixed, const SpeciesView &sv, int tile, int cell, int64_t cap, double *x,
                            double *y, double *z, double *px, double *py, double *pz, int64_t *slot, unsigned *count,
                            cudaStream_t s);
+// rebin of one species: its bins to a new layout (dead: they may hold dead
+// slots); the tiles of its outbox entries that did not fit; those entries into
+// the new bins
+cudaError_t rebin_copy(const Grid &g, int mixed, bool dead, const SpeciesView &from, const SpeciesView &to,
+                       cudaStream_t s);
+cudaError_t outbox_histogram(const StepParams &p, int species, unsigned n_out, int *counts, cudaStream_t s);
+cudaError_t insert_left(const StepParams &p, int species, unsigned n_out, const SpeciesView &to, cudaStream_t s);
 // outbox leftovers of one species (after a failed insert) -> flat list appended at offset
 cudaError_t gather_outbox(const StepParams &p, int species, unsigned n_out, unsigned *counter, int64_t offset,
                           double *x, double *y, double *z, double *px, double *py, double *pz, int *cell,

@@ -787,8 +787,9 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                     }
                     S.cell[slot] = -1;
                     const int hpos = hbase + rank;
-                    if (hpos < kHoleMax) (SPLIT ? P.holes + ((size_t)s * g.ntiles + t) * kHoleMax : sHoles)[hpos] = j;
-                    else bad |= ST_HOLES;
+                    if (!list_hole(S, t, SPLIT ? P.holes + ((size_t)s * g.ntiles + t) * kHoleMax : sHoles,
+                                   (unsigned)hpos, j))
+                        bad |= ST_HOLES;
                 }
             }
         }
@@ -816,11 +817,12 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         // front of the new count
         // (SPLIT: by the tile's last CTA, after its last species)
         const int nh = SPLIT ? 0 : sNHoles[sp];
-        if (nh > 0 && nh <= kHoleMax) {
+        const HoleList holes = hole_list(S, t, sHoles, false), fronts = hole_list(S, t, sFront, true);
+        if (nh > 0 && nh <= holes.limit()) {
             const int newcount = count - nh;
             for (int r = threadIdx.x; r < nh; r += blockDim.x) {
-                int h = sHoles[r];
-                if (h < newcount) sFront[atomicAdd(&sNFront[sp], 1)] = h;
+                int h = *holes.at(r);
+                if (h < newcount) *fronts.at(atomicAdd(&sNFront[sp], 1)) = h;
             }
             __syncthreads();
             for (int r = threadIdx.x; r < nh; r += blockDim.x) {
@@ -828,7 +830,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                 if (S.cell[src] >= 0) {
                     int mv = atomicAdd(&sNMove[sp], 1);
                     if (mv >= sNFront[sp]) { bad |= ST_BADCELL; continue; }
-                    int dst = start + sFront[mv];
+                    int dst = start + *fronts.at(mv);
                     S.cell[dst] = S.cell[src];
                     S.ox[dst] = S.ox[src]; S.oy[dst] = S.oy[src]; S.oz[dst] = S.oz[src];
                     S.fx[dst] = S.fx[src]; S.fy[dst] = S.fy[src]; S.fz[dst] = S.fz[src];

@@ -584,16 +584,9 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                 }
                 if (leave) {
                     S.cell[slot] = -1;
-                    if (SPLIT) {
-                        const size_t e = (size_t)s * g.ntiles + t;
-                        const unsigned hpos = atomicAdd(&P.hole_count[e], 1u);
-                        if (hpos < (unsigned)kHoleMax) P.holes[e * kHoleMax + hpos] = j;
-                        else bad |= ST_HOLES;
-                    } else {
-                        int hpos = atomicAdd(&sNHoles, 1);
-                        if (hpos < kHoleMax) sHoles[hpos] = j;
-                        else bad |= ST_HOLES;
-                    }
+                    const size_t e = (size_t)s * g.ntiles + t;
+                    const unsigned hpos = SPLIT ? atomicAdd(&P.hole_count[e], 1u) : (unsigned)atomicAdd(&sNHoles, 1);
+                    if (!list_hole(S, t, SPLIT ? P.holes + e * kHoleMax : sHoles, hpos, j)) bad |= ST_HOLES;
                 } else {
                     S.cell[slot] = newcell;
                     S.x[slot] = x; S.y[slot] = y; S.z[slot] = z;
@@ -630,11 +623,12 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
         __syncthreads();
         // ---- compaction of the tile bin (replaces GPU_MakeDepartureLists_rm, kernels.cu:219-242)
         const int L = sNHoles;
-        if (L > 0 && L <= kHoleMax) {
+        const HoleList holes = hole_list(S, t, sHoles, false), fronts = hole_list(S, t, sFront, true);
+        if (L > 0 && L <= holes.limit()) {
             const int newcount = count - L;
             for (int r = threadIdx.x; r < L; r += blockDim.x) {
-                int h = sHoles[r];
-                if (h < newcount) sFront[atomicAdd(&sNFront, 1)] = h;
+                int h = *holes.at(r);
+                if (h < newcount) *fronts.at(atomicAdd(&sNFront, 1)) = h;
             }
             __syncthreads();
             for (int r = threadIdx.x; r < L; r += blockDim.x) {
@@ -642,7 +636,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                 if (S.cell[src] >= 0) {
                     int m = atomicAdd(&sNMove, 1);
                     if (m >= sNFront) { bad |= ST_BADCELL; continue; }
-                    int dst = start + sFront[m];
+                    int dst = start + *fronts.at(m);
                     S.cell[dst] = S.cell[src];
                     S.x[dst] = S.x[src]; S.y[dst] = S.y[src]; S.z[dst] = S.z[src];
                     S.px[dst] = S.px[src]; S.py[dst] = S.py[src]; S.pz[dst] = S.pz[src];
