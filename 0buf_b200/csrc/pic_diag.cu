@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
+#include <algorithm>
 #include "pic0buf.h"
 #include "pic_internal.cuh"
 #include "pic_kernels.cuh"
@@ -29,46 +30,72 @@
 namespace pic {
 namespace {
 
-// One CTA per tile: every species' particles of the tile add their eight
-// weights into a shared (tx+2)(ty+2)(tz+2) node box in 64-bit fixed point
-// (exact and order-independent: q = 2^(E-62) with 2^E > sum |m| over the
-// tile's particles, each node receives at most that much), then the box is
-// added into the global rho.
-__global__ void k_charge_tile(StepParams P, double *rho) {
+// The particles of every species in a share of a tile (blockIdx.y of
+// gridDim.y) add their eight weights into a shared (tx+2)(ty+2)(tz+2) node box
+// in 64-bit fixed point (exact and order-independent: q = 2^(E-62) with 2^E >
+// sum |m| over the tile's particles, each node receives at most that much),
+// then the box is added into the global rho.
+//
+// Bound: the eight 64-bit shared adds per particle and the FP64 products in
+// front of them.  m / q is folded into the x weights, and a contribution below
+// 2^51 quanta (every tile of 2048 equal charges or more) is rounded by adding
+// 1.5 * 2^52 instead of by a conversion.  50.3M FP32-form particles (128x64x64
+// cells): 733 -> 696 us; 805M (512x128x128): 11.6 -> 9.95 ms.  The shared
+// atomics are what is left (a copy without the carry, wrong sums, timing only:
+// 635 us).  With few tiles each is dealt out to several CTAs: the reference's
+// default run (13 tiles of 500k particles) 3546 -> 143 us FP64, 2118 -> 154 us
+// FP32; 32x4x4 cells 85 -> 38 us.
+template <bool MIXED>
+__global__ void __launch_bounds__(256) k_charge_tile(StepParams P, double *rho) {
     const Grid &g = P.g;
-    const int mixed = P.mixed, nsp = P.nsp;
+    const int nsp = P.nsp;
     const SpeciesView *sp = P.sp;
-    extern __shared__ unsigned long long sR[];
+    // the nodes' low and high words: FP32 form nn low, then nn high words (32
+    // banks for either); FP64 form interleaved
+    extern __shared__ unsigned sR[];
     __shared__ double sQ, sInvQ;
+    __shared__ int sMagic;
     const int t = blockIdx.x;
     const int tk = t % g.ntz, tl = (t / g.ntz) % g.nty, ti = t / (g.ntz * g.nty);
     const int i0 = ti * g.tx, l0 = tl * g.ty, k0 = tk * g.tz;
     const int SX = g.tx + 2, SY = g.ty + 2, SZ = g.tz + 2;
     const int nn = SX * SY * SZ;
     if (threadIdx.x == 0) {
-        double bound = 0.0;
-        for (int s = 0; s < nsp; s++) bound += fabs(sp[s].m) * (double)sp[s].tile_count[t];
+        double bound = 0.0, one = 0.0;
+        for (int s = 0; s < nsp; s++) {
+            bound += fabs(sp[s].m) * (double)sp[s].tile_count[t];
+            if (sp[s].tile_count[t] > 0) one = fmax(one, fabs(sp[s].m));
+        }
         int e2;
         frexp(bound > 0.0 ? bound : 1.0, &e2);
         sQ = ldexp(1.0, e2 - 62);
         sInvQ = ldexp(1.0, 62 - e2);
+        sMagic = one * sInvQ < 0x1p51;
     }
-    for (int idx = threadIdx.x; idx < nn; idx += blockDim.x) sR[idx] = 0ull;
+    for (int idx = threadIdx.x; idx < 2 * nn; idx += blockDim.x) sR[idx] = 0u;
     __syncthreads();
     const double inv_q = sInvQ;
+    const bool magic = sMagic != 0;
     const double h[3] = {g.hx, g.hy, g.hz};
+    const int st = MIXED ? 1 : 2, hi_word = MIXED ? nn : 1;
+    // FP32 form: a warp takes 8 runs of 4 particles out of 8 different places
+    // of the block's 256, so that fewer lanes share a cell (FP64 form: its
+    // 8-byte loads would lose more than that gains)
+    const int lane_of = MIXED ? ((threadIdx.x & 31) >> 2) * 32 + (threadIdx.x >> 5) * 4 + (threadIdx.x & 3) : threadIdx.x;
     for (int s = 0; s < nsp; s++) {
         const SpeciesView &S = sp[s];
-        const int start = S.tile_start[t], count = S.tile_count[t];
-        const double m = S.m;
-        for (int j = threadIdx.x; j < count; j += blockDim.x) {
+        const int start = S.tile_start[t];
+        const long long all = S.tile_count[t];
+        const int jbeg = (int)(all * blockIdx.y / gridDim.y), jend = (int)(all * (blockIdx.y + 1) / gridDim.y);
+        const double mq = S.m * inv_q;  // exact: inv_q is a power of two
+        for (int j = jbeg + lane_of; j < jend; j += blockDim.x) {
             const int slot = start + j;
             const int c = S.cell[slot];
             if (c < 0) continue;
             int ci[3];
             g.cell_ijk(c, ci[0], ci[1], ci[2]);
             double f[3];
-            if (mixed) {
+            if (MIXED) {
                 f[0] = (double)S.ox[slot];
                 f[1] = (double)S.oy[slot];
                 f[2] = (double)S.oz[slot];
@@ -87,17 +114,26 @@ __global__ void k_charge_tile(StepParams P, double *rho) {
                 ok = ok && lo[a] >= 0 && lo[a] + 1 < (a == 0 ? SX : a == 1 ? SY : SZ);
             }
             if (!ok) continue;  // a bin entry outside its tile (never expected)
-            const int nb = (lo[0] * SY + lo[1]) * SZ + lo[2];
-            for (int b = 0; b < 8; b++) {
-                const int ax = b >> 2, ay = (b >> 1) & 1, az = b & 1;
-                const double w = (ax ? w1[0] : 1.0 - w1[0]) * (ay ? w1[1] : 1.0 - w1[1]) * (az ? w1[2] : 1.0 - w1[2]);
-                fx_add(&sR[nb + (ax * SY + ay) * SZ + az], m * w, inv_q);
+            unsigned *R = sR + st * ((lo[0] * SY + lo[1]) * SZ + lo[2]);
+            const double wx[2] = {mq * (1.0 - w1[0]), mq * w1[0]}, wy[2] = {1.0 - w1[1], w1[1]},
+                         wz[2] = {1.0 - w1[2], w1[2]};
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const double wxy = wx[b >> 1] * wy[b & 1];
+                unsigned *r = R + st * (((b >> 1) * SY + (b & 1)) * SZ);
+#pragma unroll
+                for (int az = 0; az < 2; az++) {
+                    const double v = wxy * wz[az];
+                    const long long iv = magic ? __double_as_longlong(v + 0x1.8p52) - 0x4338000000000000ll
+                                               : __double2ll_rn(v);
+                    if (iv) shared_add64(r + st * az, r + st * az + hi_word, iv);
+                }
             }
         }
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < nn; idx += blockDim.x) {
-        const long long v = (long long)sR[idx];
+        const long long v = (long long)(((unsigned long long)sR[st * idx + hi_word] << 32) | sR[st * idx]);
         if (v == 0) continue;
         const int c = idx % SZ, b = (idx / SZ) % SY, a = idx / (SZ * SY);
         if (i0 + a < g.NX && l0 + b < g.NY && k0 + c < g.NZ) atomicAdd(&rho[g.node(i0 + a, l0 + b, k0 + c)], (double)v * sQ);
@@ -126,28 +162,34 @@ __global__ void k_rho_fold(Grid g, double *rho, int dir) {
 // G = div E - rho on the interior nodes (0 on the ghosts); optional baseline
 // copy; reductions into red[0] max |G - G0|, red[1] max |rho|, red[2] sum (G - G0)^2,
 // red[3] max |G0| (non-negative doubles compared through their bit patterns)
+// (a block walks over many nodes and reduces once: one atomic per warp on the
+// same four addresses took 1.65 ms of a 512x128x128 call, this takes 0.27)
 template <typename T>
 __global__ void k_gauss(Grid g, const T *__restrict__ Ex, const T *__restrict__ Ey, const T *__restrict__ Ez,
                         const double *__restrict__ rho, double *G, double *G0, int set_baseline, double *red) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int l = blockIdx.y, i = blockIdx.z;
+    __shared__ double part[4][8];
     double dmax = 0.0, rmax = 0.0, d2 = 0.0, g0max = 0.0;
-    if (k < g.NZ) {
-        const size_t n = g.node(i, l, k);
-        const bool interior = i >= 1 && i <= g.nx && l >= 1 && l <= g.ny && k >= 1 && k <= g.nz;
-        double v = 0.0;
-        if (interior) {
-            const size_t sx = (size_t)g.NY * g.pz, sy = g.pz;
-            v = ((double)Ex[n] - (double)Ex[n - sx]) / g.hx + ((double)Ey[n] - (double)Ey[n - sy]) / g.hy +
-                ((double)Ez[n] - (double)Ez[n - 1]) / g.hz - rho[n];
-            rmax = fabs(rho[n]);
+    const size_t sx = (size_t)g.NY * g.pz, sy = g.pz;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rows = g.NX * g.NY, stride = gridDim.x * (blockDim.x >> 5);
+    for (int row = blockIdx.x * (blockDim.x >> 5) + warp; row < rows; row += stride) {
+        const int i = row / g.NY, l = row - i * g.NY;
+        const bool inner = i >= 1 && i <= g.nx && l >= 1 && l <= g.ny;
+        for (int k = lane; k < g.NZ; k += 32) {
+            const size_t n = g.node(i, l, k);
+            double v = 0.0;
+            if (inner && k >= 1 && k <= g.nz) {
+                v = ((double)Ex[n] - (double)Ex[n - sx]) / g.hx + ((double)Ey[n] - (double)Ey[n - sy]) / g.hy +
+                    ((double)Ez[n] - (double)Ez[n - 1]) / g.hz - rho[n];
+                rmax = fmax(rmax, fabs(rho[n]));
+            }
+            if (G) G[n] = v;
+            if (set_baseline) G0[n] = v;
+            const double base = set_baseline ? v : G0[n];
+            dmax = fmax(dmax, fabs(v - base));
+            d2 += (v - base) * (v - base);
+            g0max = fmax(g0max, fabs(base));
         }
-        if (G) G[n] = v;
-        if (set_baseline) G0[n] = v;
-        const double base = G0[n];
-        dmax = fabs(v - base);
-        d2 = (v - base) * (v - base);
-        g0max = fabs(base);
     }
     for (int o = 16; o > 0; o >>= 1) {
         dmax = fmax(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
@@ -155,30 +197,37 @@ __global__ void k_gauss(Grid g, const T *__restrict__ Ex, const T *__restrict__ 
         d2 += __shfl_down_sync(0xffffffffu, d2, o);
         g0max = fmax(g0max, __shfl_down_sync(0xffffffffu, g0max, o));
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax((unsigned long long *)&red[0], (unsigned long long)__double_as_longlong(dmax));
-        atomicMax((unsigned long long *)&red[1], (unsigned long long)__double_as_longlong(rmax));
-        atomicAdd(&red[2], d2);
-        atomicMax((unsigned long long *)&red[3], (unsigned long long)__double_as_longlong(g0max));
+    if (lane == 0) { part[0][warp] = dmax; part[1][warp] = rmax; part[2][warp] = d2; part[3][warp] = g0max; }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++)
+            v = threadIdx.x == 2 ? v + part[2][w] : fmax(v, part[threadIdx.x][w]);
+        if (threadIdx.x == 2) atomicAdd(&red[2], v);
+        else atomicMax((unsigned long long *)&red[threadIdx.x], (unsigned long long)__double_as_longlong(v));
     }
 }
 
 // total mechanical momentum per species, sum over particles of (m/q_m) p, in
-// FP64: one block per (tile, species), out[3 s + a]
-__global__ void k_momentum(StepParams P, double *out) {
+// FP64: a block walks over shares of tiles of one species, out[3 s + a] (one
+// atomic per block: a block per tile and species spent a c2 call, 3.1 ms, on
+// 400k atomics to nine addresses and single loads in flight; now 2.2 ms)
+__global__ void k_momentum(StepParams P, int shares, double *out) {
     __shared__ double red[3][32];
     const SpeciesView &S = P.sp[blockIdx.y];
-    const int t = blockIdx.x;
-    const int start = S.tile_start[t], n = S.tile_count[t];
     const double M = S.m / S.q_m;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const int slot = start + j;
-        if (S.cell[slot] < 0) continue;
-        if (P.mixed) {
-            acc[0] += M * (double)S.fx[slot]; acc[1] += M * (double)S.fy[slot]; acc[2] += M * (double)S.fz[slot];
-        } else {
-            acc[0] += M * S.px[slot]; acc[1] += M * S.py[slot]; acc[2] += M * S.pz[slot];
+    for (int u = blockIdx.x; u < P.g.ntiles * shares; u += gridDim.x) {
+        const int t = u / shares, q = u - t * shares;
+        const long long n = S.tile_count[t];
+        const int start = S.tile_start[t], jend = (int)(n * (q + 1) / shares);
+        for (int j = (int)(n * q / shares) + threadIdx.x; j < jend; j += 4 * blockDim.x) {
+            double p[4][3];
+            load_momenta4(P.mixed, S, start, j, jend, p);
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                acc[0] += M * p[v][0]; acc[1] += M * p[v][1]; acc[2] += M * p[v][2];
+            }
         }
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -200,7 +249,8 @@ __global__ void k_momentum(StepParams P, double *out) {
 cudaError_t momentum(const StepParams &p, double *out, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(out, 0, 3 * p.nsp * sizeof(double), s);
     if (e != cudaSuccess) return e;
-    k_momentum<<<dim3(p.g.ntiles, p.nsp), 256, 0, s>>>(p, out);
+    const int shares = tile_shares(p.g.ntiles);
+    k_momentum<<<dim3(std::min(p.g.ntiles * shares, 148 * 8), p.nsp), 256, 0, s>>>(p, shares, out);
     return cudaGetLastError();
 }
 
@@ -209,11 +259,12 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(rho, 0, g.nodes_pitched() * sizeof(double), s);
     if (e != cudaSuccess) return e;
     const size_t smem = (size_t)(g.tx + 2) * (g.ty + 2) * (g.tz + 2) * sizeof(unsigned long long);
+    auto *k = p.mixed ? k_charge_tile<true> : k_charge_tile<false>;
     if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(k_charge_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    k_charge_tile<<<g.ntiles, 256, smem, s>>>(p, rho);
+    k<<<dim3(g.ntiles, tile_shares(g.ntiles)), 256, smem, s>>>(p, rho);
     for (int dir = 0; dir < 3; dir++) {
         const int A = dir == 0 ? g.NY : g.NX;
         const int B = dir == 2 ? g.NY : g.NZ;
@@ -224,8 +275,7 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
 
 cudaError_t gauss_residual(const Grid &g, int mixed, const void *const E[3], const double *rho, double *G, double *G0,
                            int set_baseline, double *red, cudaStream_t s) {
-    const int bx = g.NZ >= 128 ? 128 : 32;
-    const dim3 grid((g.NZ + bx - 1) / bx, g.NY, g.NX);
+    const int bx = 256, grid = std::min((g.NX * g.NY + 7) / 8, 148 * 8);
     if (mixed)
         k_gauss<float><<<grid, bx, 0, s>>>(g, (const float *)E[0], (const float *)E[1], (const float *)E[2], rho, G,
                                            G0, set_baseline, red);

@@ -126,12 +126,15 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, c
 // 64-bit shared-memory atomicAdd costs about 8 atomic instructions per add
 // in the FP64 push (lanes of a warp often share a node), and the split took
 // the c2 FP64 push from 106.4 to 72.4 ms.
+__device__ __forceinline__ void shared_add64(unsigned *plo, unsigned *phi, long long v) {
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd(plo, lo);
+    const unsigned hi = (unsigned)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(phi, hi);
+}
 __device__ __forceinline__ void shared_add64(unsigned long long *w, long long v) {
     unsigned *p = (unsigned *)w;  // p[0] low word, p[1] high word
-    const unsigned lo = (unsigned)v;
-    const unsigned old = atomicAdd(p, lo);
-    const unsigned hi = (unsigned)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u);
-    if (hi) atomicAdd(p + 1, hi);
+    shared_add64(p, p + 1, v);
 }
 __device__ __forceinline__ void fx_add(unsigned long long *a, double v, double inv_q) {
     long long iv = __double2ll_rn(v * inv_q);
@@ -239,6 +242,28 @@ struct OutMixed {
     int cell, species;
 };
 
+// Momenta of the live particles among slots start + {j, j + B, j + 2B, j + 3B}
+// (B = blockDim.x) below start + jend, zeros for the others.  All loads are
+// issued before any is looked at: a reduction that loads one particle at a time
+// waits for it.
+__device__ __forceinline__ void load_momenta4(int mixed, const SpeciesView &S, int start, int j, int jend,
+                                              double p[4][3]) {
+    bool live[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const int q = j + v * (int)blockDim.x, slot = start + q;
+        live[v] = q < jend && S.cell[slot] >= 0;
+        p[v][0] = p[v][1] = p[v][2] = 0.0;
+        if (q < jend) {
+            if (mixed) { p[v][0] = S.fx[slot]; p[v][1] = S.fy[slot]; p[v][2] = S.fz[slot]; }
+            else { p[v][0] = S.px[slot]; p[v][1] = S.py[slot]; p[v][2] = S.pz[slot]; }
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; v++)
+        if (!live[v]) p[v][0] = p[v][1] = p[v][2] = 0.0;
+}
+
 struct StepParams {
     Grid g;
     int nsp;
@@ -269,6 +294,10 @@ struct StepParams {
     int *holes;
     unsigned *hole_count, *ticket;
 };
+
+// Shares that a reduction over the bins deals a tile out in: enough blocks for
+// eight per SM where the tiles alone are too few.
+inline int tile_shares(int ntiles) { return ntiles >= 148 * 8 ? 1 : (148 * 8 + ntiles - 1) / ntiles; }
 
 // The particles of one species that slice q of P.slices of tile t handles:
 // [jbeg, jend) of the bin.  The bins of all species, cut into blocks of
