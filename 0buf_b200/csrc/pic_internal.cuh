@@ -157,15 +157,19 @@ __device__ __forceinline__ void fx_addf(unsigned long long *a, float v, float in
 // (kFxMaxTileSlots guards it).
 constexpr int kFxLoBits = 40;
 constexpr long long kFxMaxTileSlots = 1ll << 23;
-__device__ __forceinline__ void fx_split(double v, double inv_q, long long &ih, long long &il) {
-    const double s = v * inv_q;
-    const double r = rint(s);
-    ih = (long long)r;
-    il = __double2ll_rn((s - r) * 1099511627776.0);  // 2^40
+// s is in quanta with |s| < 2^51 and is rounded by adding 1.5 * 2^52 (to
+// nearest even, as rint): conversions between FP64 and integers run at a
+// quarter of the FP64 add rate.
+constexpr double kRound = 0x1.8p52;
+__device__ __forceinline__ double fx_split(double s, long long &ih) {
+    const double u = s + kRound;
+    ih = __double_as_longlong(u) - 0x4338000000000000ll;
+    return s - (u - kRound);  // the exact remainder
 }
-__device__ __forceinline__ void fx_add2(unsigned long long *hi, unsigned long long *lo, double v, double inv_q) {
-    long long ih, il;
-    fx_split(v, inv_q, ih, il);
+__device__ __forceinline__ void fx_put2(unsigned long long *hi, unsigned long long *lo, double s) {
+    long long ih;
+    const double r = fx_split(s, ih);
+    const long long il = __double_as_longlong(fma(r, 1099511627776.0, kRound)) - 0x4338000000000000ll;  // 2^40
     if (ih) shared_add64(hi, ih);
     if (il) shared_add64(lo, il);
 }
@@ -185,12 +189,10 @@ __device__ __forceinline__ int fx_lo32_bits(long long n) {
     while ((1ll << b) <= n) b++;
     return 31 - b;
 }
-__device__ __forceinline__ void fx_add_lo32(unsigned long long *hi, int *lo, double v, double inv_q,
-                                            double lo_scale) {
-    const double s = v * inv_q;
-    const double r = rint(s);
-    const long long ih = (long long)r;
-    const int il = __double2int_rn((s - r) * lo_scale);  // lo_scale = 2^L: exact
+__device__ __forceinline__ void fx_put_lo32(unsigned long long *hi, int *lo, double s, double lo_scale) {
+    long long ih;
+    const double r = fx_split(s, ih);
+    const int il = __double2loint(fma(r, lo_scale, kRound));  // lo_scale = 2^L: exact
     if (ih) shared_add64(hi, ih);
     if (il) atomicAdd(lo, il);
 }
@@ -293,7 +295,17 @@ struct StepParams {
     int slices;
     int *holes;
     unsigned *hole_count, *ticket;
+    int prefetch;  // plain push: the next particle comes through shared memory (set by its launcher)
 };
+
+// one 4- or 8-byte asynchronous copy from global to shared memory
+template <int B>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(B)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Shares that a reduction over the bins deals a tile out in: enough blocks for
 // eight per SM where the tiles alone are too few.

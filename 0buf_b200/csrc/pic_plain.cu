@@ -7,8 +7,10 @@
 // where the order of the current sums differs (shared/global atomics).
 #include <cuda_runtime.h>
 #include <math.h>
+#include <algorithm>
 #include "pic_internal.cuh"
 #include "pic_kernels.cuh"
+#include "pic_plain_math.cuh"
 
 namespace pic {
 namespace {
@@ -194,64 +196,66 @@ __device__ __forceinline__ double interp_plain(const double *__restrict__ T, int
                                                int bk, int i, int l, int k, double sx, double sx1, double sy,
                                                double sy1, double sz, double sz1, unsigned &bad) {
     if (i < 2 || i > 3 || l < 2 || l > 3 || k < 2 || k > 3) { bad |= ST_STENCIL; return 0.0; }
-    int n = ((bi + i) * SY + (bl + l)) * SZ + (bk + k);
-    int dz = 1, dy = SZ, dx = SY * SZ;
-    double t_ilk = T[n], t_ilk1 = T[n + dz], t_il1k = T[n + dy], t_il1k1 = T[n + dy + dz];
-    double t_i1lk = T[n + dx], t_i1lk1 = T[n + dx + dz], t_i1l1k = T[n + dx + dy], t_i1l1k1 = T[n + dx + dy + dz];
-    double t1 = sx * (sy * (sz * t_ilk + sz1 * t_ilk1) + sy1 * (sz * t_il1k + sz1 * t_il1k1));
-    double t2 = sx1 * (sy * (sz * t_i1lk + sz1 * t_i1lk1) + sy1 * (sz * t_i1l1k + sz1 * t_i1l1k1));
-    return t2 + t1;
+    return trilinear(T + ((bi + i) * SY + (bl + l)) * SZ + (bk + k), SY * SZ, SZ, sx, sx1, sy, sy1, sz, sz1);
 }
 
 // pqr, cell.h:1511-1693, accumulating into the tile J (shared memory).  The
 // reference's divisions by 12 and by tau*h*h are multiplications by their
-// reciprocals (rc[d] = 1 / (tau * h_e * h_f), precomputed): the products feed
-// only the current's magnitude, never an index, and differ from the quotients
-// by an ulp.  LO32 selects the int32 remainder word (fx_add_lo32; words at
-// sJ + 3 nn as 3 nn ints), else the 64-bit one (fx_add2; 3 nn words).
+// reciprocals (rc[d] = 1 / (tau * h_e * h_f) times the charge weight and the
+// inverse quantum, precomputed): the products feed only the current's
+// magnitude, never an index, and differ from the quotients by an ulp.  LO32
+// selects the int32 remainder word (fx_put_lo32; words at sJ + 3 nn as 3 nn
+// ints), else the 64-bit one (fx_put2; 3 nn words).
 template <bool LO32>
-__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double inv_q, double lo_scale, int nn,
-                                          int SY, int SZ, int bi, int bl, int bk, const int iv[3], const double x[3],
-                                          const double x1[3], double a1, double hx, double hy, double hz,
-                                          const double rc[3], double x0, double y0, double z0, unsigned &bad) {
-    double dx = (0.50 * (x[0] + x1[0]) - hx * ((double)iv[0] - 2.50) - x0);
-    double dy = (0.50 * (x[1] + x1[1]) - hy * ((double)iv[1] - 2.50) - y0);
-    double dz = (0.50 * (x[2] + x1[2]) - hz * ((double)iv[2] - 2.50) - z0);
-    double a = a1;
-    double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
+__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double lo_scale, int nn, int SY, int SZ,
+                                          int bi, int bl, int bk, const int iv[3], const double x[3],
+                                          const double x1[3], double hx, double hy, double hz, const double rc[3],
+                                          double x0, double y0, double z0, unsigned &bad) {
+    const double dx = (0.50 * (x[0] + x1[0]) - hx * ((double)iv[0] - 2.50) - x0);
+    const double dy = (0.50 * (x[1] + x1[1]) - hy * ((double)iv[1] - 2.50) - y0);
+    const double dz = (0.50 * (x[2] + x1[2]) - hz * ((double)iv[2] - 2.50) - z0);
+    const double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
     double su = x1[0] - x[0], sv = x1[1] - x[1], sw = x1[2] - x[2];
     constexpr double kTwelfth = 1.0 / 12.0;
-    double s1 = sv * sw * kTwelfth, s2 = su * sw * kTwelfth, s3 = su * sv * kTwelfth;
-    su = su * a * rc[0];
-    sv = sv * a * rc[1];
-    sw = sw * a * rc[2];
+    const double s1 = sv * sw * kTwelfth, s2 = su * sw * kTwelfth, s3 = su * sv * kTwelfth;
+    su = su * rc[0];
+    sv = sv * rc[1];
+    sw = sw * rc[2];
     if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) { bad |= ST_STENCIL; return; }
     const int n = ((bi + iv[0]) * SY + (bl + iv[1])) * SZ + (bk + iv[2]);
     const int ez = 1, ey = SZ, ex = SY * SZ;
     int *lo32 = (int *)(sJ + 3 * nn);
-    // component c, node offset o from n
+    // component c, node offset o from n, contribution v in quanta
     auto add = [&](int c, int o, double v) {
         const int w = c * nn + n + o;
-        if (LO32) fx_add_lo32(&sJ[w], &lo32[w], v, inv_q, lo_scale);
-        else fx_add2(&sJ[w], &sJ[3 * nn + w], v, inv_q);
+        if (LO32) fx_put_lo32(&sJ[w], &lo32[w], v, lo_scale);
+        else fx_put2(&sJ[w], &sJ[3 * nn + w], v);
     };
-    add(0, 0, su * (dy1 * dz1 + s1));
-    add(0, ez, su * (dy1 * dz - s1));
-    add(0, ey, su * (dy * dz1 - s1));
-    add(0, ey + ez, su * (dy * dz + s1));
-    add(1, 0, sv * (dx1 * dz1 + s2));
-    add(1, ez, sv * (dx1 * dz - s2));
-    add(1, ex, sv * (dx * dz1 - s2));
-    add(1, ex + ez, sv * (dx * dz + s2));
-    add(2, 0, sw * (dx1 * dy1 + s3));
-    add(2, ey, sw * (dx1 * dy - s3));
-    add(2, ex, sw * (dx * dy1 - s3));
-    add(2, ex + ey, sw * (dx * dy + s3));
+    add(0, 0, su * fma(dy1, dz1, s1));
+    add(0, ez, su * fma(dy1, dz, -s1));
+    add(0, ey, su * fma(dy, dz1, -s1));
+    add(0, ey + ez, su * fma(dy, dz, s1));
+    add(1, 0, sv * fma(dx1, dz1, s2));
+    add(1, ez, sv * fma(dx1, dz, -s2));
+    add(1, ex, sv * fma(dx, dz1, -s2));
+    add(1, ex + ez, sv * fma(dx, dz, s2));
+    add(2, 0, sw * fma(dx1, dy1, s3));
+    add(2, ey, sw * fma(dx1, dy, -s3));
+    add(2, ex, sw * fma(dx, dy1, -s3));
+    add(2, ex + ey, sw * fma(dx, dy, s3));
 }
 
-// Reflect, cell.h:1427-1478
-__device__ __forceinline__ double reflect_plain(double x, double xm) {
-    return (x > xm) * (x - xm) + (x < 0.0) * (xm + x) + (x > 0 && x < xm) * x;
+// flyDirection (cell.h:694-701): whether the particle leaves its cell
+__device__ __forceinline__ bool moved_cell(const Grid &g, int i, int l, int k, double x, double y, double z, double x0,
+                                           double y0, double z0) {
+    const double hx = g.hx, hy = g.hy, hz = g.hz;
+    int dxd = (((x > x0 + hx) && (x < x0 + 2 * hx)) || ((x < hx) && (i == g.nx - 1)))
+                  ? 2 : (((x < x0) || ((x > g.lx - hx) && (i == 0))) ? 0 : 1);
+    int dyd = (((y > y0 + hy) && (y < y0 + 2 * hy)) || ((y < hy) && (l == g.ny - 1)))
+                  ? 2 : (((y < y0) || ((y > g.ly - hy) && (l == 0))) ? 0 : 1);
+    int dzd = (((z > z0 + hz) && (z < z0 + 2 * hz)) || ((z < hz) && (k == g.nz - 1)))
+                  ? 2 : (((z < z0) || ((z > g.lz - hz) && (k == 0))) ? 0 : 1);
+    return dxd * 9 + dyd * 3 + dzd != 13;
 }
 
 // per-axis receivers of a departing particle: the cells of {c-1, c, c+1}
@@ -275,6 +279,14 @@ __device__ __forceinline__ int receivers(double x, int c, int N, double h, int o
 // better (c2 push 208.7 ms against 246.5 at 256 threads); with the split
 // 64-bit add (shared_add64) the atomics cost nothing measurable and 256
 // threads win: 71.1 ms against 72.7 (384: 75.0, 448: 76.0).
+//
+// Bound: dependent FP64 operations (4 warps per scheduler at 128 registers;
+// `wait` is the top stall, FP64 pipe 35 %, shared-memory pipe 55 %, DRAM 15 %).
+// What shortened the chains, 256x64x64 cells, 201M particles: 17.1 ms; exact
+// cheaper quotients, truncations and roundings and fused multiply-adds
+// (pic_plain_math.cuh; 1648 -> 1367 instructions per 32 particles) 14.0 ms; the
+// next particle by cp.async instead of a load at its use 12.4 ms (then 320
+// threads 14.6, 384 15.4, 512 15.6).
 #ifndef PIC_PLAIN_THREADS
 #define PIC_PLAIN_THREADS 256
 #endif
@@ -319,8 +331,12 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     // start cell (tile-local) with the segment's centre-cell bits
     double *qd = (double *)(sHoles + 2 * kHoleMax) + warp * 6 * kQPlain;
     int *qc = (int *)((double *)(sHoles + 2 * kHoleMax) + (kPlainThreads / 32) * 6 * kQPlain) + warp * kQPlain;
+    // this thread's next particle (P.prefetch): 6 values 32 lanes apart, then the cell
+    double *sNext = (double *)(sHoles + 2 * kHoleMax + (kPlainThreads / 32) * 13 * kQPlain) + warp * (6 * 32 + 16) + lane;
+    int *sNextCell = (int *)(sNext - lane + 6 * 32) + lane;
+    const bool pre = P.prefetch != 0;
     if (threadIdx.x == 0) {
-        double bound = 0.0;
+        double bound = 0.0, one = 0.0;
         long long ntile = 0;
         for (int s = 0, first = 0; s < P.nsp; s++) {
             const int count = P.sp[s].tile_count[t];
@@ -328,12 +344,17 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
             if (SPLIT) slice_range(slice, first, count, kPlainThreads, jbeg, jend);
             first += (count + kPlainThreads - 1) / kPlainThreads;
             bound += 2.5 * fabs(P.sp[s].m) * (double)(jend - jbeg);
+            if (jend > jbeg) one = fmax(one, 1.0834 * fabs(P.sp[s].m));
             ntile += jend - jbeg;
         }
-        int e2;
+        // a quantum that holds every sum of the tile below 2^62 and every single
+        // contribution below 2^51 (fx_split)
+        int e2, e1;
         frexp(bound, &e2);  // bound < 2^e2
-        sQ = ldexp(1.0, e2 - 62);
-        sInvQ = ldexp(1.0, 62 - e2);
+        frexp(one, &e1);
+        const int eq = max(e2 - 62, e1 - 51);
+        sQ = ldexp(1.0, eq);
+        sInvQ = ldexp(1.0, -eq);
         sLoScale = LO32 ? ldexp(1.0, fx_lo32_bits(ntile)) : 1099511627776.0;  // 2^L or 2^40
     }
 
@@ -357,9 +378,8 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
     __syncthreads();
 
     const double hx = g.hx, hy = g.hy, hz = g.hz, tau = g.tau;
-    const double inv_q = sInvQ, lo_scale = sLoScale;
-    // reciprocals of the reference's tau*h*h divisors in pqr
-    const double rc[3] = {1.0 / (tau * hy * hz), 1.0 / (tau * hx * hz), 1.0 / (tau * hx * hy)};
+    const double rhx = 1.0 / hx, rhy = 1.0 / hy, rhz = 1.0 / hz;
+    const double lo_scale = sLoScale;
     unsigned bad = 0;
     double kin = 0.0;
     unsigned long long moved = 0, dropped = 0, dup = 0;
@@ -376,13 +396,32 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
             first += (all + kPlainThreads - 1) / kPlainThreads;
             if (jbeg == count) continue;
         }
-        const double q_m = S.q_m, mw = S.m, M = S.m / S.q_m;
+        const double M = S.m / S.q_m, tau1 = S.q_m * tau * 0.5;
+        // the charge weight over pqr's tau*h*h divisors, in quanta (a power of two)
+        const double mq = S.m * sInvQ;
+        const double rc[3] = {mq / (tau * hy * hz), mq / (tau * hx * hz), mq / (tau * hx * hy)};
         if (!SPLIT) {
             if (threadIdx.x == 0) { sNHoles = 0; sNFront = 0; sNMove = 0; }
             __syncthreads();
         }
         int qn = 0;  // entries in this warp's segment queue (warp-uniform)
         if (lane == 0) sQn[warp] = 0;
+        // the particle of the next iteration comes asynchronously (cp.async) into
+        // shared memory while the current one is processed: registers are full,
+        // and the loads were a fifth of the kernel's stalls
+        auto prefetch = [&](int jn) {
+            if (jn < count) {
+                const int q = start + jn;
+                cp_async<4>(sNextCell, S.cell + q);
+                cp_async<8>(sNext, S.x + q);
+                cp_async<8>(sNext + 32, S.y + q);
+                cp_async<8>(sNext + 64, S.z + q);
+                cp_async<8>(sNext + 96, S.px + q);
+                cp_async<8>(sNext + 128, S.py + q);
+                cp_async<8>(sNext + 160, S.pz + q);
+            }
+        };
+        if (pre) prefetch(jbeg + threadIdx.x);
         __syncwarp();
         // Whole warps iterate together (the queue is drained by whole warps),
         // and past the last particle until the queue is empty.
@@ -392,7 +431,22 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
             const int j = jw + lane;
             const int slot = start + j;
             // cell < 0: past the bin's end, or a dead slot left by an overflowed compaction
-            const int cell = (!tail && j < count) ? S.cell[slot] : -1;
+            int cell = -1;
+            double x = 0.0, y = 0.0, z = 0.0, p[3] = {0.0, 0.0, 0.0};
+            if (pre) {
+                cp_async_wait_all();
+                if (j < count) {
+                    cell = *sNextCell;
+                    x = sNext[0]; y = sNext[32]; z = sNext[64];
+                    p[0] = sNext[96]; p[1] = sNext[128]; p[2] = sNext[160];
+                }
+                __syncwarp();  // the reads come before the next copies into the same place
+                prefetch(j + (int)blockDim.x);
+            } else if (j < count) {
+                cell = S.cell[slot];
+                x = S.x[slot]; y = S.y[slot]; z = S.z[slot];
+                p[0] = S.px[slot]; p[1] = S.py[slot]; p[2] = S.pz[slot];
+            }
             int i = 0, l = 0, k = 0;
             if (cell >= 0) g.cell_ijk(cell, i, l, k);
             const int bi = i - i0 - 2, bl = l - l0 - 2, bk = k - k0 - 2;
@@ -401,84 +455,46 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
             if (cell >= 0 && in_tile) {
                 // Cell ctor, cell.h:731-737
                 const double x0 = (double)i * hx, y0 = (double)l * hy, z0 = (double)k * hz;
-                double x = S.x[slot], y = S.y[slot], z = S.z[slot];
-                double pu = S.px[slot], pv = S.py[slot], pw = S.pz[slot];
+                AxisTaps X, Y, Z;
+                axis_taps(x, x0, hx, rhx, X);
+                axis_taps(y, y0, hy, rhy, Y);
+                axis_taps(z, z0, hz, rhz, Z);
 
-                // (x - x0) / h per axis: GetField's tap index and CurrentToMesh's
-                // start class both truncate it (divided once, the same bits)
-                const double ux = (x - x0) / hx, uy = (y - y0) / hy, uz = (z - z0) / hz;
-
-                // ---- Cell::GetField, cell.h:1257-1290 (InverseKernel 1010-1047)
-                double fEx, fEy, fEz, fHx, fHy, fHz;
+                // ---- Cell::GetField, cell.h:1257-1290
+                double F[6];
                 if (x < 0 || y < 0 || z < 0) {
-                    fEx = fEy = fEz = fHx = fHy = fHz = 0.0;
+#pragma unroll
+                    for (int c = 0; c < 6; c++) F[c] = 0.0;
                 } else {
-                    int ix = (int)(ux + 1.0) + 1;
-                    int i1x = (int)((ux + 1.0) + 1.5);
-                    double s1 = (int)(x / hx + 1.0) - x / hx;
-                    double s2 = (int)(x / hx + 1.5) - 0.5 - x / hx;
-                    int iy = (int)(uy + 1.0) + 1;
-                    int i1y = (int)((uy + 1.0) + 1.5);
-                    double s3 = (int)(y / hy + 1.0) - y / hy;
-                    double s4 = (int)(y / hy + 1.5) - 0.5 - y / hy;
-                    int iz = (int)(uz + 1.0) + 1;
-                    int i1z = (int)((uz + 1.0) + 1.5);
-                    double s5 = (int)(z / hz + 1.0) - z / hz;
-                    double s6 = (int)(z / hz + 1.5) - 0.5 - z / hz;
-                    double s11 = 1. - s1, s21 = 1. - s2, s31 = 1. - s3, s41 = 1. - s4, s51 = 1. - s5, s61 = 1. - s6;
-                    fEx = interp_plain(sF, SY, SZ, bi, bl, bk, ix, i1y, i1z, s1, s11, s4, s41, s6, s61, bad);
-                    fEy = interp_plain(sF + nn, SY, SZ, bi, bl, bk, i1x, iy, i1z, s2, s21, s3, s31, s6, s61, bad);
-                    fEz = interp_plain(sF + 2 * nn, SY, SZ, bi, bl, bk, i1x, i1y, iz, s2, s21, s4, s41, s5, s51, bad);
-                    fHx = interp_plain(sF + 3 * nn, SY, SZ, bi, bl, bk, i1x, iy, iz, s2, s21, s3, s31, s5, s51, bad);
-                    fHy = interp_plain(sF + 4 * nn, SY, SZ, bi, bl, bk, ix, i1y, iz, s1, s11, s4, s41, s5, s51, bad);
-                    fHz = interp_plain(sF + 5 * nn, SY, SZ, bi, bl, bk, ix, iy, i1z, s1, s11, s3, s31, s6, s61, bad);
+                    const double s1 = X.wn, s2 = X.wc, s3 = Y.wn, s4 = Y.wc, s5 = Z.wn, s6 = Z.wc;
+                    const double s11 = 1. - s1, s21 = 1. - s2, s31 = 1. - s3, s41 = 1. - s4, s51 = 1. - s5, s61 = 1. - s6;
+                    F[0] = interp_plain(sF, SY, SZ, bi, bl, bk, X.tn, Y.tc, Z.tc, s1, s11, s4, s41, s6, s61, bad);
+                    F[1] = interp_plain(sF + nn, SY, SZ, bi, bl, bk, X.tc, Y.tn, Z.tc, s2, s21, s3, s31, s6, s61, bad);
+                    F[2] = interp_plain(sF + 2 * nn, SY, SZ, bi, bl, bk, X.tc, Y.tc, Z.tn, s2, s21, s4, s41, s5, s51, bad);
+                    F[3] = interp_plain(sF + 3 * nn, SY, SZ, bi, bl, bk, X.tc, Y.tn, Z.tn, s2, s21, s3, s31, s5, s51, bad);
+                    F[4] = interp_plain(sF + 4 * nn, SY, SZ, bi, bl, bk, X.tn, Y.tc, Z.tn, s1, s11, s4, s41, s5, s51, bad);
+                    F[5] = interp_plain(sF + 5 * nn, SY, SZ, bi, bl, bk, X.tn, Y.tn, Z.tc, s1, s11, s3, s31, s6, s61, bad);
                 }
                 // ---- Particle::Move, particle.h:65-202
-                double tau1 = q_m * tau * 0.5;
-                pu += tau1 * fEx;
-                pv += tau1 * fEy;
-                pw += tau1 * fEz;
-                // pow(v, -0.5) of the reference as 1 / sqrt(v): two correctly rounded
-                // operations, within an ulp of the reference's pow and without its
-                // logarithm/exponential code (16 ms of a c2 push)
-                double ps = tau1 * (1.0 / sqrt((pu * pu + pv * pv + pw * pw) * 1. + 1.0));
-                {
-                    double bx = ps * fHx, by = ps * fHy, bz = ps * fHz;
-                    double su = pu + pv * bz - pw * by;
-                    double sv = pv + pw * bx - pu * bz;
-                    double sw = pw + pu * by - pv * bx;
-                    double q1 = bx * bx, q2 = by * by, q3 = bz * bz, q4 = bx * by, q5 = by * bz, q6 = bz * bx;
-                    // the reference's three divisions by sd as one reciprocal
-                    // (continuous values only: within an ulp of the quotients)
-                    double sd = q1 + 1. + q2 + q3;
-                    const double isd = 1.0 / sd;
-                    double pu1 = ((q1 + 1.) * su + (q4 + bz) * sv + (q6 - by) * sw) * isd;
-                    double pv1 = ((q4 - bz) * su + (q2 + 1.) * sv + (q5 + bx) * sw) * isd;
-                    double pw1 = ((q6 + by) * su + (q5 - bx) * sv + (q3 + 1.) * sw) * isd;
-                    pu = pu1 + fEx * tau1;
-                    pv = pv1 + fEy * tau1;
-                    pw = pw1 + fEz * tau1;
-                }
-                // gamma = sqrt(p^2 + 1), for the new position and the kinetic energy
-                const double p2 = pu * pu + pv * pv + pw * pw;
-                const double gam = sqrt(p2 + 1.0);
-                ps = 1.0 / gam;
-                double xn[3] = {x + tau * (ps * pu), y + tau * (ps * pv), z + tau * (ps * pw)};
+                double p2;
+                const double ig = boris_move(tau1, F, p, p2);
+                const double pu = p[0], pv = p[1], pw = p[2];
+                double xn[3] = {x + tau * (ig * pu), y + tau * (ig * pv), z + tau * (ig * pw)};
                 if (!(isfinite(pu) && isfinite(pv) && isfinite(pw))) bad |= ST_NAN;
-                kin += M * (p2 / (gam + 1.0));  // gamma - 1 without cancellation
+                // gamma - 1 = p^2 / (gamma + 1) without cancellation
+                kin += M * (p2 * ig / (1.0 + ig));
 
                 // ---- Cell::CurrentToMesh, cell.h:1306-1422
                 {
                     double xo[3] = {x, y, z}, x2[3] = {0.0, 0.0, 0.0}, sr;
-                    const double h3[3] = {hx, hy, hz}, o3[3] = {x0, y0, z0}, r3[3] = {ux, uy, uz};
-                    int i1[3], i2[3];
+                    const double h3[3] = {hx, hy, hz}, r3[3] = {rhx, rhy, rhz}, o3[3] = {x0, y0, z0};
+                    const int i1[3] = {X.i1, Y.i1, Z.i1};
+                    int i2[3];
+                    bool exact = true;
 #pragma unroll
-                    for (int d = 0; d < 3; d++) {  // getCellNumberCenterCurrent, cell.h:577-578
-                        double tt = (r3[d] + 1.5);  // (xo - o3) / h3 + 1.5
-                        i1[d] = (int)(tt + 1);
-                        double t2 = ((xn[d] - o3[d]) / h3[d] + 1.5);
-                        i2[d] = (int)(t2 + 1);
-                    }
+                    for (int d = 0; d < 3; d++)  // getCellNumberCenterCurrent, cell.h:577-578
+                        i2[d] = trunc_checked((div_by(xn[d] - o3[d], h3[d], r3[d]) + 1.5) + 1, exact);
+                    if (!exact) { bad |= ST_STENCIL; i2[0] = 0; }
                     int m = 4 * abs(i2[0] - i1[0]) + 2 * abs(i2[1] - i1[1]) + abs(i2[2] - i1[2]);
 #define AVG(d) (h3[d] * (((double)i1[d] + (double)i2[d]) * 0.5 - 2.0) + o3[d])
 #define RATIO(d) ((x2[d] - xo[d]) / (xn[d] - xo[d]))
@@ -521,8 +537,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                     double sb[3];
 #pragma unroll
                     for (int d = 0; d < 3; d++) sb[d] = cross ? x2[d] : xn[d];
-                    pqr_plain<LO32>(sJ, inv_q, lo_scale, nn, SY, SZ, bi, bl, bk, i1, xo, sb, mw, hx, hy, hz, rc, x0, y0,
-                                    z0, bad);
+                    pqr_plain<LO32>(sJ, lo_scale, nn, SY, SZ, bi, bl, bk, i1, xo, sb, hx, hy, hz, rc, x0, y0, z0, bad);
                     if (cross) {
                         if (i2[0] >= 2 && i2[0] <= 3 && i2[1] >= 2 && i2[1] <= 3 && i2[2] >= 2 && i2[2] <= 3) {
                             const int e = atomicAdd(&sQn[warp], 1);  // < 15 + 32: drained at 16
@@ -542,17 +557,15 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                 y = reflect_plain(xn[1], g.ly);
                 z = reflect_plain(xn[2], g.lz);
 
-                // ---- flyDirection (cell.h:694-701) and the receivers of K8
-                int dxd = (((x > x0 + hx) && (x < x0 + 2 * hx)) || ((x < hx) && (i == g.nx - 1)))
-                              ? 2 : (((x < x0) || ((x > g.lx - hx) && (i == 0))) ? 0 : 1);
-                int dyd = (((y > y0 + hy) && (y < y0 + 2 * hy)) || ((y < hy) && (l == g.ny - 1)))
-                              ? 2 : (((y < y0) || ((y > g.ly - hy) && (l == 0))) ? 0 : 1);
-                int dzd = (((z > z0 + hz) && (z < z0 + 2 * hz)) || ((z < hz) && (k == g.nz - 1)))
-                              ? 2 : (((z < z0) || ((z > g.lz - hz) && (k == 0))) ? 0 : 1);
+                // ---- flyDirection (cell.h:694-701) and the receivers of K8.  A
+                // particle within [x0, x0 + h] on every axis stays: the wrap
+                // cases (x < h in the last cell, x > L - h in the first) lie at
+                // least a cell away from that interval.
+                const bool inside = x >= x0 && x <= x0 + hx && y >= y0 && y <= y0 + hy && z >= z0 && z <= z0 + hz;
                 int newcell = cell;
                 bool leave = false;
                 int rx[3], ry[3], rz[3], nrx = 1, nry = 1, nrz = 1;
-                if (dxd * 9 + dyd * 3 + dzd != 13) {
+                if (!inside && moved_cell(g, i, l, k, x, y, z, x0, y0, z0)) {
                     nrx = receivers(x, i, g.nx, hx, rx);
                     nry = receivers(y, l, g.ny, hy, ry);
                     nrz = receivers(z, k, g.nz, hz, rz);
@@ -610,8 +623,8 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                         sa[dd] = qd[dd * kQPlain + e];
                         sb[dd] = qd[(3 + dd) * kQPlain + e];
                     }
-                    pqr_plain<LO32>(sJ, inv_q, lo_scale, nn, SY, SZ, a - 2, b - 2, c - 2, iv, sa, sb, mw, hx, hy, hz,
-                                    rc, (double)qi * hx, (double)ql * hy, (double)qk * hz, bad);
+                    pqr_plain<LO32>(sJ, lo_scale, nn, SY, SZ, a - 2, b - 2, c - 2, iv, sa, sb, hx, hy, hz, rc,
+                                    (double)qi * hx, (double)ql * hy, (double)qk * hz, bad);
                 }
                 qn -= d;
                 __syncwarp();
@@ -754,14 +767,26 @@ void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic
     e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s);
 }
 
+// shared memory of the next particle of every thread
+constexpr size_t kPlainPrefetch = (size_t)(kPlainThreads / 32) * (6 * 32 + 16) * sizeof(double);
+
 size_t push_smem_plain(const Grid &g) {
     size_t nn = (size_t)(g.tx + 2) * (g.ty + 2) * (g.tz + 2);
     return 6 * nn * sizeof(double) + 6 * nn * sizeof(unsigned long long) + 2 * kHoleMax * sizeof(int) +
            (size_t)(kPlainThreads / 32) * kQPlain * (6 * sizeof(double) + sizeof(int));
 }
 
-cudaError_t launch_push_plain(const StepParams &p, bool lo32, cudaStream_t s) {
+cudaError_t launch_push_plain(const StepParams &in, bool lo32, cudaStream_t s) {
+    StepParams p = in;
     size_t smem = push_smem_plain(p.g);
+    // prefetch through shared memory where it leaves as many CTAs on an SM
+    int dev = 0, per_sm = 0, per_block = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    auto fit = [&](size_t b) { return std::min<size_t>(PIC_PLAIN_MIN_BLOCKS, (size_t)per_sm / (b + 2048)); };
+    p.prefetch = smem + kPlainPrefetch <= (size_t)per_block && fit(smem + kPlainPrefetch) >= fit(smem);
+    if (p.prefetch) smem += kPlainPrefetch;
     const bool split = p.slices > 1;
     auto *kern = lo32 ? (split ? k_push_plain<true, true> : k_push_plain<true, false>)
                       : (split ? k_push_plain<false, true> : k_push_plain<false, false>);

@@ -61,3 +61,25 @@ def test_sliced_push_matches_oracle(pkg, oracle_mod, cells, ppc, empty, precisio
         assert len(np.unique(got, axis=0)) == sum(n)
         if sim.layout()["tiles"] > 1:  # a box of one tile wraps inside it
             assert sim.counters()[0] > 0
+
+
+# FP64 push with and without the shared-memory copy of the next particle: the
+# copy is left out where it would cost a CTA per SM (8x6x8 cells) or does not
+# fit (16x9x8), kept otherwise (16x8x8, one CTA per SM)
+@pytest.mark.parametrize("tile", [(8, 6, 8), (16, 9, 8), (16, 8, 8)])
+def test_plain_push_tiles_of_every_staging(pkg, oracle_mod, tile):
+    cells, ppc = (20, 13, 17), 6
+    L = tuple(c * H for c in cells)
+    table = pkg.configs.species_table(ppc)
+    orc = oracle_mod.OracleSim(cells, L, TAU)
+    with pkg.PicSimulation(cells, L, TAU, table, tile=tile) as sim:
+        for i, a in enumerate(species(pkg, cells, ppc, None)):
+            sim.load_particles(i, *a)
+            orc.add_particles(i, *a, table[i][1], table[i][0])
+        for nt in range(3):
+            sim.step(nt)
+            assert orc.step() == 0
+            assert np.array_equal(sim.cell_counts(), orc.cell_counts())
+        for f in ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz", "Jx", "Jy", "Jz"):
+            want = orc.get_field(f)
+            assert np.linalg.norm(sim.get_field(f) - want) <= 1e-12 * np.linalg.norm(want), f
