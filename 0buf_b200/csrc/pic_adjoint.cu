@@ -27,6 +27,7 @@
 #include "pic_kernels.cuh"
 #include "pic_handle.cuh"
 #include "pic_adjoint.cuh"
+#include "pic_plain_math.cuh"
 
 namespace pic {
 
@@ -50,10 +51,10 @@ struct FlatOut {
 struct FlatParams {
     Grid g;
     int nsp;
+    const AdjChunk *chunks;  // one per CTA
     int64_t off[kMaxSpecies + 1];
     FlatSp sp[kMaxSpecies];
     FlatOut out[kMaxSpecies];
-    double *Fout[6];  // optional: the six interpolated field values per particle (flat index)
     const double *E[3];
     const double *H[3];
     double *J[3];
@@ -73,301 +74,182 @@ struct AdjParams {
     const double *LJ[3];  // lambda_J (after the fold's transpose)
     double *LE[3];        // lambda_E_n (scatter target)
     double *LH[3];        // lambda_H_a (scatter target)
-    double *LF[6];        // lambda of the six interpolated field values, per particle (flat index)
-    const double *Fin[6]; // the forward's interpolated fields of this step, or null (gather again)
 };
 
-// Particle handled by thread t of a 256-thread block.  Consecutive particles
-// in the fixed order mostly share a cell, so a warp of consecutive particles
-// would send its 32 current / adjoint atomics of one tap to the same few
-// nodes.  Lane quads take 4 consecutive particles (one 32-byte sector of an
-// FP64 array) and the 8 quads of a warp sit 32 particles apart, i.e. in about
-// 8 different cells: loads stay sector-coalesced and atomic conflicts drop ~8x.
-__device__ __forceinline__ int64_t spread_index(int t) {
-    return (int64_t)blockIdx.x * kT + ((t & 31) >> 2) * 32 + (t >> 5) * 4 + (t & 3);
-}
+constexpr int kW = kT / 32;        // warps per CTA
+constexpr int kQueuePlain = 48;    // queued second segments per warp, as in k_push_plain
+constexpr int kFlatWindow = 900;   // nodes of the forward's window: 109 KB of shared memory, two CTAs per SM
+constexpr int kAdjWindow = 640;    // nodes of the adjoint's: 106 KB
 
-__device__ __forceinline__ int species_of(const int64_t *off, int nsp, int64_t idx) {
-    int s = 0;
-    while (s + 1 < nsp && idx >= off[s + 1]) s++;
-    return s;
-}
-
-// staggered interpolation of one particle: lower tap (reference tile index)
-// and its weight per axis, node- and centre-staggered (InverseKernel,
-// cell.h:1010-1047, as evaluated in Cell::GetField, cell.h:1257-1290)
-struct Taps {
-    int tn[3], tc[3];
-    double wn[3], wc[3];
-};
-// the discrete part of the taps: tap indices and the integer parts of the
-// weights (nI = int(x/h + 1), cI = int(x/h + 1.5)); the weights follow from them
-struct TapInts {
-    int tn[3], tc[3], nI[3], cI[3];
-};
-__device__ __forceinline__ void tap_ints(const Grid &g, int i, int l, int k, const double x[3], TapInts &I) {
-    const double h3[3] = {g.hx, g.hy, g.hz};
-    const int c3[3] = {i, l, k};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        double x0 = (double)c3[d] * h3[d];
-        I.tn[d] = (int)((x[d] - x0) / h3[d] + 1.0) + 1;
-        I.tc[d] = (int)(((x[d] - x0) / h3[d] + 1.0) + 1.5);
-        I.nI[d] = (int)(x[d] / h3[d] + 1.0);
-        I.cI[d] = (int)(x[d] / h3[d] + 1.5);
+// shared memory of a thread's next particle (cp.async, as in k_push_plain)
+constexpr size_t kNextBytes = (size_t)kW * (6 * 32 + 16) * sizeof(double);
+struct NextParticle {
+    double *v;
+    int *c;
+    __device__ __forceinline__ NextParticle(void *base) {
+        const int lane = threadIdx.x & 31;
+        double *b = (double *)base + (threadIdx.x >> 5) * (6 * 32 + 16);
+        v = b + lane;
+        c = (int *)(b + 6 * 32) + lane;
     }
-}
-__device__ __forceinline__ void taps_from(const Grid &g, const double x[3], const TapInts &I, Taps &T) {
-    const double h3[3] = {g.hx, g.hy, g.hz};
+    __device__ __forceinline__ void start(const FlatSp &S, int64_t j) const {
+        cp_async<4>(c, S.cell + j);
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        T.tn[d] = I.tn[d];
-        T.tc[d] = I.tc[d];
-        T.wn[d] = I.nI[d] - x[d] / h3[d];
-        T.wc[d] = I.cI[d] - 0.5 - x[d] / h3[d];
+        for (int a = 0; a < 6; a++) cp_async<8>(v + 32 * a, S.v[a] + j);
     }
-}
-__device__ __forceinline__ void taps_plain(const Grid &g, int i, int l, int k, const double x[3], Taps &T) {
-    TapInts I;
-    tap_ints(g, i, l, k, x, I);
-    taps_from(g, x, I, T);
-}
+    __device__ __forceinline__ int take(double x[3], double p[3]) const {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            x[d] = v[32 * d];
+            p[d] = v[32 * (3 + d)];
+        }
+        return *c;
+    }
+};
+
+// the same for its six adjoints
+constexpr size_t kNextLamBytes = (size_t)kW * 6 * 32 * sizeof(double);
+struct NextLam {
+    double *v;
+    __device__ __forceinline__ NextLam(void *base) {
+        v = (double *)base + (threadIdx.x >> 5) * (6 * 32) + (threadIdx.x & 31);
+    }
+    __device__ __forceinline__ void start(const LamSp &L, int64_t j) const {
+#pragma unroll
+        for (int a = 0; a < 6; a++) cp_async<8>(v + 32 * a, L.v[a] + j);
+    }
+    __device__ __forceinline__ void take(double lx[3], double lp[3]) const {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            lx[d] = v[32 * d];
+            lp[d] = v[32 * (3 + d)];
+        }
+    }
+};
+
+// A particle's view of the fields: the CTA's window in shared memory (WIN) or
+// the arrays in global memory.  n0 is the node of the particle's cell.
+template <bool WIN>
+struct FieldView {
+    const double *base[6];
+    int n0, dx, dy;
+    __device__ __forceinline__ int at(int tx, int ty, int tz) const {
+        return n0 + (tx - 2) * dx + (ty - 2) * dy + (tz - 2);
+    }
+};
 // component c (0..2 E, 3..5 H) is node-staggered along axis d when
 // (E_c and d == c) or (H_c and d != c)
-__device__ __forceinline__ bool node_axis(int c, int d) { return c < 3 ? d == c : d != c - 3; }
+__device__ __forceinline__ constexpr bool node_axis(int c, int d) { return c < 3 ? d == c : d != c - 3; }
 
-// the 8 taps of one component: value (interp_plain's expression order) and
-// the tap base; false when a tap leaves the 3-node stencil (CFL violation)
-__device__ __forceinline__ bool comp_taps(const Taps &T, int c, int t[3], double w[3]) {
-    bool ok = true;
+// GetField (cell.h:1257-1290) at the particle; false if a tap left the stencil
+// (that component is then 0, as in k_push_plain)
+template <class V>
+__device__ __forceinline__ bool gather_fields(const V &A, const AxisTaps T[3], double F[6]) {
+    bool okn[3], okc[3], ok = true;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        bool nd = node_axis(c, d);
-        t[d] = nd ? T.tn[d] : T.tc[d];
-        w[d] = nd ? T.wn[d] : T.wc[d];
-        ok = ok && t[d] >= 2 && t[d] <= 3;
+        okn[d] = T[d].tn >= 2 && T[d].tn <= 3;
+        okc[d] = T[d].tc >= 2 && T[d].tc <= 3;
     }
-    return ok;
-}
-__device__ __forceinline__ size_t tap_node(const Grid &g, int i, int l, int k, const int t[3]) {
-    return g.node(i + t[0] - 2, l + t[1] - 2, k + t[2] - 2);
-}
-__device__ __forceinline__ double interp_g(const double *__restrict__ A, size_t n, size_t dx, size_t dy,
-                                           const double w[3]) {
-    const size_t dz = 1;
-    double sx = w[0], sx1 = 1. - w[0], sy = w[1], sy1 = 1. - w[1], sz = w[2], sz1 = 1. - w[2];
-    double t_ilk = A[n], t_ilk1 = A[n + dz], t_il1k = A[n + dy], t_il1k1 = A[n + dy + dz];
-    double t_i1lk = A[n + dx], t_i1lk1 = A[n + dx + dz], t_i1l1k = A[n + dx + dy], t_i1l1k1 = A[n + dx + dy + dz];
-    double t1 = sx * (sy * (sz * t_ilk + sz1 * t_ilk1) + sy1 * (sz * t_il1k + sz1 * t_il1k1));
-    double t2 = sx1 * (sy * (sz * t_i1lk + sz1 * t_i1lk1) + sy1 * (sz * t_i1l1k + sz1 * t_i1l1k1));
-    return t2 + t1;
-}
-
-// fields at the particle (all six components); false if a stencil left range
-// (negative_is_zero: the reference's GetField gives no field at a negative
-// coordinate; positions are wrapped into [0, L) so a run never meets it, and a
-// replay of frozen branches, whose wraps are fixed, leaves it out)
-__device__ __forceinline__ bool gather_fields_taps(const Grid &g, const double *const E[3],
-                                                   const double *const H[3], int i, int l, int k, const double x[3],
-                                                   const Taps &T, double F[6], bool negative_is_zero = true) {
-    if (negative_is_zero && (x[0] < 0 || x[1] < 0 || x[2] < 0)) {
-        for (int c = 0; c < 6; c++) F[c] = 0.0;
-        return true;
-    }
-    const size_t dx = (size_t)g.NY * g.pz, dy = g.pz;
-    bool ok = true;
 #pragma unroll
     for (int c = 0; c < 6; c++) {
-        int t[3];
-        double w[3];
-        if (!comp_taps(T, c, t, w)) { ok = false; F[c] = 0.0; continue; }
-        F[c] = interp_g(c < 3 ? E[c] : H[c - 3], tap_node(g, i, l, k, t), dx, dy, w);
+        const bool nx = node_axis(c, 0), ny = node_axis(c, 1), nz = node_axis(c, 2);
+        if (!((nx ? okn[0] : okc[0]) && (ny ? okn[1] : okc[1]) && (nz ? okn[2] : okc[2]))) {
+            ok = false;
+            F[c] = 0.0;
+            continue;
+        }
+        const int n = A.at(nx ? T[0].tn : T[0].tc, ny ? T[1].tn : T[1].tc, nz ? T[2].tn : T[2].tc);
+        const double wx = nx ? T[0].wn : T[0].wc, wy = ny ? T[1].wn : T[1].wc, wz = nz ? T[2].wn : T[2].wc;
+        F[c] = trilinear(A.base[c] + n, A.dx, A.dy, wx, 1. - wx, wy, 1. - wy, wz, 1. - wz);
     }
     return ok;
 }
-__device__ __forceinline__ bool gather_fields(const Grid &g, const double *const E[3], const double *const H[3],
-                                              int i, int l, int k, const double x[3], double F[6]) {
-    Taps T;
-    taps_plain(g, i, l, k, x, T);
-    return gather_fields_taps(g, E, H, i, l, k, x, T, F);
-}
 
-// Particle::Move, particle.h:65-202, with the intermediates the adjoint needs
-struct Boris {
-    double t, u[3], g1, ps, b[3], s[3], sd, up[3], pp[3], g2, x1[3];
-};
-__device__ __forceinline__ void boris_plain(double q_m, double tau, const double p[3], const double F[6],
-                                            const double x[3], Boris &B) {
-    double tau1 = q_m * tau * 0.5;
-    B.t = tau1;
-    double pu = p[0], pv = p[1], pw = p[2];
-    pu += tau1 * F[0];
-    pv += tau1 * F[1];
-    pw += tau1 * F[2];
-    B.u[0] = pu; B.u[1] = pv; B.u[2] = pw;
-    B.g1 = 1.0 / sqrt((pu * pu + pv * pv + pw * pw) * 1. + 1.0);  // pow(v, -0.5), as in k_push_plain
-    double ps = tau1 * B.g1;
-    B.ps = ps;
-    double bx = ps * F[3], by = ps * F[4], bz = ps * F[5];
-    B.b[0] = bx; B.b[1] = by; B.b[2] = bz;
-    double su = pu + pv * bz - pw * by;
-    double sv = pv + pw * bx - pu * bz;
-    double sw = pw + pu * by - pv * bx;
-    B.s[0] = su; B.s[1] = sv; B.s[2] = sw;
-    double q1 = bx * bx, q2 = by * by, q3 = bz * bz, q4 = bx * by, q5 = by * bz, q6 = bz * bx;
-    double sd = q1 + 1. + q2 + q3;
-    B.sd = sd;
-    double pu1 = ((q1 + 1.) * su + (q4 + bz) * sv + (q6 - by) * sw) / sd;
-    double pv1 = ((q4 - bz) * su + (q2 + 1.) * sv + (q5 + bx) * sw) / sd;
-    double pw1 = ((q6 + by) * su + (q5 - bx) * sv + (q3 + 1.) * sw) / sd;
-    B.up[0] = pu1; B.up[1] = pv1; B.up[2] = pw1;
-    pu = pu1 + F[0] * tau1;
-    pv = pv1 + F[1] * tau1;
-    pw = pw1 + F[2] * tau1;
-    B.pp[0] = pu; B.pp[1] = pv; B.pp[2] = pw;
-    B.g2 = 1.0 / sqrt(((pu * pu + pv * pv + pw * pw) + 1.0));
-    B.x1[0] = x[0] + tau * (B.g2 * pu);
-    B.x1[1] = x[1] + tau * (B.g2 * pv);
-    B.x1[2] = x[2] + tau * (B.g2 * pw);
-}
-
-// zigzag split of CurrentToMesh, cell.h:1306-1422 (m = 4|di| + 2|dl| + |dk|)
+// zigzag split of CurrentToMesh, cell.h:1306-1422
 struct Split {
     int m, i1[3], i2[3];
     double x2[3], sr;
 };
-// the discrete part: cell-centre indices of both end points
-// (getCellNumberCenterCurrent, cell.h:577-578)
-__device__ __forceinline__ void split_ints(const Grid &g, const double xo[3], const double xn[3], const double o3[3],
-                                           Split &S) {
-    const double h3[3] = {g.hx, g.hy, g.hz};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        double tt = ((xo[d] - o3[d]) / h3[d] + 1.5);
-        S.i1[d] = (int)(tt + 1);
-        double t2 = ((xn[d] - o3[d]) / h3[d] + 1.5);
-        S.i2[d] = (int)(t2 + 1);
-    }
-}
-// the split case and relay point from S.i1, S.i2
-__device__ __forceinline__ void split_from(const Grid &g, const double xo[3], const double xn[3], const double o3[3],
-                                           Split &S) {
-    const double h3[3] = {g.hx, g.hy, g.hz};
-    double *x2 = S.x2;
-    x2[0] = x2[1] = x2[2] = 0.0;
-    S.sr = 0.0;
-    double sr = 0.0;
-    const int *i1 = S.i1, *i2 = S.i2;
-    int m = 4 * abs(i2[0] - i1[0]) + 2 * abs(i2[1] - i1[1]) + abs(i2[2] - i1[2]);
-    S.m = m;
-#define AVG(d) (h3[d] * (((double)i1[d] + (double)i2[d]) * 0.5 - 2.0) + o3[d])
-#define RATIO(d) ((x2[d] - xo[d]) / (xn[d] - xo[d]))
-#define PROD(d) ((x2[d] - xo[d]) * (xn[d] - xo[d]))
-#define RBX(d) (xo[d] + (xn[d] - xo[d]) * sr)
-#define SQ(v) ((v) * (v))
-    switch (m) {
-        case 1: x2[2] = AVG(2); sr = RATIO(2); x2[0] = RBX(0); x2[1] = RBX(1); break;
-        case 2: x2[1] = AVG(1); sr = RATIO(1); x2[0] = RBX(0); x2[2] = RBX(2); break;
-        case 3:
-            x2[1] = AVG(1); x2[2] = AVG(2);
-            sr = (PROD(2) + PROD(1)) / (SQ(xn[2] - xo[2]) + SQ(xn[1] - xo[1]));
-            x2[0] = RBX(0);
-            break;
-        case 4: x2[0] = AVG(0); sr = RATIO(0); x2[1] = RBX(1); x2[2] = RBX(2); break;
-        case 5:
-            x2[0] = AVG(0); x2[2] = AVG(2);
-            sr = (PROD(2) + PROD(0)) / (SQ(xn[2] - xo[2]) + SQ(xn[0] - xo[0]));
-            x2[1] = RBX(1);
-            break;
-        case 6:
-            x2[0] = AVG(0); x2[1] = AVG(1);
-            sr = (PROD(1) + PROD(0)) / (SQ(xn[1] - xo[1]) + SQ(xn[0] - xo[0]));
-            x2[2] = RBX(2);
-            break;
-        case 7: x2[0] = AVG(0); x2[1] = AVG(1); x2[2] = AVG(2); break;
-        default: break;
-    }
-#undef AVG
-#undef RATIO
-#undef PROD
-#undef RBX
-#undef SQ
-    S.sr = sr;
-}
-__device__ __forceinline__ void split_plain(const Grid &g, const double xo[3], const double xn[3], const double o3[3],
-                                            Split &S) {
-    split_ints(g, xo, xn, o3, S);
-    split_from(g, xo, xn, o3, S);
-}
 
-// one pqr segment (cell.h:1511-1693) into the global J, FP64 atomics
-__device__ __forceinline__ void seg_plain(double *const J[3], const Grid &g, int ci, int cl, int ck, const int iv[3],
-                                          const double x[3], const double x1[3], double a1, const double o3[3],
-                                          unsigned &bad) {
-    const double hx = g.hx, hy = g.hy, hz = g.hz, tau = g.tau;
-    double dx = (0.50 * (x[0] + x1[0]) - hx * ((double)iv[0] - 2.50) - o3[0]);
-    double dy = (0.50 * (x[1] + x1[1]) - hy * ((double)iv[1] - 2.50) - o3[1]);
-    double dz = (0.50 * (x[2] + x1[2]) - hz * ((double)iv[2] - 2.50) - o3[2]);
-    double a = a1;
-    double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
+// one pqr segment (cell.h:1511-1693) into the global J, FP64 atomics (particles
+// outside their CTA's window); rc[d] = m / (tau * h_e * h_f)
+__device__ __forceinline__ void seg_global(double *const J[3], const Grid &g, int ci, int cl, int ck, const int iv[3],
+                                           const double x[3], const double x1[3], const double rc[3],
+                                           const double o3[3], unsigned &bad) {
+    const double hx = g.hx, hy = g.hy, hz = g.hz;
+    const double dx = (0.50 * (x[0] + x1[0]) - hx * ((double)iv[0] - 2.50) - o3[0]);
+    const double dy = (0.50 * (x[1] + x1[1]) - hy * ((double)iv[1] - 2.50) - o3[1]);
+    const double dz = (0.50 * (x[2] + x1[2]) - hz * ((double)iv[2] - 2.50) - o3[2]);
+    const double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
     double su = x1[0] - x[0], sv = x1[1] - x[1], sw = x1[2] - x[2];
-    double s1 = sv * sw / 12.0, s2 = su * sw / 12.0, s3 = su * sv / 12.0;
-    su = su * a / (tau * hy * hz);
-    sv = sv * a / (tau * hx * hz);
-    sw = sw * a / (tau * hx * hy);
+    constexpr double kTwelfth = 1.0 / 12.0;
+    const double s1 = sv * sw * kTwelfth, s2 = su * sw * kTwelfth, s3 = su * sv * kTwelfth;
+    su = su * rc[0];
+    sv = sv * rc[1];
+    sw = sw * rc[2];
     if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) { bad |= ST_STENCIL; return; }
-    size_t n = tap_node(g, ci, cl, ck, iv);
+    const size_t n = g.node(ci + iv[0] - 2, cl + iv[1] - 2, ck + iv[2] - 2);
     const size_t ez = 1, ey = g.pz, ex = (size_t)g.NY * g.pz;
     double *Jx = J[0], *Jy = J[1], *Jz = J[2];
-    atomicAdd(&Jx[n], su * (dy1 * dz1 + s1));
-    atomicAdd(&Jx[n + ez], su * (dy1 * dz - s1));
-    atomicAdd(&Jx[n + ey], su * (dy * dz1 - s1));
-    atomicAdd(&Jx[n + ey + ez], su * (dy * dz + s1));
-    atomicAdd(&Jy[n], sv * (dx1 * dz1 + s2));
-    atomicAdd(&Jy[n + ez], sv * (dx1 * dz - s2));
-    atomicAdd(&Jy[n + ex], sv * (dx * dz1 - s2));
-    atomicAdd(&Jy[n + ex + ez], sv * (dx * dz + s2));
-    atomicAdd(&Jz[n], sw * (dx1 * dy1 + s3));
-    atomicAdd(&Jz[n + ey], sw * (dx1 * dy - s3));
-    atomicAdd(&Jz[n + ex], sw * (dx * dy1 - s3));
-    atomicAdd(&Jz[n + ex + ey], sw * (dx * dy + s3));
+    atomicAdd(&Jx[n], su * fma(dy1, dz1, s1));
+    atomicAdd(&Jx[n + ez], su * fma(dy1, dz, -s1));
+    atomicAdd(&Jx[n + ey], su * fma(dy, dz1, -s1));
+    atomicAdd(&Jx[n + ey + ez], su * fma(dy, dz, s1));
+    atomicAdd(&Jy[n], sv * fma(dx1, dz1, s2));
+    atomicAdd(&Jy[n + ez], sv * fma(dx1, dz, -s2));
+    atomicAdd(&Jy[n + ex], sv * fma(dx, dz1, -s2));
+    atomicAdd(&Jy[n + ex + ez], sv * fma(dx, dz, s2));
+    atomicAdd(&Jz[n], sw * fma(dx1, dy1, s3));
+    atomicAdd(&Jz[n + ey], sw * fma(dx1, dy, -s3));
+    atomicAdd(&Jz[n + ex], sw * fma(dx, dy1, -s3));
+    atomicAdd(&Jz[n + ex + ey], sw * fma(dx, dy, s3));
 }
 
-// transpose of seg_plain: lambda_J gathered at the segment's 12 nodes gives
-// the gradient with respect to the segment's end points (added to gs, ge)
-__device__ __forceinline__ void seg_plain_rev(const double *const L[3], const Grid &g, int ci, int cl, int ck,
-                                              const int iv[3], const double xs[3], const double xe[3], double a,
-                                              const double o3[3], double gs[3], double ge[3]) {
-    if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) return;
-    const double hx = g.hx, hy = g.hy, hz = g.hz, tau = g.tau;
-    double dx = 0.5 * (xs[0] + xe[0]) - hx * ((double)iv[0] - 2.5) - o3[0];
-    double dy = 0.5 * (xs[1] + xe[1]) - hy * ((double)iv[1] - 2.5) - o3[1];
-    double dz = 0.5 * (xs[2] + xe[2]) - hz * ((double)iv[2] - 2.5) - o3[2];
-    double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
-    double Dx = xe[0] - xs[0], Dy = xe[1] - xs[1], Dz = xe[2] - xs[2];
-    double s1 = Dy * Dz / 12.0, s2 = Dx * Dz / 12.0, s3 = Dx * Dy / 12.0;
-    double cu = a / (tau * hy * hz), cv = a / (tau * hx * hz), cw = a / (tau * hx * hy);
-    double Ax = cu * Dx, Ay = cv * Dy, Az = cw * Dz;
-    size_t n = tap_node(g, ci, cl, ck, iv);
-    const size_t ez = 1, ey = g.pz, ex = (size_t)g.NY * g.pz;
-    double Lx0 = L[0][n], Lx1 = L[0][n + ez], Lx2 = L[0][n + ey], Lx3 = L[0][n + ey + ez];
-    double Ly0 = L[1][n], Ly1 = L[1][n + ez], Ly2 = L[1][n + ex], Ly3 = L[1][n + ex + ez];
-    double Lz0 = L[2][n], Lz1 = L[2][n + ey], Lz2 = L[2][n + ex], Lz3 = L[2][n + ex + ey];
-    double Fx = Lx0 * (dy1 * dz1 + s1) + Lx1 * (dy1 * dz - s1) + Lx2 * (dy * dz1 - s1) + Lx3 * (dy * dz + s1);
-    double Fy = Ly0 * (dx1 * dz1 + s2) + Ly1 * (dx1 * dz - s2) + Ly2 * (dx * dz1 - s2) + Ly3 * (dx * dz + s2);
-    double Fz = Lz0 * (dx1 * dy1 + s3) + Lz1 * (dx1 * dy - s3) + Lz2 * (dx * dy1 - s3) + Lz3 * (dx * dy + s3);
-    double Kx = Lx0 - Lx1 - Lx2 + Lx3, Ky = Ly0 - Ly1 - Ly2 + Ly3, Kz = Lz0 - Lz1 - Lz2 + Lz3;
+// transpose of a pqr segment: lambda_J (L: three components, n the segment's
+// base node, ex, ey the node strides) gathered at its 12 nodes gives the
+// gradient with respect to the segment's end points (added to gs, ge)
+__device__ __forceinline__ void seg_rev(const double *L0, const double *L1, const double *L2, int n, int ex, int ey,
+                                        const Grid &g, const int iv[3], const double xs[3], const double xe[3],
+                                        const double rc[3], const double o3[3], double gs[3], double ge[3]) {
+    constexpr double kTwelfth = 1.0 / 12.0;
+    const double hx = g.hx, hy = g.hy, hz = g.hz;
+    const double dx = 0.5 * (xs[0] + xe[0]) - hx * ((double)iv[0] - 2.5) - o3[0];
+    const double dy = 0.5 * (xs[1] + xe[1]) - hy * ((double)iv[1] - 2.5) - o3[1];
+    const double dz = 0.5 * (xs[2] + xe[2]) - hz * ((double)iv[2] - 2.5) - o3[2];
+    const double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
+    const double Dx = xe[0] - xs[0], Dy = xe[1] - xs[1], Dz = xe[2] - xs[2];
+    const double s1 = Dy * Dz * kTwelfth, s2 = Dx * Dz * kTwelfth, s3 = Dx * Dy * kTwelfth;
+    const double Ax = rc[0] * Dx, Ay = rc[1] * Dy, Az = rc[2] * Dz;
+    // per component the four nodes as sums over its two transverse axes:
+    // F = sum L (weight + or - s), K = L00 - L01 - L10 + L11, and the weights'
+    // derivatives along the two axes
+    double a, b, c, d;
+    a = L0[n]; b = L0[n + 1]; c = L0[n + ey]; d = L0[n + ey + 1];
+    const double Kx = (a - b) + (d - c);
+    const double xz0 = fma(a, dz1, b * dz), xz1 = fma(c, dz1, d * dz);   // z sums of the lower and the upper y row
+    const double Fx = fma(dy1, xz0, fma(dy, xz1, s1 * Kx));
+    const double x_dy = xz1 - xz0, x_dz = fma(dy1, b - a, dy * (d - c));
+    a = L1[n]; b = L1[n + 1]; c = L1[n + ex]; d = L1[n + ex + 1];
+    const double Ky = (a - b) + (d - c);
+    const double yz0 = fma(a, dz1, b * dz), yz1 = fma(c, dz1, d * dz);
+    const double Fy = fma(dx1, yz0, fma(dx, yz1, s2 * Ky));
+    const double y_dx = yz1 - yz0, y_dz = fma(dx1, b - a, dx * (d - c));
+    a = L2[n]; b = L2[n + ey]; c = L2[n + ex]; d = L2[n + ex + ey];
+    const double Kz = (a - b) + (d - c);
+    const double zy0 = fma(a, dy1, b * dy), zy1 = fma(c, dy1, d * dy);
+    const double Fz = fma(dx1, zy0, fma(dx, zy1, s3 * Kz));
+    const double z_dx = zy1 - zy0, z_dy = fma(dx1, b - a, dx * (d - c));
     // d/d(D): direct factor and the D-products in s1, s2, s3
-    double gDx = cu * Fx + (Ay * Ky * Dz + Az * Kz * Dy) / 12.0;
-    double gDy = cv * Fy + (Ax * Kx * Dz + Az * Kz * Dx) / 12.0;
-    double gDz = cw * Fz + (Ax * Kx * Dy + Ay * Ky * Dx) / 12.0;
+    const double kx = Ax * Kx * kTwelfth, ky = Ay * Ky * kTwelfth, kz = Az * Kz * kTwelfth;
+    const double gDx = fma(rc[0], Fx, fma(ky, Dz, kz * Dy));
+    const double gDy = fma(rc[1], Fy, fma(kx, Dz, kz * Dx));
+    const double gDz = fma(rc[2], Fz, fma(kx, Dy, ky * Dx));
     // d/d(dx, dy, dz): the bilinear node weights
-    double gdx = Ay * (-Ly0 * dz1 - Ly1 * dz + Ly2 * dz1 + Ly3 * dz) + Az * (-Lz0 * dy1 - Lz1 * dy + Lz2 * dy1 + Lz3 * dy);
-    double gdy = Ax * (-Lx0 * dz1 - Lx1 * dz + Lx2 * dz1 + Lx3 * dz) + Az * (-Lz0 * dx1 + Lz1 * dx1 - Lz2 * dx + Lz3 * dx);
-    double gdz = Ax * (-Lx0 * dy1 + Lx1 * dy1 - Lx2 * dy + Lx3 * dy) + Ay * (-Ly0 * dx1 + Ly1 * dx1 - Ly2 * dx + Ly3 * dx);
-    gs[0] += 0.5 * gdx - gDx; ge[0] += 0.5 * gdx + gDx;
-    gs[1] += 0.5 * gdy - gDy; ge[1] += 0.5 * gdy + gDy;
-    gs[2] += 0.5 * gdz - gDz; ge[2] += 0.5 * gdz + gDz;
+    const double gdx = fma(Ay, y_dx, Az * z_dx), gdy = fma(Ax, x_dy, Az * z_dy), gdz = fma(Ax, x_dz, Ay * y_dz);
+    gs[0] += fma(0.5, gdx, -gDx); ge[0] += fma(0.5, gdx, gDx);
+    gs[1] += fma(0.5, gdy, -gDy); ge[1] += fma(0.5, gdy, gDy);
+    gs[2] += fma(0.5, gdz, -gDz); ge[2] += fma(0.5, gdz, gDz);
 }
 
 // transpose of the split point x2(xo, xn): adds g2 . dx2/dxo to gx, . dx2/dxn
@@ -415,12 +297,9 @@ __device__ __forceinline__ void split_rev(const Split &S, const double xo[3], co
     }
 }
 
-// Reflect, cell.h:1427-1478
-__device__ __forceinline__ double reflect_g(double x, double xm) {
-    return (x > xm) * (x - xm) + (x < 0.0) * (xm + x) + (x > 0 && x < xm) * x;
-}
-// reflect_g as a choice (0 keep, 1 subtract xm, 2 add xm, 3 the x == xm case: 0)
-// and its application; apply_wrap(x, xm, wrap_choice(x, xm)) == reflect_g(x, xm)
+// the wrap of Reflect (cell.h:1427-1478) as a choice (0 keep, 1 subtract xm, 2
+// add xm, 3 the x == xm case: 0); apply_wrap(x, xm, wrap_choice(x, xm)) ==
+// reflect_plain(x, xm)
 __device__ __forceinline__ int wrap_choice(double x, double xm) {
     return x > xm ? 1 : (x < 0.0 ? 2 : (x == xm ? 3 : 0));
 }
@@ -486,305 +365,610 @@ __device__ __forceinline__ int new_cell_plain(const Grid &g, int cell, int i, in
     return g.cell_of(rx, ry, rz);
 }
 
+// stages the window's nodes of `n` arrays src[c] into dst (n x w.nn doubles)
+template <int N>
+__device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow &w, const double *const *src, double *dst) {
+    for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
+        const int c = e % w.SZ, ab = e / w.SZ, b = ab % w.SY, a = ab / w.SY;
+        const size_t n = g.node(w.i0 + a, w.l0 + b, w.k0 + c);
+#pragma unroll
+        for (int q = 0; q < N; q++) dst[q * w.nn + e] = src[q][n];
+    }
+}
+
 // ---- flat forward step of all particles (push + deposit + cell update).
-// Four CTAs per SM (64 registers, some spills): the kernel gathers its field
-// taps from global memory and waits on them; 32 warps per SM hide more of
-// that than 16 at 96 registers (c3 forward about 9 % faster)
-__global__ void __launch_bounds__(kT, 4) k_flat_push_plain(FlatParams P) {
-    int64_t idx = spread_index(threadIdx.x);
+//
+// One CTA per chunk of consecutive particles (they share a neighbourhood: the
+// fixed order is tile by tile at the start of the run).  The chunk's window --
+// the nodes around its cells -- is staged into shared memory, and its current
+// is summed there in the exact fixed point of k_push_plain and added to the
+// global J once; a particle outside the window gathers from and adds to
+// global memory.  Bound: dependent FP64 operations, as k_push_plain.  128x32x32
+// cells, 12.6M particles: 1.58 -> 1.12 ms per step (before: taps gathered from
+// and currents added to global memory, one particle per thread).
+template <int BMODE>
+__global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ AdjWindow sWin;
+    __shared__ int sRed[15 * kW], sQn[kW];
+    __shared__ double sQ, sInvQ;
+    double *sF = (double *)smem_raw;
+    unsigned long long *sJ = (unsigned long long *)(sF + 6 * kFlatWindow);  // 3 nn words, then 3 nn ints
+    unsigned char *sTail = smem_raw + (size_t)kFlatWindow * (6 * sizeof(double) + 3 * 12);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *qd = (double *)sTail + warp * 6 * kQueuePlain;
+    int *qc = (int *)((double *)sTail + kW * 6 * kQueuePlain) + warp * kQueuePlain;
+    const NextParticle next(sTail + (size_t)kW * kQueuePlain * 52);
+    const Grid &g = P.g;
+    const AdjChunk ch = P.chunks[blockIdx.x];
+    const int s = ch.species, count = ch.count;
+    const FlatSp &S = P.sp[s];
+    if ((int)threadIdx.x < count) next.start(S, ch.first + threadIdx.x);
+    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
+    const int nn = w.nn;
+    if (threadIdx.x == 0) {
+        // the quantum of k_push_plain's tile current, for this chunk
+        int e2, e1;
+        frexp(2.5 * fabs(S.m) * (double)count, &e2);
+        frexp(1.0834 * fabs(S.m), &e1);
+        const int eq = max(e2 - 62, e1 - 51);
+        sQ = ldexp(1.0, eq);
+        sInvQ = ldexp(1.0, -eq);
+    }
+    const double *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
+    stage_window<6>(g, w, src, sF);
+    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
+        sJ[e] = 0ull;
+        ((int *)(sJ + 3 * nn))[e] = 0;
+    }
+    if (lane == 0) sQn[warp] = 0;
+    __syncthreads();
+    const double h3[3] = {g.hx, g.hy, g.hz}, r3[3] = {1.0 / g.hx, 1.0 / g.hy, 1.0 / g.hz};
+    const double tau = g.tau, tau1 = S.q_m * tau * 0.5;
+    const double lo_scale = ldexp(1.0, fx_lo32_bits(count));
+    // the charge weight over pqr's tau*h*h divisors, and in quanta
+    const double rg[3] = {S.m / (tau * g.hy * g.hz), S.m / (tau * g.hx * g.hz), S.m / (tau * g.hx * g.hy)};
+    const double rc[3] = {rg[0] * sInvQ, rg[1] * sInvQ, rg[2] * sInvQ};
+    const double L3[3] = {g.lx, g.ly, g.lz};
+    const int n3[3] = {g.nx, g.ny, g.nz};
     unsigned bad = 0;
     unsigned long long amb = 0;
-    if (idx < P.off[P.nsp]) {
-        const Grid &g = P.g;
-        int s = species_of(P.off, P.nsp, idx);
-        const FlatSp &S = P.sp[s];
-        int64_t j = idx - P.off[s];
-        int cell = S.cell[j];
-        int i, l, k;
-        g.cell_ijk(cell, i, l, k);
-        double x[3] = {S.v[0][j], S.v[1][j], S.v[2][j]};
-        double p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
-        const int c3[3] = {i, l, k};
-        const unsigned long long rc = P.bmode == 2 ? P.branch[idx] : 0ull;
-        unsigned long long code = 0ull;
-        bool inrange = true;
-        TapInts TI;
-        if (P.bmode == 2) {
+    int qn = 0;  // entries in this warp's queue of second segments (warp-uniform)
+    for (int jw = threadIdx.x - lane;; jw += blockDim.x) {
+        const bool tail = jw >= count;
+        if (tail && qn == 0) break;
+        const int jc = jw + lane;
+        const int64_t j = ch.first + jc;
+        int cell = -1;
+        double x[3] = {0.0, 0.0, 0.0}, p[3] = {0.0, 0.0, 0.0};
+        cp_async_wait_all();
+        if (jc < count) cell = next.take(x, p);
+        __syncwarp();  // the reads come before the next copies into the same place
+        if (jc + (int)blockDim.x < count) next.start(S, j + blockDim.x);
+        if (cell >= 0) {
+            int c3[3];
+            g.cell_ijk(cell, c3[0], c3[1], c3[2]);
+            const bool in = w.holds(c3[0], c3[1], c3[2]);
+            const double o3[3] = {(double)c3[0] * h3[0], (double)c3[1] * h3[1], (double)c3[2] * h3[2]};
+            const unsigned long long rcode = BMODE == 2 ? P.branch[P.off[s] + j] : 0ull;
+            AxisTaps T[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                TI.tn[d] = unpack2(rc, 16 * d) + 1;
-                TI.tc[d] = unpack2(rc, 16 * d + 2) + 1;
-                TI.nI[d] = unpack2(rc, 16 * d + 4) + c3[d];
-                TI.cI[d] = unpack2(rc, 16 * d + 6) + c3[d];
+                if (BMODE == 2) {
+                    T[d].tn = unpack2(rcode, 16 * d) + 1;
+                    T[d].tc = unpack2(rcode, 16 * d + 2) + 1;
+                    T[d].nI = unpack2(rcode, 16 * d + 4) + c3[d];
+                    T[d].cI = unpack2(rcode, 16 * d + 6) + c3[d];
+                    T[d].i1 = unpack2(rcode, 16 * d + 8) + 1;
+                    const double q = div_by(x[d], h3[d], r3[d]);
+                    T[d].wn = (double)T[d].nI - q;
+                    T[d].wc = (double)T[d].cI - 0.5 - q;
+                } else {
+                    axis_taps(x[d], o3[d], h3[d], r3[d], T[d]);
+                }
             }
-        } else {
-            tap_ints(g, i, l, k, x, TI);
-        }
-        Taps TT;
-        taps_from(g, x, TI, TT);
-        double F[6];
-        if (!gather_fields_taps(g, P.E, P.H, i, l, k, x, TT, F, P.bmode != 2)) bad |= ST_STENCIL;
-        if (P.Fout[0]) {
+            double F[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            // the reference's GetField gives no field at a negative coordinate;
+            // positions are wrapped into [0, L) so a run never meets it, and a
+            // replay of frozen branches, whose wraps are fixed, leaves it out
+            if (BMODE == 2 || !(x[0] < 0 || x[1] < 0 || x[2] < 0)) {
+                bool ok;
+                if (in) {
+                    FieldView<true> A;
 #pragma unroll
-            for (int c = 0; c < 6; c++) P.Fout[c][idx] = F[c];
-        }
-        Boris B;
-        boris_plain(S.q_m, g.tau, p, F, x, B);
-        if (!(isfinite(B.pp[0]) && isfinite(B.pp[1]) && isfinite(B.pp[2]))) bad |= ST_NAN;
-        const double o3[3] = {(double)i * g.hx, (double)l * g.hy, (double)k * g.hz};
-        Split SP;
-        if (P.bmode == 2) {
+                    for (int c = 0; c < 6; c++) A.base[c] = sF + c * nn;
+                    A.n0 = w.node(c3[0], c3[1], c3[2]); A.dx = w.SY * w.SZ; A.dy = w.SZ;
+                    ok = gather_fields(A, T, F);
+                } else {
+                    FieldView<false> A;
+#pragma unroll
+                    for (int c = 0; c < 6; c++) A.base[c] = src[c] + g.node(c3[0], c3[1], c3[2]);
+                    A.n0 = 0; A.dx = g.NY * g.pz; A.dy = g.pz;
+                    ok = gather_fields(A, T, F);
+                }
+                if (!ok) bad |= ST_STENCIL;
+            }
+            double p2;
+            const double ig = boris_move(tau1, F, p, p2);
+            if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) bad |= ST_NAN;
+            Split SP;
+            double x1[3];
+            bool exact = true;
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                SP.i1[d] = unpack2(rc, 16 * d + 8) + 1;
-                SP.i2[d] = unpack2(rc, 16 * d + 10) + 1;
+                x1[d] = x[d] + tau * (ig * p[d]);
+                SP.i1[d] = T[d].i1;
+                SP.i2[d] = BMODE == 2 ? unpack2(rcode, 16 * d + 10) + 1
+                                      : trunc_checked((div_by(x1[d] - o3[d], h3[d], r3[d]) + 1.5) + 1, exact);
             }
-        } else {
-            split_ints(g, x, B.x1, o3, SP);
-        }
-        split_from(g, x, B.x1, o3, SP);
-        if (SP.m >= 1 && SP.m <= 7) {
-            seg_plain(P.J, g, i, l, k, SP.i1, x, SP.x2, S.m, o3, bad);
-            seg_plain(P.J, g, i, l, k, SP.i2, SP.x2, B.x1, S.m, o3, bad);
-        } else {
-            seg_plain(P.J, g, i, l, k, SP.i1, x, B.x1, S.m, o3, bad);
-        }
-        const double L3[3] = {g.lx, g.ly, g.lz};
-        const int n3[3] = {g.nx, g.ny, g.nz};
-        int wr[3];
-        double xr[3];
+            if (!exact) { bad |= ST_STENCIL; SP.i2[0] = 0; }
+            SP.m = relay_point(x, x1, o3, h3, SP.i1, SP.i2, SP.x2, SP.sr);
+            const bool cross = SP.m >= 1 && SP.m <= 7;
+            double sb[3];
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            wr[d] = P.bmode == 2 ? unpack2(rc, 16 * d + 12) : wrap_choice(B.x1[d], L3[d]);
-            xr[d] = apply_wrap(B.x1[d], L3[d], wr[d]);
-        }
-        const FlatOut &O = P.out[s];
-        int ncell;
-        if (P.bmode == 2) {
-            int r[3];
+            for (int d = 0; d < 3; d++) sb[d] = cross ? SP.x2[d] : x1[d];
+            if (in) {
+                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, c3[0] - w.i0 - 2, c3[1] - w.l0 - 2, c3[2] - w.k0 - 2, SP.i1,
+                                x, sb, g.hx, g.hy, g.hz, rc, o3[0], o3[1], o3[2], bad);
+                if (cross) {
+                    if (SP.i2[0] >= 2 && SP.i2[0] <= 3 && SP.i2[1] >= 2 && SP.i2[1] <= 3 && SP.i2[2] >= 2 &&
+                        SP.i2[2] <= 3) {
+                        const int e = atomicAdd(&sQn[warp], 1);  // < 15 + 32: drained at 16
 #pragma unroll
-            for (int d = 0; d < 3; d++) {
-                r[d] = c3[d] + unpack2(rc, 16 * d + 14) - 1;
-                r[d] = r[d] < 0 ? r[d] + n3[d] : (r[d] >= n3[d] ? r[d] - n3[d] : r[d]);
+                        for (int d = 0; d < 3; d++) {
+                            qd[d * kQueuePlain + e] = SP.x2[d];
+                            qd[(3 + d) * kQueuePlain + e] = x1[d];
+                        }
+                        // window-local cell, 9 bits each (a window has at most kFlatWindow nodes), and class bits
+                        qc[e] = ((c3[0] - w.i0) << 21) | ((c3[1] - w.l0) << 12) | ((c3[2] - w.k0) << 3) | (SP.i2[0] - 2) |
+                                ((SP.i2[1] - 2) << 1) | ((SP.i2[2] - 2) << 2);
+                    } else {
+                        bad |= ST_STENCIL;
+                    }
+                }
+            } else {
+                seg_global(P.J, g, c3[0], c3[1], c3[2], SP.i1, x, sb, rg, o3, bad);
+                if (cross) seg_global(P.J, g, c3[0], c3[1], c3[2], SP.i2, SP.x2, x1, rg, o3, bad);
             }
-            ncell = g.cell_of(r[0], r[1], r[2]);
-        } else {
-            ncell = new_cell_plain(g, cell, i, l, k, xr, amb);
-        }
-        if (P.bmode == 1) {
-            int r[3];
-            g.cell_ijk(ncell, r[0], r[1], r[2]);
+            int wr[3];
+            double xr[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                int mv = r[d] - c3[d];
-                mv = mv > 1 ? mv - n3[d] : (mv < -1 ? mv + n3[d] : mv);
-                inrange &= pack2(code, TI.tn[d] - 1, 16 * d);
-                inrange &= pack2(code, TI.tc[d] - 1, 16 * d + 2);
-                inrange &= pack2(code, TI.nI[d] - c3[d], 16 * d + 4);
-                inrange &= pack2(code, TI.cI[d] - c3[d], 16 * d + 6);
-                inrange &= pack2(code, SP.i1[d] - 1, 16 * d + 8);
-                inrange &= pack2(code, SP.i2[d] - 1, 16 * d + 10);
-                inrange &= pack2(code, wr[d], 16 * d + 12);
-                inrange &= pack2(code, mv + 1, 16 * d + 14);
+                wr[d] = BMODE == 2 ? unpack2(rcode, 16 * d + 12) : wrap_choice(x1[d], L3[d]);
+                xr[d] = apply_wrap(x1[d], L3[d], wr[d]);
             }
-            P.branch[idx] = code;
-            if (!inrange) bad |= ST_BRANCH_RANGE;
+            int ncell;
+            if (BMODE == 2) {
+                int r[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    r[d] = c3[d] + unpack2(rcode, 16 * d + 14) - 1;
+                    r[d] = r[d] < 0 ? r[d] + n3[d] : (r[d] >= n3[d] ? r[d] - n3[d] : r[d]);
+                }
+                ncell = g.cell_of(r[0], r[1], r[2]);
+            } else {
+                // within [x0, x0 + h] on every axis: stays (see k_push_plain)
+                const bool inside = xr[0] >= o3[0] && xr[0] <= o3[0] + h3[0] && xr[1] >= o3[1] &&
+                                    xr[1] <= o3[1] + h3[1] && xr[2] >= o3[2] && xr[2] <= o3[2] + h3[2];
+                ncell = inside ? cell : new_cell_plain(g, cell, c3[0], c3[1], c3[2], xr, amb);
+            }
+            if (BMODE == 1) {
+                unsigned long long code = 0ull;
+                bool inrange = true;
+                int r[3];
+                g.cell_ijk(ncell, r[0], r[1], r[2]);
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    int mv = r[d] - c3[d];
+                    mv = mv > 1 ? mv - n3[d] : (mv < -1 ? mv + n3[d] : mv);
+                    inrange &= pack2(code, T[d].tn - 1, 16 * d);
+                    inrange &= pack2(code, T[d].tc - 1, 16 * d + 2);
+                    inrange &= pack2(code, T[d].nI - c3[d], 16 * d + 4);
+                    inrange &= pack2(code, T[d].cI - c3[d], 16 * d + 6);
+                    inrange &= pack2(code, SP.i1[d] - 1, 16 * d + 8);
+                    inrange &= pack2(code, SP.i2[d] - 1, 16 * d + 10);
+                    inrange &= pack2(code, wr[d], 16 * d + 12);
+                    inrange &= pack2(code, mv + 1, 16 * d + 14);
+                }
+                P.branch[P.off[s] + j] = code;
+                if (!inrange) bad |= ST_BRANCH_RANGE;
+            }
+            const FlatOut &O = P.out[s];
+            O.cell[j] = ncell;
+            O.v[0][j] = xr[0]; O.v[1][j] = xr[1]; O.v[2][j] = xr[2];
+            O.v[3][j] = p[0]; O.v[4][j] = p[1]; O.v[5][j] = p[2];
         }
-        O.cell[j] = ncell;
-        O.v[0][j] = xr[0]; O.v[1][j] = xr[1]; O.v[2][j] = xr[2];
-        O.v[3][j] = B.pp[0]; O.v[4][j] = B.pp[1]; O.v[5][j] = B.pp[2];
+        // ---- the warp's queued second segments, one per lane
+        __syncwarp();
+        qn = sQn[warp];
+        if (qn >= (tail ? 1 : 16)) {
+            const int d = qn < 32 ? qn : 32;
+            if (lane < d) {
+                const int e = qn - d + lane;
+                const int code = qc[e], a = code >> 21, b = (code >> 12) & 511, c = (code >> 3) & 511;
+                const int iv[3] = {2 + (code & 1), 2 + ((code >> 1) & 1), 2 + ((code >> 2) & 1)};
+                double sa[3], se[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    sa[q] = qd[q * kQueuePlain + e];
+                    se[q] = qd[(3 + q) * kQueuePlain + e];
+                }
+                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
+                                (double)(w.i0 + a) * g.hx, (double)(w.l0 + b) * g.hy, (double)(w.k0 + c) * g.hz, bad);
+            }
+            qn -= d;
+            __syncwarp();
+            if (lane == 0) sQn[warp] = qn;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
+        const long long ih = (long long)sJ[e];
+        const int il = ((const int *)(sJ + 3 * nn))[e];
+        if (ih == 0 && il == 0) continue;
+        const int comp = e / nn, r = e - comp * nn;
+        const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
+        atomicAdd(&P.J[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], ((double)ih + (double)il / lo_scale) * sQ);
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (amb) atomicAdd(&P.st->ambiguous, amb);
 }
 
-// ---- adjoint of the particle part of one step, first pass: recompute the
-// push, transpose the deposit and the push; lambda_F goes to a scratch array
-// (two CTAs per SM: the register cap spills a little but doubles the warps
-// that hide the latency of the lambda_J gathers; measured faster)
-template <bool STORED>
-__global__ void __launch_bounds__(kT, 2) k_adj_push_plain(AdjParams A) {
-    const FlatParams &P = A.f;
-    int64_t idx = spread_index(threadIdx.x);
-    if (idx >= P.off[P.nsp]) return;
-    const Grid &g = P.g;
-    int s = species_of(P.off, P.nsp, idx);
-    const FlatSp &S = P.sp[s];
-    const LamSp &Lm = A.lam[s];
-    int64_t j = idx - P.off[s];
-    int i, l, k;
-    g.cell_ijk(S.cell[j], i, l, k);
-    double x[3] = {S.v[0][j], S.v[1][j], S.v[2][j]};
-    double p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
-    // recompute the forward
-    double F[6];
-    if (STORED) {
+// The taps in few registers: bit d tn - 2, bit 3 + d tc - 2, bit 6 + d cI - nI
+// (wc = wn -+ 1/2), bit 9: a tap left the stencil (the forward has reported it)
+struct PackedTaps {
+    unsigned bits;
+    double wn[3];
+    __device__ __forceinline__ int tap(bool node, int d) const { return (int)(bits >> (node ? d : 3 + d)) & 1; }
+    __device__ __forceinline__ double weight(bool node, int d) const {
+        return node ? wn[d] : wn[d] + (bits >> (6 + d) & 1u ? 0.5 : -0.5);
+    }
+};
+__device__ __forceinline__ PackedTaps pack_taps(const AxisTaps T[3]) {
+    PackedTaps P;
+    P.bits = 0u;
 #pragma unroll
-        for (int c = 0; c < 6; c++) F[c] = A.Fin[c][idx];
-    } else {
-        gather_fields(g, P.E, P.H, i, l, k, x, F);
-    }
-    Boris B;
-    boris_plain(S.q_m, g.tau, p, F, x, B);
-    const double o3[3] = {(double)i * g.hx, (double)l * g.hy, (double)k * g.hz};
-    Split SP;
-    split_plain(g, x, B.x1, o3, SP);
-    // incoming adjoint of the particle's state after the step (Reflect: identity)
-    double lx[3] = {Lm.v[0][j], Lm.v[1][j], Lm.v[2][j]};
-    double lp[3] = {Lm.v[3][j], Lm.v[4][j], Lm.v[5][j]};
-    double gx[3] = {0.0, 0.0, 0.0}, gn[3] = {lx[0], lx[1], lx[2]};
-    // deposit transpose
-    if (SP.m >= 1 && SP.m <= 7) {
-        double g2[3] = {0.0, 0.0, 0.0};
-        seg_plain_rev(A.LJ, g, i, l, k, SP.i1, x, SP.x2, S.m, o3, gx, g2);
-        seg_plain_rev(A.LJ, g, i, l, k, SP.i2, SP.x2, B.x1, S.m, o3, g2, gn);
-        split_rev(SP, x, B.x1, g2, gx, gn);
-    } else {
-        seg_plain_rev(A.LJ, g, i, l, k, SP.i1, x, B.x1, S.m, o3, gx, gn);
-    }
-    // x1 = x + tau g2 p'
-    const double tau = g.tau;
-    for (int d = 0; d < 3; d++) gx[d] += gn[d];
-    double dot = gn[0] * B.pp[0] + gn[1] * B.pp[1] + gn[2] * B.pp[2];
-    double g23 = B.g2 * B.g2 * B.g2;
-    double lP[3];
-    for (int d = 0; d < 3; d++) lP[d] = lp[d] + tau * B.g2 * gn[d] - tau * g23 * dot * B.pp[d];
-    // p' = u' + t E
-    double lF[6];
-    for (int d = 0; d < 3; d++) lF[d] = B.t * lP[d];
-    // u' = (s + b (b.s) + s x b) / sd
-    const double *b = B.b, *sv = B.s, *up = B.up, *u = B.u;
-    double bl = b[0] * lP[0] + b[1] * lP[1] + b[2] * lP[2];
-    double bs = b[0] * sv[0] + b[1] * sv[1] + b[2] * sv[2];
-    double lu_ = lP[0] * up[0] + lP[1] * up[1] + lP[2] * up[2];
-    double inv = 1.0 / B.sd;
-    double bxl[3] = {b[1] * lP[2] - b[2] * lP[1], b[2] * lP[0] - b[0] * lP[2], b[0] * lP[1] - b[1] * lP[0]};
-    double lxs[3] = {lP[1] * sv[2] - lP[2] * sv[1], lP[2] * sv[0] - lP[0] * sv[2], lP[0] * sv[1] - lP[1] * sv[0]};
-    double ls[3], lb[3];
     for (int d = 0; d < 3; d++) {
-        ls[d] = (lP[d] + b[d] * bl + bxl[d]) * inv;
-        lb[d] = (bs * lP[d] + bl * sv[d] + lxs[d] - 2.0 * lu_ * b[d]) * inv;
+        P.bits |= ((unsigned)(T[d].tn - 2) & 1u) << d;
+        P.bits |= ((unsigned)(T[d].tc - 2) & 1u) << (3 + d);
+        P.bits |= ((unsigned)(T[d].cI - T[d].nI) & 1u) << (6 + d);
+        if ((unsigned)(T[d].tn - 2) > 1u || (unsigned)(T[d].tc - 2) > 1u) P.bits |= 512u;
+        P.wn[d] = T[d].wn;
     }
-    // s = u + u x b
-    double lu[3] = {ls[0] + (b[1] * ls[2] - b[2] * ls[1]), ls[1] + (b[2] * ls[0] - b[0] * ls[2]),
-                    ls[2] + (b[0] * ls[1] - b[1] * ls[0])};
-    lb[0] += ls[1] * u[2] - ls[2] * u[1];
-    lb[1] += ls[2] * u[0] - ls[0] * u[2];
-    lb[2] += ls[0] * u[1] - ls[1] * u[0];
-    // b = ps H, ps = t (1 + u^2)^-1/2
-    double lps = 0.0;
-    for (int d = 0; d < 3; d++) {
-        lF[3 + d] = B.ps * lb[d];
-        lps += lb[d] * F[3 + d];
-    }
-    double cps = -B.t * B.g1 * B.g1 * B.g1 * lps;
-    for (int d = 0; d < 3; d++) lu[d] += cps * u[d];
-    // u = p + t E
-    double lpo[3];
-    for (int d = 0; d < 3; d++) {
-        lpo[d] = lu[d];
-        lF[d] += B.t * lu[d];
-    }
-    for (int d = 0; d < 3; d++) {
-        Lm.v[d][j] = gx[d];
-        Lm.v[3 + d][j] = lpo[d];
-    }
-#pragma unroll
-    for (int c = 0; c < 6; c++) A.LF[c][idx] = lF[c];
+    return P;
 }
 
-// ---- adjoint of the interpolation (second pass, few registers): scatter
-// lambda_F into lambda_E / lambda_H and add F's position gradient to lambda_x.
-// Four CTAs per SM (64 registers): it waits on global gathers, and 32 warps
-// per SM hide them better than 16 (c3 backward 591 -> 500 ms for 100 steps)
-__global__ void __launch_bounds__(kT, 4) k_adj_interp_plain(AdjParams A) {
-    __shared__ int sHi[6 * kBoxNodes], sLo[6 * kBoxNodes];
-    __shared__ int sRed[6 * (kT / 32)];
-    __shared__ unsigned sMax[kT / 32], sMaxOut;
-    __shared__ NodeBox sBox;
+// The reverse of one particle's step up to the adjoint of its interpolated
+// fields: recomputes the push (cell indices c3, o3 the cell's corner, fields and
+// lambda_J from V and LJ, L0 the cell's node in LJ with strides lx, ly), and
+// transposes the deposit and the push.  In: gn, lP the incoming lambda_x and
+// lambda_p (Reflect: identity).  Out: gx = lambda_x without the interpolation's
+// part, lu = lambda_p, lF, the taps.  false: the push saw no field here.
+struct ReverseConst {
+    double h3[3], r3[3], rg[3], tau, tau1;
+};
+__device__ __forceinline__ ReverseConst reverse_const(const Grid &g, const FlatSp &S) {
+    ReverseConst K;
+    K.h3[0] = g.hx; K.h3[1] = g.hy; K.h3[2] = g.hz;
+#pragma unroll
+    for (int d = 0; d < 3; d++) K.r3[d] = 1.0 / K.h3[d];
+    K.tau = g.tau;
+    K.tau1 = S.q_m * g.tau * 0.5;
+    K.rg[0] = S.m / (g.tau * g.hy * g.hz);
+    K.rg[1] = S.m / (g.tau * g.hx * g.hz);
+    K.rg[2] = S.m / (g.tau * g.hx * g.hy);
+    return K;
+}
+template <class V>
+__device__ __forceinline__ bool reverse_particle(const Grid &g, const ReverseConst &K, const V &A, const double *L0,
+                                                 const double *L1, const double *L2, int ln, int lx, int ly,
+                                                 const int c3[3], const double x[3], const double p[3], double gn[3],
+                                                 double lP[3], PackedTaps &PT, double gx[3], double lu[3],
+                                                 double lF[6]) {
+    const double *h3 = K.h3, *r3 = K.r3;
+    AxisTaps T[3];
+    const double o3[3] = {(double)c3[0] * h3[0], (double)c3[1] * h3[1], (double)c3[2] * h3[2]};
+    const bool seen = !(x[0] < 0 || x[1] < 0 || x[2] < 0);  // else the push saw zero fields
+#pragma unroll
+    for (int d = 0; d < 3; d++) axis_taps(x[d], o3[d], h3[d], r3[d], T[d]);
+    double F[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (seen) gather_fields(A, T, F);
+    BorisPlain B;
+    boris_plain(K.tau1, F, p, B);
+    Split SP;
+    double x1[3];
+    bool exact = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        x1[d] = x[d] + K.tau * (B.g2 * B.pp[d]);
+        SP.i1[d] = T[d].i1;
+        SP.i2[d] = trunc_checked((div_by(x1[d] - o3[d], h3[d], r3[d]) + 1.5) + 1, exact);
+        gx[d] = 0.0;
+    }
+    PT = pack_taps(T);
+    if (!exact) SP.i2[0] = 0;
+    SP.m = relay_point(x, x1, o3, h3, SP.i1, SP.i2, SP.x2, SP.sr);
+    // deposit transpose
+    {
+        auto rev = [&](const int iv[3], const double a[3], const double b[3], double ga[3], double gb[3]) {
+            if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) return;
+            seg_rev(L0, L1, L2, ln + (iv[0] - 2) * lx + (iv[1] - 2) * ly + (iv[2] - 2), lx, ly, g, iv, a, b, K.rg, o3, ga,
+                    gb);
+        };
+        const bool cross = SP.m >= 1 && SP.m <= 7;
+        double sb[3], g2[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < 3; d++) sb[d] = cross ? SP.x2[d] : x1[d];
+        rev(SP.i1, x, sb, gx, g2);
+        if (cross) {
+            rev(SP.i2, SP.x2, x1, g2, gn);
+            split_rev(SP, x, x1, g2, gx, gn);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; d++) gn[d] += g2[d];
+        }
+    }
+    // x1 = x + tau g2 p'
+#pragma unroll
+    for (int d = 0; d < 3; d++) gx[d] += gn[d];
+    const double tg = K.tau * B.g2;
+    const double dot = tg * B.g2 * B.g2 * fma(gn[0], B.pp[0], fma(gn[1], B.pp[1], gn[2] * B.pp[2]));
+#pragma unroll
+    for (int d = 0; d < 3; d++) lP[d] = fma(tg, gn[d], fma(-dot, B.pp[d], lP[d]));
+    // p' = u' + t E, u' = (s + b (b.s) + s x b) / sd
+    const double *b = B.b, *sv = B.s, *up = B.up, *u = B.u;
+    const double inv = B.isd;
+    const double bl = fma(b[0], lP[0], fma(b[1], lP[1], b[2] * lP[2]));
+    const double bs = fma(b[0], sv[0], fma(b[1], sv[1], b[2] * sv[2]));
+    const double lu_ = -2.0 * fma(lP[0], up[0], fma(lP[1], up[1], lP[2] * up[2]));
+    double ls[3], lb[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int e = (d + 1) % 3, f = (d + 2) % 3;
+        ls[d] = fma(b[d], bl, fma(b[e], lP[f], fma(-b[f], lP[e], lP[d]))) * inv;
+        lb[d] = fma(bs, lP[d], fma(bl, sv[d], fma(lP[e], sv[f], fma(-lP[f], sv[e], lu_ * b[d])))) * inv;
+    }
+    // s = u + u x b
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int e = (d + 1) % 3, f = (d + 2) % 3;
+        lu[d] = fma(b[e], ls[f], fma(-b[f], ls[e], ls[d]));
+        lb[d] = fma(ls[e], u[f], fma(-ls[f], u[e], lb[d]));
+    }
+    // b = ps H, ps = t (1 + u^2)^-1/2; u = p + t E
+    const double lps = fma(lb[0], F[3], fma(lb[1], F[4], lb[2] * F[5]));
+    const double cps = -K.tau1 * B.g1 * B.g1 * B.g1 * lps;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        lu[d] = fma(cps, u[d], lu[d]);
+        lF[d] = K.tau1 * (lP[d] + lu[d]);
+        lF[3 + d] = B.ps * lb[d];
+    }
+    return seen && !(PT.bits & 512u);
+}
+
+// One component of the interpolation's transpose: gi += lam * dF/dx (V: the
+// cell's node in the component's array, strides dX, dY), add(o, w): weight w
+// belongs to the node o = (x, y, z) bits away from the tap base.
+template <int C, class Add>
+__device__ __forceinline__ void reverse_component(const double *V, int dX, int dY, const PackedTaps &T, double lam,
+                                                  double gi[3], Add add) {
+    constexpr bool nx = node_axis(C, 0), ny = node_axis(C, 1), nz = node_axis(C, 2);
+    const int tx = T.tap(nx, 0), ty = T.tap(ny, 1), tz = T.tap(nz, 2);
+    const double wx = T.weight(nx, 0), wy = T.weight(ny, 1), wz = T.weight(nz, 2);
+    const double vx = 1. - wx, vy = 1. - wy, vz = 1. - wz;
+    V += tx * dX + ty * dY + tz;
+    // z, then y, then x: sums and differences
+    double yl[2], yd[2], yz[2];
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        const double v0 = V[a * dX], v1 = V[a * dX + 1], v2 = V[a * dX + dY], v3 = V[a * dX + dY + 1];
+        const double z0 = fma(vz, v1, wz * v0), z1 = fma(vz, v3, wz * v2);
+        yl[a] = fma(vy, z1, wy * z0);
+        yd[a] = z1 - z0;
+        yz[a] = fma(vy, v3 - v2, wy * (v1 - v0));
+    }
+    gi[0] = fma(lam, yl[1] - yl[0], gi[0]);
+    gi[1] = fma(lam, fma(vx, yd[1], wx * yd[0]), gi[1]);
+    gi[2] = fma(lam, fma(vx, yz[1], wx * yz[0]), gi[2]);
+#pragma unroll
+    for (int t = 0; t < 4; t++) add(tx + (t >> 1), ty + (t & 1), tz, (t >> 1 ? vx : wx) * (t & 1 ? vy : wy), wz, vz);
+}
+
+// a particle outside its chunk's window: everything through global memory
+__device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
     const FlatParams &P = A.f;
     const Grid &g = P.g;
-    int64_t idx = spread_index(threadIdx.x);
-    bool valid = idx < P.off[P.nsp];
-    int s = 0, i = 0, l = 0, k = 0;
-    int64_t j = 0;
-    double x[3] = {0.0, 0.0, 0.0};
-    if (valid) {
-        s = species_of(P.off, P.nsp, idx);
-        const FlatSp &S = P.sp[s];
-        j = idx - P.off[s];
-        x[0] = S.v[0][j]; x[1] = S.v[1][j]; x[2] = S.v[2][j];
-        g.cell_ijk(S.cell[j], i, l, k);
-        valid = !(x[0] < 0 || x[1] < 0 || x[2] < 0);  // else the push saw zero fields
-    }
-    double lam6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    float amax = 0.f;
-    if (valid) {
+    const FlatSp &S = P.sp[s];
+    const LamSp &Lm = A.lam[s];
+    const ReverseConst K = reverse_const(g, S);
+    double x[3] = {S.v[0][j], S.v[1][j], S.v[2][j]}, p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
+    double gn[3] = {Lm.v[0][j], Lm.v[1][j], Lm.v[2][j]}, lP[3] = {Lm.v[3][j], Lm.v[4][j], Lm.v[5][j]};
+    int c3[3];
+    g.cell_ijk(S.cell[j], c3[0], c3[1], c3[2]);
+    const size_t n = g.node(c3[0], c3[1], c3[2]);
+    FieldView<false> V;
 #pragma unroll
-        for (int c = 0; c < 6; c++) {
-            lam6[c] = A.LF[c][idx];
-            amax = fmaxf(amax, (float)fabs(lam6[c]));
-        }
+    for (int c = 0; c < 3; c++) { V.base[c] = P.E[c] + n; V.base[3 + c] = P.H[c] + n; }
+    V.n0 = 0; V.dx = g.NY * g.pz; V.dy = g.pz;
+    PackedTaps T;
+    double gx[3], lu[3], lF[6], gi[3] = {0.0, 0.0, 0.0};
+    if (reverse_particle(g, K, V, A.LJ[0] + n, A.LJ[1] + n, A.LJ[2] + n, 0, V.dx, V.dy, c3, x, p, gn, lP, T, gx, lu, lF)) {
+        auto put = [&](double *L, double lam) {
+            return [=](int tx, int ty, int tz, double xy, double wz, double vz) {
+                double *r = L + tx * V.dx + ty * V.dy + tz;
+                atomicAdd(r, lam * xy * wz);
+                atomicAdd(r + 1, lam * xy * vz);
+            };
+        };
+        reverse_component<0>(V.base[0], V.dx, V.dy, T, lF[0], gi, put(A.LE[0] + n, lF[0]));
+        reverse_component<1>(V.base[1], V.dx, V.dy, T, lF[1], gi, put(A.LE[1] + n, lF[1]));
+        reverse_component<2>(V.base[2], V.dx, V.dy, T, lF[2], gi, put(A.LE[2] + n, lF[2]));
+        reverse_component<3>(V.base[3], V.dx, V.dy, T, lF[3], gi, put(A.LH[0] + n, lF[3]));
+        reverse_component<4>(V.base[4], V.dx, V.dy, T, lF[4], gi, put(A.LH[1] + n, lF[4]));
+        reverse_component<5>(V.base[5], V.dx, V.dy, T, lF[5], gi, put(A.LH[2] + n, lF[5]));
     }
-    const NodeBox box = block_node_box(i, l, k, valid, sRed, &sBox);
-    const float bmax = block_max_abs(amax, sMax, &sMaxOut);
-    if (bmax == 0.f) return;  // no adjoint reaches the particles of this block
-    const int E = box_exponent(bmax);
-    const double inv_q = pow2_d(22 - E);
-    for (int e = threadIdx.x; e < 6 * box.nodes; e += blockDim.x) sHi[e] = sLo[e] = 0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        Lm.v[d][j] = fma(gi[d], K.r3[d], gx[d]);
+        Lm.v[3 + d][j] = lu[d];
+    }
+}
+
+// ---- adjoint of the particle part of one step: recompute the push, transpose
+// the deposit and the push, transpose the interpolation.
+//
+// One CTA per chunk, with the chunk's window of E, H and lambda_J staged and
+// lambda_E, lambda_H summed in shared memory (64-bit fixed point, added to the
+// global arrays once); particles outside the window are done at the end through
+// global memory.  The interpolated fields are formed again from the staged
+// window instead of being kept by the forward (48 B written and read per
+// particle and step).  The quantum follows the largest |lambda of a field
+// value| of the 256 particles at hand: where that outgrows the quantum in use,
+// the sums so far are added to the global arrays and start again at one that
+// leaves 2^-48 of it.
+// Bound: latency at 16 warps per SM (128 registers, some spills) and the shared
+// memory pipe (64 %: 91 shared atomics and 110 loads per particle).  128x32x32
+// cells: 3.3 -> 2.3 ms per reverse step (before: two kernels, lambda of the
+// field values and the fields themselves passed through global memory).
+__global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_constant__ AdjParams A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ AdjWindow sWin;
+    __shared__ int sRed[15 * kW], sFar;
+    __shared__ unsigned sMax[2];
+    const FlatParams &P = A.f;
+    const Grid &g = P.g;
+    const AdjChunk ch = P.chunks[blockIdx.x];
+    const int s = ch.species, count = ch.count;
+    const FlatSp &S = P.sp[s];
+    const LamSp &Lm = A.lam[s];
+    const NextParticle next(smem_raw + (size_t)kAdjWindow * 120);
+    const NextLam lnext(smem_raw + (size_t)kAdjWindow * 120 + kNextBytes);
+    unsigned short *sList =
+        (unsigned short *)(smem_raw + (size_t)kAdjWindow * 120 + kNextBytes + kNextLamBytes);  // kAdjChunk entries
+    __shared__ ReverseConst sK;  // in shared memory: registers are short
+    // a warp takes 4 runs of 8 particles out of 4 places of the block's 256:
+    // consecutive particles mostly share a cell, and adds to one address queue
+    // up (one run of 32: 254 ps per particle and reverse step, 8 of 4: 189, 16 of
+    // 2: 208, 4 of 8: 185; c3's 12.6M particles)
+    const int lane = threadIdx.x & 31, mine = (lane >> 3) * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
+    if (mine < count) {
+        next.start(S, ch.first + mine);
+        lnext.start(Lm, ch.first + mine);
+    }
+    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kAdjWindow, sRed, &sWin);
+    const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
+    double *sF = (double *)smem_raw, *sL = sF + 6 * nn;
+    unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
+    const double *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
+    stage_window<6>(g, w, src, sF);
+    stage_window<3>(g, w, A.LJ, sL);
+    for (int e = threadIdx.x; e < 12 * nn; e += blockDim.x) sLo[e] = 0u;
+    if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = 0u; sK = reverse_const(g, S); }
     __syncthreads();
-    if (valid) {
-        Taps T;
-        taps_plain(g, i, l, k, x, T);
-        const size_t dX = (size_t)g.NY * g.pz, dY = g.pz, dZ = 1;
-        double gx[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            int t[3];
-            double w[3];
-            const double lam = lam6[c];
-            if (!comp_taps(T, c, t, w) || lam == 0.0) continue;
-            size_t n = tap_node(g, i, l, k, t);
-            const double *Arr = c < 3 ? P.E[c] : P.H[c - 3];
-            double *LA = c < 3 ? A.LE[c] : A.LH[c - 3];
-            const int b0 = box.nodes ? c * box.nodes + box_index(box, i + t[0] - 2, l + t[1] - 2, k + t[2] - 2) : 0;
-            const double W0[2] = {w[0], 1. - w[0]}, W1[2] = {w[1], 1. - w[1]}, W2[2] = {w[2], 1. - w[2]};
-            double gr[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-            for (int a = 0; a < 2; a++)
-#pragma unroll
-                for (int bb = 0; bb < 2; bb++)
-#pragma unroll
-                    for (int cc = 0; cc < 2; cc++) {
-                        size_t m = n + a * dX + bb * dY + cc * dZ;
-                        double v = Arr[m];
-                        double add = lam * (W0[a] * W1[bb] * W2[cc]);
-                        if (box.nodes) {
-                            const int e = b0 + (a * box.by + bb) * box.bz + cc;
-                            double vq = add * inv_q;
-                            int hi = __double2int_rn(vq);
-                            int lo = __double2int_rn((vq - (double)hi) * 0x1p22);
-                            if (hi) atomicAdd(&sHi[e], hi);
-                            if (lo) atomicAdd(&sLo[e], lo);
-                        } else {
-                            atomicAdd(&LA[m], add);
-                        }
-                        gr[0] += (a ? 1.0 : -1.0) * W1[bb] * W2[cc] * v;
-                        gr[1] += (bb ? 1.0 : -1.0) * W0[a] * W2[cc] * v;
-                        gr[2] += (cc ? 1.0 : -1.0) * W0[a] * W1[bb] * v;
-                    }
-            gx[0] += lam * gr[0] / g.hx;
-            gx[1] += lam * gr[1] / g.hy;
-            gx[2] += lam * gr[2] / g.hz;
+    const ReverseConst &K = sK;
+    // contributions below 2^50 quanta, at most kAdjChunk per node and component: sums below 2^61
+    int E = -1000;  // none yet
+    double limit = 0.0, inv_q = 0.0;
+    auto flush = [&](bool again) {
+        if (E > -1000) {
+            const double q = pow2_d(E - 50);
+            double *const dst[6] = {A.LE[0], A.LE[1], A.LE[2], A.LH[0], A.LH[1], A.LH[2]};
+            for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
+                const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
+                if (v == 0) continue;
+                if (again) sHi[e] = sLo[e] = 0u;
+                const int comp = e / nn, r = e - comp * nn;
+                const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
+                atomicAdd(&dst[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * q);
+            }
         }
-        const LamSp &Lm = A.lam[s];
-        for (int d = 0; d < 3; d++) Lm.v[d][j] += gx[d];
-    }
-    if (box.nodes) {
+    };
+    for (int base = 0, it = 0; base < count; base += blockDim.x, it++) {
+        const int jc = base + mine;
+        const int64_t j = ch.first + jc;
+        int cell = -1;
+        double x[3], p[3], gn[3], lP[3];
+        cp_async_wait_all();
+        if (jc < count) {
+            cell = next.take(x, p);
+            lnext.take(gn, lP);
+        }
+        __syncwarp();
+        if (jc + (int)blockDim.x < count) {
+            next.start(S, j + blockDim.x);
+            lnext.start(Lm, j + blockDim.x);
+        }
+        int c3[3] = {w.i0, w.l0, w.k0};
+        bool near = cell >= 0;
+        if (near) {
+            g.cell_ijk(cell, c3[0], c3[1], c3[2]);
+            if (!w.holds(c3[0], c3[1], c3[2])) {
+                near = false;
+                sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
+            }
+        }
+        PackedTaps T;
+        double gx[3], lu[3], lF[6], gi[3] = {0.0, 0.0, 0.0};
+        bool seen = false;
+        float amax = 0.f;
+        const int n0 = w.node(c3[0], c3[1], c3[2]);
+        if (near) {
+            FieldView<true> V;
+#pragma unroll
+            for (int c = 0; c < 6; c++) V.base[c] = sF + c * nn;
+            V.n0 = n0; V.dx = dX; V.dy = dY;
+            seen = reverse_particle(g, K, V, sL, sL + nn, sL + 2 * nn, n0, dX, dY, c3, x, p, gn, lP, T, gx, lu, lF);
+            double am = 0.0;
+#pragma unroll
+            for (int c = 0; c < 6; c++) am = fmax(am, fabs(lF[c]));
+            if (seen) amax = (float)am;
+        }
+        // the block's largest |lambda_F| against the quantum in use
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+        if (lane == 0 && wm) atomicMax(&sMax[it & 1], wm);
         __syncthreads();
-        double *const dst[6] = {A.LE[0], A.LE[1], A.LE[2], A.LH[0], A.LH[1], A.LH[2]};
-        flush_node_box(box, sHi, sLo, pow2_d(E - 22), g, dst);
+        const float bm = __uint_as_float(sMax[it & 1]);
+        if (threadIdx.x == 0) sMax[(it & 1) ^ 1] = 0u;
+        if ((double)bm >= limit && bm > 0.f) {  // block-uniform
+            flush(true);
+            E = adj_exponent(bm) + 2;
+            // a float rounded down from a larger double stays below 2^E
+            limit = pow2_d(E - 1);
+            inv_q = pow2_d(50 - E);
+            __syncthreads();
+        }
+        if (near && seen && amax > 0.f) {
+            auto put = [&](int c) {
+                const double lam = lF[c] * inv_q;
+                unsigned *lo = sLo + c * nn + n0;
+                return [=](int tx, int ty, int tz, double xy, double wz, double vz) {
+                    unsigned *r = lo + tx * dX + ty * dY + tz;
+                    const double v = lam * xy;
+                    shared_add64(r, r + 6 * nn, __double_as_longlong(fma(v, wz, kRound)) - 0x4338000000000000ll);
+                    shared_add64(r + 1, r + 1 + 6 * nn, __double_as_longlong(fma(v, vz, kRound)) - 0x4338000000000000ll);
+                };
+            };
+            const double *V = sF + n0;
+            reverse_component<0>(V, dX, dY, T, lF[0], gi, put(0));
+            reverse_component<1>(V + nn, dX, dY, T, lF[1], gi, put(1));
+            reverse_component<2>(V + 2 * nn, dX, dY, T, lF[2], gi, put(2));
+            reverse_component<3>(V + 3 * nn, dX, dY, T, lF[3], gi, put(3));
+            reverse_component<4>(V + 4 * nn, dX, dY, T, lF[4], gi, put(4));
+            reverse_component<5>(V + 5 * nn, dX, dY, T, lF[5], gi, put(5));
+        }
+        if (near) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                Lm.v[d][j] = fma(gi[d], K.r3[d], gx[d]);
+                Lm.v[3 + d][j] = lu[d];
+            }
+        }
     }
+    __syncthreads();
+    flush(false);
+    for (int e = threadIdx.x; e < sFar; e += blockDim.x) reverse_far(A, s, ch.first + sList[e]);
 }
 
 // ------------------------------------------------------------- fields --
@@ -1106,6 +1290,7 @@ FlatParams flat_params(pic_handle *h, AdjState &A, char *state, void *const F[PI
         P.out[s].cell = cell[s];
         for (int a = 0; a < 6; a++) P.out[s].v[a] = (double *)v[s][a];
     }
+    P.chunks = A.chunks;
     P.st = A.st;
     P.branch = A.step_branch;
     P.bmode = A.step_branch ? A.step_bmode : 0;
@@ -1120,17 +1305,19 @@ int64_t total_particles(const AdjState &A) {
 
 // one forward step of the flat state on the field set F (plain): particles
 // read from `state`, written to `out` (the same buffer when out is null)
-int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out = nullptr,
-                    double *Fout = nullptr) {
+int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out = nullptr) {
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
     yee_b_half_plain(g, (double *const *)F, s);
     size_t nodes = g.nodes_pitched();
     for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(F[PIC_JX + c], 0, nodes * sizeof(double), s), "zero J");
     FlatParams P = flat_params(h, A, state, F, out);
-    int64_t n = total_particles(A);
-    for (int c = 0; c < 6; c++) P.Fout[c] = Fout ? Fout + (size_t)c * n : nullptr;
-    if (n > 0) k_flat_push_plain<<<blocks_of(n), kT, 0, s>>>(P);
+    if (A.nchunks > 0) {
+        auto *kern = P.bmode == 0 ? k_flat_push_plain<0> : (P.bmode == 1 ? k_flat_push_plain<1> : k_flat_push_plain<2>);
+        const size_t smem = (size_t)kFlatWindow * (6 * sizeof(double) + 3 * 12) + (size_t)kW * kQueuePlain * 52 + kNextBytes;
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "flat push");
+        kern<<<A.nchunks, kT, smem, s>>>(P);
+    }
     CK(cudaGetLastError(), "flat push");
     j_fold(g, (double *)F[PIC_JX], (double *)F[PIC_JY], (double *)F[PIC_JZ], s);
     yee_b_complete_plain(g, (double *const *)F, s);
@@ -1196,7 +1383,7 @@ void adj_free(pic_handle *h) {
     if (!h || !h->adj) return;
     AdjState *A = h->adj;
     void *bufs[] = {A->cur, A->ckp, A->ckf, A->segp, A->segf, A->subp, A->subf, A->lamp, A->lamf, A->rf, A->ha,
-                    A->hist, A->st, A->red, A->lamF, A->segF, A->branch};
+                    A->hist, A->st, A->red, A->lamF, A->segF, A->branch, A->chunks};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (A->e0) cudaEventDestroy(A->e0);
@@ -1257,7 +1444,7 @@ MixParams mix_params(pic_handle *h, AdjState &A, char *state, void *const F[PIC_
 // read from `state`, written to `out` (same buffer when null); Fout, when
 // given, receives the interpolated fields of every particle
 int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, void *Fout) {
-    if (!h->mixed) return flat_step_plain(h, A, state, F, out, (double *)Fout);
+    if (!h->mixed) return flat_step_plain(h, A, state, F, out);
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
     float *const *E = (float *const *)&F[PIC_EX];
@@ -1377,14 +1564,11 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
             o += 6 * (size_t)A.n[s];
         }
         for (int c = 0; c < 3; c++) { P.LJ[c] = LJ[c]; P.LE[c] = LE[c]; P.LH[c] = LH[c]; }
-        for (int c = 0; c < 6; c++) {
-            P.LF[c] = (double *)A.lamF + (size_t)c * np;
-            P.Fin[c] = Fin ? (const double *)Fin + (size_t)c * np : nullptr;
-        }
-        if (np > 0) {
-            if (Fin) k_adj_push_plain<true><<<blocks_of(np), kT, 0, st>>>(P);
-            else k_adj_push_plain<false><<<blocks_of(np), kT, 0, st>>>(P);
-            k_adj_interp_plain<<<blocks_of(np), kT, 0, st>>>(P);
+        if (A.nchunks > 0) {
+            const size_t smem = (size_t)kAdjWindow * 120 + kNextBytes + kNextLamBytes + kAdjChunk * sizeof(unsigned short);
+            CK(cudaFuncSetAttribute(k_adj_particles_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+               "adjoint particles");
+            k_adj_particles_plain<<<A.nchunks, kT, smem, st>>>(P);
         }
     } else {
         const float *En = (const float *)EHn, *Hn = (const float *)EHn + 3 * N;
@@ -1510,6 +1694,25 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
         A.n[s] = t;
     }
     A.pbytes = adj_state_bytes(A);
+    std::vector<AdjChunk> chunks;
+    {
+        // each tile's particles of a species in equal chunks: large enough to
+        // pay for a chunk's window, small enough to fill the GPU a few times
+        const int64_t per = total_particles(A) / (8 * h->sms);
+        const int most = (int)std::min<int64_t>(kAdjChunk, std::max<int64_t>(kT, (per + kT - 1) / kT * kT));
+        for (int s = 0; s < A.nsp; s++) {
+            int64_t at = 0;
+            for (int c : counts[s]) {
+                const int pieces = (c + most - 1) / most;
+                for (int q = 0; q < pieces; q++) {
+                    const int64_t a = (int64_t)c * q / pieces, b = (int64_t)c * (q + 1) / pieces;
+                    chunks.push_back(AdjChunk{at + a, (int)(b - a), s});
+                }
+                at += c;
+            }
+        }
+        A.nchunks = (int)chunks.size();
+    }
     const size_t fbytes = g.nodes_pitched() * (h->mixed ? sizeof(float) : sizeof(double));
     if (src) {
         const AdjState *S = src->adj;
@@ -1536,6 +1739,10 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     if ((rc = adj_alloc(h, (void **)&A.hist, sizeof(double) * 3 * steps, "the history"))) return rc;
     if ((rc = adj_alloc(h, (void **)&A.st, sizeof(AdjStatus), "the status"))) return rc;
     if ((rc = adj_alloc(h, (void **)&A.red, sizeof(double) * 8, "the reduction scratch"))) return rc;
+    if ((rc = adj_alloc(h, (void **)&A.chunks, sizeof(AdjChunk) * chunks.size(), "the chunk table"))) return rc;
+    CK(cudaMemcpyAsync(A.chunks, chunks.data(), sizeof(AdjChunk) * chunks.size(), cudaMemcpyHostToDevice, h->stream),
+       "chunk table");
+    CK(cudaStreamSynchronize(h->stream), "sync");
     CK(cudaMemsetAsync(A.hist, 0, sizeof(double) * 3 * steps, h->stream), "zero history");
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     // bins -> flat order
@@ -1684,13 +1891,15 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
         if ((rc = adj_alloc(h, (void **)&A.rf, N * sizeof(double) * PIC_FIELD_COUNT, "the recompute fields")))
             return rc;
         if ((rc = adj_alloc(h, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
-        if ((rc = adj_alloc(h, (void **)&A.lamF, (size_t)np * 6 * A.elem, "the interpolation adjoints"))) return rc;
+        if (h->mixed &&
+            (rc = adj_alloc(h, (void **)&A.lamF, (size_t)np * 6 * A.elem, "the interpolation adjoints")))
+            return rc;
         // optional: the interpolated fields of every step of a segment, so the
         // adjoint does not gather them again (skipped when memory is short)
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
         size_t want = (size_t)np * 6 * A.elem * (size_t)A.K2;
-        if (want + ((size_t)4 << 30) < free_b && cudaMalloc((void **)&A.segF, want) != cudaSuccess) {
+        if (h->mixed && want + ((size_t)4 << 30) < free_b && cudaMalloc((void **)&A.segF, want) != cudaSuccess) {
             A.segF = nullptr;
             cudaGetLastError();
         }

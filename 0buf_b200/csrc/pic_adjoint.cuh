@@ -18,6 +18,14 @@ struct AdjStatus {
     unsigned long long ambiguous;  // cell changes with zero or several receiving cells (resolved, counted)
 };
 
+// a run of consecutive particles of one species in the fixed order, all from
+// one tile at the start: the work of one CTA of the particle kernels
+constexpr int kAdjChunk = 2048;  // particles at most
+struct AdjChunk {
+    int64_t first;  // index within the species
+    int count, species;
+};
+
 // Buffers live until pic_adjoint_free / the next pic_forward / pic_destroy.
 // A "particle state" is the whole population in the fixed order of the run:
 // per species the packed cells then 6 value arrays (plain: FP64 global
@@ -44,6 +52,8 @@ struct AdjState {
     void *segF;        // optional: K x the 6 interpolated field values per particle of the segment
     char *rf;          // field set of the recompute (form's layout: 12 arrays)
     char *ha;          // B after the half step of the step being reversed (3 arrays)
+    AdjChunk *chunks;  // nchunks of them, device
+    int nchunks;
     double *hist;      // steps x 3: sum over nodes 1..N of E_c^2 after each step
     // frozen branches (plain form): mode 1 records every step's discrete
     // choices into branch (steps x particles codes), mode 2 replays those of
@@ -63,6 +73,102 @@ struct AdjState {
 };
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+
+// ---- a chunk's window: the box of cells whose nodes a CTA keeps in shared memory
+struct AdjWindow {
+    int i0, l0, k0, cx, cy, cz;  // first cell and cells per axis
+    int SY, SZ, nn;              // node strides and nodes: (cx+2)(cy+2)(cz+2)
+    __device__ __forceinline__ bool holds(int i, int l, int k) const {
+        return (unsigned)(i - i0) < (unsigned)cx && (unsigned)(l - l0) < (unsigned)cy && (unsigned)(k - k0) < (unsigned)cz;
+    }
+    // window-local node of a cell (its lower corner)
+    __device__ __forceinline__ int node(int i, int l, int k) const { return ((i - i0) * SY + (l - l0)) * SZ + (k - k0); }
+};
+// The window of `count` particles' cells with at most `cap` nodes: their
+// bounding box where that fits.  Otherwise (particles that wandered off, or a
+// chunk that lies on both sides of a periodic boundary) a box around their mean
+// position, taken periodically, cut at the grid's edge and shrunk on its longest
+// axis until it fits; the particles outside it use global memory.  Every thread
+// of the CTA calls it; red holds 15 ints per warp.
+__device__ __forceinline__ AdjWindow chunk_window(const Grid &g, const int *__restrict__ cell, int count, int cap,
+                                                  int *red, AdjWindow *out) {
+    const unsigned FULL = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int n3[3] = {g.nx, g.ny, g.nz};
+    int at[3];  // the middle particle's cell: the others' periodic distances are taken from it
+    g.cell_ijk(cell[count / 2], at[0], at[1], at[2]);
+    int lo[3], hi[3], dlo[3], dhi[3], sum[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) { lo[d] = dlo[d] = 0x7fffffff; hi[d] = dhi[d] = -0x7fffffff; sum[d] = 0; }
+    for (int j = threadIdx.x; j < count; j += blockDim.x) {
+        int c[3];
+        g.cell_ijk(cell[j], c[0], c[1], c[2]);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            int e = c[d] - at[d];
+            if (2 * e > n3[d]) e -= n3[d];
+            else if (2 * e < -n3[d]) e += n3[d];
+            lo[d] = min(lo[d], c[d]); hi[d] = max(hi[d], c[d]);
+            dlo[d] = min(dlo[d], e); dhi[d] = max(dhi[d], e);
+            sum[d] += e;
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int r[5] = {__reduce_min_sync(FULL, lo[d]), __reduce_max_sync(FULL, hi[d]), __reduce_min_sync(FULL, dlo[d]),
+                          __reduce_max_sync(FULL, dhi[d]), __reduce_add_sync(FULL, sum[d])};
+        if ((threadIdx.x & 31) == 0)
+            for (int q = 0; q < 5; q++) red[(5 * d + q) * nw + warp] = r[q];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int a[3], b[3];
+        int64_t nodes = 1;
+        for (int d = 0; d < 3; d++) {
+            const int *r = red + 5 * d * nw;
+            a[d] = r[0];
+            b[d] = r[nw];
+            for (int w = 1; w < nw; w++) { a[d] = min(a[d], r[w]); b[d] = max(b[d], r[nw + w]); }
+            nodes *= b[d] - a[d] + 3;
+        }
+        if (nodes > cap) {
+            int mid[3];
+            for (int d = 0; d < 3; d++) {
+                const int *r = red + 5 * d * nw;
+                int mn = r[2 * nw], mx = r[3 * nw], sm = r[4 * nw];
+                for (int w = 1; w < nw; w++) {
+                    mn = min(mn, r[2 * nw + w]); mx = max(mx, r[3 * nw + w]); sm += r[4 * nw + w];
+                }
+                const int m = at[d] + (int)rintf((float)sm / (float)count);
+                mid[d] = m < 0 ? m + n3[d] : (m >= n3[d] ? m - n3[d] : m);
+                a[d] = max(max(at[d] + mn + mid[d] - m, 0), mid[d] - 15);
+                b[d] = min(min(at[d] + mx + mid[d] - m, n3[d] - 1), mid[d] + 15);
+                a[d] = min(a[d], mid[d]);
+                b[d] = max(b[d], mid[d]);
+            }
+            while ((b[0] - a[0] + 3) * (b[1] - a[1] + 3) * (b[2] - a[2] + 3) > cap) {
+                int d = 0;
+                for (int e = 1; e < 3; e++)
+                    if (b[e] - a[e] > b[d] - a[d]) d = e;
+                if (b[d] - mid[d] >= mid[d] - a[d]) b[d]--;
+                else a[d]++;
+            }
+        }
+        AdjWindow w;
+        w.i0 = a[0]; w.l0 = a[1]; w.k0 = a[2];
+        w.cx = b[0] - a[0] + 1; w.cy = b[1] - a[1] + 1; w.cz = b[2] - a[2] + 1;
+        w.SY = w.cy + 2; w.SZ = w.cz + 2;
+        w.nn = (w.cx + 2) * w.SY * w.SZ;
+        *out = w;
+    }
+    __syncthreads();
+    return *out;
+}
+// e with 2^(e-1) <= x < 2^e for a positive normal float, at least -120
+__device__ __forceinline__ int adj_exponent(float x) {
+    const int e = x > 0.f ? (int)((__float_as_uint(x) >> 23) & 0xff) - 126 : -120;
+    return max(e, -120);
+}
 
 // ---- per-block node box for scatters (adjoint of the interpolation).
 // Global atomics cost one L2 sector update each; the 256 particles of a block

@@ -199,52 +199,6 @@ __device__ __forceinline__ double interp_plain(const double *__restrict__ T, int
     return trilinear(T + ((bi + i) * SY + (bl + l)) * SZ + (bk + k), SY * SZ, SZ, sx, sx1, sy, sy1, sz, sz1);
 }
 
-// pqr, cell.h:1511-1693, accumulating into the tile J (shared memory).  The
-// reference's divisions by 12 and by tau*h*h are multiplications by their
-// reciprocals (rc[d] = 1 / (tau * h_e * h_f) times the charge weight and the
-// inverse quantum, precomputed): the products feed only the current's
-// magnitude, never an index, and differ from the quotients by an ulp.  LO32
-// selects the int32 remainder word (fx_put_lo32; words at sJ + 3 nn as 3 nn
-// ints), else the 64-bit one (fx_put2; 3 nn words).
-template <bool LO32>
-__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double lo_scale, int nn, int SY, int SZ,
-                                          int bi, int bl, int bk, const int iv[3], const double x[3],
-                                          const double x1[3], double hx, double hy, double hz, const double rc[3],
-                                          double x0, double y0, double z0, unsigned &bad) {
-    const double dx = (0.50 * (x[0] + x1[0]) - hx * ((double)iv[0] - 2.50) - x0);
-    const double dy = (0.50 * (x[1] + x1[1]) - hy * ((double)iv[1] - 2.50) - y0);
-    const double dz = (0.50 * (x[2] + x1[2]) - hz * ((double)iv[2] - 2.50) - z0);
-    const double dx1 = hx - dx, dy1 = hy - dy, dz1 = hz - dz;
-    double su = x1[0] - x[0], sv = x1[1] - x[1], sw = x1[2] - x[2];
-    constexpr double kTwelfth = 1.0 / 12.0;
-    const double s1 = sv * sw * kTwelfth, s2 = su * sw * kTwelfth, s3 = su * sv * kTwelfth;
-    su = su * rc[0];
-    sv = sv * rc[1];
-    sw = sw * rc[2];
-    if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) { bad |= ST_STENCIL; return; }
-    const int n = ((bi + iv[0]) * SY + (bl + iv[1])) * SZ + (bk + iv[2]);
-    const int ez = 1, ey = SZ, ex = SY * SZ;
-    int *lo32 = (int *)(sJ + 3 * nn);
-    // component c, node offset o from n, contribution v in quanta
-    auto add = [&](int c, int o, double v) {
-        const int w = c * nn + n + o;
-        if (LO32) fx_put_lo32(&sJ[w], &lo32[w], v, lo_scale);
-        else fx_put2(&sJ[w], &sJ[3 * nn + w], v);
-    };
-    add(0, 0, su * fma(dy1, dz1, s1));
-    add(0, ez, su * fma(dy1, dz, -s1));
-    add(0, ey, su * fma(dy, dz1, -s1));
-    add(0, ey + ez, su * fma(dy, dz, s1));
-    add(1, 0, sv * fma(dx1, dz1, s2));
-    add(1, ez, sv * fma(dx1, dz, -s2));
-    add(1, ex, sv * fma(dx, dz1, -s2));
-    add(1, ex + ez, sv * fma(dx, dz, s2));
-    add(2, 0, sw * fma(dx1, dy1, s3));
-    add(2, ey, sw * fma(dx1, dy, -s3));
-    add(2, ex, sw * fma(dx, dy1, -s3));
-    add(2, ex + ey, sw * fma(dx, dy, s3));
-}
-
 // flyDirection (cell.h:694-701): whether the particle leaves its cell
 __device__ __forceinline__ bool moved_cell(const Grid &g, int i, int l, int k, double x, double y, double z, double x0,
                                            double y0, double z0) {
@@ -486,7 +440,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
 
                 // ---- Cell::CurrentToMesh, cell.h:1306-1422
                 {
-                    double xo[3] = {x, y, z}, x2[3] = {0.0, 0.0, 0.0}, sr;
+                    double xo[3] = {x, y, z}, x2[3], sr;
                     const double h3[3] = {hx, hy, hz}, r3[3] = {rhx, rhy, rhz}, o3[3] = {x0, y0, z0};
                     const int i1[3] = {X.i1, Y.i1, Z.i1};
                     int i2[3];
@@ -495,39 +449,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
                     for (int d = 0; d < 3; d++)  // getCellNumberCenterCurrent, cell.h:577-578
                         i2[d] = trunc_checked((div_by(xn[d] - o3[d], h3[d], r3[d]) + 1.5) + 1, exact);
                     if (!exact) { bad |= ST_STENCIL; i2[0] = 0; }
-                    int m = 4 * abs(i2[0] - i1[0]) + 2 * abs(i2[1] - i1[1]) + abs(i2[2] - i1[2]);
-#define AVG(d) (h3[d] * (((double)i1[d] + (double)i2[d]) * 0.5 - 2.0) + o3[d])
-#define RATIO(d) ((x2[d] - xo[d]) / (xn[d] - xo[d]))
-#define PROD(d) ((x2[d] - xo[d]) * (xn[d] - xo[d]))
-#define RBX(d) (xo[d] + (xn[d] - xo[d]) * sr)
-#define SQ(v) ((v) * (v))
-                    switch (m) {
-                        case 1: x2[2] = AVG(2); sr = RATIO(2); x2[0] = RBX(0); x2[1] = RBX(1); break;
-                        case 2: x2[1] = AVG(1); sr = RATIO(1); x2[0] = RBX(0); x2[2] = RBX(2); break;
-                        case 3:
-                            x2[1] = AVG(1); x2[2] = AVG(2);
-                            sr = (PROD(2) + PROD(1)) / (SQ(xn[2] - xo[2]) + SQ(xn[1] - xo[1]));
-                            x2[0] = RBX(0);
-                            break;
-                        case 4: x2[0] = AVG(0); sr = RATIO(0); x2[1] = RBX(1); x2[2] = RBX(2); break;
-                        case 5:
-                            x2[0] = AVG(0); x2[2] = AVG(2);
-                            sr = (PROD(2) + PROD(0)) / (SQ(xn[2] - xo[2]) + SQ(xn[0] - xo[0]));
-                            x2[1] = RBX(1);
-                            break;
-                        case 6:
-                            x2[0] = AVG(0); x2[1] = AVG(1);
-                            sr = (PROD(1) + PROD(0)) / (SQ(xn[1] - xo[1]) + SQ(xn[0] - xo[0]));
-                            x2[2] = RBX(2);
-                            break;
-                        case 7: x2[0] = AVG(0); x2[1] = AVG(1); x2[2] = AVG(2); break;
-                        default: break;
-                    }
-#undef AVG
-#undef RATIO
-#undef PROD
-#undef RBX
-#undef SQ
+                    const int m = relay_point(xo, xn, o3, h3, i1, i2, x2, sr);
                     // the first segment here: xo -> xn, or xo -> x2 when the step
                     // crosses a cell-centre plane.  The second, x2 -> xn, goes to
                     // the warp's queue and is deposited with the warp's other
