@@ -1383,7 +1383,7 @@ void adj_free(pic_handle *h) {
     if (!h || !h->adj) return;
     AdjState *A = h->adj;
     void *bufs[] = {A->cur, A->ckp, A->ckf, A->segp, A->segf, A->subp, A->subf, A->lamp, A->lamf, A->rf, A->ha,
-                    A->hist, A->st, A->red, A->lamF, A->segF, A->branch, A->chunks};
+                    A->hist, A->st, A->red, A->branch, A->chunks};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (A->e0) cudaEventDestroy(A->e0);
@@ -1436,14 +1436,14 @@ MixParams mix_params(pic_handle *h, AdjState &A, char *state, void *const F[PIC_
         P.H[c] = (const float *)F[PIC_HX + c];
         P.J[c] = (double *)F[PIC_JX + c];
     }
+    P.chunks = A.chunks;
     P.st = A.st;
     return P;
 }
 
 // one forward step of the fixed-order state on the field set F: particles
-// read from `state`, written to `out` (same buffer when null); Fout, when
-// given, receives the interpolated fields of every particle
-int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, void *Fout) {
+// read from `state`, written to `out` (same buffer when null)
+int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out) {
     if (!h->mixed) return flat_step_plain(h, A, state, F, out);
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
@@ -1453,9 +1453,7 @@ int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_C
     const size_t nodes = g.nodes_pitched();
     for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(F[PIC_JX + c], 0, nodes * sizeof(double), s), "zero J");
     MixParams P = mix_params(h, A, state, F, out);
-    const int64_t n = total_particles(A);
-    for (int c = 0; c < 6; c++) P.Fout[c] = Fout ? (float *)Fout + (size_t)c * n : nullptr;
-    CK(launch_flat_push_mixed(P, s), "flat push");
+    CK(launch_flat_push_mixed(P, A.nchunks, s), "flat push");
     j_fold(g, (double *)F[PIC_JX], (double *)F[PIC_JY], (double *)F[PIC_JZ], s);
     yee_b_half_mixed(g, E, H, s);  // completion: the same Q again
     yee_e_update_mixed(g, E, H, (double *const *)&F[PIC_JX], s);
@@ -1485,7 +1483,7 @@ int forward_run(pic_handle *h, AdjState &A) {
             A.step_branch = const_cast<unsigned long long *>(A.branch_src) + (size_t)n * np_all;
             A.step_bmode = 2;
         }
-        int rc = flat_step(h, A, A.cur, h->f, nullptr, nullptr);
+        int rc = flat_step(h, A, A.cur, h->f, nullptr);
         A.step_branch = nullptr;
         A.step_bmode = 0;
         if (rc) return rc;
@@ -1503,9 +1501,9 @@ int forward_run(pic_handle *h, AdjState &A) {
 }
 
 // reverse of step n: EHn = E_n, H_n of the step (form's type, 6 arrays),
-// Enext = E after the step, Fin = the push's interpolated fields (or null)
+// Enext = E after the step
 int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *state, const char *EHn,
-                 const char *Enext, const void *Fin) {
+                 const char *Enext) {
     const Grid &g = h->g;
     cudaStream_t st = h->stream;
     const size_t N = g.nodes_pitched();
@@ -1543,7 +1541,6 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
         int a = dir == 0 ? g.NY : g.NX, b = dir == 2 ? g.NY : g.NZ;
         k_adj_j_fold<<<(a * b + 127) / 128, 128, 0, st>>>(g, LJ[0], LJ[1], LJ[2], dir);
     }
-    const int64_t np = total_particles(A);
     if (!h->mixed) {
         // H_a of step n
         const double *En = (const double *)EHn, *Hn = (const double *)EHn + 3 * N;
@@ -1586,11 +1583,7 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
             o += 6 * (size_t)A.n[s];
         }
         for (int c = 0; c < 3; c++) { P.LJ[c] = LJ[c]; P.LE[c] = LE[c]; P.LH[c] = LH[c]; }
-        for (int c = 0; c < 6; c++) {
-            P.LF[c] = (float *)A.lamF + (size_t)c * np;
-            P.Fin[c] = Fin ? (const float *)Fin + (size_t)c * np : nullptr;
-        }
-        CK(launch_adj_particles_mixed(P, st), "adjoint particles");
+        CK(launch_adj_particles_mixed(P, A.nchunks, st), "adjoint particles");
     }
     k_adj_b_half<<<node_grid(g), 32, 0, st>>>(FA);
     CK(cudaGetLastError(), "reverse step");
@@ -1602,8 +1595,6 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
     cudaStream_t st = h->stream;
     const size_t N = g.nodes_pitched();
     const size_t fbytes = field_bytes(h);
-    const int64_t np = total_particles(A);
-    const size_t Fstep = (size_t)6 * np * A.elem;  // interpolated fields of one step
     CK(cudaMemsetAsync(A.lamp, 0, A.lamp_bytes, st), "zero lambda");
     CK(cudaMemsetAsync(A.lamf, 0, 12 * N * sizeof(double), st), "zero lambda fields");
     void *RF[PIC_FIELD_COUNT];
@@ -1628,7 +1619,7 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
                        "sub-checkpoint fields");
                     if (q == nsub - 1) break;  // the last sub-segment starts here
                 }
-                int rc = flat_step(h, A, A.segp, RF, nullptr, nullptr);
+                int rc = flat_step(h, A, A.segp, RF, nullptr);
                 if (rc) return rc;
             }
         }
@@ -1640,15 +1631,13 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
             CK(cudaMemcpyAsync(A.rf, sf, ehb, cudaMemcpyDeviceToDevice, st), "restore fields");
             for (int j = 0; j < slen; j++) {
                 CK(cudaMemcpyAsync(A.segf + (size_t)j * ehb, A.rf, ehb, cudaMemcpyDeviceToDevice, st), "keep fields");
-                void *Fj = A.segF ? (char *)A.segF + (size_t)j * Fstep : nullptr;
-                int rc = flat_step(h, A, A.segp + (size_t)j * A.pbytes, RF, A.segp + (size_t)(j + 1) * A.pbytes, Fj);
+                int rc = flat_step(h, A, A.segp + (size_t)j * A.pbytes, RF, A.segp + (size_t)(j + 1) * A.pbytes);
                 if (rc) return rc;
             }
             CK(cudaMemcpyAsync(A.segf + (size_t)slen * ehb, A.rf, ehb, cudaMemcpyDeviceToDevice, st), "keep fields");
             for (int j = slen - 1; j >= 0; j--) {
                 int rc = reverse_step(h, A, L, s0 + j, A.segp + (size_t)j * A.pbytes, A.segf + (size_t)j * ehb,
-                                      A.segf + (size_t)(j + 1) * ehb,
-                                      A.segF ? (const char *)A.segF + (size_t)j * Fstep : nullptr);
+                                      A.segf + (size_t)(j + 1) * ehb);
                 if (rc) return rc;
             }
         }
@@ -1891,18 +1880,6 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
         if ((rc = adj_alloc(h, (void **)&A.rf, N * sizeof(double) * PIC_FIELD_COUNT, "the recompute fields")))
             return rc;
         if ((rc = adj_alloc(h, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
-        if (h->mixed &&
-            (rc = adj_alloc(h, (void **)&A.lamF, (size_t)np * 6 * A.elem, "the interpolation adjoints")))
-            return rc;
-        // optional: the interpolated fields of every step of a segment, so the
-        // adjoint does not gather them again (skipped when memory is short)
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        size_t want = (size_t)np * 6 * A.elem * (size_t)A.K2;
-        if (h->mixed && want + ((size_t)4 << 30) < free_b && cudaMalloc((void **)&A.segF, want) != cudaSuccess) {
-            A.segF = nullptr;
-            cudaGetLastError();
-        }
     }
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     rc = backward_run(h, A, *loss);

@@ -17,17 +17,6 @@ namespace {
 constexpr int kT = 256;
 constexpr float kOneBelow = 0.99999994f;  // largest float < 1
 
-// see spread_index in pic_adjoint.cu: lane quads take 4 consecutive particles,
-// the 8 quads of a warp sit 32 particles apart (about 8 different cells)
-__device__ __forceinline__ int64_t spread_index(int t) {
-    return (int64_t)blockIdx.x * kT + ((t & 31) >> 2) * 32 + (t >> 5) * 4 + (t & 3);
-}
-__device__ __forceinline__ int species_of(const int64_t *off, int nsp, int64_t idx) {
-    int s = 0;
-    while (s + 1 < nsp && idx >= off[s + 1]) s++;
-    return s;
-}
-
 // GetField in cell units (k_push_mixed): the node-staggered tap is 2 with
 // weight 1 - o, the centre-staggered tap 2 + (o >= 1/2) with weight
 // (1/2 or 3/2) - o; component c is node-staggered along d when
@@ -52,30 +41,32 @@ __device__ __forceinline__ void comp_taps_m(const MTaps &T, int c, int t[3], flo
         w[d] = nd ? T.wn[d] : T.wc[d];
     }
 }
-__device__ __forceinline__ size_t tap_node(const Grid &g, int i, int l, int k, const int t[3]) {
-    return g.node(i + t[0] - 2, l + t[1] - 2, k + t[2] - 2);
-}
-// interp_mixed's expression order
-__device__ __forceinline__ float interp_gm(const float *__restrict__ A, size_t n, size_t dx, size_t dy,
-                                           const float w[3]) {
-    const size_t dz = 1;
+// interp_mixed's expression order; the eight taps at A, A + dx, ...
+__device__ __forceinline__ float interp_gm(const float *__restrict__ A, int dx, int dy, const float w[3]) {
+    const int dz = 1;
     float sx = w[0], sy = w[1], sz = w[2];
     float sx1 = 1.f - sx, sy1 = 1.f - sy, sz1 = 1.f - sz;
-    float t1 = sx * (sy * (sz * A[n] + sz1 * A[n + dz]) + sy1 * (sz * A[n + dy] + sz1 * A[n + dy + dz]));
-    float t2 = sx1 * (sy * (sz * A[n + dx] + sz1 * A[n + dx + dz]) + sy1 * (sz * A[n + dx + dy] + sz1 * A[n + dx + dy + dz]));
+    float t1 = sx * (sy * (sz * A[0] + sz1 * A[dz]) + sy1 * (sz * A[dy] + sz1 * A[dy + dz]));
+    float t2 = sx1 * (sy * (sz * A[dx] + sz1 * A[dx + dz]) + sy1 * (sz * A[dx + dy] + sz1 * A[dx + dy + dz]));
     return t1 + t2;
 }
-__device__ __forceinline__ void gather_fields_m(const Grid &g, const float *const E[3], const float *const H[3],
-                                                int i, int l, int k, const float x[3], float F[6]) {
+// A particle's view of the fields: the CTA's window in shared memory (WIN) or
+// the arrays in global memory; base[c] points at the node of its cell
+template <bool WIN>
+struct FieldViewM {
+    const float *base[6];
+    int dx, dy;
+};
+template <class V>
+__device__ __forceinline__ void gather_fields_m(const V &A, const float x[3], float F[6]) {
     MTaps T;
     taps_mixed(x, T);
-    const size_t dx = (size_t)g.NY * g.pz, dy = g.pz;
 #pragma unroll
     for (int c = 0; c < 6; c++) {
         int t[3];
         float w[3];
         comp_taps_m(T, c, t, w);
-        F[c] = interp_gm(c < 3 ? E[c] : H[c - 3], tap_node(g, i, l, k, t), dx, dy, w);
+        F[c] = interp_gm(A.base[c] + (t[0] - 2) * A.dx + (t[1] - 2) * A.dy + (t[2] - 2), A.dx, A.dy, w);
     }
 }
 
@@ -146,9 +137,11 @@ __device__ __forceinline__ bool stencil_ok(const int iv[3]) {
     return iv[0] >= 2 && iv[0] <= 3 && iv[1] >= 2 && iv[1] <= 3 && iv[2] >= 2 && iv[2] <= 3;
 }
 
-// pqr_mixed (pic_mixed.cu) into the FP64 global J
-__device__ __forceinline__ void seg_mixed(double *const J[3], const Grid &g, int ci, int cl, int ck, const int iv[3],
-                                          const float xs[3], const float xe[3], float wx, float wy, float wz) {
+// pqr_mixed (pic_mixed.cu): add(component, x, y, z node offset from the
+// particle's cell, FP32 contribution); false when the segment has no length
+template <class Add>
+__device__ __forceinline__ void seg_mixed(const int iv[3], const float xs[3], const float xe[3], float wx, float wy,
+                                          float wz, Add add) {
     float dx = 0.5f * (xs[0] + xe[0]) - ((float)iv[0] - 2.5f);
     float dy = 0.5f * (xs[1] + xe[1]) - ((float)iv[1] - 2.5f);
     float dz = 0.5f * (xs[2] + xe[2]) - ((float)iv[2] - 2.5f);
@@ -160,27 +153,27 @@ __device__ __forceinline__ void seg_mixed(double *const J[3], const Grid &g, int
     sv *= wy;
     sw *= wz;
     if (su == 0.f && sv == 0.f && sw == 0.f) return;
-    size_t n = tap_node(g, ci, cl, ck, iv);
-    const size_t ez = 1, ey = g.pz, ex = (size_t)g.NY * g.pz;
-    double *Jx = J[0], *Jy = J[1], *Jz = J[2];
-    atomicAdd(&Jx[n], (double)(su * (dy1 * dz1 + s1)));
-    atomicAdd(&Jx[n + ez], (double)(su * (dy1 * dz - s1)));
-    atomicAdd(&Jx[n + ey], (double)(su * (dy * dz1 - s1)));
-    atomicAdd(&Jx[n + ey + ez], (double)(su * (dy * dz + s1)));
-    atomicAdd(&Jy[n], (double)(sv * (dx1 * dz1 + s2)));
-    atomicAdd(&Jy[n + ez], (double)(sv * (dx1 * dz - s2)));
-    atomicAdd(&Jy[n + ex], (double)(sv * (dx * dz1 - s2)));
-    atomicAdd(&Jy[n + ex + ez], (double)(sv * (dx * dz + s2)));
-    atomicAdd(&Jz[n], (double)(sw * (dx1 * dy1 + s3)));
-    atomicAdd(&Jz[n + ey], (double)(sw * (dx1 * dy - s3)));
-    atomicAdd(&Jz[n + ex], (double)(sw * (dx * dy1 - s3)));
-    atomicAdd(&Jz[n + ex + ey], (double)(sw * (dx * dy + s3)));
+    const int a = iv[0] - 2, b = iv[1] - 2, c = iv[2] - 2;
+    add(0, a, b, c, su * (dy1 * dz1 + s1));
+    add(0, a, b, c + 1, su * (dy1 * dz - s1));
+    add(0, a, b + 1, c, su * (dy * dz1 - s1));
+    add(0, a, b + 1, c + 1, su * (dy * dz + s1));
+    add(1, a, b, c, sv * (dx1 * dz1 + s2));
+    add(1, a, b, c + 1, sv * (dx1 * dz - s2));
+    add(1, a + 1, b, c, sv * (dx * dz1 - s2));
+    add(1, a + 1, b, c + 1, sv * (dx * dz + s2));
+    add(2, a, b, c, sw * (dx1 * dy1 + s3));
+    add(2, a, b + 1, c, sw * (dx1 * dy - s3));
+    add(2, a + 1, b, c, sw * (dx * dy1 - s3));
+    add(2, a + 1, b + 1, c, sw * (dx * dy + s3));
 }
 
-// transpose of seg_mixed (cell units: h = 1, weights wx, wy, wz)
-__device__ __forceinline__ void seg_mixed_rev(const double *const L[3], const Grid &g, int ci, int cl, int ck,
-                                              const int iv[3], const float xs[3], const float xe[3], float cu,
-                                              float cv, float cw, float gs[3], float ge[3]) {
+// transpose of seg_mixed (cell units: h = 1, weights wx, wy, wz); L: lambda_J
+// at the particle's cell (float in the window, double in global memory)
+template <class T>
+__device__ __forceinline__ void seg_mixed_rev(const T *L0, const T *L1, const T *L2, int ex, int ey, const int iv[3],
+                                              const float xs[3], const float xe[3], float cu, float cv, float cw,
+                                              float gs[3], float ge[3]) {
     float dx = 0.5f * (xs[0] + xe[0]) - ((float)iv[0] - 2.5f);
     float dy = 0.5f * (xs[1] + xe[1]) - ((float)iv[1] - 2.5f);
     float dz = 0.5f * (xs[2] + xe[2]) - ((float)iv[2] - 2.5f);
@@ -189,11 +182,11 @@ __device__ __forceinline__ void seg_mixed_rev(const double *const L[3], const Gr
     const float r12 = 1.f / 12.f;
     float s1 = Dy * Dz * r12, s2 = Dx * Dz * r12, s3 = Dx * Dy * r12;
     float Ax = cu * Dx, Ay = cv * Dy, Az = cw * Dz;
-    size_t n = tap_node(g, ci, cl, ck, iv);
-    const size_t ez = 1, ey = g.pz, ex = (size_t)g.NY * g.pz;
-    float Lx0 = (float)L[0][n], Lx1 = (float)L[0][n + ez], Lx2 = (float)L[0][n + ey], Lx3 = (float)L[0][n + ey + ez];
-    float Ly0 = (float)L[1][n], Ly1 = (float)L[1][n + ez], Ly2 = (float)L[1][n + ex], Ly3 = (float)L[1][n + ex + ez];
-    float Lz0 = (float)L[2][n], Lz1 = (float)L[2][n + ey], Lz2 = (float)L[2][n + ex], Lz3 = (float)L[2][n + ex + ey];
+    const int n = (iv[0] - 2) * ex + (iv[1] - 2) * ey + (iv[2] - 2);
+    const int ez = 1;
+    float Lx0 = (float)L0[n], Lx1 = (float)L0[n + ez], Lx2 = (float)L0[n + ey], Lx3 = (float)L0[n + ey + ez];
+    float Ly0 = (float)L1[n], Ly1 = (float)L1[n + ez], Ly2 = (float)L1[n + ex], Ly3 = (float)L1[n + ex + ez];
+    float Lz0 = (float)L2[n], Lz1 = (float)L2[n + ey], Lz2 = (float)L2[n + ex], Lz3 = (float)L2[n + ex + ey];
     float Fx = Lx0 * (dy1 * dz1 + s1) + Lx1 * (dy1 * dz - s1) + Lx2 * (dy * dz1 - s1) + Lx3 * (dy * dz + s1);
     float Fy = Ly0 * (dx1 * dz1 + s2) + Ly1 * (dx1 * dz - s2) + Ly2 * (dx * dz1 - s2) + Ly3 * (dx * dz + s2);
     float Fz = Lz0 * (dx1 * dy1 + s3) + Lz1 * (dx1 * dy - s3) + Lz2 * (dx * dy1 - s3) + Lz3 * (dx * dy + s3);
@@ -252,104 +245,253 @@ __device__ __forceinline__ void split_rev_m(const SplitM &S, const float xo[3], 
     }
 }
 
-// ---- fixed-order push of the FP32 form
-__global__ void __launch_bounds__(kT) k_flat_push_mixed(MixParams P) {
-    int64_t idx = spread_index(threadIdx.x);
-    unsigned bad = 0;
-    unsigned long long amb = 0;
-    if (idx < P.off[P.nsp]) {
-        const Grid &g = P.g;
-        int s = species_of(P.off, P.nsp, idx);
-        const MixSp &S = P.sp[s];
-        int64_t j = idx - P.off[s];
-        int cell = S.cell[j];
-        int i, l, k;
-        g.cell_ijk(cell, i, l, k);
-        float xs[3] = {S.v[0][j], S.v[1][j], S.v[2][j]};
-        float p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
-        float F[6];
-        gather_fields_m(g, P.E, P.H, i, l, k, xs, F);
-        if (P.Fout[0]) {
-#pragma unroll
-            for (int c = 0; c < 6; c++) P.Fout[c][idx] = F[c];
-        }
-        const float tau1 = (float)(S.q_m * g.tau * 0.5);
-        const float ct[3] = {(float)(g.tau / g.hx), (float)(g.tau / g.hy), (float)(g.tau / g.hz)};
-        BorisM B;
-        boris_mixed(tau1, ct, p, F, xs, B);
-        if (!(isfinite(B.pp[0]) && isfinite(B.pp[1]) && isfinite(B.pp[2]))) bad |= ST_NAN;
-        float xe[3] = {B.xe[0], B.xe[1], B.xe[2]};
-        SplitM SP;
-        split_mixed(xs, xe, SP);
-        const float wx = (float)(S.m * g.hx / g.tau), wy = (float)(S.m * g.hy / g.tau), wz = (float)(S.m * g.hz / g.tau);
-        if (!stencil_ok(SP.i2) || !(isfinite(xe[0]) && isfinite(xe[1]) && isfinite(xe[2]))) {
-            bad |= ST_STENCIL;
-        } else {
-            seg_mixed(P.J, g, i, l, k, SP.i1, xs, SP.x2, wx, wy, wz);
-            seg_mixed(P.J, g, i, l, k, SP.i2, SP.x2, xe, wx, wy, wz);
-        }
-        // new cell (Reflect and migration in cell units, as k_push_mixed)
-        int ci[3] = {i, l, k};
-        const int nc[3] = {g.nx, g.ny, g.nz};
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            if (xe[d] >= 1.f) {
-                xe[d] -= 1.f;
-                ci[d] = ci[d] + 1 == nc[d] ? 0 : ci[d] + 1;
-            } else if (xe[d] < 0.f) {
-                xe[d] += 1.f;
-                ci[d] = ci[d] == 0 ? nc[d] - 1 : ci[d] - 1;
-            }
-            xe[d] = fminf(fmaxf(xe[d], 0.f), kOneBelow);
-        }
-        const MixOut &O = P.out[s];
-        O.cell[j] = g.cell_of(ci[0], ci[1], ci[2]);
-        O.v[0][j] = xe[0]; O.v[1][j] = xe[1]; O.v[2][j] = xe[2];
-        O.v[3][j] = B.pp[0]; O.v[4][j] = B.pp[1]; O.v[5][j] = B.pp[2];
-    }
-    if (bad) atomicOr(&P.st->flags, bad);
-    if (amb) atomicAdd(&P.st->ambiguous, amb);
+// per-species constants of the particle kernels (formed once per CTA: the FP64
+// divisions behind them cost more than a particle's FP32 work)
+struct MixConst {
+    float tau1, ct[3], w[3];
+};
+__device__ __forceinline__ MixConst mix_const(const Grid &g, const MixSp &S) {
+    MixConst K;
+    K.tau1 = (float)(S.q_m * g.tau * 0.5);
+    K.ct[0] = (float)(g.tau / g.hx); K.ct[1] = (float)(g.tau / g.hy); K.ct[2] = (float)(g.tau / g.hz);
+    K.w[0] = (float)(S.m * g.hx / g.tau); K.w[1] = (float)(S.m * g.hy / g.tau); K.w[2] = (float)(S.m * g.hz / g.tau);
+    return K;
 }
 
-// ---- adjoint, first pass: recompute, deposit and push transposes
-template <bool STORED>
-__global__ void __launch_bounds__(kT, 2) k_adj_push_mixed(MixParams P) {
-    int64_t idx = spread_index(threadIdx.x);
-    if (idx >= P.off[P.nsp]) return;
-    const Grid &g = P.g;
-    int s = species_of(P.off, P.nsp, idx);
-    const MixSp &S = P.sp[s];
-    int64_t j = idx - P.off[s];
-    int i, l, k;
-    g.cell_ijk(S.cell[j], i, l, k);
-    float xs[3] = {S.v[0][j], S.v[1][j], S.v[2][j]};
-    float p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
-    float F[6];
-    if (STORED) {
-#pragma unroll
-        for (int c = 0; c < 6; c++) F[c] = P.Fin[c][idx];
-    } else {
-        gather_fields_m(g, P.E, P.H, i, l, k, xs, F);
+constexpr int kW = kT / 32;          // warps per CTA
+constexpr int kQueueMix = 48;        // queued second segments per warp: drained at 16, at most 15 + 32
+constexpr int kFlatWindowMix = 800;  // nodes of the forward's window: 56 KB of shared memory, three CTAs per SM (80 registers)
+constexpr int kAdjWindowMix = 640;   // nodes of the adjoint's: 71 KB, three
+
+// shared memory of a thread's next particle (cp.async, as in k_push_plain): N values, then the cell
+template <int N>
+struct NextMix {
+    float *v;
+    __device__ __forceinline__ NextMix(void *base) {
+        v = (float *)base + (threadIdx.x >> 5) * ((N + 1) * 32) + (threadIdx.x & 31);
     }
-    const float tau1 = (float)(S.q_m * g.tau * 0.5);
-    const float ct[3] = {(float)(g.tau / g.hx), (float)(g.tau / g.hy), (float)(g.tau / g.hz)};
+    static constexpr size_t bytes = (size_t)kW * (N + 1) * 32 * sizeof(float);
+    __device__ __forceinline__ void start(const MixSp &S, float *const *lam, int64_t j) const {
+#pragma unroll
+        for (int a = 0; a < 6; a++) cp_async<4>(v + 32 * a, S.v[a] + j);
+        if (N > 6)
+#pragma unroll
+            for (int a = 0; a < 6; a++) cp_async<4>(v + 32 * (6 + a), lam[a] + j);
+        cp_async<4>(v + 32 * N, S.cell + j);
+    }
+    __device__ __forceinline__ int cell() const { return __float_as_int(v[32 * N]); }
+    __device__ __forceinline__ void take3(int from, float x[3]) const {
+#pragma unroll
+        for (int d = 0; d < 3; d++) x[d] = v[32 * (from + d)];
+    }
+};
+
+// stages the window's nodes of N arrays src[c] into dst (N x w.nn floats)
+template <int N, class T>
+__device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow &w, const T *const *src, float *dst) {
+    for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
+        const int c = e % w.SZ, ab = e / w.SZ, b = ab % w.SY, a = ab / w.SY;
+        const size_t n = g.node(w.i0 + a, w.l0 + b, w.k0 + c);
+#pragma unroll
+        for (int q = 0; q < N; q++) dst[q * w.nn + e] = (float)src[q][n];
+    }
+}
+
+// ---- fixed-order push of the FP32 form.  One CTA per chunk of consecutive
+// particles with the chunk's window staged in shared memory, as
+// k_flat_push_plain; the FP32 contributions are summed in 64-bit fixed point
+// (quantum 2^-50 of the light-speed bound of the chunk, or 2^-51 of one
+// particle's) and added to the FP64 global J once.
+// Bound: instruction issue (1104 instructions per 32 particles, issue slots 70 %
+// busy).  128x32x32 cells, 12.6M particles: 0.916 -> 0.635 ms per step (before:
+// taps gathered from and currents added to global memory; four CTAs per SM at
+// 64 registers: 0.688; lanes spread over 4 or 8 places: 0.625, 0.660, and slower
+// at 3M particles).
+__global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant__ MixParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ AdjWindow sWin;
+    __shared__ int sRed[15 * kW], sQn[kW];
+    __shared__ double sQ, sInvQ;
+    __shared__ MixConst sK;
+    const Grid &g = P.g;
+    const AdjChunk ch = P.chunks[blockIdx.x];
+    const int s = ch.species, count = ch.count;
+    const MixSp &S = P.sp[s];
+    unsigned char *sTail = smem_raw + (size_t)kFlatWindowMix * 48;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *qd = (float *)sTail + warp * 7 * kQueueMix;  // x2, xe, then the cell and class code
+    const NextMix<6> next(sTail + (size_t)kW * 7 * kQueueMix * sizeof(float));
+    if ((int)threadIdx.x < count) next.start(S, nullptr, ch.first + threadIdx.x);
+    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
+    const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
+    unsigned *sLo = (unsigned *)smem_raw, *sHi = sLo + 3 * nn;
+    float *sF = (float *)(sHi + 3 * nn);
+    if (threadIdx.x == 0) {
+        int e2, e1;
+        frexp(2.5 * fabs(S.m) * (double)count, &e2);
+        frexp(1.0834 * fabs(S.m), &e1);
+        const int eq = max(e2 - 62, e1 - 51);
+        sQ = ldexp(1.0, eq);
+        sInvQ = ldexp(1.0, -eq);
+        sK = mix_const(g, S);
+    }
+    const float *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
+    stage_window_m<6>(g, w, src, sF);
+    for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) sLo[e] = 0u;
+    if (lane == 0) sQn[warp] = 0;
+    __syncthreads();
+    const MixConst &K = sK;
+    const double inv_q = sInvQ;
+    const int nc[3] = {g.nx, g.ny, g.nz};
+    unsigned bad = 0;
+    int qn = 0;
+    auto put = [&](int n0) {
+        return [=](int c, int a, int b, int k, float v) {
+            const int n = c * nn + n0 + a * dX + b * dY + k;
+            const long long iv = __double_as_longlong(fma((double)v, inv_q, kRound)) - 0x4338000000000000ll;
+            if (iv) shared_add64(sLo + n, sHi + n, iv);
+        };
+    };
+    for (int jw = threadIdx.x - lane;; jw += blockDim.x) {
+        const bool tail = jw >= count;
+        if (tail && qn == 0) break;
+        const int jc = jw + lane;
+        const int64_t j = ch.first + jc;
+        int cell = -1;
+        float xs[3], p[3];
+        cp_async_wait_all();
+        if (jc < count) {
+            cell = next.cell();
+            next.take3(0, xs);
+            next.take3(3, p);
+        }
+        __syncwarp();  // the reads come before the next copies into the same place
+        if (jc + (int)blockDim.x < count) next.start(S, nullptr, j + blockDim.x);
+        if (cell >= 0) {
+            int c3[3];
+            g.cell_ijk(cell, c3[0], c3[1], c3[2]);
+            const bool in = w.holds(c3[0], c3[1], c3[2]);
+            const int n0 = w.node(c3[0], c3[1], c3[2]);
+            float F[6];
+            if (in) {
+                FieldViewM<true> V;
+#pragma unroll
+                for (int c = 0; c < 6; c++) V.base[c] = sF + c * nn + n0;
+                V.dx = dX; V.dy = dY;
+                gather_fields_m(V, xs, F);
+            } else {
+                FieldViewM<false> V;
+#pragma unroll
+                for (int c = 0; c < 6; c++) V.base[c] = src[c] + g.node(c3[0], c3[1], c3[2]);
+                V.dx = g.NY * g.pz; V.dy = g.pz;
+                gather_fields_m(V, xs, F);
+            }
+            BorisM B;
+            boris_mixed(K.tau1, K.ct, p, F, xs, B);
+            if (!(isfinite(B.pp[0]) && isfinite(B.pp[1]) && isfinite(B.pp[2]))) bad |= ST_NAN;
+            float xe[3] = {B.xe[0], B.xe[1], B.xe[2]};
+            SplitM SP;
+            split_mixed(xs, xe, SP);
+            if (!stencil_ok(SP.i2) || !(isfinite(xe[0]) && isfinite(xe[1]) && isfinite(xe[2]))) {
+                bad |= ST_STENCIL;
+            } else if (in) {
+                seg_mixed(SP.i1, xs, SP.x2, K.w[0], K.w[1], K.w[2], put(n0));
+                // the second segment: from a cell-centre plane, or the rounding of
+                // x2 = xs + (xe - xs) where none is crossed
+                if (SP.x2[0] != xe[0] || SP.x2[1] != xe[1] || SP.x2[2] != xe[2]) {
+                    const int e = atomicAdd(&sQn[warp], 1);
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        qd[d * kQueueMix + e] = SP.x2[d];
+                        qd[(3 + d) * kQueueMix + e] = xe[d];
+                    }
+                    qd[6 * kQueueMix + e] =
+                        __int_as_float((n0 << 3) | (SP.i2[0] - 2) | ((SP.i2[1] - 2) << 1) | ((SP.i2[2] - 2) << 2));
+                }
+            } else {
+                auto far = [&](int c, int a, int b, int k, float v) {
+                    atomicAdd(&P.J[c][g.node(c3[0] + a, c3[1] + b, c3[2] + k)], (double)v);
+                };
+                seg_mixed(SP.i1, xs, SP.x2, K.w[0], K.w[1], K.w[2], far);
+                seg_mixed(SP.i2, SP.x2, xe, K.w[0], K.w[1], K.w[2], far);
+            }
+            // new cell (Reflect and migration in cell units, as k_push_mixed)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                if (xe[d] >= 1.f) {
+                    xe[d] -= 1.f;
+                    c3[d] = c3[d] + 1 == nc[d] ? 0 : c3[d] + 1;
+                } else if (xe[d] < 0.f) {
+                    xe[d] += 1.f;
+                    c3[d] = c3[d] == 0 ? nc[d] - 1 : c3[d] - 1;
+                }
+                xe[d] = fminf(fmaxf(xe[d], 0.f), kOneBelow);
+            }
+            const MixOut &O = P.out[s];
+            O.cell[j] = g.cell_of(c3[0], c3[1], c3[2]);
+            O.v[0][j] = xe[0]; O.v[1][j] = xe[1]; O.v[2][j] = xe[2];
+            O.v[3][j] = B.pp[0]; O.v[4][j] = B.pp[1]; O.v[5][j] = B.pp[2];
+        }
+        // ---- the warp's queued second segments, one per lane
+        __syncwarp();
+        qn = sQn[warp];
+        if (qn >= (tail ? 1 : 16)) {
+            const int d = qn < 32 ? qn : 32;
+            if (lane < d) {
+                const int e = qn - d + lane, code = __float_as_int(qd[6 * kQueueMix + e]);
+                const int iv[3] = {2 + (code & 1), 2 + ((code >> 1) & 1), 2 + ((code >> 2) & 1)};
+                float sa[3], sb[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    sa[q] = qd[q * kQueueMix + e];
+                    sb[q] = qd[(3 + q) * kQueueMix + e];
+                }
+                seg_mixed(iv, sa, sb, K.w[0], K.w[1], K.w[2], put(code >> 3));
+            }
+            qn -= d;
+            __syncwarp();
+            if (lane == 0) sQn[warp] = qn;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
+        const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
+        if (v == 0) continue;
+        const int comp = e / nn, r = e - comp * nn;
+        const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
+        atomicAdd(&P.J[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * sQ);
+    }
+    if (bad) atomicOr(&P.st->flags, bad);
+}
+
+// The reverse of one particle's step up to the adjoint of its interpolated
+// fields (reverse_particle in pic_adjoint.cu): in gn, lP the incoming lambda_x
+// and lambda_p, out gx, lu and lF
+template <class V, class T>
+__device__ __forceinline__ void reverse_particle_m(const MixConst &K, const V &A, const T *L0, const T *L1, const T *L2,
+                                                   int lx, int ly, const float xs[3], const float p[3], float gn[3],
+                                                   float lP[3], float gx[3], float lu[3], float lF[6]) {
+    float F[6];
+    gather_fields_m(A, xs, F);
     BorisM B;
-    boris_mixed(tau1, ct, p, F, xs, B);
+    boris_mixed(K.tau1, K.ct, p, F, xs, B);
     SplitM SP;
     split_mixed(xs, B.xe, SP);
-    float *const *Lm = P.lam[s];
-    float lx[3] = {Lm[0][j], Lm[1][j], Lm[2][j]};
-    float lp[3] = {Lm[3][j], Lm[4][j], Lm[5][j]};
-    float gx[3] = {0.f, 0.f, 0.f}, gn[3] = {lx[0], lx[1], lx[2]};
-    const float wx = (float)(S.m * g.hx / g.tau), wy = (float)(S.m * g.hy / g.tau), wz = (float)(S.m * g.hz / g.tau);
+#pragma unroll
+    for (int d = 0; d < 3; d++) gx[d] = 0.f;
     if (stencil_ok(SP.i2)) {
+        float g2[3] = {0.f, 0.f, 0.f}, sb[3];
+        // without a crossing the first segment is the whole step
+#pragma unroll
+        for (int d = 0; d < 3; d++) sb[d] = SP.m != 0 ? SP.x2[d] : B.xe[d];
+        seg_mixed_rev(L0, L1, L2, lx, ly, SP.i1, xs, sb, K.w[0], K.w[1], K.w[2], gx, g2);
         if (SP.m != 0) {
-            float g2[3] = {0.f, 0.f, 0.f};
-            seg_mixed_rev(P.LJ, g, i, l, k, SP.i1, xs, SP.x2, wx, wy, wz, gx, g2);
-            seg_mixed_rev(P.LJ, g, i, l, k, SP.i2, SP.x2, B.xe, wx, wy, wz, g2, gn);
+            seg_mixed_rev(L0, L1, L2, lx, ly, SP.i2, SP.x2, B.xe, K.w[0], K.w[1], K.w[2], g2, gn);
             split_rev_m(SP, xs, B.xe, g2, gx, gn);
-        } else {  // no crossing: x2 = xe, one segment
-            seg_mixed_rev(P.LJ, g, i, l, k, SP.i1, xs, B.xe, wx, wy, wz, gx, gn);
+        } else {
+#pragma unroll
+            for (int d = 0; d < 3; d++) gn[d] += g2[d];
         }
     }
     // xe = xs + ct * ig * p'
@@ -360,10 +502,8 @@ __global__ void __launch_bounds__(kT, 2) k_adj_push_mixed(MixParams P) {
         dot += gn[d] * B.ct[d] * B.pp[d];
     }
     const float ig3 = B.ig * B.ig * B.ig;
-    float lP[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) lP[d] = lp[d] + B.ig * B.ct[d] * gn[d] - ig3 * dot * B.pp[d];
-    float lF[6];
+    for (int d = 0; d < 3; d++) lP[d] = lP[d] + B.ig * B.ct[d] * gn[d] - ig3 * dot * B.pp[d];
 #pragma unroll
     for (int d = 0; d < 3; d++) lF[d] = B.t * lP[d];
     const float *b = B.b, *sv = B.s, *up = B.up, *u = B.u;
@@ -379,8 +519,9 @@ __global__ void __launch_bounds__(kT, 2) k_adj_push_mixed(MixParams P) {
         ls[d] = (lP[d] + b[d] * bl + bxl[d]) * inv;
         lb[d] = (bs * lP[d] + bl * sv[d] + lxs[d] - 2.f * lu_ * b[d]) * inv;
     }
-    float lu[3] = {ls[0] + (b[1] * ls[2] - b[2] * ls[1]), ls[1] + (b[2] * ls[0] - b[0] * ls[2]),
-                   ls[2] + (b[0] * ls[1] - b[1] * ls[0])};
+    lu[0] = ls[0] + (b[1] * ls[2] - b[2] * ls[1]);
+    lu[1] = ls[1] + (b[2] * ls[0] - b[0] * ls[2]);
+    lu[2] = ls[2] + (b[0] * ls[1] - b[1] * ls[0]);
     lb[0] += ls[1] * u[2] - ls[2] * u[1];
     lb[1] += ls[2] * u[0] - ls[0] * u[2];
     lb[2] += ls[0] * u[1] - ls[1] * u[0];
@@ -396,100 +537,203 @@ __global__ void __launch_bounds__(kT, 2) k_adj_push_mixed(MixParams P) {
         lu[d] += cps * u[d];
         lF[d] += B.t * lu[d];
     }
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        Lm[d][j] = gx[d];
-        Lm[3 + d][j] = lu[d];
-    }
-#pragma unroll
-    for (int c = 0; c < 6; c++) P.LF[c][idx] = lF[c];
 }
 
-// ---- adjoint, second pass: interpolation transpose
-__global__ void __launch_bounds__(kT) k_adj_interp_mixed(MixParams P) {
-    __shared__ int sHi[6 * kBoxNodes];
-    __shared__ int sRed[6 * (kT / 32)];
-    __shared__ unsigned sMax[kT / 32], sMaxOut;
-    __shared__ NodeBox sBox;
+// One component of the interpolation's transpose: gi += lam * dF/dx (V: the
+// particle's cell in the component's array, strides dX, dY), add(x, y, z, lam
+// times the x and y weights, lower and upper z weight)
+template <int C, class Add>
+__device__ __forceinline__ void reverse_component_m(const float *V, int dX, int dY, const float xs[3], float lam,
+                                                    float gi[3], Add add) {
+    MTaps T;
+    taps_mixed(xs, T);
+    int t[3];
+    float w[3];
+    comp_taps_m(T, C, t, w);
+    const int tx = t[0] - 2, ty = t[1] - 2, tz = t[2] - 2;
+    const float wx = w[0], wy = w[1], wz = w[2], vx = 1.f - wx, vy = 1.f - wy, vz = 1.f - wz;
+    V += tx * dX + ty * dY + tz;
+    float yl[2], yd[2], yz[2];
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        const float v0 = V[a * dX], v1 = V[a * dX + 1], v2 = V[a * dX + dY], v3 = V[a * dX + dY + 1];
+        const float z0 = wz * v0 + vz * v1, z1 = wz * v2 + vz * v3;
+        yl[a] = wy * z0 + vy * z1;
+        yd[a] = z1 - z0;
+        yz[a] = wy * (v1 - v0) + vy * (v3 - v2);
+    }
+    gi[0] += lam * (yl[1] - yl[0]);
+    gi[1] += lam * (wx * yd[0] + vx * yd[1]);
+    gi[2] += lam * (wx * yz[0] + vx * yz[1]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) add(tx + (q >> 1), ty + (q & 1), tz, lam * ((q >> 1 ? vx : wx) * (q & 1 ? vy : wy)), wz, vz);
+}
+
+// a particle outside its chunk's window: everything through global memory
+__device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j) {
     const Grid &g = P.g;
-    int64_t idx = spread_index(threadIdx.x);
-    const bool valid = idx < P.off[P.nsp];
-    int s = 0, i = 0, l = 0, k = 0;
-    int64_t j = 0;
-    float xs[3] = {0.f, 0.f, 0.f};
-    if (valid) {
-        s = species_of(P.off, P.nsp, idx);
-        const MixSp &S = P.sp[s];
-        j = idx - P.off[s];
-        xs[0] = S.v[0][j]; xs[1] = S.v[1][j]; xs[2] = S.v[2][j];
-        g.cell_ijk(S.cell[j], i, l, k);
-    }
-    float lam6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    float amax = 0.f;
-    if (valid) {
+    const MixSp &S = P.sp[s];
+    float *const *Lm = P.lam[s];
+    const MixConst K = mix_const(g, S);
+    float xs[3] = {S.v[0][j], S.v[1][j], S.v[2][j]}, p[3] = {S.v[3][j], S.v[4][j], S.v[5][j]};
+    float gn[3] = {Lm[0][j], Lm[1][j], Lm[2][j]}, lP[3] = {Lm[3][j], Lm[4][j], Lm[5][j]};
+    int c3[3];
+    g.cell_ijk(S.cell[j], c3[0], c3[1], c3[2]);
+    const size_t n = g.node(c3[0], c3[1], c3[2]);
+    FieldViewM<false> V;
 #pragma unroll
-        for (int c = 0; c < 6; c++) {
-            lam6[c] = P.LF[c][idx];
-            amax = fmaxf(amax, fabsf(lam6[c]));
-        }
+    for (int c = 0; c < 3; c++) { V.base[c] = P.E[c] + n; V.base[3 + c] = P.H[c] + n; }
+    V.dx = g.NY * g.pz; V.dy = g.pz;
+    float gx[3], lu[3], lF[6], gi[3] = {0.f, 0.f, 0.f};
+    reverse_particle_m(K, V, P.LJ[0] + n, P.LJ[1] + n, P.LJ[2] + n, V.dx, V.dy, xs, p, gn, lP, gx, lu, lF);
+    auto put = [&](double *L) {
+        return [=](int a, int b, int c, float v, float wz, float vz) {
+            double *r = L + a * V.dx + b * V.dy + c;
+            atomicAdd(r, (double)(v * wz));
+            atomicAdd(r + 1, (double)(v * vz));
+        };
+    };
+    reverse_component_m<0>(V.base[0], V.dx, V.dy, xs, lF[0], gi, put(P.LE[0] + n));
+    reverse_component_m<1>(V.base[1], V.dx, V.dy, xs, lF[1], gi, put(P.LE[1] + n));
+    reverse_component_m<2>(V.base[2], V.dx, V.dy, xs, lF[2], gi, put(P.LE[2] + n));
+    reverse_component_m<3>(V.base[3], V.dx, V.dy, xs, lF[3], gi, put(P.LH[0] + n));
+    reverse_component_m<4>(V.base[4], V.dx, V.dy, xs, lF[4], gi, put(P.LH[1] + n));
+    reverse_component_m<5>(V.base[5], V.dx, V.dy, xs, lF[5], gi, put(P.LH[2] + n));
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        Lm[d][j] = gx[d] + gi[d];
+        Lm[3 + d][j] = lu[d];
     }
-    const NodeBox box = block_node_box(i, l, k, valid, sRed, &sBox);
-    const float bmax = block_max_abs(amax, sMax, &sMaxOut);
-    if (bmax == 0.f) return;  // no adjoint reaches the particles of this block
-    const int E = box_exponent(bmax);
-    const float inv_q = __uint_as_float((unsigned)(22 - E + 127) << 23);
-    for (int e = threadIdx.x; e < 6 * box.nodes; e += blockDim.x) sHi[e] = 0;
+}
+
+// ---- adjoint of the particle part of one step (k_adj_particles_plain in FP32):
+// one CTA per chunk with its window of E, H and lambda_J staged; lambda_E and
+// lambda_H are summed there in 64-bit words in units of 2^-30 of the largest
+// |lambda of a field value| (at most 4 times the block's) and added to the FP64
+// global arrays once.  A contribution fits an int32, so its add touches the high
+// word only when the low one carries or borrows.
+// Bound: instruction issue and the shared-memory pipe.  128x32x32 cells: 1.90 ->
+// 1.37 ms per reverse step (two CTAs per SM at 128 registers: 1.46; before: two
+// kernels that gathered from global memory).
+__global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_constant__ MixParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ AdjWindow sWin;
+    __shared__ int sRed[15 * kW], sFar;
+    __shared__ unsigned sMax[2];
+    __shared__ MixConst sK;
+    const Grid &g = P.g;
+    const AdjChunk ch = P.chunks[blockIdx.x];
+    const int s = ch.species, count = ch.count;
+    const MixSp &S = P.sp[s];
+    float *const *Lm = P.lam[s];
+    const NextMix<12> next(smem_raw + (size_t)kAdjWindowMix * 84);
+    unsigned short *sList = (unsigned short *)(smem_raw + (size_t)kAdjWindowMix * 84 + NextMix<12>::bytes);
+    // lanes as in k_adj_particles_plain
+    const int lane = threadIdx.x & 31, mine = (lane >> 3) * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
+    if (mine < count) next.start(S, Lm, ch.first + mine);
+    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kAdjWindowMix, sRed, &sWin);
+    const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
+    float *sF = (float *)smem_raw, *sL = sF + 6 * nn;
+    unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
+    const float *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
+    stage_window_m<6>(g, w, src, sF);
+    stage_window_m<3>(g, w, P.LJ, sL);
+    for (int e = threadIdx.x; e < 12 * nn; e += blockDim.x) sLo[e] = 0u;
+    if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = 0u; sK = mix_const(g, S); }
     __syncthreads();
-    if (valid) {
-        MTaps T;
-        taps_mixed(xs, T);
-        const size_t dX = (size_t)g.NY * g.pz, dY = g.pz, dZ = 1;
-        float gx[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            int t[3];
-            float w[3];
-            const float lam = lam6[c];
-            if (lam == 0.f) continue;
-            comp_taps_m(T, c, t, w);
-            size_t n = tap_node(g, i, l, k, t);
-            const float *Arr = c < 3 ? P.E[c] : P.H[c - 3];
-            double *LA = c < 3 ? P.LE[c] : P.LH[c - 3];
-            const int b0 = box.nodes ? c * box.nodes + box_index(box, i + t[0] - 2, l + t[1] - 2, k + t[2] - 2) : 0;
-            const float W0[2] = {w[0], 1.f - w[0]}, W1[2] = {w[1], 1.f - w[1]}, W2[2] = {w[2], 1.f - w[2]};
-            float gr[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-            for (int a = 0; a < 2; a++)
-#pragma unroll
-                for (int bb = 0; bb < 2; bb++)
-#pragma unroll
-                    for (int cc = 0; cc < 2; cc++) {
-                        size_t m = n + a * dX + bb * dY + cc * dZ;
-                        float v = Arr[m];
-                        float add = lam * (W0[a] * W1[bb] * W2[cc]);
-                        if (box.nodes) {
-                            int hi = __float2int_rn(add * inv_q);
-                            if (hi) atomicAdd(&sHi[b0 + (a * box.by + bb) * box.bz + cc], hi);
-                        } else {
-                            atomicAdd(&LA[m], (double)add);
-                        }
-                        gr[0] += (a ? 1.f : -1.f) * W1[bb] * W2[cc] * v;
-                        gr[1] += (bb ? 1.f : -1.f) * W0[a] * W2[cc] * v;
-                        gr[2] += (cc ? 1.f : -1.f) * W0[a] * W1[bb] * v;
-                    }
-            gx[0] += lam * gr[0];
-            gx[1] += lam * gr[1];
-            gx[2] += lam * gr[2];
-        }
-        float *const *Lm = P.lam[s];
-#pragma unroll
-        for (int d = 0; d < 3; d++) Lm[d][j] += gx[d];
-    }
-    if (box.nodes) {
-        __syncthreads();
+    const MixConst &K = sK;
+    int E = -1000;  // contributions below 2^E = 2^30 quanta; none yet
+    float limit = 0.f, inv_q = 0.f;
+    auto flush = [&](bool again) {
+        if (E == -1000) return;
+        const double q = pow2_d(E - 30);
         double *const dst[6] = {P.LE[0], P.LE[1], P.LE[2], P.LH[0], P.LH[1], P.LH[2]};
-        flush_node_box(box, sHi, nullptr, pow2_d(E - 22), g, dst);
+        for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
+            const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
+            if (v == 0) continue;
+            if (again) sHi[e] = sLo[e] = 0u;
+            const int comp = e / nn, r = e - comp * nn;
+            const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
+            atomicAdd(&dst[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * q);
+        }
+    };
+    for (int base = 0, it = 0; base < count; base += blockDim.x, it++) {
+        const int jc = base + mine;
+        const int64_t j = ch.first + jc;
+        int cell = -1;
+        float xs[3], p[3], gn[3], lP[3];
+        cp_async_wait_all();
+        if (jc < count) {
+            cell = next.cell();
+            next.take3(0, xs);
+            next.take3(3, p);
+            next.take3(6, gn);
+            next.take3(9, lP);
+        }
+        __syncwarp();
+        if (jc + (int)blockDim.x < count) next.start(S, Lm, j + blockDim.x);
+        int c3[3] = {w.i0, w.l0, w.k0};
+        bool near = cell >= 0;
+        if (near) {
+            g.cell_ijk(cell, c3[0], c3[1], c3[2]);
+            if (!w.holds(c3[0], c3[1], c3[2])) {
+                near = false;
+                sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
+            }
+        }
+        float gx[3], lu[3], lF[6], gi[3] = {0.f, 0.f, 0.f}, amax = 0.f;
+        const int n0 = w.node(c3[0], c3[1], c3[2]);
+        if (near) {
+            FieldViewM<true> V;
+#pragma unroll
+            for (int c = 0; c < 6; c++) V.base[c] = sF + c * nn + n0;
+            V.dx = dX; V.dy = dY;
+            reverse_particle_m(K, V, sL + n0, sL + nn + n0, sL + 2 * nn + n0, dX, dY, xs, p, gn, lP, gx, lu, lF);
+#pragma unroll
+            for (int c = 0; c < 6; c++) amax = fmaxf(amax, fabsf(lF[c]));
+        }
+        // the block's largest |lambda_F| against the quantum in use
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+        if (lane == 0 && wm) atomicMax(&sMax[it & 1], wm);
+        __syncthreads();
+        const float bm = __uint_as_float(sMax[it & 1]);
+        if (threadIdx.x == 0) sMax[(it & 1) ^ 1] = 0u;
+        if (bm >= limit && bm > 0.f) {  // block-uniform
+            flush(true);
+            E = max(adj_exponent(bm), -90) + 2;
+            limit = __uint_as_float((unsigned)(E + 127) << 23);
+            inv_q = __uint_as_float((unsigned)(30 - E + 127) << 23);
+            __syncthreads();
+        }
+        if (near && amax > 0.f) {
+            auto put = [&](int c) {
+                unsigned *lo = sLo + c * nn + n0;
+                return [=](int a, int b, int k, float v, float wz, float vz) {
+                    unsigned *r = lo + a * dX + b * dY + k;
+                    const float vq = v * inv_q;
+                    shared_add64_small(r, r + 6 * nn, __float2int_rn(vq * wz));
+                    shared_add64_small(r + 1, r + 1 + 6 * nn, __float2int_rn(vq * vz));
+                };
+            };
+            const float *V = sF + n0;
+            reverse_component_m<0>(V, dX, dY, xs, lF[0], gi, put(0));
+            reverse_component_m<1>(V + nn, dX, dY, xs, lF[1], gi, put(1));
+            reverse_component_m<2>(V + 2 * nn, dX, dY, xs, lF[2], gi, put(2));
+            reverse_component_m<3>(V + 3 * nn, dX, dY, xs, lF[3], gi, put(3));
+            reverse_component_m<4>(V + 4 * nn, dX, dY, xs, lF[4], gi, put(4));
+            reverse_component_m<5>(V + 5 * nn, dX, dY, xs, lF[5], gi, put(5));
+        }
+        if (near) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                Lm[d][j] = gx[d] + gi[d];
+                Lm[3 + d][j] = lu[d];
+            }
+        }
     }
+    __syncthreads();
+    flush(false);
+    for (int e = threadIdx.x; e < sFar; e += blockDim.x) reverse_far_m(P, s, ch.first + sList[e]);
 }
 
 __global__ void k_h_half_m(Grid g, const float *__restrict__ Ex, const float *__restrict__ Ey,
@@ -533,22 +777,23 @@ __global__ void k_widen(const float *__restrict__ lp, const float *__restrict__ 
     out[5 * n + j] = c[j];
 }
 
-inline unsigned blocks_of(int64_t n) { return (unsigned)((n + kT - 1) / kT); }
-
 }  // namespace
 
-cudaError_t launch_flat_push_mixed(const MixParams &P, cudaStream_t s) {
-    int64_t n = P.off[P.nsp];
-    if (n > 0) k_flat_push_mixed<<<blocks_of(n), kT, 0, s>>>(P);
+cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, cudaStream_t s) {
+    if (nchunks <= 0) return cudaSuccess;
+    const size_t smem = (size_t)kFlatWindowMix * 48 + (size_t)kW * 7 * kQueueMix * sizeof(float) + NextMix<6>::bytes;
+    cudaError_t e = cudaFuncSetAttribute(k_flat_push_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_flat_push_mixed<<<nchunks, kT, smem, s>>>(P);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_particles_mixed(const MixParams &P, cudaStream_t s) {
-    int64_t n = P.off[P.nsp];
-    if (n <= 0) return cudaSuccess;
-    if (P.Fin[0]) k_adj_push_mixed<true><<<blocks_of(n), kT, 0, s>>>(P);
-    else k_adj_push_mixed<false><<<blocks_of(n), kT, 0, s>>>(P);
-    k_adj_interp_mixed<<<blocks_of(n), kT, 0, s>>>(P);
+cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStream_t s) {
+    if (nchunks <= 0) return cudaSuccess;
+    const size_t smem = (size_t)kAdjWindowMix * 84 + NextMix<12>::bytes + kAdjChunk * sizeof(unsigned short);
+    cudaError_t e = cudaFuncSetAttribute(k_adj_particles_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_adj_particles_mixed<<<nchunks, kT, smem, s>>>(P);
     return cudaGetLastError();
 }
 

@@ -136,6 +136,14 @@ __device__ __forceinline__ void shared_add64(unsigned long long *w, long long v)
     unsigned *p = (unsigned *)w;  // p[0] low word, p[1] high word
     shared_add64(p, p + 1, v);
 }
+// a 32-bit addend: the high word changes only when the low one carries (or, for
+// a negative addend, does not)
+__device__ __forceinline__ void shared_add64_small(unsigned *plo, unsigned *phi, int v) {
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd(plo, lo);
+    const unsigned hi = (unsigned)(v >> 31) + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(phi, hi);
+}
 __device__ __forceinline__ void fx_add(unsigned long long *a, double v, double inv_q) {
     long long iv = __double2ll_rn(v * inv_q);
     if (iv) shared_add64(a, iv);
