@@ -1363,15 +1363,28 @@ int check_adj_status(pic_handle *h, AdjState &A, const char *where) {
     return PIC_OK;
 }
 
-int adj_alloc(pic_handle *h, void **p, size_t bytes, const char *what) {
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 256);
-    if (e != cudaSuccess) {
-        char msg[200];
-        snprintf(msg, sizeof(msg), "differentiable run: cannot allocate %s (%.2f GB); use a larger ckpt_every or "
-                 "fewer particles", what, bytes / 1e9);
-        cudaGetLastError();
-        return set_err(h, PIC_ERR_NOMEM, msg);
+// a buffer of the run: the one kept for this use when its size suits, else a new one
+int adj_alloc(pic_handle *h, AdjSlot slot, void **p, size_t bytes, const char *what) {
+    AdjState::Buf &b = h->adj->pool[slot];
+    if (bytes == 0) bytes = 256;
+    if (b.p && (b.cap < bytes || b.cap > 2 * bytes + (1 << 20))) {
+        cudaFree(b.p);
+        b.p = nullptr;
     }
+    if (!b.p) {
+        cudaError_t e = dev_alloc(h, &b.p, bytes);
+        if (e != cudaSuccess) {
+            b.p = nullptr;
+            char msg[200];
+            snprintf(msg, sizeof(msg), "differentiable run: cannot allocate %s (%.2f GB); use a larger ckpt_every or "
+                     "fewer particles", what, bytes / 1e9);
+            cudaGetLastError();
+            return set_err(h, PIC_ERR_NOMEM, msg);
+        }
+        b.cap = bytes;
+    }
+    b.used = 1;
+    *p = b.p;
     return PIC_OK;
 }
 
@@ -1382,14 +1395,24 @@ namespace pic_host {
 void adj_free(pic_handle *h) {
     if (!h || !h->adj) return;
     AdjState *A = h->adj;
-    void *bufs[] = {A->cur, A->ckp, A->ckf, A->segp, A->segf, A->subp, A->subf, A->lamp, A->lamf, A->rf, A->ha,
-                    A->hist, A->st, A->red, A->branch, A->chunks};
-    for (void *b : bufs)
-        if (b) cudaFree(b);
+    for (AdjState::Buf &b : A->pool)
+        if (b.p) cudaFree(b.p);
     if (A->e0) cudaEventDestroy(A->e0);
     if (A->e1) cudaEventDestroy(A->e1);
     delete A;
     h->adj = nullptr;
+}
+
+bool adj_reclaim(pic_handle *h) {
+    if (!h || !h->adj) return false;
+    bool any = false;
+    for (AdjState::Buf &b : h->adj->pool)
+        if (b.p && !b.used) {
+            cudaFree(b.p);
+            b.p = nullptr;
+            any = true;
+        }
+    return any;
 }
 
 }  // namespace pic_host
@@ -1663,8 +1686,16 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     int rc = set_device(h);
     if (rc) return rc;
     if ((rc = need_particles(h))) return rc;
-    adj_free(h);
+    // the last run's buffers stay for this one
     AdjState *Ap = new AdjState();
+    if (h->adj) {
+        for (int q = 0; q < kAdjSlots; q++) {
+            Ap->pool[q] = h->adj->pool[q];
+            Ap->pool[q].used = 0;
+            h->adj->pool[q].p = nullptr;
+        }
+        adj_free(h);
+    }
     h->adj = Ap;
     AdjState &A = *Ap;
     A.mixed = h->mixed;
@@ -1714,7 +1745,7 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
         A.branch_mode = 2;
         A.branch_src = S->branch;
     } else if (h->branch_record && !h->mixed) {
-        if ((rc = adj_alloc(h, (void **)&A.branch,
+        if ((rc = adj_alloc(h, kAdjBranch, (void **)&A.branch,
                             (size_t)steps * (size_t)total_particles(A) * sizeof(unsigned long long),
                             "the branch record")))
             return rc;
@@ -1722,24 +1753,28 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     }
     CK(cudaEventCreate(&A.e0), "event");
     CK(cudaEventCreate(&A.e1), "event");
-    if ((rc = adj_alloc(h, (void **)&A.cur, A.pbytes, "the particle state"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.ckp, A.pbytes * A.nseg, "the particle checkpoints"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.ckf, fbytes * 6 * A.nseg, "the field checkpoints"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.hist, sizeof(double) * 3 * steps, "the history"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.st, sizeof(AdjStatus), "the status"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.red, sizeof(double) * 8, "the reduction scratch"))) return rc;
-    if ((rc = adj_alloc(h, (void **)&A.chunks, sizeof(AdjChunk) * chunks.size(), "the chunk table"))) return rc;
+    if ((rc = adj_alloc(h, kAdjCur, (void **)&A.cur, A.pbytes, "the particle state"))) return rc;
+    if ((rc = adj_alloc(h, kAdjCkp, (void **)&A.ckp, A.pbytes * A.nseg, "the particle checkpoints"))) return rc;
+    if ((rc = adj_alloc(h, kAdjCkf, (void **)&A.ckf, fbytes * 6 * A.nseg, "the field checkpoints"))) return rc;
+    if ((rc = adj_alloc(h, kAdjHist, (void **)&A.hist, sizeof(double) * 3 * steps, "the history"))) return rc;
+    if ((rc = adj_alloc(h, kAdjSt, (void **)&A.st, sizeof(AdjStatus), "the status"))) return rc;
+    if ((rc = adj_alloc(h, kAdjRed, (void **)&A.red, sizeof(double) * 8, "the reduction scratch"))) return rc;
+    if ((rc = adj_alloc(h, kAdjChunks, (void **)&A.chunks, sizeof(AdjChunk) * chunks.size(), "the chunk table"))) return rc;
     CK(cudaMemcpyAsync(A.chunks, chunks.data(), sizeof(AdjChunk) * chunks.size(), cudaMemcpyHostToDevice, h->stream),
        "chunk table");
     CK(cudaStreamSynchronize(h->stream), "sync");
+    // kept buffers that this run has no use for
+    if (!A.branch && A.pool[kAdjBranch].p) { cudaFree(A.pool[kAdjBranch].p); A.pool[kAdjBranch].p = nullptr; }
+    if (A.K2 == A.K)
+        for (int q : {kAdjSubp, kAdjSubf})
+            if (A.pool[q].p) { cudaFree(A.pool[q].p); A.pool[q].p = nullptr; }
     CK(cudaMemsetAsync(A.hist, 0, sizeof(double) * 3 * steps, h->stream), "zero history");
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     // bins -> flat order
     int *cell[kMaxSpecies];
     void *v[kMaxSpecies][6];
     adj_state_view(A, A.cur, cell, v);
-    int64_t *d0 = nullptr;
-    CK(cudaMalloc(&d0, (g.ntiles + 1) * sizeof(int64_t)), "alloc");
+    int64_t *d0 = (int64_t *)h->dense;  // I/O staging, free between calls: a double per node, more than one per tile
     for (int s = 0; s < A.nsp; s++) {
         std::vector<int64_t> start(g.ntiles + 1);
         int64_t acc = 0;
@@ -1757,7 +1792,6 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
         CK(cudaGetLastError(), "flat gather");
         CK(cudaStreamSynchronize(h->stream), "sync");
     }
-    cudaFree(d0);
     rc = forward_run(h, A);
     if (rc) return rc;
     if ((rc = check_adj_status(h, A, "pic_forward"))) return rc;
@@ -1867,19 +1901,19 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
     const size_t fbytes = N * (h->mixed ? sizeof(float) : sizeof(double));
     int64_t np = total_particles(A);
     if (!A.segp) {
-        if ((rc = adj_alloc(h, (void **)&A.segp, A.pbytes * (size_t)(A.K2 + 1), "the segment states"))) return rc;
-        if ((rc = adj_alloc(h, (void **)&A.segf, fbytes * 6 * (size_t)(A.K2 + 1), "the segment fields"))) return rc;
+        if ((rc = adj_alloc(h, kAdjSegp, (void **)&A.segp, A.pbytes * (size_t)(A.K2 + 1), "the segment states"))) return rc;
+        if ((rc = adj_alloc(h, kAdjSegf, (void **)&A.segf, fbytes * 6 * (size_t)(A.K2 + 1), "the segment fields"))) return rc;
         if (A.K2 < A.K) {
             const size_t nsub = (size_t)(A.K + A.K2 - 1) / A.K2;
-            if ((rc = adj_alloc(h, (void **)&A.subp, A.pbytes * nsub, "the sub-checkpoint states"))) return rc;
-            if ((rc = adj_alloc(h, (void **)&A.subf, fbytes * 6 * nsub, "the sub-checkpoint fields"))) return rc;
+            if ((rc = adj_alloc(h, kAdjSubp, (void **)&A.subp, A.pbytes * nsub, "the sub-checkpoint states"))) return rc;
+            if ((rc = adj_alloc(h, kAdjSubf, (void **)&A.subf, fbytes * 6 * nsub, "the sub-checkpoint fields"))) return rc;
         }
         A.lamp_bytes = (size_t)np * 6 * A.elem;
-        if ((rc = adj_alloc(h, (void **)&A.lamp, A.lamp_bytes, "the particle adjoints"))) return rc;
-        if ((rc = adj_alloc(h, (void **)&A.lamf, N * sizeof(double) * 12, "the field adjoints"))) return rc;
-        if ((rc = adj_alloc(h, (void **)&A.rf, N * sizeof(double) * PIC_FIELD_COUNT, "the recompute fields")))
+        if ((rc = adj_alloc(h, kAdjLamp, (void **)&A.lamp, A.lamp_bytes, "the particle adjoints"))) return rc;
+        if ((rc = adj_alloc(h, kAdjLamf, (void **)&A.lamf, N * sizeof(double) * 12, "the field adjoints"))) return rc;
+        if ((rc = adj_alloc(h, kAdjRf, (void **)&A.rf, N * sizeof(double) * PIC_FIELD_COUNT, "the recompute fields")))
             return rc;
-        if ((rc = adj_alloc(h, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
+        if ((rc = adj_alloc(h, kAdjHa, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
     }
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     rc = backward_run(h, A, *loss);
@@ -1898,6 +1932,13 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
     double out4[4] = {0.0, 0.0, 0.0, 0.0};
     double *lp = nullptr;  // FP64 copies of lambda_p (and p0) for the mixed form
     if (n > 0) {
+        // their place, and the interleaved gradient's: the segment's states,
+        // which the sweep is done with, where they are large enough
+        ScratchGuard guard(h);
+        const size_t lp_bytes = h->mixed ? align256((size_t)n * 6 * sizeof(double)) : 0;
+        const size_t need = lp_bytes + (size_t)n * 3 * sizeof(double);
+        char *stage = A.segp;
+        if (A.pool[kAdjSegp].cap < need) CK(guard.alloc(&stage, need), "alloc");
         CK(cudaMemsetAsync(A.red, 0, 4 * sizeof(double), h->stream), "zero");
         const double *l3[3], *p3[3];
         if (!h->mixed) {
@@ -1906,7 +1947,7 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
                 p3[a] = (const double *)v0[s][3 + a];
             }
         } else {
-            CK(cudaMalloc(&lp, (size_t)n * 6 * sizeof(double)), "alloc");
+            lp = (double *)stage;
             adj_widen_mixed((const float *)A.lamp + o + 3 * (size_t)n, (const float *const *)&v0[s][3], n, lp,
                             h->stream);
             for (int a = 0; a < 3; a++) {
@@ -1918,16 +1959,12 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
                                                  loss->drift[1], loss->drift[2], A.red);
         CK(cudaMemcpyAsync(out4, A.red, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
         if (grads->d_p0 && grads->n >= n) {
-            double *tmp = nullptr;
-            CK(cudaMalloc(&tmp, (size_t)n * 3 * sizeof(double)), "alloc");
+            double *tmp = (double *)(stage + lp_bytes);
             k_interleave<<<blocks_of(n), kT, 0, h->stream>>>(n, l3[0], l3[1], l3[2], tmp);
             CK(cudaMemcpyAsync(grads->d_p0, tmp, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream),
                "D2H");
-            CK(cudaStreamSynchronize(h->stream), "sync");
-            cudaFree(tmp);
         }
         CK(cudaStreamSynchronize(h->stream), "sync");
-        if (lp) cudaFree(lp);
     }
     bool fits = grads->n >= n;
     grads->n = n;

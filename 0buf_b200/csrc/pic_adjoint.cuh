@@ -26,11 +26,25 @@ struct AdjChunk {
     int count, species;
 };
 
-// Buffers live until pic_adjoint_free / the next pic_forward / pic_destroy.
+// the device buffers of the run, by use
+enum AdjSlot {
+    kAdjBranch, kAdjCur, kAdjCkp, kAdjCkf, kAdjHist, kAdjSt, kAdjRed, kAdjChunks, kAdjSegp, kAdjSegf, kAdjSubp, kAdjSubf,
+    kAdjLamp, kAdjLamf, kAdjRf, kAdjHa, kAdjSlots
+};
+
+// Buffers live until pic_adjoint_free / pic_destroy; the next pic_forward takes
+// over those of about its own size (an optimiser's evaluations then allocate
+// nothing) and frees the others.  Buffers that no run uses at the moment are
+// given back when a device allocation of the handle fails (adj_reclaim).
 // A "particle state" is the whole population in the fixed order of the run:
 // per species the packed cells then 6 value arrays (plain: FP64 global
 // positions and momenta; mixed: FP32 in-cell offsets and momenta).
 struct AdjState {
+    struct Buf {
+        void *p;
+        size_t cap;
+        int used;  // by the current run
+    } pool[kAdjSlots];
     int mixed;
     size_t elem;       // bytes per particle value (8 plain, 4 mixed)
     int nsp;

@@ -41,8 +41,12 @@ int cuda_err(pic_handle *h, cudaError_t e, const char *where) {
 }
 
 cudaError_t dev_alloc(pic_handle *h, void **p, size_t bytes) {
-    (void)h;
-    return cudaMalloc(p, bytes > 0 ? bytes : 16);
+    cudaError_t e = cudaMalloc(p, bytes > 0 ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation && adj_reclaim(h)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes > 0 ? bytes : 16);
+    }
+    return e;
 }
 
 void dev_free(pic_handle *h, void *p) {
@@ -81,10 +85,14 @@ StepParams make_params(pic_handle *h) {
     return p;
 }
 
-void free_species(pic_handle *h, int s) {
+// empties a species; its arrays stay for alloc_species unless `give_back`
+void free_species(pic_handle *h, int s, bool give_back) {
     SpeciesView &v = h->sp[s].v;
-    dev_free(h, h->sp[s].arena);
-    h->sp[s].arena = nullptr;
+    if (give_back) {
+        dev_free(h, h->sp[s].arena);
+        h->sp[s].arena = nullptr;
+        h->sp[s].arena_bytes = 0;
+    }
     double q_m = v.q_m, m = v.m;
     memset(&v, 0, sizeof(v));
     v.q_m = q_m;
@@ -120,9 +128,12 @@ int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> 
     return PIC_OK;
 }
 
-// a species' arrays for `slots` slots, carved from one allocation (a driver
-// call per array costs a rebin of a small run more than its copies)
-cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **arena) {
+// A species' arrays for `slots` slots, carved from one allocation (a driver
+// call per array costs a rebin of a small run more than its copies).  *arena of
+// `have` bytes is used again when it is large enough and at most twice what is
+// needed (a program that loads its species anew for every run then allocates
+// nothing), and is freed otherwise.
+cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **arena, size_t *have) {
     const size_t n = (size_t)slots, el = h->mixed ? sizeof(float) : sizeof(double);
     size_t o = 0;
     auto room = [&](size_t bytes) { size_t a = o; o += (bytes + 255) / 256 * 256; return a; };
@@ -131,8 +142,16 @@ cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **a
     for (size_t &a : val) a = room(n * el);
     const size_t st = room(((size_t)h->g.ntiles + 1) * sizeof(int)), ct = room((size_t)h->g.ntiles * sizeof(int));
     const size_t sp = room(n / (kHoleSpill / 2) * sizeof(int));
-    cudaError_t e = dev_alloc(h, arena, o);
-    if (e != cudaSuccess) return e;
+    if (*arena && (*have < o || *have > 2 * o + (1 << 20))) {
+        dev_free(h, *arena);
+        *arena = nullptr;
+    }
+    if (!*arena) {
+        *have = 0;
+        cudaError_t e = dev_alloc(h, arena, o);
+        if (e != cudaSuccess) { *arena = nullptr; return e; }
+        *have = o;
+    }
     char *b = (char *)*arena;
     v.cell = (int *)(b + cell);
     v.tile_start = (int *)(b + st);
@@ -153,10 +172,10 @@ int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
     std::vector<int> start;
     int rc = layout_bins(h, counts, start);
     if (rc) return rc;
-    free_species(h, s);
+    free_species(h, s, false);
     SpeciesView &v = h->sp[s].v;
     const int64_t acc = start[g.ntiles];
-    CK(carve_species(h, acc, v, &h->sp[s].arena), "alloc particles");
+    CK(carve_species(h, acc, v, &h->sp[s].arena, &h->sp[s].arena_bytes), "alloc particles");
     CK(cudaMemcpyAsync(v.tile_start, start.data(), (g.ntiles + 1) * sizeof(int), cudaMemcpyHostToDevice, h->stream),
        "upload tile_start");
     CK(cudaMemsetAsync(v.cell, 0xff, (size_t)acc * sizeof(int), h->stream), "clear cells");
@@ -194,13 +213,6 @@ int push_slices(pic_handle *h) {
 
 size_t split_ints(const pic_handle *h) { return (size_t)h->cfg.nspecies * h->g.ntiles * kHoleMax; }
 
-int ensure_split(pic_handle *h) {
-    if (h->split_buf) return PIC_OK;
-    const size_t n = split_ints(h) + (size_t)(h->cfg.nspecies + 1) * h->g.ntiles;
-    CK(cudaMalloc(&h->split_buf, n * sizeof(int)), "alloc hole lists");
-    return PIC_OK;
-}
-
 int ensure_outbox(pic_handle *h) {
     if (h->outbox_pinned) return PIC_OK;  // leftovers of an overflowing insert still live in it
     int64_t total = 0;
@@ -212,10 +224,14 @@ int ensure_outbox(pic_handle *h) {
     const int slices = push_slices(h);
     if (h->mixed && slices > 1) want += (int64_t)h->g.ntiles * slices * (kPushThreads / 32) * kOutboxChunk;
     if (want > 0x7fffffffLL) want = 0x7fffffffLL;
-    if (h->outbox && (int64_t)h->out_cap >= want) return PIC_OK;
+    if (h->outbox && (int64_t)h->out_cap >= want && (slices == 1 || h->split_buf)) return PIC_OK;
     if (h->outbox) cudaFree(h->outbox);
     h->outbox = nullptr;
-    CK(cudaMalloc(&h->outbox, (size_t)want * h->out_elem), "alloc outbox");
+    h->split_buf = nullptr;
+    const size_t ob = ((size_t)want * h->out_elem + 255) / 256 * 256;
+    const size_t sb = slices > 1 ? (split_ints(h) + (size_t)(h->cfg.nspecies + 1) * h->g.ntiles) * sizeof(int) : 0;
+    CK(dev_alloc(h, &h->outbox, ob + sb), "alloc outbox");
+    if (sb) h->split_buf = (int *)((char *)h->outbox + ob);
     h->out_cap = (unsigned)want;
     return PIC_OK;
 }
@@ -225,9 +241,7 @@ using ScatterFn = std::function<cudaError_t(const SpeciesView &, int *)>;
 
 int build_bins_with(pic_handle *h, int s, int64_t n, int *cell, const ScatterFn &scatter, int64_t *inserted) {
     const Grid &g = h->g;
-    ScratchGuard guard(h);
-    int *tc = nullptr;
-    CK(guard.alloc(&tc, (size_t)g.ntiles), "alloc tile counts");
+    int *tc = h->dcounts;  // scratch between calls: an int per cell, more than one per tile
     CK(cudaMemsetAsync(tc, 0, g.ntiles * sizeof(int), h->stream), "memset");
     CK(tile_histogram(g, n, cell, tc, h->stream), "tile histogram");
     std::vector<int> counts(g.ntiles);
@@ -295,9 +309,7 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     const Grid &g = h->g;
     auto &sp = h->sp[s];
     StepParams p = make_params(h);
-    ScratchGuard guard(h);
-    int *extra = nullptr;
-    CK(guard.alloc(&extra, (size_t)g.ntiles), "rebin counts");
+    int *extra = h->dcounts;  // scratch between calls: an int per cell, more than one per tile
     CK(cudaMemsetAsync(extra, 0, g.ntiles * sizeof(int), h->stream), "memset");
     CK(outbox_histogram(p, s, n_out, extra, h->stream), "outbox histogram");
     std::vector<int> counts(g.ntiles), left(g.ntiles);
@@ -311,7 +323,8 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     if (rc) return rc;
     SpeciesView v = sp.v;
     void *arena = nullptr;
-    const cudaError_t e = carve_species(h, start[g.ntiles], v, &arena);
+    size_t bytes = 0;
+    const cudaError_t e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         return rebin_flat(h, s, n_out);
@@ -333,6 +346,7 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     }
     dev_free(h, sp.arena);
     sp.arena = arena;
+    sp.arena_bytes = bytes;
     sp.v = v;
     sp.cap_total = start[g.ntiles];
     sp.h_start = std::move(start);
@@ -488,9 +502,8 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
     }
     StepParams p = make_params(h);
     p.b_half = b_half_in_push;
-    p.slices = push_slices(h);
+    p.slices = h->split_buf ? push_slices(h) : 1;
     if (p.slices > 1) {
-        if ((rc = ensure_split(h))) return rc;
         const size_t nc = (size_t)h->cfg.nspecies * h->g.ntiles;
         p.holes = h->split_buf;
         p.hole_count = (unsigned *)(h->split_buf + split_ints(h));
@@ -685,7 +698,7 @@ int pic_destroy(pic_handle *h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     adj_free(h);
-    for (int s = 0; s < h->cfg.nspecies; s++) free_species(h, s);
+    for (int s = 0; s < h->cfg.nspecies; s++) free_species(h, s, true);
     for (int fi = 0; fi < PIC_FIELD_COUNT; fi++)
         if (h->f[fi]) cudaFree(h->f[fi]);
     if (h->dense) cudaFree(h->dense);
@@ -696,7 +709,6 @@ int pic_destroy(pic_handle *h) {
     if (h->hred) cudaFreeHost(h->hred);
     if (h->dcounts) cudaFree(h->dcounts);
     if (h->lb_buf) cudaFree(h->lb_buf);
-    if (h->split_buf) cudaFree(h->split_buf);
     release_load_scratch(h);
 
     double *diag[3] = {h->rho, h->gauss, h->gauss0};

@@ -24,6 +24,7 @@ struct pic_handle {
     struct Sp {
         pic::SpeciesView v;
         void *arena;  // the one allocation that holds v's arrays
+        size_t arena_bytes;
         int64_t cap_total;
         int loaded;
         std::vector<int> h_start;
@@ -75,7 +76,8 @@ struct pic_handle {
     void *load_buf;
     size_t load_bytes;
     // pushes with several CTAs per tile (StepParams::slices): hole lists and,
-    // after them, hole counts and tickets; allocated at the first such push
+    // after them, hole counts and tickets; the tail of the outbox's allocation
+    // (null: it has none)
     int *split_buf;
     int sms;  // SMs of the device
 };
@@ -126,6 +128,8 @@ int build_bins_f(pic_handle *h, int s, int64_t n, int *cell, const float *ox, co
 int tile_counts(pic_handle *h, int s, std::vector<int> &counts);
 // the differentiable run's buffers (pic_adjoint.cu)
 void adj_free(pic_handle *h);
+// frees the differentiable run's buffers that no run uses; false if there were none
+bool adj_reclaim(pic_handle *h);
 
 }  // namespace pic_host
 

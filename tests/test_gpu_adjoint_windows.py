@@ -52,3 +52,37 @@ def test_gradient_does_not_depend_on_the_tiling(pkg, cells, ppc, vth, precision)
     assert np.linalg.norm(got[0][0]) > 0
     assert rel(got[1][0], got[0][0]) < tol
     assert rel(got[1][1], got[0][1]) < tol and abs(got[1][2] - got[0][2]) < tol * abs(got[0][2])
+
+
+def test_kept_buffers_serve_runs_of_other_shapes(pkg):
+    """One handle through runs of growing and shrinking length, one and two
+    checkpoint levels, with and without a record, other particle numbers and a
+    release in between: each gives the gradient of a fresh handle (1e-9, the
+    order of FP64 sums)."""
+    loss = dict(field="Ex", window=3, species=2, drift=(0.2, 0.0, 0.0), vth=0.002)
+
+    def start(sim, ppc):
+        for s, sp in enumerate(pkg.configs.SPECIES_BEAM_PLASMA):
+            sim.init_species(s, ppc, drift=sp["drift"], vth=max(sp["vth"], 0.02), seed=3 + s)
+        for f in ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz"):
+            sim.set_field(f, np.zeros(int(np.prod(sim.shape))))
+
+    def fresh():
+        cells = (16, 8, 8)
+        return pkg.PicSimulation(cells, tuple(c * H for c in cells), 0.02, pkg.configs.species_table(4))
+
+    with fresh() as kept:
+        for ppc, steps, every, sub, record in ((4, 9, 4, None, False), (4, 20, 6, 2, False), (12, 5, 5, None, True),
+                                               (4, 20, 20, None, False), (1, 4, 2, None, False)):
+            start(kept, ppc)
+            kept.branch_record(record)
+            kept.forward(steps, every, sub)
+            g = kept.backward(**loss)
+            with fresh() as sim:
+                start(sim, ppc)
+                sim.forward(steps, every, sub)
+                w = sim.backward(**loss)
+            assert rel(g["d_p0"], w["d_p0"]) < 1e-9 and rel(g["d_drift"], w["d_drift"]) < 1e-9
+            assert g["loss"] == pytest.approx(w["loss"], rel=1e-12)
+            if steps == 5:
+                kept.adjoint_free()
