@@ -28,6 +28,7 @@
 #include "pic_handle.cuh"
 #include "pic_adjoint.cuh"
 #include "pic_plain_math.cuh"
+#include "pic_fold.cuh"
 
 namespace pic {
 
@@ -1068,29 +1069,11 @@ __device__ __forceinline__ void line_g(const Grid &g, int dir, int a, int b, siz
     else { base = ((size_t)a * g.NY + b) * g.pz; stride = 1; }
 }
 
-// transpose of the J fold along one axis (periodicCurrentElement, kernels.cu:1124-1146)
-__global__ void k_adj_j_fold(Grid g, double *Lx, double *Ly, double *Lz, int dir) {
-    int A = dir == 0 ? g.NY : g.NX;
-    int B = dir == 2 ? g.NY : g.NZ;
-    int N = dir == 0 ? g.NX : (dir == 1 ? g.NY : g.NZ);
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= A * B) return;
-    size_t base, st;
-    line_g(g, dir, idx / B, idx % B, base, st);
-    double *L3[3] = {Lx, Ly, Lz};
-    for (int comp = 0; comp < 3; comp++) {
-        double *L = L3[comp] + base;
-        size_t n1 = st, nm1 = (size_t)(N - 1) * st, nm2 = (size_t)(N - 2) * st;
-        // forward: J1 += J[N-1] (dir != comp); J[N-1] = J1 (not y/y); J0 += J[N-2]; J[N-2] = J0
-        L[0] += L[nm2];
-        L[nm2] = 0.0;
-        L[nm2] += L[0];
-        if (dir != 1 || comp != 1) {
-            L[n1] += L[nm1];
-            L[nm1] = 0.0;
-        }
-        if (dir != comp) L[nm1] += L[n1];
-    }
+// transpose of the J fold (pic_fold.cuh)
+__global__ void k_adj_j_fold(Grid g, double *Lx, double *Ly, double *Lz) {
+    double *const L[3] = {Lx, Ly, Lz};
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < fold_orbits(g)) fold_adjoint(g, L, idx);
 }
 
 // transpose of the E ghost copies E[0] = E[N], E[N+1] = E[1] (periodicElement, kernels.cu:1104-1110)
@@ -1310,7 +1293,7 @@ int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_F
     cudaStream_t s = h->stream;
     yee_b_half_plain(g, (double *const *)F, s);
     size_t nodes = g.nodes_pitched();
-    for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(F[PIC_JX + c], 0, nodes * sizeof(double), s), "zero J");
+    CK(cudaMemsetAsync(F[PIC_JX], 0, 3 * nodes * sizeof(double), s), "zero J");  // the three lie one after another
     FlatParams P = flat_params(h, A, state, F, out);
     if (A.nchunks > 0) {
         auto *kern = P.bmode == 0 ? k_flat_push_plain<0> : (P.bmode == 1 ? k_flat_push_plain<1> : k_flat_push_plain<2>);
@@ -1319,8 +1302,7 @@ int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_F
         kern<<<A.nchunks, kT, smem, s>>>(P);
     }
     CK(cudaGetLastError(), "flat push");
-    j_fold(g, (double *)F[PIC_JX], (double *)F[PIC_JY], (double *)F[PIC_JZ], s);
-    yee_b_complete_plain(g, (double *const *)F, s);
+    fold_b_plain(g, (double *const *)F, s);
     yee_e_update_plain(g, (double *const *)F, s);
     e_ghosts_plain(g, (double *)F[PIC_EX], (double *)F[PIC_EY], (double *)F[PIC_EZ],
                    h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s);
@@ -1474,7 +1456,7 @@ int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_C
     float *const *H = (float *const *)&F[PIC_HX];
     yee_b_half_mixed(g, E, H, s);
     const size_t nodes = g.nodes_pitched();
-    for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(F[PIC_JX + c], 0, nodes * sizeof(double), s), "zero J");
+    CK(cudaMemsetAsync(F[PIC_JX], 0, 3 * nodes * sizeof(double), s), "zero J");  // the three lie one after another
     MixParams P = mix_params(h, A, state, F, out);
     CK(launch_flat_push_mixed(P, A.nchunks, s), "flat push");
     j_fold(g, (double *)F[PIC_JX], (double *)F[PIC_JY], (double *)F[PIC_JZ], s);
@@ -1560,10 +1542,7 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
     FA.tau = g.tau;
     for (int c = 0; c < 3; c++) { FA.LE[c] = LE[c]; FA.LH[c] = LH[c]; FA.LJ[c] = LJ[c]; FA.LQ[c] = LQ[c]; }
     k_adj_e_update<<<node_grid(g), 32, 0, st>>>(FA);
-    for (int dir = 2; dir >= 0; dir--) {
-        int a = dir == 0 ? g.NY : g.NX, b = dir == 2 ? g.NY : g.NZ;
-        k_adj_j_fold<<<(a * b + 127) / 128, 128, 0, st>>>(g, LJ[0], LJ[1], LJ[2], dir);
-    }
+    k_adj_j_fold<<<(fold_orbits(g) + 127) / 128, 128, 0, st>>>(g, LJ[0], LJ[1], LJ[2]);
     if (!h->mixed) {
         // H_a of step n
         const double *En = (const double *)EHn, *Hn = (const double *)EHn + 3 * N;

@@ -390,9 +390,15 @@ int rebin_flat(pic_handle *h, int s, unsigned n_out) {
     return build_bins(h, s, acc + extra, cell, x, y, z, px, py, pz, nullptr);
 }
 
+// acts on the status of the last push, which is in st_host
+int handle_status(pic_handle *h);
 int check_status(pic_handle *h) {
     CK(cudaMemcpyAsync(h->st_host, h->st, sizeof(DevStatus), cudaMemcpyDeviceToHost, h->stream), "status");
     CK(cudaStreamSynchronize(h->stream), "sync");
+    return handle_status(h);
+}
+
+int handle_status(pic_handle *h) {
     const DevStatus &st = *h->st_host;
     h->counters[0] = (int64_t)st.moved;
     h->counters[1] = (int64_t)st.dropped;
@@ -483,9 +489,6 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
     // the outbox is sized once for all species (the loads leave that to the
     // first push)
     if ((rc = ensure_outbox(h))) return rc;
-    size_t nodes = h->g.nodes_pitched();
-    for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(h->f[PIC_JX + c], 0, nodes * sizeof(double), h->stream), "zero J");
-    CK(cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream), "reset status");
     if (h->mixed) {
         // species loaded since the last push: their contribution bound from their momenta
         float *prev = h->lb_buf + h->lb_par * kMaxSpecies;
@@ -497,8 +500,6 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
             h->launches += 1;
             h->sp[s].lb_known = 1;
         }
-        CK(cudaMemsetAsync(h->lb_buf + (h->lb_par ^ 1) * kMaxSpecies, 0, kMaxSpecies * sizeof(float), h->stream),
-           "reset bounds");
     }
     StepParams p = make_params(h);
     p.b_half = b_half_in_push;
@@ -508,8 +509,9 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
         p.holes = h->split_buf;
         p.hole_count = (unsigned *)(h->split_buf + split_ints(h));
         p.ticket = p.hole_count + nc;
-        CK(cudaMemsetAsync(p.hole_count, 0, (nc + h->g.ntiles) * sizeof(unsigned), h->stream), "reset hole counts");
     }
+    CK(begin_push(p, h->g.nodes_pitched(), h->stream), "begin push");
+    h->launches += 1;
     cudaEventRecord(h->ev[2], h->stream);
     CK(h->mixed ? launch_push_mixed(p, h->maps, h->stream) : launch_push_plain(p, plain_lo32(h), h->stream),
        "push_deposit");
@@ -544,12 +546,16 @@ int do_e_update(pic_handle *h) {
     return PIC_OK;
 }
 
-int do_e_ghosts(pic_handle *h) {
+// with_status: the step's status goes to st_host with this launch
+int do_e_ghosts(pic_handle *h, bool with_status = false) {
     int per = h->cfg.ghosts == PIC_GHOSTS_PERIODIC;
+    DevStatus *out = with_status ? h->st_host : nullptr;
     if (!h->mixed)
-        e_ghosts_plain(h->g, (double *)h->f[PIC_EX], (double *)h->f[PIC_EY], (double *)h->f[PIC_EZ], per, h->stream);
+        e_ghosts_plain(h->g, (double *)h->f[PIC_EX], (double *)h->f[PIC_EY], (double *)h->f[PIC_EZ], per, h->stream,
+                       h->st, out);
     else
-        e_ghosts_mixed(h->g, (float *)h->f[PIC_EX], (float *)h->f[PIC_EY], (float *)h->f[PIC_EZ], per, h->stream);
+        e_ghosts_mixed(h->g, (float *)h->f[PIC_EX], (float *)h->f[PIC_EY], (float *)h->f[PIC_EZ], per, h->stream, h->st,
+                       out);
     CK(cudaGetLastError(), "e_ghosts");
     h->launches += 1;
     return PIC_OK;
@@ -558,7 +564,7 @@ int do_e_ghosts(pic_handle *h) {
 int do_j_fold(pic_handle *h) {
     j_fold(h->g, (double *)h->f[PIC_JX], (double *)h->f[PIC_JY], (double *)h->f[PIC_JZ], h->stream);
     CK(cudaGetLastError(), "j_fold");
-    h->launches += 3;
+    h->launches += 1;
     return PIC_OK;
 }
 
@@ -666,6 +672,11 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
             if (fi >= PIC_QX) continue;
             if (fi < PIC_JX) es = sizeof(float);
         }
+        if (fi == PIC_JY || fi == PIC_JZ) {  // the three currents lie one after another: cleared in one pass
+            h->f[fi] = (double *)h->f[PIC_JX] + (fi - PIC_JX) * nodes;
+            continue;
+        }
+        if (fi == PIC_JX) es *= 3;
         if ((e = cudaMalloc(&h->f[fi], nodes * es)) != cudaSuccess) return fail(e);
         // on the handle's stream: the legacy-stream cudaMemset does not order
         // before work on a non-blocking stream
@@ -685,7 +696,8 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
     if ((e = cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream)) != cudaSuccess) return fail(e);
     if ((e = cudaMallocHost(&h->st_host, sizeof(DevStatus))) != cudaSuccess) return fail(e);
     memset(h->st_host, 0, sizeof(DevStatus));
-    if ((e = cudaMalloc(&h->dred, 8 * sizeof(double))) != cudaSuccess) return fail(e);
+    if ((e = cudaMalloc(&h->dred, kEnergyScratch * sizeof(double))) != cudaSuccess) return fail(e);
+    if ((e = cudaMemsetAsync(h->dred, 0, kEnergyScratch * sizeof(double), h->stream)) != cudaSuccess) return fail(e);
     if ((e = cudaMallocHost(&h->hred, 8 * sizeof(double))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->dcounts, (size_t)g.ncells() * sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return fail(e);
@@ -700,7 +712,7 @@ int pic_destroy(pic_handle *h) {
     adj_free(h);
     for (int s = 0; s < h->cfg.nspecies; s++) free_species(h, s, true);
     for (int fi = 0; fi < PIC_FIELD_COUNT; fi++)
-        if (h->f[fi]) cudaFree(h->f[fi]);
+        if (h->f[fi] && fi != PIC_JY && fi != PIC_JZ) cudaFree(h->f[fi]);
     if (h->dense) cudaFree(h->dense);
     if (h->outbox) cudaFree(h->outbox);
     if (h->st) cudaFree(h->st);
@@ -1067,9 +1079,28 @@ int pic_b_complete(pic_handle *h) { return h ? (set_device(h) ? h->status : do_b
 int pic_e_update(pic_handle *h) { return h ? (set_device(h) ? h->status : do_e_update(h)) : PIC_ERR_ARG; }
 int pic_e_ghosts(pic_handle *h) { return h ? (set_device(h) ? h->status : do_e_ghosts(h)) : PIC_ERR_ARG; }
 
-int pic_step(pic_handle *h, int nt) {
-    (void)nt;
-    if (!h) return PIC_ERR_ARG;
+}  // extern "C"
+
+namespace {
+
+// enqueues the field energies, and the kinetic energy of the last push where it
+// is current, into hred
+int enqueue_energy(pic_handle *h, bool kinetic) {
+    const void *E[3] = {h->f[PIC_EX], h->f[PIC_EY], h->f[PIC_EZ]};
+    const void *H[3] = {h->f[PIC_HX], h->f[PIC_HY], h->f[PIC_HZ]};
+    CK(field_energy(h->g, h->mixed, E, H, kinetic ? h->st : nullptr, h->dred, h->hred, h->stream), "field energy");
+    return PIC_OK;
+}
+void energies_of(const pic_handle *h, double *out4) {
+    out4[0] = 0.5 * h->hred[0];
+    out4[1] = 0.5 * h->hred[1];
+    out4[2] = h->hred[3];
+    out4[3] = out4[0] + out4[1] + out4[2];
+}
+
+// one step; energies (may be null) receives pic_energy's four numbers after it,
+// with the same wait
+int step_impl(pic_handle *h, double *energies) {
     int rc = set_device(h);
     if (rc) return rc;
     h->launches = 0;
@@ -1080,42 +1111,45 @@ int pic_step(pic_handle *h, int nt) {
     if ((rc = do_push_deposit(h, h->mixed))) return rc;  // records ev[2], ev[3] around the kernel
     StepParams p = make_params(h);
     CK(launch_insert(p, h->stream), "insert");
-    h->launches += 2;
     cudaEventRecord(h->ev[4], h->stream);
-    if ((rc = do_j_fold(h))) return rc;
-    if (h->mixed) {
-        // H in memory is still the full-step field: both half steps in one pass
-        yee_b_both_mixed(h->g, (float *const *)&h->f[PIC_EX], (float *const *)&h->f[PIC_HX], h->stream);
-        CK(cudaGetLastError(), "b_complete");
-        h->launches += 1;
-    } else if ((rc = do_b_complete(h))) {
-        return rc;
-    }
+    // (FP32 form: H in memory is still the full-step field, both half steps in one pass)
+    if (h->mixed)
+        fold_b_mixed(h->g, (float *const *)&h->f[PIC_EX], (float *const *)&h->f[PIC_HX], (double *const *)&h->f[PIC_JX],
+                     h->stream);
+    else
+        fold_b_plain(h->g, (double *const *)h->f, h->stream);
+    CK(cudaGetLastError(), "fold and b_complete");
+    h->launches += 2;
     if ((rc = do_e_update(h))) return rc;
-    if ((rc = do_e_ghosts(h))) return rc;
+    if ((rc = do_e_ghosts(h, true))) return rc;
     cudaEventRecord(h->ev[5], h->stream);
-    rc = check_status(h);
+    if (energies && (rc = enqueue_energy(h, true))) return rc;
+    h->timed = h->timed ? 2 : 0;
+    CK(cudaStreamSynchronize(h->stream), "sync");
+    rc = handle_status(h);
     h->counters[3] = h->launches;
     if (!rc) {
-        cudaEventElapsedTime(&h->timings[0], h->ev[0], h->ev[1]);
-        cudaEventElapsedTime(&h->timings[1], h->ev[2], h->ev[3]);
-        cudaEventElapsedTime(&h->timings[2], h->ev[3], h->ev[4]);
-        cudaEventElapsedTime(&h->timings[3], h->ev[4], h->ev[5]);
-        cudaEventElapsedTime(&h->timings[4], h->ev[0], h->ev[5]);
-        h->timed = 1;
+        h->timed = 1;  // pic_step_timings reads the events
+        if (energies) energies_of(h, energies);
     }
     return rc;
+}
+
+}  // namespace
+
+extern "C" {
+
+int pic_step(pic_handle *h, int nt) {
+    (void)nt;
+    if (!h) return PIC_ERR_ARG;
+    return step_impl(h, nullptr);
 }
 
 int pic_run(pic_handle *h, int nsteps, double *energies) {
     if (!h || nsteps < 0) return PIC_ERR_ARG;
     for (int n = 0; n < nsteps; n++) {
-        int rc = pic_step(h, n + 1);
+        int rc = step_impl(h, energies ? energies + 4 * n : nullptr);
         if (rc) return rc;
-        if (energies) {
-            rc = pic_energy(h, energies + 4 * n);
-            if (rc) return rc;
-        }
     }
     return PIC_OK;
 }
@@ -1265,22 +1299,16 @@ int pic_energy(pic_handle *h, double *out4) {
     if (rc) return rc;
     rc = need_particles(h);
     if (rc) return rc;
-    CK(cudaMemsetAsync(h->dred, 0, 8 * sizeof(double), h->stream), "memset");
-    const void *E[3] = {h->f[PIC_EX], h->f[PIC_EY], h->f[PIC_EZ]};
-    const void *H[3] = {h->f[PIC_HX], h->f[PIC_HY], h->f[PIC_HZ]};
-    CK(field_energy(h->g, h->mixed, E, H, h->dred, h->stream), "field energy");
+    if ((rc = enqueue_energy(h, h->kin_valid))) return rc;
     if (!h->kin_valid) {
+        double *kin = h->dred + 4;
+        CK(cudaMemsetAsync(kin, 0, sizeof(double), h->stream), "memset");
         StepParams p = make_params(h);
-        CK(kinetic_energy(p, h->dred + 3, h->stream), "kinetic");
-    } else {
-        CK(cudaMemcpyAsync(h->dred + 3, &h->st->kinetic, sizeof(double), cudaMemcpyDeviceToDevice, h->stream), "kin");
+        CK(kinetic_energy(p, kin, h->stream), "kinetic");
+        CK(cudaMemcpyAsync(h->hred + 3, kin, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
     }
-    CK(cudaMemcpyAsync(h->hred, h->dred, 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
     CK(cudaStreamSynchronize(h->stream), "sync");
-    out4[0] = 0.5 * h->hred[0];
-    out4[1] = 0.5 * h->hred[1];
-    out4[2] = h->hred[3];
-    out4[3] = out4[0] + out4[1] + out4[2];
+    energies_of(h, out4);
     return PIC_OK;
 }
 
@@ -1288,11 +1316,7 @@ int pic_energy_reference(pic_handle *h, double *out) {
     if (!h || !out) return set_err(h, PIC_ERR_ARG, "bad argument");
     int rc = set_device(h);
     if (rc) return rc;
-    CK(cudaMemsetAsync(h->dred, 0, 8 * sizeof(double), h->stream), "memset");
-    const void *E[3] = {h->f[PIC_EX], h->f[PIC_EY], h->f[PIC_EZ]};
-    const void *H[3] = {h->f[PIC_HX], h->f[PIC_HY], h->f[PIC_HZ]};
-    CK(field_energy(h->g, h->mixed, E, H, h->dred, h->stream), "field energy");
-    CK(cudaMemcpyAsync(h->hred, h->dred, 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
+    if ((rc = enqueue_energy(h, false))) return rc;
     CK(cudaStreamSynchronize(h->stream), "sync");
     *out = h->hred[2];
     return PIC_OK;
@@ -1334,6 +1358,12 @@ int pic_step_counters(pic_handle *h, int64_t *out4) {
 
 int pic_step_timings(pic_handle *h, float *out5) {
     if (!h || !out5) return PIC_ERR_ARG;
+    if (h->timed == 1) {
+        cudaSetDevice(h->device);
+        const int of[5][2] = {{0, 1}, {2, 3}, {3, 4}, {4, 5}, {0, 5}};
+        for (int i = 0; i < 5; i++) cudaEventElapsedTime(&h->timings[i], h->ev[of[i][0]], h->ev[of[i][1]]);
+        h->timed = 2;
+    }
     for (int i = 0; i < 5; i++) out5[i] = h->timings[i];
     return h->timed ? PIC_OK : PIC_ERR_STATE;
 }

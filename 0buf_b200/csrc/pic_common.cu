@@ -158,7 +158,10 @@ __global__ void k_gather_f(Grid g, int mixed, SpeciesView S, const int64_t *__re
 
 // Arrivals of the migration (replaces GPU_ArrangeFlights' Insert, kernels.cu:316-370):
 // every outbox entry is appended to its destination tile.  Entries that fit
-// are marked done (cell = -1); the rest stay for a rebin.
+// are marked done (cell = -1); the rest stay for a rebin.  An entry that finds
+// its tile full takes its count back: a tile's count passes its capacity only
+// while such entries are under way, so no slot is handed out twice and the
+// counts end at the capacity.
 template <class Out, bool MIXED>
 __global__ void k_insert(StepParams P) {
     unsigned n = P.st->out_count;
@@ -188,6 +191,7 @@ __global__ void k_insert(StepParams P) {
             }
             ob[e].cell = -1;
         } else {
+            atomicSub(&S.tile_count[t], 1);
             atomicAdd(&P.st->overflow_count, 1u);
             atomicOr(&P.st->flags, (unsigned)ST_TILE_FULL);
             atomicOr(&P.st->full_species, 1u << o.species);
@@ -262,14 +266,15 @@ __global__ void k_insert_left(Grid g, Out *ob, unsigned n, int species, SpeciesV
     ob[e].cell = -1;
 }
 
-// clamp tile counts after an overflowing insert so the bins stay consistent
-__global__ void k_clamp_counts(StepParams P) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.g.ntiles) return;
-    for (int s = 0; s < P.nsp; s++) {
-        int cap = P.sp[s].tile_start[t + 1] - P.sp[s].tile_start[t];
-        if (P.sp[s].tile_count[t] > cap) P.sp[s].tile_count[t] = cap;
-    }
+// see begin_push: one launch in place of a memset per array (five of them at
+// 2 us each in a small step)
+__global__ void k_begin_push(double2 *J, size_t n2, unsigned *st, int nst, unsigned *lb, int nlb, unsigned *holes,
+                             int nholes) {
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = i0; i < n2; i += stride) J[i] = make_double2(0.0, 0.0);
+    for (size_t i = i0; i < (size_t)nholes; i += stride) holes[i] = 0u;
+    if (i0 < (size_t)nst) st[i0] = 0u;
+    if (i0 < (size_t)nlb) lb[i0] = 0u;
 }
 
 // per interior cell counts over all species (blockIdx.y = species)
@@ -454,13 +459,16 @@ __device__ __forceinline__ void load4(const double *p, double v[4]) {
 }
 
 // Bound by reading E and H once.  A block walks over many quads of nodes and
-// adds its three sums once: a block per 128 nodes sent 400k FP64 atomics to
-// three addresses at 512x128x128 (634 us per call, now 56).
+// leaves its three sums, and the last block to finish adds them up in order and
+// writes them to the host (a block per 128 nodes that added to three addresses
+// sent them 400k FP64 atomics at 512x128x128: 634 us per call, now 56).
 template <typename T>
 __global__ void k_field_energy(Grid g, const T *__restrict__ Ex, const T *__restrict__ Ey, const T *__restrict__ Ez,
                                const T *__restrict__ Hx, const T *__restrict__ Hy, const T *__restrict__ Hz,
-                               double *out) {
+                               const DevStatus *st, double *scratch, double *host) {
+    chain_enter();
     __shared__ double red[32];
+    __shared__ int last;
     double we = 0.0, wb = 0.0, wr = 0.0;
     const int nq = g.pz / 4;
     const int64_t quads = (int64_t)g.NX * g.NY * nq;
@@ -485,10 +493,28 @@ __global__ void k_field_energy(Grid g, const T *__restrict__ Ex, const T *__rest
     double a = block_sum(we, red);
     double b = block_sum(wb, red);
     double c = block_sum(wr, red);
+    unsigned *ticket = (unsigned *)scratch;
+    double *part = scratch + 8;
     if (threadIdx.x == 0) {
-        atomicAdd(&out[0], a);
-        atomicAdd(&out[1], b);
-        atomicAdd(&out[2], c);
+        part[3 * blockIdx.x] = a;
+        part[3 * blockIdx.x + 1] = b;
+        part[3 * blockIdx.x + 2] = c;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int u = threadIdx.x; u < (int)gridDim.x; u += blockDim.x)
+        for (int q = 0; q < 3; q++) v[q] += __ldcg(&part[3 * u + q]);
+    for (int q = 0; q < 3; q++) {
+        const double t = block_sum(v[q], red);
+        if (threadIdx.x == 0) ((volatile double *)host)[q] = t;
+    }
+    if (threadIdx.x == 0) {
+        if (st) ((volatile double *)host)[3] = st->kinetic;
+        *ticket = 0u;  // for the next call
     }
 }
 
@@ -582,7 +608,6 @@ cudaError_t launch_insert(const StepParams &p, cudaStream_t s) {
     int blocks = 148 * 4;
     if (p.mixed) k_insert<OutMixed, true><<<blocks, 256, 0, s>>>(p);
     else k_insert<OutPlain, false><<<blocks, 256, 0, s>>>(p);
-    k_clamp_counts<<<blocks_for(p.g.ntiles, 256), 256, 0, s>>>(p);
     return cudaGetLastError();
 }
 
@@ -658,18 +683,27 @@ cudaError_t init_cells(const Grid &g, int mixed, SpeciesView sv, int species_ind
     return cudaGetLastError();
 }
 
-cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], double *out3,
-                         cudaStream_t s) {
+cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], const DevStatus *st,
+                         double *scratch, double *host, cudaStream_t s) {
     const int bx = 256;
     const int64_t quads = (int64_t)g.NX * g.NY * (g.pz / 4);
-    const int grid = (int)std::min<int64_t>((quads + bx - 1) / bx, 148 * 8);
+    const dim3 grid((unsigned)std::min<int64_t>((quads + bx - 1) / bx, kEnergyBlocks));
     if (mixed)
-        k_field_energy<float><<<grid, bx, 0, s>>>(g, (const float *)E[0], (const float *)E[1], (const float *)E[2],
-                                                  (const float *)H[0], (const float *)H[1], (const float *)H[2], out3);
-    else
-        k_field_energy<double><<<grid, bx, 0, s>>>(g, (const double *)E[0], (const double *)E[1],
-                                                   (const double *)E[2], (const double *)H[0], (const double *)H[1],
-                                                   (const double *)H[2], out3);
+        return launch_chained(k_field_energy<float>, grid, dim3(bx), s, g, (const float *)E[0], (const float *)E[1],
+                              (const float *)E[2], (const float *)H[0], (const float *)H[1], (const float *)H[2], st,
+                              scratch, host);
+    return launch_chained(k_field_energy<double>, grid, dim3(bx), s, g, (const double *)E[0], (const double *)E[1],
+                          (const double *)E[2], (const double *)H[0], (const double *)H[1], (const double *)H[2], st,
+                          scratch, host);
+}
+
+cudaError_t begin_push(const StepParams &p, size_t nodes, cudaStream_t s) {
+    const size_t n2 = 3 * nodes / 2;  // a multiple of four nodes per row
+    const int nholes = p.slices > 1 ? (p.nsp + 1) * p.g.ntiles : 0;
+    const int nlb = p.lb_cur ? kMaxSpecies : 0;
+    const int blocks = (int)std::min<size_t>((n2 + 255) / 256, 148 * 16);
+    k_begin_push<<<blocks, 256, 0, s>>>((double2 *)p.J[0], n2, (unsigned *)p.st, (int)(sizeof(DevStatus) / 4), p.lb_cur,
+                                        nlb, p.hole_count, nholes);
     return cudaGetLastError();
 }
 

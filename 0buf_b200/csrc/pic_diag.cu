@@ -317,11 +317,12 @@ int run_gauss(pic_handle *h, int set_baseline, double *red4) {
     int rc = compute_rho(h);
     if (rc) return rc;
     const void *E[3] = {h->f[PIC_EX], h->f[PIC_EY], h->f[PIC_EZ]};
-    CK(cudaMemsetAsync(h->dred, 0, 4 * sizeof(double), h->stream), "memset");
-    CK(gauss_residual(h->g, h->mixed, E, h->rho, h->gauss, h->gauss0, set_baseline, h->dred, h->stream), "gauss");
+    double *red = h->dred + 4;  // the first word counts the blocks of field_energy
+    CK(cudaMemsetAsync(red, 0, 4 * sizeof(double), h->stream), "memset");
+    CK(gauss_residual(h->g, h->mixed, E, h->rho, h->gauss, h->gauss0, set_baseline, red, h->stream), "gauss");
     if (set_baseline) h->gauss_has_base = 1;
     if (red4) {
-        CK(cudaMemcpyAsync(h->hred, h->dred, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
+        CK(cudaMemcpyAsync(h->hred, red, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
         CK(cudaStreamSynchronize(h->stream), "sync");
         for (int i = 0; i < 4; i++) red4[i] = h->hred[i];
     }

@@ -10,8 +10,13 @@ void yee_b_half_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void yee_b_complete_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void yee_e_update_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void j_fold(const Grid &g, double *Jx, double *Jy, double *Jz, cudaStream_t s);
-void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s);
-void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s);
+// the J fold and the B completion in one launch
+void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s);
+// st, out: device status and pinned host memory that receives it (null: none)
+void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr);
+void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s,
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr);
 size_t push_smem_plain(const Grid &g);
 // lo32: the tile current's int32 remainder word (every tile holds fewer than
 // 2^(31 - kFxLo32MinBits) particles), else the 64-bit one
@@ -22,8 +27,9 @@ cudaError_t place_particles_plain(const Grid &g, int64_t n, const double *x, con
 
 // mixed form (pic_mixed.cu, FP32 with FP64 global J)
 void yee_b_half_mixed(const Grid &g, float *const E[3], float *const H[3], cudaStream_t s);
-// both B half steps of a step in one pass, H = (H + Q(E)) + Q(E) (pic_step: the push forms the first in shared memory)
-void yee_b_both_mixed(const Grid &g, float *const E[3], float *const H[3], cudaStream_t s);
+// the J fold, and both B half steps of a step in one pass, H = (H + Q(E)) + Q(E) (pic_step: the push forms the first
+// in shared memory), in one launch
+void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s);
 void yee_e_update_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s);
 size_t push_smem_mixed(const Grid &g);
 // dynamic + static shared memory of the mixed push kernel ((size_t)-1 if it cannot be queried)
@@ -36,6 +42,9 @@ cudaError_t encode_field_maps(const Grid &g, float *const E[3], float *const H[3
 
 // form-independent (pic_common.cu, FP64 parts with -fmad=false)
 cudaError_t launch_insert(const StepParams &p, cudaStream_t s);
+// what a push starts from: J (3 components of `nodes`, one after another), the
+// status, the contribution bounds it records and the hole counts, all zero
+cudaError_t begin_push(const StepParams &p, size_t nodes, cudaStream_t s);
 cudaError_t cell_histogram(const StepParams &p, int *counts, cudaStream_t s);
 // native 28-byte layout (reference cell number, FP32 offsets and momenta)
 cudaError_t place_particles_cells(const Grid &g, int64_t n, const int *ref_cell, const float *ox, const float *oy,
@@ -75,9 +84,12 @@ cudaError_t init_species_bins(const Grid &g, int mixed, SpeciesView sv, int spec
 // seeded generator with per-cell counts (count, first slot per dense cell)
 cudaError_t init_cells(const Grid &g, int mixed, SpeciesView sv, int species_index, const int *count,
                        const int *first, double dx, double dy, double dz, double vth, uint64_t seed, cudaStream_t s);
-// FP64 reductions: out[0] sum E^2, out[1] sum H^2 over nodes 1..N, out[2] sum E^2 all nodes (reference)
-cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], double *out3,
-                         cudaStream_t s);
+// FP64 reductions: host[0] sum E^2, host[1] sum H^2 over nodes 1..N, host[2] sum E^2 all nodes (reference), host[3]
+// st->kinetic (st null: left alone).  host: pinned memory, written by the kernel; scratch: kEnergyScratch doubles,
+// the first zero before the first call
+constexpr int kEnergyBlocks = 148 * 8, kEnergyScratch = 8 + 3 * kEnergyBlocks;
+cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], const DevStatus *st,
+                         double *scratch, double *host, cudaStream_t s);
 cudaError_t kinetic_energy(const StepParams &p, double *out, cudaStream_t s);
 // charge-conservation diagnostic (pic_diag.cu, FP64): rho on the cell-centre
 // nodes, folded; G = div E - rho on interior nodes with reductions

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include "pic_internal.cuh"
 #include "pic_kernels.cuh"
+#include "pic_fold.cuh"
 
 namespace pic {
 namespace {
@@ -48,14 +49,12 @@ __device__ __forceinline__ void un4(float4 a, float v[4]) { v[0] = a.x; v[1] = a
 // half step the push formed in shared memory only (the same bits as the two
 // separate passes of the sub-step calls)
 template <bool TWICE>
-__global__ void k_b_half_mixed(Grid g, const float *__restrict__ Ex, const float *__restrict__ Ey,
-                               const float *__restrict__ Ez, float *Hx, float *Hy, float *Hz, float cx, float cy,
-                               float cz) {
-    chain_enter();
+__device__ __forceinline__ void b_half_nodes(const Grid &g, int i, int q, const float *__restrict__ Ex,
+                                             const float *__restrict__ Ey, const float *__restrict__ Ez, float *Hx,
+                                             float *Hy, float *Hz, float cx, float cy, float cz) {
     const int nq = g.pz / 4;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= g.NY * nq) return;
-    const int l = q / nq, k0 = (q - l * nq) * 4, i = blockIdx.y;
+    const int l = q / nq, k0 = (q - l * nq) * 4;
     const size_t n = g.node(i, l, k0);
     const size_t sx = (size_t)g.NY * g.pz, sy = g.pz;
     float ex[5], ey[5], ez[4], hx[4], hy[4], hz[4], ezy[4] = {}, exy[4] = {}, ezx[4] = {}, eyx[4] = {};
@@ -85,6 +84,29 @@ __global__ void k_b_half_mixed(Grid g, const float *__restrict__ Ex, const float
         }
     }
     st4(Hx + n, hx); st4(Hy + n, hy); st4(Hz + n, hz);
+}
+
+template <bool TWICE>
+__global__ void k_b_half_mixed(Grid g, const float *__restrict__ Ex, const float *__restrict__ Ey,
+                               const float *__restrict__ Ez, float *Hx, float *Hy, float *Hz, float cx, float cy,
+                               float cz) {
+    chain_enter();
+    b_half_nodes<TWICE>(g, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, cx, cy, cz);
+}
+// the J fold and both B half steps, which touch different arrays, in one launch:
+// the first `folds` blocks fold, the others step
+__global__ void k_fold_b_mixed(Grid g, int folds, int per_plane, double *Jx, double *Jy, double *Jz,
+                               const float *__restrict__ Ex, const float *__restrict__ Ey, const float *__restrict__ Ez,
+                               float *Hx, float *Hy, float *Hz, float cx, float cy, float cz) {
+    chain_enter();
+    if ((int)blockIdx.x < folds) {
+        double *const J[3] = {Jx, Jy, Jz};
+        const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+        if (idx < fold_orbits(g)) fold_current(g, J, idx);
+        return;
+    }
+    const int b = blockIdx.x - folds, i = b / per_plane;
+    b_half_nodes<true>(g, i, (b - i * per_plane) * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, cx, cy, cz);
 }
 
 // emeElement (kernels.cu:1091-1102) in FP32, tau*J formed in FP64
@@ -919,10 +941,12 @@ void yee_b_half_mixed(const Grid &g, float *const E[3], float *const H[3], cudaS
                    cx, cy, cz);
 }
 
-void yee_b_both_mixed(const Grid &g, float *const E[3], float *const H[3], cudaStream_t s) {
+void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s) {
     float cx = (float)(g.tau / g.hx), cy = (float)(g.tau / g.hy), cz = (float)(g.tau / g.hz);
-    launch_chained(k_b_half_mixed<true>, plane_grid(g), dim3(kPlaneThreads), s, g, E[0], E[1], E[2], H[0], H[1], H[2],
-                   cx, cy, cz);
+    const int folds = (fold_orbits(g) + kPlaneThreads - 1) / kPlaneThreads;
+    const dim3 plane = plane_grid(g);
+    launch_chained(k_fold_b_mixed, dim3(folds + plane.x * plane.y), dim3(kPlaneThreads), s, g, folds, (int)plane.x, J[0],
+                   J[1], J[2], E[0], E[1], E[2], H[0], H[1], H[2], cx, cy, cz);
 }
 
 void yee_e_update_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s) {
