@@ -40,11 +40,21 @@ int cuda_err(pic_handle *h, cudaError_t e, const char *where) {
     return set_err(h, (int)e, buf);
 }
 
+static void release_spare(pic_handle *h) {
+    if (h->spare) cudaFree(h->spare);
+    h->spare = nullptr;
+    h->spare_bytes = 0;
+}
+
 cudaError_t dev_alloc(pic_handle *h, void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes > 0 ? bytes : 16);
-    if (e == cudaErrorMemoryAllocation && adj_reclaim(h)) {
-        cudaGetLastError();
-        e = cudaMalloc(p, bytes > 0 ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation) {
+        const bool spare = h->spare != nullptr;
+        release_spare(h);
+        if (adj_reclaim(h) || spare) {
+            cudaGetLastError();
+            e = cudaMalloc(p, bytes > 0 ? bytes : 16);
+        }
     }
     return e;
 }
@@ -104,8 +114,17 @@ void free_species(pic_handle *h, int s, bool give_back) {
 }
 
 // tile starts from particle counts: the capacity of every tile (start has
-// ntiles + 1 entries).  Slots start on multiples of 32 particles.
-int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> &start) {
+// ntiles + 1 entries).  Slots start on multiples of 32 particles.  old (may be
+// null): the starts of the bins that a rebin replaces.  Bins that overflowed once
+// would overflow again soon, so there
+//   - a tile that fills 9/10 of its old bin or more gets three times the slack
+//     (it is filling up: dense regions that spread overflow tile after tile);
+//   - a tile whose count has fallen keeps its capacity, up to kKeepCapacity times
+//     what its count asks for (particles that slosh between tiles).
+// 256x64x64 cells, stress configuration: 15 -> 9 rebuilds in 240 steps.
+constexpr double kKeepCapacity = 1.5;
+int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> &start,
+                const std::vector<int> *old = nullptr) {
     const Grid &g = h->g;
     double slack = h->cfg.capacity_slack > 0 ? h->cfg.capacity_slack : 0.25;
     start.resize(g.ntiles + 1);
@@ -113,7 +132,10 @@ int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> 
     for (int t = 0; t < g.ntiles; t++) {
         start[t] = (int)acc;
         int64_t pad = h->cfg.capacity_pad >= 0 ? h->cfg.capacity_pad : 64;
-        int64_t cap = (int64_t)counts[t] + (int64_t)ceil(counts[t] * slack) + pad;
+        const int64_t was = old ? (*old)[t + 1] - (*old)[t] : 0;
+        const bool filling = old && 10 * (int64_t)counts[t] > 9 * was;
+        int64_t cap = (int64_t)counts[t] + (int64_t)ceil(counts[t] * (filling ? 3.0 * slack : slack)) + pad;
+        if (old) cap = std::max(cap, std::min<int64_t>(was, (int64_t)(kKeepCapacity * cap)));
         if (pad > 0) cap = (cap + 31) / 32 * 32;
         // the FP32 push reads and writes particles in 8-byte pairs: every tile starts on an even slot
         if (h->mixed) cap = (cap + 1) / 2 * 2;
@@ -218,6 +240,15 @@ int ensure_outbox(pic_handle *h) {
     int64_t total = 0;
     for (int s = 0; s < h->cfg.nspecies; s++) total += h->sp[s].cap_total;
     double frac = h->cfg.outbox_fraction > 0 ? h->cfg.outbox_fraction : 0.04;
+    // species still to be loaded, in a small run: room for as many slots as the
+    // largest so far, so that loading one after the other allocates once
+    int64_t most = 0;
+    int missing = 0;
+    for (int s = 0; s < h->cfg.nspecies; s++) {
+        most = std::max(most, h->sp[s].cap_total);
+        missing += !h->sp[s].loaded;
+    }
+    if (frac * (double)(missing * most) * h->out_elem < (double)(16 << 20)) total += missing * most;
     int64_t want = (int64_t)(frac * (double)total) + 65536;
     // the FP32 push leaves up to a chunk per warp unused: keep that out of the
     // share of the particles when several CTAs work on a tile
@@ -225,7 +256,10 @@ int ensure_outbox(pic_handle *h) {
     if (h->mixed && slices > 1) want += (int64_t)h->g.ntiles * slices * (kPushThreads / 32) * kOutboxChunk;
     if (want > 0x7fffffffLL) want = 0x7fffffffLL;
     if (h->outbox && (int64_t)h->out_cap >= want && (slices == 1 || h->split_buf)) return PIC_OK;
-    if (h->outbox) cudaFree(h->outbox);
+    if (h->outbox) {
+        cudaFree(h->outbox);
+        want = std::min<int64_t>(want + want / 8, 0x7fffffffLL);  // growing: not again at the next rebin
+    }
     h->outbox = nullptr;
     h->split_buf = nullptr;
     const size_t ob = ((size_t)want * h->out_elem + 255) / 256 * 256;
@@ -305,6 +339,7 @@ int load_device(pic_handle *h, int s, int64_t n, const double *x, const double *
 // old and the new arrays do not fit side by side, the particles go through a
 // flat list instead (rebin_flat).
 int rebin_flat(pic_handle *h, int s, unsigned n_out);
+constexpr size_t kSpareBytes = (size_t)512 << 20;
 int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     const Grid &g = h->g;
     auto &sp = h->sp[s];
@@ -319,12 +354,23 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     CK(cudaStreamSynchronize(h->stream), "sync");
     for (int t = 0; t < g.ntiles; t++) counts[t] += left[t];
     std::vector<int> start;
-    int rc = layout_bins(h, counts, start);
-    if (rc) return rc;
     SpeciesView v = sp.v;
-    void *arena = nullptr;
-    size_t bytes = 0;
-    const cudaError_t e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
+    // the new arrays: the last rebin's old ones where they fit
+    void *arena = h->spare;
+    size_t bytes = h->spare_bytes;
+    h->spare = nullptr;
+    h->spare_bytes = 0;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!layout_bins(h, counts, start, &sp.h_start)) e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
+    if (e == cudaErrorMemoryAllocation) {  // no room for kept capacities
+        cudaGetLastError();
+        const int rc = layout_bins(h, counts, start);
+        if (rc) {
+            if (arena) dev_free(h, arena);
+            return rc;
+        }
+        e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
+    }
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         return rebin_flat(h, s, n_out);
@@ -344,7 +390,12 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
         dev_free(h, arena);
         return cuda_err(h, r, "rebin");
     }
-    dev_free(h, sp.arena);
+    if (sp.arena_bytes <= kSpareBytes) {
+        h->spare = sp.arena;
+        h->spare_bytes = sp.arena_bytes;
+    } else {
+        dev_free(h, sp.arena);
+    }
     sp.arena = arena;
     sp.arena_bytes = bytes;
     sp.v = v;
@@ -694,11 +745,13 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
     }
     if ((e = cudaMalloc(&h->st, sizeof(DevStatus))) != cudaSuccess) return fail(e);
     if ((e = cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream)) != cudaSuccess) return fail(e);
-    if ((e = cudaMallocHost(&h->st_host, sizeof(DevStatus))) != cudaSuccess) return fail(e);
-    memset(h->st_host, 0, sizeof(DevStatus));
+    // pinned: the status, then the reductions
+    if ((e = cudaMallocHost(&h->st_host, 256 + 8 * sizeof(double))) != cudaSuccess) return fail(e);
+    static_assert(sizeof(DevStatus) <= 256, "the reductions start 256 bytes behind the status");
+    memset(h->st_host, 0, 256);
+    h->hred = (double *)((char *)h->st_host + 256);
     if ((e = cudaMalloc(&h->dred, kEnergyScratch * sizeof(double))) != cudaSuccess) return fail(e);
     if ((e = cudaMemsetAsync(h->dred, 0, kEnergyScratch * sizeof(double), h->stream)) != cudaSuccess) return fail(e);
-    if ((e = cudaMallocHost(&h->hred, 8 * sizeof(double))) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc(&h->dcounts, (size_t)g.ncells() * sizeof(int))) != cudaSuccess) return fail(e);
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return fail(e);
     *out = h;
@@ -718,10 +771,10 @@ int pic_destroy(pic_handle *h) {
     if (h->st) cudaFree(h->st);
     if (h->st_host) cudaFreeHost(h->st_host);
     if (h->dred) cudaFree(h->dred);
-    if (h->hred) cudaFreeHost(h->hred);
     if (h->dcounts) cudaFree(h->dcounts);
     if (h->lb_buf) cudaFree(h->lb_buf);
     release_load_scratch(h);
+    release_spare(h);
 
     double *diag[3] = {h->rho, h->gauss, h->gauss0};
     for (double *d : diag)

@@ -80,6 +80,10 @@ struct pic_handle {
     // (null: it has none)
     int *split_buf;
     int sms;  // SMs of the device
+    // the arrays that the last rebin left, for the next one (at most
+    // kSpareBytes; given back when a device allocation fails)
+    void *spare;
+    size_t spare_bytes;
 };
 
 namespace pic_host {
