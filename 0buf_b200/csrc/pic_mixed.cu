@@ -279,13 +279,22 @@ struct PartM {
     float x, y, z, px, py, pz;
 };
 
-__device__ __forceinline__ PartM load_part(const SpeciesView &S, int slot) {
-    PartM p;
-    p.cell = S.cell[slot];
-    p.x = S.ox[slot]; p.y = S.oy[slot]; p.z = S.oz[slot];
-    p.px = S.fx[slot]; p.py = S.fy[slot]; p.pz = S.fz[slot];
-    return p;
-}
+// One bin's arrays: CTA-uniform pointers to its first slot, indexed by 32-bit
+// offsets within the bin (no 64-bit address arithmetic per particle)
+struct BinM {
+    int *cell;
+    float *x, *y, *z, *px, *py, *pz;
+    __device__ __forceinline__ BinM(const SpeciesView &S, int start)
+        : cell(S.cell + start), x(S.ox + start), y(S.oy + start), z(S.oz + start), px(S.fx + start), py(S.fy + start),
+          pz(S.fz + start) {}
+    __device__ __forceinline__ PartM load(unsigned j) const {
+        PartM p;
+        p.cell = cell[j];
+        p.x = x[j]; p.y = y[j]; p.z = z[j];
+        p.px = px[j]; p.py = py[j]; p.pz = pz[j];
+        return p;
+    }
+};
 
 // ------------------------------------------------- tensor-memory staging --
 // The CTA's field tile (6 components, tile + 2-node halo, plus one row in y
@@ -325,20 +334,24 @@ constexpr int kTmaWaitLimit = 1 << 20;
 
 // Deposit of the tile current, two levels:
 //  1. the first zigzag segment of every particle goes, with native int32
-//     shared-memory atomics, into a tile-sized int32 current that two warps
-//     share (kJCopies per CTA).  Its quantum q_s = 2^e_s is static per
-//     species: cmax bounds one contribution (twice the largest of the species
-//     in the last push, or from its momenta before its first push; at most
-//     the light-speed bound) and q_s >= 2^-22 cmax keeps the FMA
-//     magic-number rounding of a contribution exact.  Each warp adds up, per
-//     iteration, the bounds of its lanes' contributions (redux.sync): its
-//     share of any node's int32 sum never exceeds that running total.  Before
-//     the total could pass 2^30 the warp moves the current into the tile's
-//     exact 64-bit fixed-point J (atomicExch, so the other warp's concurrent
-//     adds are never lost; rescaled exactly: both quanta are powers of two)
-//     and starts its total again at zero, so two warps' shares stay below
-//     2^31.  At the end of the species the copies are summed per node into
-//     the tile J.
+//     shared-memory atomics, into one of kJCopies tile-sized int32 currents, lane
+//     l of every warp into copy l mod kJCopies.  Consecutive particles mostly
+//     share a cell, and adds of one warp to one address take turns: with a copy
+//     per pair of warps an add took about 8 turns and the shared-memory pipe was
+//     75 % busy; with the lanes spread over the copies, whose nodes lie 8 banks
+//     apart, it is 59 % (50.3M particles: push 1.233 -> 1.122 ms; after 400 steps,
+//     bins no longer in cell order, 1.262 -> 1.213).
+//     The quantum q_s = 2^e_s is static per species: cmax bounds one contribution
+//     (twice the largest of the species in the last push, or from its momenta
+//     before its first push; at most the light-speed bound) and q_s >= 2^-22 cmax
+//     keeps the FMA magic-number rounding of a contribution exact.  Each lane
+//     adds up the bounds of its contributions: its share of any node's int32 sum
+//     never exceeds that.  Before a lane's total could pass kRunLimit its warp
+//     moves the copies into the tile's exact 64-bit fixed-point J (atomicExch, so
+//     the other warps' concurrent adds are never lost; rescaled exactly: both
+//     quanta are powers of two) and its lanes start again at zero, so the
+//     kMixedThreads / kJCopies lanes of a copy stay below 2^31 together.  At the
+//     end of the species the copies are summed per node into the tile J.
 //  2. the second segment of a particle that crosses a cell-centre plane
 //     (1-4% of particles), and both segments of a particle whose contribution
 //     bound exceeds cmax, are queued per warp and deposited 32 at a time, one
@@ -356,7 +369,10 @@ constexpr int kTmaWaitLimit = 1 << 20;
 #endif
 constexpr int kMixedThreads = PIC_MIXED_THREADS;  // threads per CTA of k_push_mixed
 constexpr int kMixedWarps = kMixedThreads / 32;
-constexpr int kJCopies = kMixedWarps / 2;         // int32 tile currents per CTA: one per two warps
+constexpr int kJCopies = kMixedWarps / 2;         // int32 tile currents per CTA
+constexpr int kJPad = 8;                          // words between the copies: 8 banks
+constexpr float kRunLimit = 0x1.fp30f / (kMixedThreads / kJCopies);  // quanta per lane
+static_assert(kRunLimit < 0x1p25f, "floats 2 apart");
 constexpr int kQueue = PIC_MIXED_QUEUE;           // queued segments per warp
 constexpr unsigned kOutChunk = kOutboxChunk;      // outbox slots a warp takes from the global counter at once
 static_assert(kMixedThreads == kPushThreads, "the slices of a tile are cut in blocks of kPushThreads particles");
@@ -384,7 +400,7 @@ __host__ __device__ inline MixedSmem mixed_smem(int tx, int ty, int tz) {
     m.raw_e = round_up_sz(box_e * sizeof(float), 128);
     m.raw_h = round_up_sz(box_h * sizeof(float), 128);
     const size_t raw_bytes = 3 * m.raw_e + 3 * m.raw_h;
-    const size_t jw_bytes = (size_t)kJCopies * 3 * nn * sizeof(int);
+    const size_t jw_bytes = (size_t)kJCopies * (3 * nn + kJPad) * sizeof(int);
     // the raw TMA staging area is consumed (into the quads) before the int32
     // currents are cleared, so the two share memory
     m.raw = 0;
@@ -436,7 +452,8 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
     int *sJw = (int *)(smem_raw + L.jw);
     int *sHoles = (int *)(smem_raw + L.holes);
     int *sFront = sHoles + kHoleMax;  // the compaction's holes in front of the new count
-    int *myJ = sJw + (warp % kJCopies) * 3 * nn;
+    const int JS = 3 * nn + kJPad;  // words per int32 current
+    int *myJ = sJw + (lane % kJCopies) * JS;
 
     // a TMA destination starts on a 128-byte boundary (block-uniform check)
     if (smem_u32(smem_raw + L.raw) & 127u) {
@@ -508,7 +525,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         sF[idx] = make_float4(R[0], R[1], R[BZ], R[BZ + 1]);
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < kJCopies * 3 * nn; idx += blockDim.x) sJw[idx] = 0;
+    for (int idx = threadIdx.x; idx < kJCopies * JS; idx += blockDim.x) sJw[idx] = 0;
     if (threadIdx.x < kMaxSpecies) sLbMax[threadIdx.x] = 0u;
     if (threadIdx.x < 3) { sNHoles[threadIdx.x] = 0; sNFront[threadIdx.x] = 0; sNMove[threadIdx.x] = 0; }
     __syncthreads();
@@ -557,16 +574,18 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         const int e_s = max(exponent_above(cmax * 0x1p-22f), -100);
         const float inv_qs = pow2f(-e_s);
         const int sh = e_s - tile_e;  // int32 quantum / tile quantum = 2^sh
-        // running bound of this warp's share of any node's int32 sum, in quanta
-        unsigned run = 0;
+        // running bound of this lane's share of any node's int32 sum, in quanta
+        float run = 0.f;
         auto flush_current = [&]() {
             __syncwarp();
-            for (int idx = lane; idx < 3 * nn; idx += 32) {
-                if (myJ[idx]) {
-                    const int w = atomicExch(&myJ[idx], 0);
-                    if (w) shared_add64(&sJ[idx], rescale(w, sh));
+            for (int c = 0; c < kJCopies; c++)
+                for (int idx = lane; idx < 3 * nn; idx += 32) {
+                    int *p = sJw + c * JS + idx;
+                    if (*p) {
+                        const int w = atomicExch(p, 0);
+                        if (w) shared_add64(&sJ[idx], rescale(w, sh));
+                    }
                 }
-            }
             __syncwarp();
         };
         int qn = 0;  // segments in this warp's queue (warp-uniform)
@@ -589,31 +608,30 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         // warp-synchronous loop: every lane of a warp runs the same iterations;
         // the next particle is loaded before the current one is processed
         const int stride = blockDim.x;
-        PartM nxt;
-        nxt.cell = -1;
-        if (jbeg + warp * 32 + lane < count) nxt = load_part(S, start + jbeg + warp * 32 + lane);
+        // (lanes past the bin's end keep finite values that nothing uses)
+        const BinM bin(S, start);
+        PartM nxt = {-1, 0.25f, 0.25f, 0.25f, 0.f, 0.f, 0.f};
+        if (jbeg + warp * 32 + lane < count) nxt = bin.load(jbeg + warp * 32 + lane);
         for (int base = jbeg + warp * 32; base < count; base += stride) {
             const int j = base + lane;
-            const int slot = start + j;
             PartM cur = nxt;
-            if (j + stride < count) nxt = load_part(S, slot + stride);
+            if (j + stride < count) nxt = bin.load(j + stride);
             bool active = j < count && cur.cell >= 0;
-            int i = i0, l = l0, k = k0;
-            if (active) {
-                g.cell_ijk(cur.cell, i, l, k);
-                if ((unsigned)(i - i0) >= (unsigned)tx || (unsigned)(l - l0) >= (unsigned)ty ||
-                    (unsigned)(k - k0) >= (unsigned)tz) {
-                    bad |= ST_BADCELL;  // a bin entry outside its tile: never index the tile with it
-                    active = false;
-                    i = i0; l = l0; k = k0;
-                }
+            // tile-local cell; the packed indices of a tile's cells differ field
+            // by field from its first cell's
+            int i, l, k;
+            g.cell_ijk(cur.cell, i, l, k);
+            i -= i0; l -= l0; k -= k0;
+            if (active && ((unsigned)i >= (unsigned)tx || (unsigned)l >= (unsigned)ty || (unsigned)k >= (unsigned)tz)) {
+                bad |= ST_BADCELL;  // a bin entry outside its tile: never index the tile with it
+                active = false;
             }
             // tile-local node of the particle's cell and of reference tile index (0,0,0)
-            const int lc = ((i - i0) * SY + (l - l0)) * SZ + (k - k0);
+            const int lc = active ? (i * SY + l) * SZ + k : 0;
             const int n0 = lc - 2 * (SYZ + SZ + 1);
-            float xs[3] = {cur.x, cur.y, cur.z};
-            if (!active) xs[0] = xs[1] = xs[2] = 0.25f;
-            float pu = active ? cur.px : 0.f, pv = active ? cur.py : 0.f, pw = active ? cur.pz : 0.f;
+            // (an inactive lane computes on, from values that nothing uses)
+            const float xs[3] = {cur.x, cur.y, cur.z};
+            float pu = cur.px, pv = cur.py, pw = cur.pz;
 
             // ---- GetField (cell.h:1257-1290) in cell units: getCellNumber = 2,
             // getCellNumberCenter = 2 + (offset >= 1/2), weights s1 = 1-o, s2 = 1/2-o (+1)
@@ -690,11 +708,13 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
             lbmax = fmaxf(lbmax, lb);
             const bool fast = dep && lb <= cmax;
             {
-                // |round(v/q_s)| <= lb/q_s + 1/2 per contribution, one contribution per node and lane
-                const unsigned add = __reduce_add_sync(FULL, fast ? (unsigned)(lb * inv_qs) + 1u : 0u);
-                if (run + add > 0x40000000u) {
+                // |round(v/q_s)| <= lb/q_s + 1/2 per contribution, one contribution
+                // per node and lane.  The sum stays below 2^25, where floats are 2
+                // apart: rounded to nearest, it never counts less than that.
+                const float add = fmaf(lb, inv_qs, 1.f);
+                if (__any_sync(FULL, run + add > kRunLimit)) {
                     flush_current();
-                    run = 0;
+                    run = 0.f;
                 }
                 run += add;
             }
@@ -755,12 +775,13 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                 dl[d] = (int)up - (int)dn;
                 xw[d] = fminf(fmaxf(xe[d] + (up ? -1.f : (dn ? 1.f : 0.f)), 0.f), kOneBelow);
             }
-            const bool stay = (unsigned)(i - i0 + dl[0]) < (unsigned)txe && (unsigned)(l - l0 + dl[1]) < (unsigned)tye &&
-                              (unsigned)(k - k0 + dl[2]) < (unsigned)tze;
+            const bool stay = (unsigned)(i + dl[0]) < (unsigned)txe && (unsigned)(l + dl[1]) < (unsigned)tye &&
+                              (unsigned)(k + dl[2]) < (unsigned)tze;
             if (active && stay) {
-                S.cell[slot] = cur.cell + dl[0] * cstr_x + dl[1] * cstr_y + dl[2];
-                S.ox[slot] = xw[0]; S.oy[slot] = xw[1]; S.oz[slot] = xw[2];
-                S.fx[slot] = pu; S.fy[slot] = pv; S.fz[slot] = pw;
+                const unsigned u = (unsigned)j;
+                bin.cell[u] = cur.cell + dl[0] * cstr_x + dl[1] * cstr_y + dl[2];
+                bin.x[u] = xw[0]; bin.y[u] = xw[1]; bin.z[u] = xw[2];
+                bin.px[u] = pu; bin.py[u] = pv; bin.pz[u] = pw;
             }
             // leavers: outbox slots from the warp's chunk (a new run of chunks
             // from the global counter only when it is used up) and one
@@ -793,7 +814,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                 }
                 if (leave) {
                     // the new cell, wrapped periodically
-                    int ci[3] = {i + dl[0], l + dl[1], k + dl[2]};
+                    int ci[3] = {i0 + i + dl[0], l0 + l + dl[1], k0 + k + dl[2]};
                     const int nc[3] = {g.nx, g.ny, g.nz};
 #pragma unroll
                     for (int d = 0; d < 3; d++) ci[d] = ci[d] == nc[d] ? 0 : (ci[d] < 0 ? nc[d] - 1 : ci[d]);
@@ -807,7 +828,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
                     } else {
                         bad |= ST_OUTBOX;
                     }
-                    S.cell[slot] = -1;
+                    bin.cell[(unsigned)j] = -1;
                     const int hpos = hbase + rank;
                     if (!list_hole(S, t, SPLIT ? P.holes + ((size_t)s * g.ntiles + t) * kHoleMax : sHoles,
                                    (unsigned)hpos, j))
@@ -830,8 +851,8 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
             long long sum = 0;
 #pragma unroll
             for (int c = 0; c < kJCopies; c++) {
-                sum += sJw[c * 3 * nn + idx];
-                sJw[c * 3 * nn + idx] = 0;
+                sum += sJw[c * JS + idx];
+                sJw[c * JS + idx] = 0;
             }
             if (sum) sJ[idx] += (unsigned long long)rescale(sum, sh);
         }
