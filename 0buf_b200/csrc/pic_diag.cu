@@ -22,36 +22,42 @@
 #include <math.h>
 #include <string.h>
 #include <algorithm>
+#include <type_traits>
 #include "pic0buf.h"
 #include "pic_internal.cuh"
 #include "pic_kernels.cuh"
+#include "pic_plain_math.cuh"
 #include "pic_handle.cuh"
 
 namespace pic {
 namespace {
 
 // The particles of every species in a share of a tile (blockIdx.y of
-// gridDim.y) add their eight weights into a shared (tx+2)(ty+2)(tz+2) node box
+// gridDim.y) add their eight weights into shared (tx+2)(ty+2)(tz+2) node boxes
 // in 64-bit fixed point (exact and order-independent: q = 2^(E-62) with 2^E >
-// sum |m| over the tile's particles, each node receives at most that much),
-// then the box is added into the global rho.
+// sum |m| over the tile's particles, each node receives at most that much), and
+// the boxes are added into the global rho.  A contribution below 2^51 quanta
+// (every tile of 2048 equal charges or more) is rounded by adding 1.5 * 2^52
+// instead of by a conversion.
 //
-// Bound: the eight 64-bit shared adds per particle and the FP64 products in
-// front of them.  m / q is folded into the x weights, and a contribution below
-// 2^51 quanta (every tile of 2048 equal charges or more) is rounded by adding
-// 1.5 * 2^52 instead of by a conversion.  50.3M FP32-form particles (128x64x64
-// cells): 733 -> 696 us; 805M (512x128x128): 11.6 -> 9.95 ms.  The shared
-// atomics are what is left (a copy without the carry, wrong sums, timing only:
-// 635 us).  With few tiles each is dealt out to several CTAs: the reference's
-// default run (13 tiles of 500k particles) 3546 -> 143 us FP64, 2118 -> 154 us
-// FP32; 32x4x4 cells 85 -> 38 us.
+// Bound: the 16 shared atomics per particle, before them same-address conflicts
+// and the loads.  Consecutive particles mostly share a cell, so lanes add into
+// `copies` boxes in turn, whose nodes lie 4 banks apart, and the next particle is
+// loaded before the current one is processed.  50.3M particles, 6x4x8 and 8x4x8
+// tiles: FP32 696 -> 399 us, FP64 752 -> 447 us (one box 714 and 712, two 637,
+// four 483 and 491; 16 boxes leave too few CTAs per SM); 805M FP32 9.95 -> 5.45 ms.
+// With few tiles each is dealt out to several CTAs: the reference's default run
+// (13 tiles of 500k particles) 3546 -> 101 us FP64, 2118 -> 87 us FP32.
+// The copies: as many as five CTAs per SM leave room for.
+constexpr int kRhoCopies = 8, kRhoBytes = 40 * 1024;
+// words of a copy: nn low, nn high, and a pad
+__host__ __device__ inline int rho_stride(int nn) { return (2 * nn + 31) / 32 * 32 + 4; }
 template <bool MIXED>
-__global__ void __launch_bounds__(256) k_charge_tile(StepParams P, double *rho) {
+__global__ void __launch_bounds__(256) k_charge_tile(StepParams P, int copies, double *rho) {
+    using T = typename std::conditional<MIXED, float, double>::type;
     const Grid &g = P.g;
     const int nsp = P.nsp;
     const SpeciesView *sp = P.sp;
-    // the nodes' low and high words: FP32 form nn low, then nn high words (32
-    // banks for either); FP64 form interleaved
     extern __shared__ unsigned sR[];
     __shared__ double sQ, sInvQ;
     __shared__ int sMagic;
@@ -59,7 +65,7 @@ __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, double *rho) 
     const int tk = t % g.ntz, tl = (t / g.ntz) % g.nty, ti = t / (g.ntz * g.nty);
     const int i0 = ti * g.tx, l0 = tl * g.ty, k0 = tk * g.tz;
     const int SX = g.tx + 2, SY = g.ty + 2, SZ = g.tz + 2;
-    const int nn = SX * SY * SZ;
+    const int nn = SX * SY * SZ, stride = rho_stride(nn);
     if (threadIdx.x == 0) {
         double bound = 0.0, one = 0.0;
         for (int s = 0; s < nsp; s++) {
@@ -72,68 +78,72 @@ __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, double *rho) 
         sInvQ = ldexp(1.0, 62 - e2);
         sMagic = one * sInvQ < 0x1p51;
     }
-    for (int idx = threadIdx.x; idx < 2 * nn; idx += blockDim.x) sR[idx] = 0u;
+    for (int idx = threadIdx.x; idx < copies * stride; idx += blockDim.x) sR[idx] = 0u;
     __syncthreads();
     const double inv_q = sInvQ;
-    const bool magic = sMagic != 0;
-    const double h[3] = {g.hx, g.hy, g.hz};
-    const int st = MIXED ? 1 : 2, hi_word = MIXED ? nn : 1;
-    // FP32 form: a warp takes 8 runs of 4 particles out of 8 different places
-    // of the block's 256, so that fewer lanes share a cell (FP64 form: its
-    // 8-byte loads would lose more than that gains)
-    const int lane_of = MIXED ? ((threadIdx.x & 31) >> 2) * 32 + (threadIdx.x >> 5) * 4 + (threadIdx.x & 3) : threadIdx.x;
+    const bool magic = sMagic;
+    const double rhx = 1.0 / g.hx, rhy = 1.0 / g.hy, rhz = 1.0 / g.hz;
+    unsigned *mine = sR + (threadIdx.x & (copies - 1)) * stride;
     for (int s = 0; s < nsp; s++) {
         const SpeciesView &S = sp[s];
         const int start = S.tile_start[t];
         const long long all = S.tile_count[t];
-        const int jbeg = (int)(all * blockIdx.y / gridDim.y), jend = (int)(all * (blockIdx.y + 1) / gridDim.y);
+        const unsigned jbeg = (unsigned)(all * blockIdx.y / gridDim.y), jend = (unsigned)(all * (blockIdx.y + 1) / gridDim.y);
         const double mq = S.m * inv_q;  // exact: inv_q is a power of two
-        for (int j = jbeg + lane_of; j < jend; j += blockDim.x) {
-            const int slot = start + j;
-            const int c = S.cell[slot];
-            if (c < 0) continue;
-            int ci[3];
-            g.cell_ijk(c, ci[0], ci[1], ci[2]);
-            double f[3];
+        const int *cell = S.cell + start;
+        const T *px = MIXED ? (const T *)(S.ox + start) : (const T *)(S.x + start);
+        const T *py = MIXED ? (const T *)(S.oy + start) : (const T *)(S.y + start);
+        const T *pz = MIXED ? (const T *)(S.oz + start) : (const T *)(S.z + start);
+        int nc = -1;
+        T nx = 0, ny = 0, nz = 0;
+        auto load = [&](unsigned j) {
+            nc = -1;
+            if (j < jend) { nc = cell[j]; nx = px[j]; ny = py[j]; nz = pz[j]; }
+        };
+        load(jbeg + threadIdx.x);
+        for (unsigned j = jbeg + threadIdx.x; j < jend; j += blockDim.x) {
+            const int c = nc;
+            const T x = nx, y = ny, z = nz;
+            load(j + blockDim.x);
+            int i, l, k;
+            g.cell_ijk(c, i, l, k);
+            double fx, fy, fz;
             if (MIXED) {
-                f[0] = (double)S.ox[slot];
-                f[1] = (double)S.oy[slot];
-                f[2] = (double)S.oz[slot];
+                fx = (double)x; fy = (double)y; fz = (double)z;
             } else {
-                const double x[3] = {S.x[slot], S.y[slot], S.z[slot]};
-                for (int a = 0; a < 3; a++) f[a] = x[a] / h[a] - (double)ci[a];
+                fx = div_by(x, g.hx, rhx) - (double)i;
+                fy = div_by(y, g.hy, rhy) - (double)l;
+                fz = div_by(z, g.hz, rhz) - (double)k;
             }
-            int lo[3];
-            double w1[3];
-            const int org[3] = {i0, l0, k0};
-            bool ok = true;
-            for (int a = 0; a < 3; a++) {
-                const int up = f[a] >= 0.5;
-                w1[a] = f[a] + 0.5 - (double)up;
-                lo[a] = ci[a] + up - org[a];  // tile-local index of the lower node
-                ok = ok && lo[a] >= 0 && lo[a] + 1 < (a == 0 ? SX : a == 1 ? SY : SZ);
-            }
-            if (!ok) continue;  // a bin entry outside its tile (never expected)
-            unsigned *R = sR + st * ((lo[0] * SY + lo[1]) * SZ + lo[2]);
-            const double wx[2] = {mq * (1.0 - w1[0]), mq * w1[0]}, wy[2] = {1.0 - w1[1], w1[1]},
-                         wz[2] = {1.0 - w1[2], w1[2]};
+            const bool ux = fx >= 0.5, uy = fy >= 0.5, uz = fz >= 0.5;
+            // weights of the upper node
+            const double ax = fx + (ux ? -0.5 : 0.5), ay = fy + (uy ? -0.5 : 0.5), az = fz + (uz ? -0.5 : 0.5);
+            // tile-local lower node
+            i += (int)ux - i0; l += (int)uy - l0; k += (int)uz - k0;
+            // a dead slot, or a bin entry outside its tile (never expected)
+            if (c < 0 || (unsigned)i >= (unsigned)SX - 1u || (unsigned)l >= (unsigned)SY - 1u || (unsigned)k >= (unsigned)SZ - 1u)
+                continue;
+            unsigned *R = mine + (i * SY + l) * SZ + k;
+            const double wx[2] = {mq * (1.0 - ax), mq * ax}, wy[2] = {1.0 - ay, ay}, wz[2] = {1.0 - az, az};
 #pragma unroll
             for (int b = 0; b < 4; b++) {
                 const double wxy = wx[b >> 1] * wy[b & 1];
-                unsigned *r = R + st * (((b >> 1) * SY + (b & 1)) * SZ);
-#pragma unroll
-                for (int az = 0; az < 2; az++) {
-                    const double v = wxy * wz[az];
-                    const long long iv = magic ? __double_as_longlong(v + 0x1.8p52) - 0x4338000000000000ll
-                                               : __double2ll_rn(v);
-                    if (iv) shared_add64(r + st * az, r + st * az + hi_word, iv);
+                unsigned *r = R + ((b >> 1) * SY + (b & 1)) * SZ;
+                if (magic) {
+                    shared_add_rounded(r, r + nn, fma(wxy, wz[0], kRound));
+                    shared_add_rounded(r + 1, r + 1 + nn, fma(wxy, wz[1], kRound));
+                } else {
+                    shared_add64(r, r + nn, __double2ll_rn(wxy * wz[0]));
+                    shared_add64(r + 1, r + 1 + nn, __double2ll_rn(wxy * wz[1]));
                 }
             }
         }
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < nn; idx += blockDim.x) {
-        const long long v = (long long)(((unsigned long long)sR[st * idx + hi_word] << 32) | sR[st * idx]);
+        long long v = 0;
+        for (int q = 0; q < copies; q++)
+            v += (long long)(((unsigned long long)sR[q * stride + nn + idx] << 32) | sR[q * stride + idx]);
         if (v == 0) continue;
         const int c = idx % SZ, b = (idx / SZ) % SY, a = idx / (SZ * SY);
         if (i0 + a < g.NX && l0 + b < g.NY && k0 + c < g.NZ) atomicAdd(&rho[g.node(i0 + a, l0 + b, k0 + c)], (double)v * sQ);
@@ -258,13 +268,16 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
     const Grid &g = p.g;
     cudaError_t e = cudaMemsetAsync(rho, 0, g.nodes_pitched() * sizeof(double), s);
     if (e != cudaSuccess) return e;
-    const size_t smem = (size_t)(g.tx + 2) * (g.ty + 2) * (g.tz + 2) * sizeof(unsigned long long);
+    const size_t box = rho_stride((g.tx + 2) * (g.ty + 2) * (g.tz + 2)) * sizeof(unsigned);
+    int copies = kRhoCopies;
+    while (copies > 1 && copies * box > (size_t)kRhoBytes) copies /= 2;
+    const size_t smem = copies * box;
     auto *k = p.mixed ? k_charge_tile<true> : k_charge_tile<false>;
     if (smem > 48 * 1024) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<dim3(g.ntiles, tile_shares(g.ntiles)), 256, smem, s>>>(p, rho);
+    k<<<dim3(g.ntiles, tile_shares(g.ntiles)), 256, smem, s>>>(p, copies, rho);
     for (int dir = 0; dir < 3; dir++) {
         const int A = dir == 0 ? g.NY : g.NX;
         const int B = dir == 2 ? g.NY : g.NZ;

@@ -174,6 +174,13 @@ __device__ __forceinline__ double fx_split(double s, long long &ih) {
     ih = __double_as_longlong(u) - 0x4338000000000000ll;
     return s - (u - kRound);  // the exact remainder
 }
+// a contribution rounded by u = s + kRound, into a node's low and high word
+__device__ __forceinline__ void shared_add_rounded(unsigned *plo, unsigned *phi, double u) {
+    const unsigned lo = (unsigned)__double2loint(u);
+    const unsigned old = atomicAdd(plo, lo);
+    const unsigned hi = (unsigned)__double2hiint(u) - 0x43380000u + (old + lo < old ? 1u : 0u);
+    if (hi) atomicAdd(phi, hi);
+}
 __device__ __forceinline__ void fx_put2(unsigned long long *hi, unsigned long long *lo, double s) {
     long long ih;
     const double r = fx_split(s, ih);

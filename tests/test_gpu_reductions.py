@@ -55,3 +55,24 @@ def test_reductions_match_numpy(pkg, oracle_mod, cells, ppc, precision):
     b = 0.5 * sum((F[f][inner] ** 2).sum() for f in ("Hx", "Hy", "Hz"))
     np.testing.assert_allclose(en, [e, b, kin, e + b + kin], rtol=1e-12)
     np.testing.assert_allclose(ref, sum((F[f] ** 2).sum() for f in ("Ex", "Ey", "Ez")), rtol=1e-12)
+
+
+@pytest.mark.parametrize("tile,precision", [((1, 1, 4), "fp64"), ((1, 1, 4), "fp32"), ((4, 4, 8), "fp64"), ((8, 8, 8), "fp64"),
+                                            ((8, 8, 8), "fp32"), ((10, 8, 12), "fp64")])
+def test_rho_boxes_per_block(pkg, oracle_mod, tile, precision):
+    # 8, 8, 4 and 2 boxes fit (the FP32 push takes no tile as large as the
+    # last); ragged tiles, both ways to round a contribution
+    cells, ppc, h = (21, 9, 25), 40, (0.1, 0.1, 0.1)
+    L = tuple(c * v for c, v in zip(cells, h))
+    table = pkg.configs.species_table(ppc)
+    with pkg.PicSimulation(cells, L, 0.01, table, precision=precision, tile=tile) as sim:
+        for i in range(3):
+            sim.init_species(i, ppc, (0.1, 0.0, -0.05), 0.3, 9 + i)
+        parts = [sim.particles(i) for i in range(3)]
+        rho = sim.charge_density()
+    x = [np.concatenate([p[k] for p in parts]) for k in "xyz"]
+    m = np.concatenate([np.full(p["x"].size, table[i][1]) for i, p in enumerate(parts)])
+    # the neutral sum cancels: against the sum of |charge| each node receives
+    want = oracle_mod.charge_density(*x, m, cells, h)
+    scale = oracle_mod.charge_density(*x, np.abs(m), cells, h)
+    assert np.linalg.norm(rho - want) <= 1e-12 * np.linalg.norm(scale)
