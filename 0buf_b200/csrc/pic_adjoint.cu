@@ -389,6 +389,7 @@ __device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow &w, 
 // and currents added to global memory, one particle per thread).
 template <int BMODE>
 __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow sWin;
     __shared__ int sRed[15 * kW], sQn[kW];
@@ -834,6 +835,7 @@ __device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
 // cells: 3.3 -> 2.3 ms per reverse step (before: two kernels, lambda of the
 // field values and the fields themselves passed through global memory).
 __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_constant__ AdjParams A) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow sWin;
     __shared__ int sRed[15 * kW], sFar;
@@ -996,10 +998,12 @@ struct FieldAdj {
 // E update transpose (5) and the start of B completion's transpose (4):
 //   lambda_J = -tau lambda_E on the E ranges, lambda_H += C^T lambda_E,
 //   lambda_Q = lambda_H (new) on the H ranges
-__global__ void k_adj_e_update(FieldAdj A) {
+__global__ void k_adj_e_update(const __grid_constant__ FieldAdj A) {
+    chain_enter();
     const Grid &g = A.g;
-    int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
-    if (k >= g.NZ) return;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;  // node of an x plane
+    if (q >= g.NY * g.NZ) return;
+    const int l = q / g.NZ, k = q - l * g.NZ, i = blockIdx.y;
     size_t m = g.node(i, l, k);
     auto LEv = [&](int c, int di, int dl, int dk) -> double {
         return in_E(g, c, i + di, l + dl, k + dk) ? A.LE[c][g.node(i + di, l + dl, k + dk)] : 0.0;
@@ -1021,11 +1025,16 @@ __global__ void k_adj_e_update(FieldAdj A) {
 
 // transpose of the B half step (1): lambda_Q += lambda_H_a on the H ranges,
 // lambda_E += A^T lambda_Q (gather form: each E node collects from the Q
-// nodes whose difference reads it)
-__global__ void k_adj_b_half(FieldAdj A) {
+// nodes whose difference reads it).  Then the loss injection of the step before
+// (inject: its E after the step, of component comp; null: none):
+// lambda_E_comp += w2 E on nodes 1..N
+template <typename T>
+__global__ void k_adj_b_half(const __grid_constant__ FieldAdj A, const T *__restrict__ inject, int comp, double w2) {
+    chain_enter();
     const Grid &g = A.g;
-    int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
-    if (k >= g.NZ) return;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;  // node of an x plane
+    if (q >= g.NY * g.NZ) return;
+    const int l = q / g.NZ, k = q - l * g.NZ, i = blockIdx.y;
     size_t m = g.node(i, l, k);
     auto LQt = [&](int c, int di, int dl, int dk) -> double {
         int a = i + di, b = l + dl, cc = k + dk;
@@ -1043,23 +1052,7 @@ __global__ void k_adj_b_half(FieldAdj A) {
     A.LE[0][m] += lex;
     A.LE[1][m] += ley;
     A.LE[2][m] += lez;
-}
-
-// H_a = H + Q(E) (the forward B half step, out of place, same rounding)
-__global__ void k_h_half(Grid g, const double *__restrict__ Ex, const double *__restrict__ Ey,
-                         const double *__restrict__ Ez, const double *__restrict__ Hx, const double *__restrict__ Hy,
-                         const double *__restrict__ Hz, double *Ax, double *Ay, double *Az, double cx, double cy,
-                         double cz) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
-    if (k >= g.NZ) return;
-    size_t n = g.node(i, l, k), sx = (size_t)g.NY * g.pz, sy = g.pz;
-    double hx = Hx[n], hy = Hy[n], hz = Hz[n];
-    if (i <= g.nx + 1 && l <= g.ny && k <= g.nz) hx += 0.5 * (cz * (Ey[n + 1] - Ey[n]) - cy * (Ez[n + sy] - Ez[n]));
-    if (i <= g.nx && l <= g.ny + 1 && k <= g.nz) hy += 0.5 * (cx * (Ez[n + sx] - Ez[n]) - cz * (Ex[n + 1] - Ex[n]));
-    if (i <= g.nx && l <= g.ny && k <= g.nz + 1) hz += 0.5 * (cy * (Ex[n + sy] - Ex[n]) - cx * (Ey[n + sx] - Ey[n]));
-    Ax[n] = hx;
-    Ay[n] = hy;
-    Az[n] = hz;
+    if (inject && k >= 1 && k <= g.nz && l >= 1 && l <= g.ny && i >= 1 && i <= g.nx) A.LE[comp][m] += w2 * (double)inject[m];
 }
 
 // lines of one axis (getGlobalBoundaryCellNumber, cell.h:885-889)
@@ -1071,6 +1064,7 @@ __device__ __forceinline__ void line_g(const Grid &g, int dir, int a, int b, siz
 
 // transpose of the J fold (pic_fold.cuh)
 __global__ void k_adj_j_fold(Grid g, double *Lx, double *Ly, double *Lz) {
+    chain_enter();
     double *const L[3] = {Lx, Ly, Lz};
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < fold_orbits(g)) fold_adjoint(g, L, idx);
@@ -1086,6 +1080,7 @@ struct GPasses {
     int n;
 };
 __global__ void k_adj_ghosts(Grid g, GPasses P) {
+    chain_enter();
     if ((int)blockIdx.y >= P.n) return;
     GPass q = P.p[blockIdx.y];
     int A = q.e1 - q.s1 + 1, B = q.e2 - q.s2 + 1;
@@ -1101,39 +1096,13 @@ __global__ void k_adj_ghosts(Grid g, GPasses P) {
     L[0] = 0.0;
 }
 
-// loss injection: lambda_E_c += 2 w E_c on nodes 1..N; history sums
+// loss injection of the last step: lambda_E_c += 2 w E_c on nodes 1..N
 template <typename T>
 __global__ void k_inject(Grid g, const T *__restrict__ E, double *LE, double w2) {
     int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
     if (k < 1 || k > g.nz || l < 1 || l > g.ny || i < 1 || i > g.nx) return;
     size_t n = g.node(i, l, k);
     LE[n] += w2 * (double)E[n];
-}
-
-template <typename T>
-__global__ void k_history(Grid g, const T *__restrict__ Ex, const T *__restrict__ Ey, const T *__restrict__ Ez,
-                          double *out3) {
-    __shared__ double red[3][kT / 32];
-    int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
-    double a = 0.0, b = 0.0, c = 0.0;
-    if (k >= 1 && k <= g.nz && l >= 1 && l <= g.ny && i >= 1 && i <= g.nx) {
-        size_t n = g.node(i, l, k);
-        double ex = (double)Ex[n], ey = (double)Ey[n], ez = (double)Ez[n];
-        a = ex * ex; b = ey * ey; c = ez * ez;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-    }
-    int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if ((threadIdx.x & 31) == 0) { red[0][w] = a; red[1][w] = b; red[2][w] = c; }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double s = 0.0;
-        for (int q = 0; q < nw; q++) s += red[threadIdx.x][q];
-        atomicAdd(&out3[threadIdx.x], s);
-    }
 }
 
 // bins -> flat order (tile by tile, slot order): packed cell and FP64 values
@@ -1210,6 +1179,7 @@ __global__ void k_interleave(int64_t n, const double *__restrict__ a, const doub
 }
 
 inline dim3 node_grid(const Grid &g) { return dim3((g.NZ + 31) / 32, g.NY, g.NX); }
+inline dim3 plane_blocks(const Grid &g) { return dim3((g.NY * g.NZ + kT - 1) / kT, g.NX); }
 inline unsigned blocks_of(int64_t n) { return (unsigned)((n + kT - 1) / kT); }
 
 }  // namespace
@@ -1286,26 +1256,35 @@ int64_t total_particles(const AdjState &A) {
     return t;
 }
 
-// one forward step of the flat state on the field set F (plain): particles
-// read from `state`, written to `out` (the same buffer when out is null)
-int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out = nullptr) {
+// one forward step of the flat state on the field set F (plain): particles read
+// from `state`, written to `out` (the same buffer when out is null).  keep: E and
+// the half-step H of the step go there (six arrays; null: the half-step H to A.ha).
+// hist: receives the sums of E_c^2 after the step (null: none).
+// Five chained launches (before: eight operations, one after the other, and a
+// copy of the fields in a recompute); the reverse of a step is six (before:
+// eight).  Small runs wait on them: 16x8x8 cells, 24.6k particles, FP64 forward
+// 33.0 -> 26.1 us per step, backward 93.8 -> 70.7; 64x32x32 cells, 3.1M FP32
+// 201 -> 187 and 662 -> 630.
+int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, char *keep,
+                    double *hist) {
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
-    yee_b_half_plain(g, (double *const *)F, s);
-    size_t nodes = g.nodes_pitched();
-    CK(cudaMemsetAsync(F[PIC_JX], 0, 3 * nodes * sizeof(double), s), "zero J");  // the three lie one after another
+    const size_t N = g.nodes_pitched();
+    double *Ha = keep ? (double *)keep + 3 * N : (double *)A.ha;
+    flat_begin_plain(g, (const double *const *)&F[PIC_EX], (const double *const *)&F[PIC_HX], Ha, (double *)F[PIC_JX],
+                     (double *)keep, s);  // J: the three arrays lie one after another
     FlatParams P = flat_params(h, A, state, F, out);
+    for (int c = 0; c < 3; c++) P.H[c] = Ha + c * N;
     if (A.nchunks > 0) {
         auto *kern = P.bmode == 0 ? k_flat_push_plain<0> : (P.bmode == 1 ? k_flat_push_plain<1> : k_flat_push_plain<2>);
         const size_t smem = (size_t)kFlatWindow * (6 * sizeof(double) + 3 * 12) + (size_t)kW * kQueuePlain * 52 + kNextBytes;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "flat push");
-        kern<<<A.nchunks, kT, smem, s>>>(P);
+        CK(launch_chained_smem(kern, dim3(A.nchunks), dim3(kT), smem, s, P), "flat push");
     }
-    CK(cudaGetLastError(), "flat push");
-    fold_b_plain(g, (double *const *)F, s);
+    fold_b_twice_plain(g, (double *const *)F, s);
     yee_e_update_plain(g, (double *const *)F, s);
     e_ghosts_plain(g, (double *)F[PIC_EX], (double *)F[PIC_EY], (double *)F[PIC_EZ],
-                   h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s);
+                   h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist);
     CK(cudaGetLastError(), "flat step fields");
     return PIC_OK;
 }
@@ -1446,23 +1425,23 @@ MixParams mix_params(pic_handle *h, AdjState &A, char *state, void *const F[PIC_
     return P;
 }
 
-// one forward step of the fixed-order state on the field set F: particles
-// read from `state`, written to `out` (same buffer when null)
-int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out) {
-    if (!h->mixed) return flat_step_plain(h, A, state, F, out);
+// one forward step of the fixed-order state on the field set F (see flat_step_plain)
+int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, char *keep,
+              double *hist) {
+    if (!h->mixed) return flat_step_plain(h, A, state, F, out, keep, hist);
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
     float *const *E = (float *const *)&F[PIC_EX];
     float *const *H = (float *const *)&F[PIC_HX];
-    yee_b_half_mixed(g, E, H, s);
-    const size_t nodes = g.nodes_pitched();
-    CK(cudaMemsetAsync(F[PIC_JX], 0, 3 * nodes * sizeof(double), s), "zero J");  // the three lie one after another
+    const size_t N = g.nodes_pitched();
+    float *Ha = keep ? (float *)keep + 3 * N : (float *)A.ha;
+    flat_begin_mixed(g, (const float *const *)E, (const float *const *)H, Ha, (double *)F[PIC_JX], (float *)keep, s);
     MixParams P = mix_params(h, A, state, F, out);
+    for (int c = 0; c < 3; c++) P.H[c] = Ha + c * N;
     CK(launch_flat_push_mixed(P, A.nchunks, s), "flat push");
-    j_fold(g, (double *)F[PIC_JX], (double *)F[PIC_JY], (double *)F[PIC_JZ], s);
-    yee_b_half_mixed(g, E, H, s);  // completion: the same Q again
+    fold_b_mixed(g, E, H, (double *const *)&F[PIC_JX], s);
     yee_e_update_mixed(g, E, H, (double *const *)&F[PIC_JX], s);
-    e_ghosts_mixed(g, E[0], E[1], E[2], h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s);
+    e_ghosts_mixed(g, E[0], E[1], E[2], h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist);
     CK(cudaGetLastError(), "flat step fields");
     return PIC_OK;
 }
@@ -1488,27 +1467,20 @@ int forward_run(pic_handle *h, AdjState &A) {
             A.step_branch = const_cast<unsigned long long *>(A.branch_src) + (size_t)n * np_all;
             A.step_bmode = 2;
         }
-        int rc = flat_step(h, A, A.cur, h->f, nullptr);
+        int rc = flat_step(h, A, A.cur, h->f, nullptr, nullptr, A.hist + 3 * n);
         A.step_branch = nullptr;
         A.step_bmode = 0;
         if (rc) return rc;
-        if (h->mixed)
-            k_history<float><<<node_grid(g), 32, 0, st>>>(g, (const float *)h->f[PIC_EX], (const float *)h->f[PIC_EY],
-                                                          (const float *)h->f[PIC_EZ], A.hist + 3 * n);
-        else
-            k_history<double><<<node_grid(g), 32, 0, st>>>(g, (const double *)h->f[PIC_EX],
-                                                           (const double *)h->f[PIC_EY],
-                                                           (const double *)h->f[PIC_EZ], A.hist + 3 * n);
-        CK(cudaGetLastError(), "history");
     }
     CK(cudaEventRecord(A.e1, st), "event");
     return PIC_OK;
 }
 
-// reverse of step n: EHn = E_n, H_n of the step (form's type, 6 arrays),
-// Enext = E after the step
-int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *state, const char *EHn,
-                 const char *Enext) {
+// reverse of step n: EH = E before the step and H after its half step (form's
+// type, 6 arrays); last: E after the step, for the last step of the run (else null).
+// The loss of the other steps is injected at the end of the reverse of the step
+// after them, whose E before the step is their E after it.
+int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *state, const char *EH, const char *last) {
     const Grid &g = h->g;
     cudaStream_t st = h->stream;
     const size_t N = g.nodes_pitched();
@@ -1520,10 +1492,9 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
         LJ[c] = A.lamf + (6 + c) * N;
         LQ[c] = A.lamf + (9 + c) * N;
     }
-    // loss injection at E_{n+1}
-    if (n >= A.steps - L.window) {
-        double w2 = 2.0 * g.hx * g.hy * g.hz;
-        const char *Ec = Enext + (size_t)L.field * fb;
+    const double w2 = 2.0 * g.hx * g.hy * g.hz;
+    if (last && L.window >= 1) {
+        const char *Ec = last + (size_t)L.field * fb;
         if (h->mixed) k_inject<float><<<node_grid(g), 32, 0, st>>>(g, (const float *)Ec, LE[L.field], w2);
         else k_inject<double><<<node_grid(g), 32, 0, st>>>(g, (const double *)Ec, LE[L.field], w2);
     }
@@ -1532,8 +1503,8 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
     int maxn;
     ghost_passes(g, LE, h->cfg.ghosts == PIC_GHOSTS_PERIODIC, GA, GB, maxn);
     dim3 gg((maxn + 127) / 128, 3);
-    k_adj_ghosts<<<gg, 128, 0, st>>>(g, GB);
-    k_adj_ghosts<<<gg, 128, 0, st>>>(g, GA);
+    launch_chained(k_adj_ghosts, gg, dim3(128), st, g, GB);
+    launch_chained(k_adj_ghosts, gg, dim3(128), st, g, GA);
     FieldAdj FA;
     FA.g = g;
     FA.cx = g.tau / g.hx;
@@ -1541,23 +1512,17 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
     FA.cz = g.tau / g.hz;
     FA.tau = g.tau;
     for (int c = 0; c < 3; c++) { FA.LE[c] = LE[c]; FA.LH[c] = LH[c]; FA.LJ[c] = LJ[c]; FA.LQ[c] = LQ[c]; }
-    k_adj_e_update<<<node_grid(g), 32, 0, st>>>(FA);
-    k_adj_j_fold<<<(fold_orbits(g) + 127) / 128, 128, 0, st>>>(g, LJ[0], LJ[1], LJ[2]);
+    launch_chained(k_adj_e_update, plane_blocks(g), dim3(kT), st, FA);
+    launch_chained(k_adj_j_fold, dim3((fold_orbits(g) + 127) / 128), dim3(128), st, g, LJ[0], LJ[1], LJ[2]);
+    void *F[PIC_FIELD_COUNT] = {};
+    for (int c = 0; c < 6; c++) F[PIC_EX + c] = (void *)(EH + c * fb);
+    // E before this step, where the step before it has a loss term
+    const char *inject = n >= 1 && n - 1 >= A.steps - L.window ? EH + (size_t)L.field * fb : nullptr;
+    size_t o = 0;
     if (!h->mixed) {
-        // H_a of step n
-        const double *En = (const double *)EHn, *Hn = (const double *)EHn + 3 * N;
-        double *Ha = (double *)A.ha;
-        k_h_half<<<node_grid(g), 32, 0, st>>>(g, En, En + N, En + 2 * N, Hn, Hn + N, Hn + 2 * N, Ha, Ha + N,
-                                              Ha + 2 * N, FA.cx, FA.cy, FA.cz);
-        void *F[PIC_FIELD_COUNT] = {};
-        for (int c = 0; c < 3; c++) {
-            F[PIC_EX + c] = (void *)(En + c * N);
-            F[PIC_HX + c] = (void *)(Ha + c * N);
-        }
         AdjParams P;
         memset(&P, 0, sizeof(P));
         P.f = flat_params(h, A, state, F);
-        size_t o = 0;
         for (int s = 0; s < A.nsp; s++) {
             for (int a = 0; a < 6; a++) P.lam[s].v[a] = (double *)A.lamp + o + (size_t)a * A.n[s];
             o += 6 * (size_t)A.n[s];
@@ -1567,27 +1532,19 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
             const size_t smem = (size_t)kAdjWindow * 120 + kNextBytes + kNextLamBytes + kAdjChunk * sizeof(unsigned short);
             CK(cudaFuncSetAttribute(k_adj_particles_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "adjoint particles");
-            k_adj_particles_plain<<<A.nchunks, kT, smem, st>>>(P);
+            CK(launch_chained_smem(k_adj_particles_plain, dim3(A.nchunks), dim3(kT), smem, st, P), "adjoint particles");
         }
+        launch_chained(k_adj_b_half<double>, plane_blocks(g), dim3(kT), st, FA, (const double *)inject, L.field, w2);
     } else {
-        const float *En = (const float *)EHn, *Hn = (const float *)EHn + 3 * N;
-        float *Ha = (float *)A.ha;
-        CK(launch_h_half_mixed(g, En, Hn, Ha, N, st), "half step");
-        void *F[PIC_FIELD_COUNT] = {};
-        for (int c = 0; c < 3; c++) {
-            F[PIC_EX + c] = (void *)(En + c * N);
-            F[PIC_HX + c] = (void *)(Ha + c * N);
-        }
         MixParams P = mix_params(h, A, state, F, nullptr);
-        size_t o = 0;
         for (int s = 0; s < A.nsp; s++) {
             for (int a = 0; a < 6; a++) P.lam[s][a] = (float *)A.lamp + o + (size_t)a * A.n[s];
             o += 6 * (size_t)A.n[s];
         }
         for (int c = 0; c < 3; c++) { P.LJ[c] = LJ[c]; P.LE[c] = LE[c]; P.LH[c] = LH[c]; }
         CK(launch_adj_particles_mixed(P, A.nchunks, st), "adjoint particles");
+        launch_chained(k_adj_b_half<float>, plane_blocks(g), dim3(kT), st, FA, (const float *)inject, L.field, w2);
     }
-    k_adj_b_half<<<node_grid(g), 32, 0, st>>>(FA);
     CK(cudaGetLastError(), "reverse step");
     return PIC_OK;
 }
@@ -1621,7 +1578,7 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
                        "sub-checkpoint fields");
                     if (q == nsub - 1) break;  // the last sub-segment starts here
                 }
-                int rc = flat_step(h, A, A.segp, RF, nullptr);
+                int rc = flat_step(h, A, A.segp, RF, nullptr, nullptr, nullptr);
                 if (rc) return rc;
             }
         }
@@ -1632,14 +1589,13 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
             CK(cudaMemcpyAsync(A.segp, sp, A.pbytes, cudaMemcpyDeviceToDevice, st), "restore");
             CK(cudaMemcpyAsync(A.rf, sf, ehb, cudaMemcpyDeviceToDevice, st), "restore fields");
             for (int j = 0; j < slen; j++) {
-                CK(cudaMemcpyAsync(A.segf + (size_t)j * ehb, A.rf, ehb, cudaMemcpyDeviceToDevice, st), "keep fields");
-                int rc = flat_step(h, A, A.segp + (size_t)j * A.pbytes, RF, A.segp + (size_t)(j + 1) * A.pbytes);
+                int rc = flat_step(h, A, A.segp + (size_t)j * A.pbytes, RF, A.segp + (size_t)(j + 1) * A.pbytes,
+                                   A.segf + (size_t)j * ehb, nullptr);
                 if (rc) return rc;
             }
-            CK(cudaMemcpyAsync(A.segf + (size_t)slen * ehb, A.rf, ehb, cudaMemcpyDeviceToDevice, st), "keep fields");
             for (int j = slen - 1; j >= 0; j--) {
                 int rc = reverse_step(h, A, L, s0 + j, A.segp + (size_t)j * A.pbytes, A.segf + (size_t)j * ehb,
-                                      A.segf + (size_t)(j + 1) * ehb);
+                                      s0 + j == A.steps - 1 ? A.rf : nullptr);
                 if (rc) return rc;
             }
         }
@@ -1738,6 +1694,7 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     if ((rc = adj_alloc(h, kAdjHist, (void **)&A.hist, sizeof(double) * 3 * steps, "the history"))) return rc;
     if ((rc = adj_alloc(h, kAdjSt, (void **)&A.st, sizeof(AdjStatus), "the status"))) return rc;
     if ((rc = adj_alloc(h, kAdjRed, (void **)&A.red, sizeof(double) * 8, "the reduction scratch"))) return rc;
+    if ((rc = adj_alloc(h, kAdjHa, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
     if ((rc = adj_alloc(h, kAdjChunks, (void **)&A.chunks, sizeof(AdjChunk) * chunks.size(), "the chunk table"))) return rc;
     CK(cudaMemcpyAsync(A.chunks, chunks.data(), sizeof(AdjChunk) * chunks.size(), cudaMemcpyHostToDevice, h->stream),
        "chunk table");
@@ -1881,7 +1838,7 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
     int64_t np = total_particles(A);
     if (!A.segp) {
         if ((rc = adj_alloc(h, kAdjSegp, (void **)&A.segp, A.pbytes * (size_t)(A.K2 + 1), "the segment states"))) return rc;
-        if ((rc = adj_alloc(h, kAdjSegf, (void **)&A.segf, fbytes * 6 * (size_t)(A.K2 + 1), "the segment fields"))) return rc;
+        if ((rc = adj_alloc(h, kAdjSegf, (void **)&A.segf, fbytes * 6 * (size_t)A.K2, "the segment fields"))) return rc;
         if (A.K2 < A.K) {
             const size_t nsub = (size_t)(A.K + A.K2 - 1) / A.K2;
             if ((rc = adj_alloc(h, kAdjSubp, (void **)&A.subp, A.pbytes * nsub, "the sub-checkpoint states"))) return rc;
@@ -1892,7 +1849,6 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
         if ((rc = adj_alloc(h, kAdjLamf, (void **)&A.lamf, N * sizeof(double) * 12, "the field adjoints"))) return rc;
         if ((rc = adj_alloc(h, kAdjRf, (void **)&A.rf, N * sizeof(double) * PIC_FIELD_COUNT, "the recompute fields")))
             return rc;
-        if ((rc = adj_alloc(h, kAdjHa, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
     }
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     rc = backward_run(h, A, *loss);

@@ -56,14 +56,14 @@ struct AdjState {
     char *ckp;         // nseg particle checkpoints
     char *ckf;         // nseg x (E, H): 6 field arrays each, in the form's field type
     char *segp;        // K2+1 particle states of the (sub-)segment being reversed
-    char *segf;        // K2+1 x (E, H) of that (sub-)segment
+    char *segf;        // K2 x (E, H after the half step) of that (sub-)segment's steps
     char *subp;        // two levels: ceil(K/K2) sub-checkpoint states of the segment being reversed
     char *subf;        // two levels: their (E, H)
     char *lamp;        // per species lambda_x (3) and lambda_p (3), form's element type
     size_t lamp_bytes;
     double *lamf;      // FP64 lambda_E, lambda_H, lambda_J, lambda_Q (12 arrays)
     char *rf;          // field set of the recompute (form's layout: 12 arrays)
-    char *ha;          // B after the half step of the step being reversed (3 arrays)
+    char *ha;          // B after the half step of a step whose fields are not kept (3 arrays)
     AdjChunk *chunks;  // nchunks of them, device
     int nchunks;
     double *hist;      // steps x 3: sum over nodes 1..N of E_c^2 after each step
@@ -216,8 +216,6 @@ struct MixParams {
 };
 cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, cudaStream_t s);
 cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStream_t s);
-// Ha = H + Q(E) in FP32 (the forward's half step, out of place); E, H, Ha: 3 arrays of N each
-cudaError_t launch_h_half_mixed(const Grid &g, const float *E, const float *H, float *Ha, size_t N, cudaStream_t s);
 void adj_gather_mixed(const Grid &g, const SpeciesView &S, const int64_t *d0, int *cell, void *const v[6],
                       cudaStream_t s);
 // lambda_p (3 FP32 arrays of n) and p0 (3 FP32 arrays) -> 6 FP64 arrays of n

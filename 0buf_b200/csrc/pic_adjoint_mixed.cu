@@ -308,6 +308,7 @@ __device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow &w
 // 64 registers: 0.688; lanes spread over 4 or 8 places: 0.625, 0.660, and slower
 // at 3M particles).
 __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant__ MixParams P) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow sWin;
     __shared__ int sRed[15 * kW], sQn[kW];
@@ -616,6 +617,7 @@ __device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j)
 // 1.37 ms per reverse step (two CTAs per SM at 128 registers: 1.46; before: two
 // kernels that gathered from global memory).
 __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_constant__ MixParams P) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow sWin;
     __shared__ int sRed[15 * kW], sFar;
@@ -736,22 +738,6 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     for (int e = threadIdx.x; e < sFar; e += blockDim.x) reverse_far_m(P, s, ch.first + sList[e]);
 }
 
-__global__ void k_h_half_m(Grid g, const float *__restrict__ Ex, const float *__restrict__ Ey,
-                           const float *__restrict__ Ez, const float *__restrict__ Hx, const float *__restrict__ Hy,
-                           const float *__restrict__ Hz, float *Ax, float *Ay, float *Az, float cx, float cy,
-                           float cz) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, i = blockIdx.z;
-    if (k >= g.NZ) return;
-    size_t n = g.node(i, l, k), sx = (size_t)g.NY * g.pz, sy = g.pz;
-    float hx = Hx[n], hy = Hy[n], hz = Hz[n];
-    if (i <= g.nx + 1 && l <= g.ny && k <= g.nz) hx += 0.5f * (cz * (Ey[n + 1] - Ey[n]) - cy * (Ez[n + sy] - Ez[n]));
-    if (i <= g.nx && l <= g.ny + 1 && k <= g.nz) hy += 0.5f * (cx * (Ez[n + sx] - Ez[n]) - cz * (Ex[n + 1] - Ex[n]));
-    if (i <= g.nx && l <= g.ny && k <= g.nz + 1) hz += 0.5f * (cy * (Ex[n + sy] - Ex[n]) - cx * (Ey[n + sx] - Ey[n]));
-    Ax[n] = hx;
-    Ay[n] = hy;
-    Az[n] = hz;
-}
-
 __global__ void k_gather_native(SpeciesView S, const int64_t *__restrict__ d0, int *cell, float *ox, float *oy,
                                 float *oz, float *px, float *py, float *pz) {
     int t = blockIdx.x;
@@ -784,8 +770,7 @@ cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, cudaStream_t
     const size_t smem = (size_t)kFlatWindowMix * 48 + (size_t)kW * 7 * kQueueMix * sizeof(float) + NextMix<6>::bytes;
     cudaError_t e = cudaFuncSetAttribute(k_flat_push_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_flat_push_mixed<<<nchunks, kT, smem, s>>>(P);
-    return cudaGetLastError();
+    return launch_chained_smem(k_flat_push_mixed, dim3(nchunks), dim3(kT), smem, s, P);
 }
 
 cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStream_t s) {
@@ -793,15 +778,7 @@ cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStre
     const size_t smem = (size_t)kAdjWindowMix * 84 + NextMix<12>::bytes + kAdjChunk * sizeof(unsigned short);
     cudaError_t e = cudaFuncSetAttribute(k_adj_particles_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_adj_particles_mixed<<<nchunks, kT, smem, s>>>(P);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_h_half_mixed(const Grid &g, const float *E, const float *H, float *Ha, size_t N, cudaStream_t s) {
-    float cx = (float)(g.tau / g.hx), cy = (float)(g.tau / g.hy), cz = (float)(g.tau / g.hz);
-    dim3 grid((g.NZ + 31) / 32, g.NY, g.NX);
-    k_h_half_m<<<grid, 32, 0, s>>>(g, E, E + N, E + 2 * N, H, H + N, H + 2 * N, Ha, Ha + N, Ha + 2 * N, cx, cy, cz);
-    return cudaGetLastError();
+    return launch_chained_smem(k_adj_particles_mixed, dim3(nchunks), dim3(kT), smem, s, P);
 }
 
 void adj_gather_mixed(const Grid &g, const SpeciesView &S, const int64_t *d0, int *cell, void *const v[6],

@@ -95,11 +95,12 @@ __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&... args) {
+inline cudaError_t launch_chained_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                       A &&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -107,6 +108,10 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, c
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&... args) {
+    return launch_chained_smem(kernel, grid, block, 0, s, std::forward<A>(args)...);
 }
 
 // Tile current accumulation in 64-bit fixed point.  Each contribution is

@@ -12,11 +12,23 @@ void yee_e_update_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void j_fold(const Grid &g, double *Jx, double *Jy, double *Jz, cudaStream_t s);
 // the J fold and the B completion in one launch
 void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s);
-// st, out: device status and pinned host memory that receives it (null: none)
+// st, out: device status and pinned host memory that receives it (null: none);
+// hist: three sums that receive E_c^2 over the nodes 1..N (null: none)
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st = nullptr, DevStatus *out = nullptr);
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr);
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st = nullptr, DevStatus *out = nullptr);
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr);
+// The differentiable run's step.  Before its push, in one launch: Ha = H + Q(E)
+// (the B half step, out of place, the bits of yee_b_half_*), J = 0 (three arrays
+// one after another) and, where keepE is given, a copy of E (three arrays).
+// Ha: three arrays of g.nodes_pitched()
+void flat_begin_plain(const Grid &g, const double *const E[3], const double *const H[3], double *Ha, double *J,
+                      double *keepE, cudaStream_t s);
+void flat_begin_mixed(const Grid &g, const float *const E[3], const float *const H[3], float *Ha, double *J,
+                      float *keepE, cudaStream_t s);
+// after its push: the J fold and both B half steps, H = (H + Q(E)) + Q(E), in one
+// launch (the FP32 form has fold_b_mixed); Q is kept where the field set has it
+void fold_b_twice_plain(const Grid &g, double *const F[12], cudaStream_t s);
 size_t push_smem_plain(const Grid &g);
 // lo32: the tile current's int32 remainder word (every tile holds fewer than
 // 2^(31 - kFxLo32MinBits) particles), else the 64-bit one

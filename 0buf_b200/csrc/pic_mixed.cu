@@ -50,8 +50,9 @@ __device__ __forceinline__ void un4(float4 a, float v[4]) { v[0] = a.x; v[1] = a
 // separate passes of the sub-step calls)
 template <bool TWICE>
 __device__ __forceinline__ void b_half_nodes(const Grid &g, int i, int q, const float *__restrict__ Ex,
-                                             const float *__restrict__ Ey, const float *__restrict__ Ez, float *Hx,
-                                             float *Hy, float *Hz, float cx, float cy, float cz) {
+                                             const float *__restrict__ Ey, const float *__restrict__ Ez, const float *Hx,
+                                             const float *Hy, const float *Hz, float *Ox, float *Oy, float *Oz,
+                                             float cx, float cy, float cz) {
     const int nq = g.pz / 4;
     if (q >= g.NY * nq) return;
     const int l = q / nq, k0 = (q - l * nq) * 4;
@@ -83,7 +84,7 @@ __device__ __forceinline__ void b_half_nodes(const Grid &g, int i, int q, const 
             if (TWICE) hz[j] = __fadd_rn(hz[j], q);
         }
     }
-    st4(Hx + n, hx); st4(Hy + n, hy); st4(Hz + n, hz);
+    st4(Ox + n, hx); st4(Oy + n, hy); st4(Oz + n, hz);
 }
 
 template <bool TWICE>
@@ -91,7 +92,8 @@ __global__ void k_b_half_mixed(Grid g, const float *__restrict__ Ex, const float
                                const float *__restrict__ Ez, float *Hx, float *Hy, float *Hz, float cx, float cy,
                                float cz) {
     chain_enter();
-    b_half_nodes<TWICE>(g, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, cx, cy, cz);
+    b_half_nodes<TWICE>(g, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, Hx, Hy,
+                        Hz, cx, cy, cz);
 }
 // the J fold and both B half steps, which touch different arrays, in one launch:
 // the first `folds` blocks fold, the others step
@@ -106,8 +108,32 @@ __global__ void k_fold_b_mixed(Grid g, int folds, int per_plane, double *Jx, dou
         return;
     }
     const int b = blockIdx.x - folds, i = b / per_plane;
-    b_half_nodes<true>(g, i, (b - i * per_plane) * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, cx, cy, cz);
+    b_half_nodes<true>(g, i, (b - i * per_plane) * blockDim.x + threadIdx.x, Ex, Ey, Ez, Hx, Hy, Hz, Hx, Hy, Hz, cx, cy,
+                       cz);
 }
+// (see flat_begin_mixed) four z nodes per thread, as the other field kernels
+__global__ void k_flat_begin_mixed(Grid g, const float *__restrict__ Ex, const float *__restrict__ Ey,
+                                   const float *__restrict__ Ez, const float *__restrict__ Hx,
+                                   const float *__restrict__ Hy, const float *__restrict__ Hz, float *Ha, double *J,
+                                   float *keepE, float cx, float cy, float cz) {
+    chain_enter();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, nq = g.pz / 4;
+    if (q >= g.NY * nq) return;
+    const size_t n = g.node(blockIdx.y, q / nq, (q % nq) * 4), N = g.nodes_pitched();
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        double2 *j = reinterpret_cast<double2 *>(J + c * N + n);
+        j[0] = j[1] = make_double2(0.0, 0.0);
+    }
+    if (keepE) {
+        float4 *k = reinterpret_cast<float4 *>(keepE + n);
+        k[0] = ld4(Ex + n);
+        k[N / 4] = ld4(Ey + n);
+        k[N / 2] = ld4(Ez + n);
+    }
+    b_half_nodes<false>(g, blockIdx.y, q, Ex, Ey, Ez, Hx, Hy, Hz, Ha, Ha + N, Ha + 2 * N, cx, cy, cz);
+}
+
 
 // emeElement (kernels.cu:1091-1102) in FP32, tau*J formed in FP64
 __global__ void k_e_update_mixed(Grid g, float *Ex, float *Ey, float *Ez, const float *__restrict__ Hx,
@@ -960,6 +986,13 @@ void yee_b_half_mixed(const Grid &g, float *const E[3], float *const H[3], cudaS
     float cx = (float)(g.tau / g.hx), cy = (float)(g.tau / g.hy), cz = (float)(g.tau / g.hz);
     launch_chained(k_b_half_mixed<false>, plane_grid(g), dim3(kPlaneThreads), s, g, E[0], E[1], E[2], H[0], H[1], H[2],
                    cx, cy, cz);
+}
+
+void flat_begin_mixed(const Grid &g, const float *const E[3], const float *const H[3], float *Ha, double *J,
+                      float *keepE, cudaStream_t s) {
+    const float cx = (float)(g.tau / g.hx), cy = (float)(g.tau / g.hy), cz = (float)(g.tau / g.hz);
+    launch_chained(k_flat_begin_mixed, plane_grid(g), dim3(kPlaneThreads), s, g, E[0], E[1], E[2], H[0], H[1], H[2], Ha, J,
+                   keepE, cx, cy, cz);
 }
 
 void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s) {

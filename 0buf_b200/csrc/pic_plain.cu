@@ -85,6 +85,78 @@ __global__ void k_fold_b_plain(Grid g, int folds, int per_plane, double *Jx, dou
     b_complete_node(g, i, (b - i * per_plane) * blockDim.x + threadIdx.x, Hx, Hy, Hz, Qx, Qy, Qz);
 }
 
+
+// Q of emh1_Element at a node of the given component's range (k_b_half_plain's expressions)
+template <int C>
+__device__ __forceinline__ double q_plain(const double *__restrict__ Ex, const double *__restrict__ Ey,
+                                          const double *__restrict__ Ez, size_t n, size_t sx, size_t sy, double cx,
+                                          double cy, double cz) {
+    if (C == 0) return 0.5 * (cz * (Ey[n + 1] - Ey[n]) - cy * (Ez[n + sy] - Ez[n]));
+    if (C == 1) return 0.5 * (cx * (Ez[n + sx] - Ez[n]) - cz * (Ex[n + 1] - Ex[n]));
+    return 0.5 * (cy * (Ex[n + sy] - Ex[n]) - cx * (Ey[n + sx] - Ey[n]));
+}
+// (see flat_begin_plain) one thread per node of an x plane, z pads included
+__global__ void k_flat_begin_plain(Grid g, const double *__restrict__ Ex, const double *__restrict__ Ey,
+                                   const double *__restrict__ Ez, const double *__restrict__ Hx,
+                                   const double *__restrict__ Hy, const double *__restrict__ Hz, double *Ha, double *J,
+                                   double *keepE, double cx, double cy, double cz) {
+    chain_enter();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= g.NY * g.pz) return;
+    const int l = q / g.pz, k = q - l * g.pz, i = blockIdx.y;
+    const size_t n = g.node(i, l, k), N = g.nodes_pitched();
+    J[n] = 0.0;
+    J[N + n] = 0.0;
+    J[2 * N + n] = 0.0;
+    if (k >= g.NZ) return;
+    const size_t sx = (size_t)g.NY * g.pz, sy = g.pz;
+    double hx = Hx[n], hy = Hy[n], hz = Hz[n];
+    if (i <= g.nx + 1 && l <= g.ny && k <= g.nz) hx += q_plain<0>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+    if (i <= g.nx && l <= g.ny + 1 && k <= g.nz) hy += q_plain<1>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+    if (i <= g.nx && l <= g.ny && k <= g.nz + 1) hz += q_plain<2>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+    Ha[n] = hx;
+    Ha[N + n] = hy;
+    Ha[2 * N + n] = hz;
+    if (keepE) {
+        keepE[n] = Ex[n];
+        keepE[N + n] = Ey[n];
+        keepE[2 * N + n] = Ez[n];
+    }
+}
+// (see fold_b_twice_plain) the first `folds` blocks fold, the others step B
+__global__ void k_fold_b_twice_plain(Grid g, int folds, int per_plane, double *Jx, double *Jy, double *Jz,
+                                     const double *__restrict__ Ex, const double *__restrict__ Ey,
+                                     const double *__restrict__ Ez, double *Hx, double *Hy, double *Hz, double *Qx,
+                                     double *Qy, double *Qz, double cx, double cy, double cz) {
+    chain_enter();
+    if ((int)blockIdx.x < folds) {
+        double *const J[3] = {Jx, Jy, Jz};
+        const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+        if (idx < fold_orbits(g)) fold_current(g, J, idx);
+        return;
+    }
+    const int b = blockIdx.x - folds, i = b / per_plane;
+    const int q = (b - i * per_plane) * blockDim.x + threadIdx.x;
+    if (q >= g.NY * g.NZ) return;
+    const int l = q / g.NZ, k = q - l * g.NZ;
+    const size_t n = g.node(i, l, k), sx = (size_t)g.NY * g.pz, sy = g.pz;
+    if (i <= g.nx + 1 && l <= g.ny && k <= g.nz) {
+        const double t = q_plain<0>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+        if (Qx) Qx[n] = t;
+        Hx[n] = (Hx[n] + t) + t;
+    }
+    if (i <= g.nx && l <= g.ny + 1 && k <= g.nz) {
+        const double t = q_plain<1>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+        if (Qy) Qy[n] = t;
+        Hy[n] = (Hy[n] + t) + t;
+    }
+    if (i <= g.nx && l <= g.ny && k <= g.nz + 1) {
+        const double t = q_plain<2>(Ex, Ey, Ez, n, sx, sy, cx, cy, cz);
+        if (Qz) Qz[n] = t;
+        Hz[n] = (Hz[n] + t) + t;
+    }
+}
+
 // emeElement (kernels.cu:1091-1102) over GetElectricFieldStartsDirs ranges
 // (gpu_plasma.h:286-304) as called by ElectricFieldEvaluate (gpu_plasma.h:455-483):
 //   Ex: i in [0,Nx], l in [1,Ny], k in [1,Nz]: += tau/hy*(Hz-Hz[-y]) - tau/hz*(Hy-Hy[-z]) - tau*Jx
@@ -163,13 +235,42 @@ __device__ __forceinline__ size_t ghost_source(const Grid &g, const GhostPasses 
     return g.node(c[0], c[1], c[2]);
 }
 // out (pinned host memory, may be null): the step's status goes there with this
-// last kernel of a step instead of by a copy after it
+// last kernel of a step instead of by a copy after it.  hist (may be null):
+// the sums over nodes 1..N of E_c^2, which no pass writes, are added to it by
+// the rows of blocks after the passes'
+constexpr int kHistRows = 4;
 template <typename T>
-__global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus *out) {
+__global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus *out, const T *__restrict__ Ex,
+                           const T *__restrict__ Ey, const T *__restrict__ Ez, double *hist) {
     chain_enter();
     if (out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(DevStatus) / sizeof(unsigned))
         ((volatile unsigned *)out)[threadIdx.x] = ((const unsigned *)st)[threadIdx.x];
-    if ((int)blockIdx.y >= P.n) return;
+    if ((int)blockIdx.y >= P.n) {
+        __shared__ double red[3][4];
+        double a[3] = {0.0, 0.0, 0.0};
+        const int inner = g.nx * g.ny * g.nz, rows = gridDim.y - P.n;
+        for (int q = ((blockIdx.y - P.n) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; q < inner;
+             q += rows * gridDim.x * blockDim.x) {
+            const int k = q % g.nz, il = q / g.nz, l = il % g.ny, i = il / g.ny;
+            const size_t n = g.node(i + 1, l + 1, k + 1);
+            const double ex = (double)Ex[n], ey = (double)Ey[n], ez = (double)Ez[n];
+            a[0] += ex * ex;
+            a[1] += ey * ey;
+            a[2] += ez * ez;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            for (int o = 16; o > 0; o >>= 1) a[c] += __shfl_down_sync(0xffffffffu, a[c], o);
+            if ((threadIdx.x & 31) == 0) red[c][threadIdx.x >> 5] = a[c];
+        }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double sum = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) sum += red[threadIdx.x][w];
+            atomicAdd(&hist[threadIdx.x], sum);
+        }
+        return;
+    }
     const GhostPass q = P.p[blockIdx.y];
     const int A = q.e1 - q.s1 + 1, B = q.e2 - q.s2 + 1;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -672,9 +773,25 @@ void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s) {
 // arguments gpu_plasma.h:486-505).  Reference mode skips the y pass of Ex and
 // Ez; periodic mode performs it.  Round A holds the first pass of each
 // component, round B the second; both run in one launch (GhostPasses).
+void flat_begin_plain(const Grid &g, const double *const E[3], const double *const H[3], double *Ha, double *J,
+                      double *keepE, cudaStream_t s) {
+    const double cx = g.tau / g.hx, cy = g.tau / g.hy, cz = g.tau / g.hz;
+    launch_chained(k_flat_begin_plain, dim3((g.NY * g.pz + kPlaneThreads - 1) / kPlaneThreads, g.NX), dim3(kPlaneThreads),
+                   s, g, E[0], E[1], E[2], H[0], H[1], H[2], Ha, J, keepE, cx, cy, cz);
+}
+
+void fold_b_twice_plain(const Grid &g, double *const F[12], cudaStream_t s) {
+    const double cx = g.tau / g.hx, cy = g.tau / g.hy, cz = g.tau / g.hz;
+    const int folds = (fold_orbits(g) + kPlaneThreads - 1) / kPlaneThreads;
+    const dim3 plane = plane_grid(g);
+    launch_chained(k_fold_b_twice_plain, dim3(folds + plane.x * plane.y), dim3(kPlaneThreads), s, g, folds, (int)plane.x,
+                   F[PIC_JX], F[PIC_JY], F[PIC_JZ], F[PIC_EX], F[PIC_EY], F[PIC_EZ], F[PIC_HX], F[PIC_HY], F[PIC_HZ],
+                   F[PIC_QX], F[PIC_QY], F[PIC_QZ], cx, cy, cz);
+}
+
 template <typename T>
 static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                       DevStatus *out) {
+                       DevStatus *out, double *hist) {
     int Nx = g.nx, Ny = g.ny, Nz = g.nz;
     GhostPasses P{};
     int maxn = 0;
@@ -692,15 +809,16 @@ static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStr
     add(Ex, 2, 0, Nx, 0, Ny + 1, Nz);
     add(Ey, 2, 0, Nx + 1, 0, Ny, Nz);
     if (periodic) add(Ez, 1, 0, Nx + 1, 0, Nz, Ny);
-    launch_chained(k_e_ghosts<T>, dim3((maxn + 127) / 128, P.n), dim3(128), s, g, P, st, out);
+    launch_chained(k_e_ghosts<T>, dim3((maxn + 127) / 128, P.n + (hist ? kHistRows : 0)), dim3(128), s, g, P, st, out, Ex, Ey,
+                   Ez, hist);
 }
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st, DevStatus *out) {
-    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out);
+                    const DevStatus *st, DevStatus *out, double *hist) {
+    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out, hist);
 }
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                    DevStatus *out) {
-    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out);
+                    DevStatus *out, double *hist) {
+    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out, hist);
 }
 
 // shared memory of the next particle of every thread

@@ -42,12 +42,16 @@ def test_gradient_does_not_depend_on_the_tiling(pkg, cells, ppc, vth, precision)
             sim.forward(STEPS, 8)
             g = sim.backward(**loss)
             order = np.lexsort([p0[k] for k in KEYS])
-            got.append((g["d_p0"][order], g["d_drift"], g["d_vth"], sim.get_field("Ex"), sim.get_field("Jy")))
+            got.append((g["d_p0"][order], g["d_drift"], g["d_vth"], sim.get_field("Ex"), sim.get_field("Jy"),
+                        sim.get_field("Hz"), sim.get_field("Qx") if precision == "fp64" else None))
     with make(pkg, cells, ppc, vth, precision) as sim:
         sim.run(STEPS)
         tol = 1e-12 if precision == "fp64" else 1e-4
         assert rel(got[0][3], sim.get_field("Ex")) < tol and rel(got[1][3], sim.get_field("Ex")) < tol
         assert rel(got[0][4], sim.get_field("Jy")) < tol
+        assert rel(got[0][5], sim.get_field("Hz")) < tol
+        if precision == "fp64":
+            assert rel(got[0][6], sim.get_field("Qx")) < tol
     tol = 1e-9 if precision == "fp64" else 1e-4
     assert np.linalg.norm(got[0][0]) > 0
     assert rel(got[1][0], got[0][0]) < tol
