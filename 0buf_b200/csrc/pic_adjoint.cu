@@ -80,7 +80,7 @@ struct AdjParams {
 constexpr int kW = kT / 32;        // warps per CTA
 constexpr int kQueuePlain = 48;    // queued second segments per warp, as in k_push_plain
 constexpr int kFlatWindow = 900;   // nodes of the forward's window: 109 KB of shared memory, two CTAs per SM
-constexpr int kAdjWindow = 640;    // nodes of the adjoint's: 106 KB
+constexpr int kAdjWindow = 704;    // nodes of the adjoint's: 112 KB
 
 // shared memory of a thread's next particle (cp.async, as in k_push_plain)
 constexpr size_t kNextBytes = (size_t)kW * (6 * 32 + 16) * sizeof(double);
@@ -367,11 +367,10 @@ __device__ __forceinline__ int new_cell_plain(const Grid &g, int cell, int i, in
 }
 
 // stages the window's nodes of `n` arrays src[c] into dst (n x w.nn doubles)
-template <int N>
-__device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow &w, const double *const *src, double *dst) {
+template <int N, bool WRAP>
+__device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow<WRAP> &w, const double *const *src, double *dst) {
     for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
-        const int c = e % w.SZ, ab = e / w.SZ, b = ab % w.SY, a = ab / w.SY;
-        const size_t n = g.node(w.i0 + a, w.l0 + b, w.k0 + c);
+        const size_t n = w.grid_node(g, e);
 #pragma unroll
         for (int q = 0; q < N; q++) dst[q * w.nn + e] = src[q][n];
     }
@@ -391,7 +390,7 @@ template <int BMODE>
 __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ AdjWindow sWin;
+    __shared__ AdjWindow<false> sWin;
     __shared__ int sRed[15 * kW], sQn[kW];
     __shared__ double sQ, sInvQ;
     double *sF = (double *)smem_raw;
@@ -406,7 +405,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     const int s = ch.species, count = ch.count;
     const FlatSp &S = P.sp[s];
     if ((int)threadIdx.x < count) next.start(S, ch.first + threadIdx.x);
-    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
+    const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
     const int nn = w.nn;
     if (threadIdx.x == 0) {
         // the quantum of k_push_plain's tile current, for this chunk
@@ -450,7 +449,8 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
         if (cell >= 0) {
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            const bool in = w.holds(c3[0], c3[1], c3[2]);
+            int u3[3], n0;
+            const bool in = w.place(c3, u3, n0);
             const double o3[3] = {(double)c3[0] * h3[0], (double)c3[1] * h3[1], (double)c3[2] * h3[2]};
             const unsigned long long rcode = BMODE == 2 ? P.branch[P.off[s] + j] : 0ull;
             AxisTaps T[3];
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                     FieldView<true> A;
 #pragma unroll
                     for (int c = 0; c < 6; c++) A.base[c] = sF + c * nn;
-                    A.n0 = w.node(c3[0], c3[1], c3[2]); A.dx = w.SY * w.SZ; A.dy = w.SZ;
+                    A.n0 = n0; A.dx = w.SY * w.SZ; A.dy = w.SZ;
                     ok = gather_fields(A, T, F);
                 } else {
                     FieldView<false> A;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
 #pragma unroll
             for (int d = 0; d < 3; d++) sb[d] = cross ? SP.x2[d] : x1[d];
             if (in) {
-                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, c3[0] - w.i0 - 2, c3[1] - w.l0 - 2, c3[2] - w.k0 - 2, SP.i1,
+                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, u3[0] - 2, u3[1] - 2, u3[2] - 2, SP.i1,
                                 x, sb, g.hx, g.hy, g.hz, rc, o3[0], o3[1], o3[2], bad);
                 if (cross) {
                     if (SP.i2[0] >= 2 && SP.i2[0] <= 3 && SP.i2[1] >= 2 && SP.i2[1] <= 3 && SP.i2[2] >= 2 &&
@@ -521,8 +521,8 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                             qd[d * kQueuePlain + e] = SP.x2[d];
                             qd[(3 + d) * kQueuePlain + e] = x1[d];
                         }
-                        // window-local cell, 9 bits each (a window has at most kFlatWindow nodes), and class bits
-                        qc[e] = ((c3[0] - w.i0) << 21) | ((c3[1] - w.l0) << 12) | ((c3[2] - w.k0) << 3) | (SP.i2[0] - 2) |
+                        // window-local node of the cell, 9 bits each (a window has at most kFlatWindow nodes), and class bits
+                        qc[e] = (u3[0] << 21) | (u3[1] << 12) | (u3[2] << 3) | (SP.i2[0] - 2) |
                                 ((SP.i2[1] - 2) << 1) | ((SP.i2[2] - 2) << 2);
                     } else {
                         bad |= ST_STENCIL;
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                     se[q] = qd[(3 + q) * kQueuePlain + e];
                 }
                 pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
-                                (double)(w.i0 + a) * g.hx, (double)(w.l0 + b) * g.hy, (double)(w.k0 + c) * g.hz, bad);
+                                (double)w.at(0, a) * g.hx, (double)w.at(1, b) * g.hy, (double)w.at(2, c) * g.hz, bad);
             }
             qn -= d;
             __syncwarp();
@@ -610,8 +610,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
         const int il = ((const int *)(sJ + 3 * nn))[e];
         if (ih == 0 && il == 0) continue;
         const int comp = e / nn, r = e - comp * nn;
-        const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
-        atomicAdd(&P.J[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], ((double)ih + (double)il / lo_scale) * sQ);
+        atomicAdd(&P.J[comp][w.grid_node(g, r)], ((double)ih + (double)il / lo_scale) * sQ);
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (amb) atomicAdd(&P.st->ambiguous, amb);
@@ -837,7 +836,7 @@ __device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
 __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_constant__ AdjParams A) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ AdjWindow sWin;
+    __shared__ AdjWindow<true> sWin;
     __shared__ int sRed[15 * kW], sFar;
     __shared__ unsigned sMax[2];
     const FlatParams &P = A.f;
@@ -860,7 +859,7 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
         next.start(S, ch.first + mine);
         lnext.start(Lm, ch.first + mine);
     }
-    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kAdjWindow, sRed, &sWin);
+    const AdjWindow<true> w = chunk_window(g, S.cell + ch.first, count, kAdjWindow, sRed, &sWin);
     const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
     double *sF = (double *)smem_raw, *sL = sF + 6 * nn;
     unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
@@ -883,8 +882,7 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
                 if (v == 0) continue;
                 if (again) sHi[e] = sLo[e] = 0u;
                 const int comp = e / nn, r = e - comp * nn;
-                const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
-                atomicAdd(&dst[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * q);
+                        atomicAdd(&dst[comp][w.grid_node(g, r)], (double)v * q);
             }
         }
     };
@@ -903,11 +901,12 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
             next.start(S, j + blockDim.x);
             lnext.start(Lm, j + blockDim.x);
         }
-        int c3[3] = {w.i0, w.l0, w.k0};
+        int c3[3] = {0, 0, 0}, n0 = 0;
         bool near = cell >= 0;
         if (near) {
+            int u[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            if (!w.holds(c3[0], c3[1], c3[2])) {
+            if (!w.place(c3, u, n0)) {
                 near = false;
                 sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
             }
@@ -916,7 +915,6 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
         double gx[3], lu[3], lF[6], gi[3] = {0.0, 0.0, 0.0};
         bool seen = false;
         float amax = 0.f;
-        const int n0 = w.node(c3[0], c3[1], c3[2]);
         if (near) {
             FieldView<true> V;
 #pragma unroll

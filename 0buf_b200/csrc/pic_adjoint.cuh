@@ -86,24 +86,52 @@ struct AdjState {
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-// ---- a chunk's window: the box of cells whose nodes a CTA keeps in shared memory
+// ---- a chunk's window: the periodic box of cells whose nodes a CTA keeps in shared memory
+// WRAP: an axis whose cells run past the grid's end and go on at 0 has the nodes of
+// its cells up to the end (two more than cells), then those of its cells from 0 on.
+template <bool WRAP>
 struct AdjWindow {
-    int i0, l0, k0, cx, cy, cz;  // first cell and cells per axis
-    int SY, SZ, nn;              // node strides and nodes: (cx+2)(cy+2)(cz+2)
-    __device__ __forceinline__ bool holds(int i, int l, int k) const {
-        return (unsigned)(i - i0) < (unsigned)cx && (unsigned)(l - l0) < (unsigned)cy && (unsigned)(k - k0) < (unsigned)cz;
+    int lo[3], cells[3], n[3];  // per axis: first cell, cells, the grid's cells
+    int SY, SZ, nn;             // node strides and nodes
+    // window-local node of a cell (its lower corner); false: outside
+    __device__ __forceinline__ bool place(const int c[3], int u[3], int &node) const {
+        bool in = true;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const int v = c[d] - lo[d], on = WRAP && v < 0 ? n[d] : 0;  // on: past the end
+            in = in && (unsigned)(v + on) < (unsigned)cells[d];
+            u[d] = v + on + (on ? 2 : 0);
+        }
+        node = (u[0] * SY + u[1]) * SZ + u[2];
+        return in;
     }
-    // window-local node of a cell (its lower corner)
-    __device__ __forceinline__ int node(int i, int l, int k) const { return ((i - i0) * SY + (l - l0)) * SZ + (k - k0); }
+    // the grid's node at position u of axis d; for the lower corner of a cell, its cell
+    __device__ __forceinline__ int at(int d, int u) const {
+        const int end = n[d] - lo[d] + 2;
+        return !WRAP || u < end ? lo[d] + u : u - end;
+    }
+    __device__ __forceinline__ size_t grid_node(const Grid &g, int e) const {
+        const int c = e % SZ, ab = e / SZ, b = ab % SY, a = ab / SY;
+        return g.node(at(0, a), at(1, b), at(2, c));
+    }
 };
-// The window of `count` particles' cells with at most `cap` nodes: their
-// bounding box where that fits.  Otherwise (particles that wandered off, or a
-// chunk that lies on both sides of a periodic boundary) a box around their mean
-// position, taken periodically, cut at the grid's edge and shrunk on its longest
-// axis until it fits; the particles outside it use global memory.  Every thread
-// of the CTA calls it; red holds 15 ints per warp.
-__device__ __forceinline__ AdjWindow chunk_window(const Grid &g, const int *__restrict__ cell, int count, int cap,
-                                                  int *red, AdjWindow *out) {
+// nodes of an axis whose window starts at cell lo
+__device__ __forceinline__ int window_nodes(int lo, int cells, int n) { return cells + 2 + (lo + cells > n ? 2 : 0); }
+
+// The window of `count` particles' cells with at most `cap` nodes: per axis the
+// smaller of their bounding box and the periodic one, where that fits; else the
+// periodic box around their mean, cut at the grid's ends and then shrunk on its
+// longest axis until it fits, and the particles outside it use global memory.  Every thread of the CTA calls it;
+// red holds 15 ints per warp.
+// Particles that crossed the grid's end would else go through global memory, one
+// at a time, while their CTA waits: with WRAP in the adjoint kernels (and 704
+// instead of 640 nodes in FP64, 672 in FP32) 16x8x8 cells 45.2 -> 30.4 us per
+// reverse step (FP64), 128x32x32 2.298 -> 2.273 ms (FP64), 1.350 -> 1.314
+// (FP32).  The forward pushes don't gain: particles outside take little longer
+// there (FP32 64x32x32 cells 187 us without, 191 with).
+template <bool WRAP>
+__device__ __forceinline__ AdjWindow<WRAP> chunk_window(const Grid &g, const int *__restrict__ cell, int count, int cap,
+                                                        int *red, AdjWindow<WRAP> *out) {
     const unsigned FULL = 0xffffffffu;
     const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int n3[3] = {g.nx, g.ny, g.nz};
@@ -133,44 +161,79 @@ __device__ __forceinline__ AdjWindow chunk_window(const Grid &g, const int *__re
             for (int q = 0; q < 5; q++) red[(5 * d + q) * nw + warp] = r[q];
     }
     __syncthreads();
+    if (threadIdx.x < 15) {  // the warps' results, one of the 15 per lane
+        int *r = red + threadIdx.x * nw, v = r[0];
+        const int kind = threadIdx.x % 5;
+        for (int q = 1; q < nw; q++) v = kind == 4 ? v + r[q] : (kind & 1 ? max(v, r[q]) : min(v, r[q]));
+        r[0] = v;
+    }
+    if (threadIdx.x < 32) __syncwarp();
     if (threadIdx.x == 0) {
-        int a[3], b[3];
+        AdjWindow<WRAP> w;
+        int a[3], b[3], m[3];  // periodic box and mean, as distances from at
         int64_t nodes = 1;
         for (int d = 0; d < 3; d++) {
             const int *r = red + 5 * d * nw;
-            a[d] = r[0];
-            b[d] = r[nw];
-            for (int w = 1; w < nw; w++) { a[d] = min(a[d], r[w]); b[d] = max(b[d], r[nw + w]); }
-            nodes *= b[d] - a[d] + 3;
+            const int l0 = r[0], h0 = r[nw], sm = r[4 * nw];
+            a[d] = r[2 * nw];
+            b[d] = r[3 * nw];
+            m[d] = (int)rintf((float)sm / (float)count);
+            w.n[d] = n3[d];
+            w.lo[d] = at[d] + a[d];
+            if (w.lo[d] < 0) w.lo[d] += n3[d];
+            w.cells[d] = b[d] - a[d] + 1;
+            if ((!WRAP && w.lo[d] + w.cells[d] > n3[d]) || window_nodes(w.lo[d], w.cells[d], n3[d]) >= h0 - l0 + 3) {
+                w.lo[d] = l0;
+                w.cells[d] = h0 - l0 + 1;
+            }
+            nodes *= window_nodes(w.lo[d], w.cells[d], n3[d]);
         }
         if (nodes > cap) {
-            int mid[3];
+            int s[3];
             for (int d = 0; d < 3; d++) {
-                const int *r = red + 5 * d * nw;
-                int mn = r[2 * nw], mx = r[3 * nw], sm = r[4 * nw];
-                for (int w = 1; w < nw; w++) {
-                    mn = min(mn, r[2 * nw + w]); mx = max(mx, r[3 * nw + w]); sm += r[4 * nw + w];
+                m[d] = min(max(m[d], a[d]), b[d]);
+                a[d] = max(a[d], m[d] - 15);
+                b[d] = min(b[d], m[d] + 15);
+                if (b[d] - a[d] + 1 > n3[d]) {  // both ends half the axis away: the same cell
+                    if (b[d] > m[d]) b[d]--;
+                    else a[d]++;
                 }
-                const int m = at[d] + (int)rintf((float)sm / (float)count);
-                mid[d] = m < 0 ? m + n3[d] : (m >= n3[d] ? m - n3[d] : m);
-                a[d] = max(max(at[d] + mn + mid[d] - m, 0), mid[d] - 15);
-                b[d] = min(min(at[d] + mx + mid[d] - m, n3[d] - 1), mid[d] + 15);
-                a[d] = min(a[d], mid[d]);
-                b[d] = max(b[d], mid[d]);
             }
-            while ((b[0] - a[0] + 3) * (b[1] - a[1] + 3) * (b[2] - a[2] + 3) > cap) {
+            for (;;) {
+                nodes = 1;
+                for (int d = 0; d < 3; d++) {
+                    s[d] = at[d] + a[d];
+                    s[d] = s[d] < 0 ? s[d] + n3[d] : (s[d] >= n3[d] ? s[d] - n3[d] : s[d]);
+                    nodes *= window_nodes(s[d], b[d] - a[d] + 1, n3[d]);
+                }
+                if (WRAP && nodes <= cap) break;
+                // first what lies past the grid's end, few particles for three nodes or more
+                int cut = -1, lost = WRAP ? 4 : 0x7fffffff;
+                for (int d = 0; d < 3; d++) {
+                    const int len = b[d] - a[d] + 1, before = n3[d] - s[d];
+                    const int l = m[d] - a[d] < before ? len - before : before;
+                    if (before < len && l < lost) { cut = d; lost = l; }
+                }
+                if (cut >= 0) {
+                    if (m[cut] - a[cut] < n3[cut] - s[cut]) b[cut] -= lost;
+                    else a[cut] += lost;
+                    continue;
+                }
+                if (nodes <= cap) break;
                 int d = 0;
                 for (int e = 1; e < 3; e++)
                     if (b[e] - a[e] > b[d] - a[d]) d = e;
-                if (b[d] - mid[d] >= mid[d] - a[d]) b[d]--;
+                if (b[d] - m[d] >= m[d] - a[d]) b[d]--;
                 else a[d]++;
             }
+            for (int d = 0; d < 3; d++) {
+                w.lo[d] = s[d];
+                w.cells[d] = b[d] - a[d] + 1;
+            }
         }
-        AdjWindow w;
-        w.i0 = a[0]; w.l0 = a[1]; w.k0 = a[2];
-        w.cx = b[0] - a[0] + 1; w.cy = b[1] - a[1] + 1; w.cz = b[2] - a[2] + 1;
-        w.SY = w.cy + 2; w.SZ = w.cz + 2;
-        w.nn = (w.cx + 2) * w.SY * w.SZ;
+        w.SY = window_nodes(w.lo[1], w.cells[1], n3[1]);
+        w.SZ = window_nodes(w.lo[2], w.cells[2], n3[2]);
+        w.nn = window_nodes(w.lo[0], w.cells[0], n3[0]) * w.SY * w.SZ;
         *out = w;
     }
     __syncthreads();

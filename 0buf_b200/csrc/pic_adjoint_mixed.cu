@@ -261,7 +261,7 @@ __device__ __forceinline__ MixConst mix_const(const Grid &g, const MixSp &S) {
 constexpr int kW = kT / 32;          // warps per CTA
 constexpr int kQueueMix = 48;        // queued second segments per warp: drained at 16, at most 15 + 32
 constexpr int kFlatWindowMix = 800;  // nodes of the forward's window: 56 KB of shared memory, three CTAs per SM (80 registers)
-constexpr int kAdjWindowMix = 640;   // nodes of the adjoint's: 71 KB, three
+constexpr int kAdjWindowMix = 672;   // nodes of the adjoint's: 73 KB, three
 
 // shared memory of a thread's next particle (cp.async, as in k_push_plain): N values, then the cell
 template <int N>
@@ -287,11 +287,10 @@ struct NextMix {
 };
 
 // stages the window's nodes of N arrays src[c] into dst (N x w.nn floats)
-template <int N, class T>
-__device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow &w, const T *const *src, float *dst) {
+template <int N, class T, bool WRAP>
+__device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WRAP> &w, const T *const *src, float *dst) {
     for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
-        const int c = e % w.SZ, ab = e / w.SZ, b = ab % w.SY, a = ab / w.SY;
-        const size_t n = g.node(w.i0 + a, w.l0 + b, w.k0 + c);
+        const size_t n = w.grid_node(g, e);
 #pragma unroll
         for (int q = 0; q < N; q++) dst[q * w.nn + e] = (float)src[q][n];
     }
@@ -310,7 +309,7 @@ __device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow &w
 __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant__ MixParams P) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ AdjWindow sWin;
+    __shared__ AdjWindow<false> sWin;
     __shared__ int sRed[15 * kW], sQn[kW];
     __shared__ double sQ, sInvQ;
     __shared__ MixConst sK;
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
     float *qd = (float *)sTail + warp * 7 * kQueueMix;  // x2, xe, then the cell and class code
     const NextMix<6> next(sTail + (size_t)kW * 7 * kQueueMix * sizeof(float));
     if ((int)threadIdx.x < count) next.start(S, nullptr, ch.first + threadIdx.x);
-    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
+    const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
     const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
     unsigned *sLo = (unsigned *)smem_raw, *sHi = sLo + 3 * nn;
     float *sF = (float *)(sHi + 3 * nn);
@@ -371,8 +370,8 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         if (cell >= 0) {
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            const bool in = w.holds(c3[0], c3[1], c3[2]);
-            const int n0 = w.node(c3[0], c3[1], c3[2]);
+            int u3[3], n0;
+            const bool in = w.place(c3, u3, n0);
             float F[6];
             if (in) {
                 FieldViewM<true> V;
@@ -460,8 +459,7 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
         if (v == 0) continue;
         const int comp = e / nn, r = e - comp * nn;
-        const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
-        atomicAdd(&P.J[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * sQ);
+        atomicAdd(&P.J[comp][w.grid_node(g, r)], (double)v * sQ);
     }
     if (bad) atomicOr(&P.st->flags, bad);
 }
@@ -619,7 +617,7 @@ __device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j)
 __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_constant__ MixParams P) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ AdjWindow sWin;
+    __shared__ AdjWindow<true> sWin;
     __shared__ int sRed[15 * kW], sFar;
     __shared__ unsigned sMax[2];
     __shared__ MixConst sK;
@@ -633,7 +631,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     // lanes as in k_adj_particles_plain
     const int lane = threadIdx.x & 31, mine = (lane >> 3) * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
     if (mine < count) next.start(S, Lm, ch.first + mine);
-    const AdjWindow w = chunk_window(g, S.cell + ch.first, count, kAdjWindowMix, sRed, &sWin);
+    const AdjWindow<true> w = chunk_window(g, S.cell + ch.first, count, kAdjWindowMix, sRed, &sWin);
     const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
     float *sF = (float *)smem_raw, *sL = sF + 6 * nn;
     unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
@@ -655,8 +653,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
             if (v == 0) continue;
             if (again) sHi[e] = sLo[e] = 0u;
             const int comp = e / nn, r = e - comp * nn;
-            const int c = r % w.SZ, b = (r / w.SZ) % w.SY, a = r / (w.SZ * w.SY);
-            atomicAdd(&dst[comp][g.node(w.i0 + a, w.l0 + b, w.k0 + c)], (double)v * q);
+                atomicAdd(&dst[comp][w.grid_node(g, r)], (double)v * q);
         }
     };
     for (int base = 0, it = 0; base < count; base += blockDim.x, it++) {
@@ -674,17 +671,17 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
         }
         __syncwarp();
         if (jc + (int)blockDim.x < count) next.start(S, Lm, j + blockDim.x);
-        int c3[3] = {w.i0, w.l0, w.k0};
+        int c3[3] = {0, 0, 0}, n0 = 0;
         bool near = cell >= 0;
         if (near) {
+            int u[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            if (!w.holds(c3[0], c3[1], c3[2])) {
+            if (!w.place(c3, u, n0)) {
                 near = false;
                 sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
             }
         }
         float gx[3], lu[3], lF[6], gi[3] = {0.f, 0.f, 0.f}, amax = 0.f;
-        const int n0 = w.node(c3[0], c3[1], c3[2]);
         if (near) {
             FieldViewM<true> V;
 #pragma unroll
