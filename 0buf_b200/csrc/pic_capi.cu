@@ -503,8 +503,9 @@ int need_particles(pic_handle *h) {
     return PIC_OK;
 }
 
-int do_b_half(pic_handle *h) {
-    if (!h->mixed) yee_b_half_plain(h->g, (double *const *)h->f, h->stream);
+// stamps (here and below): the time stamps of a step (null: a sub-step call)
+int do_b_half(pic_handle *h, unsigned long long *stamps = nullptr) {
+    if (!h->mixed) yee_b_half_plain(h->g, (double *const *)h->f, h->stream, stamps);
     else yee_b_half_mixed(h->g, (float *const *)&h->f[PIC_EX], (float *const *)&h->f[PIC_HX], h->stream);
     CK(cudaGetLastError(), "b_half");
     h->launches += 1;
@@ -534,7 +535,7 @@ bool plain_lo32(pic_handle *h) {
     return 31 - b >= kFxLo32MinBits;
 }
 
-int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
+int do_push_deposit(pic_handle *h, int b_half_in_push = 0, unsigned long long *stamps = nullptr) {
     int rc = need_particles(h);
     if (rc) return rc;
     // the outbox is sized once for all species (the loads leave that to the
@@ -554,6 +555,7 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
     }
     StepParams p = make_params(h);
     p.b_half = b_half_in_push;
+    p.stamps = stamps;
     p.slices = h->split_buf ? push_slices(h) : 1;
     if (p.slices > 1) {
         const size_t nc = (size_t)h->cfg.nspecies * h->g.ntiles;
@@ -563,10 +565,8 @@ int do_push_deposit(pic_handle *h, int b_half_in_push = 0) {
     }
     CK(begin_push(p, h->g.nodes_pitched(), h->stream), "begin push");
     h->launches += 1;
-    cudaEventRecord(h->ev[2], h->stream);
     CK(h->mixed ? launch_push_mixed(p, h->maps, h->stream) : launch_push_plain(p, plain_lo32(h), h->stream),
        "push_deposit");
-    cudaEventRecord(h->ev[3], h->stream);
     if (h->mixed) h->lb_par ^= 1;
     h->launches += 1;
     h->kin_valid = 1;
@@ -597,16 +597,16 @@ int do_e_update(pic_handle *h) {
     return PIC_OK;
 }
 
-// with_status: the step's status goes to st_host with this launch
-int do_e_ghosts(pic_handle *h, bool with_status = false) {
+// of a step (stamps): its status goes to st_host with this launch
+int do_e_ghosts(pic_handle *h, unsigned long long *stamps = nullptr) {
     int per = h->cfg.ghosts == PIC_GHOSTS_PERIODIC;
-    DevStatus *out = with_status ? h->st_host : nullptr;
+    DevStatus *out = stamps ? h->st_host : nullptr;
     if (!h->mixed)
         e_ghosts_plain(h->g, (double *)h->f[PIC_EX], (double *)h->f[PIC_EY], (double *)h->f[PIC_EZ], per, h->stream,
-                       h->st, out);
+                       h->st, out, nullptr, stamps);
     else
         e_ghosts_mixed(h->g, (float *)h->f[PIC_EX], (float *)h->f[PIC_EY], (float *)h->f[PIC_EZ], per, h->stream, h->st,
-                       out);
+                       out, nullptr, stamps);
     CK(cudaGetLastError(), "e_ghosts");
     h->launches += 1;
     return PIC_OK;
@@ -712,7 +712,6 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
     auto fail = [&](cudaError_t e) { pic_destroy(h); return e == cudaErrorMemoryAllocation ? PIC_ERR_NOMEM : (int)e; };
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e) { delete h; return (int)e; }
-    for (int i = 0; i < 6; i++) cudaEventCreate(&h->ev[i]);
     if ((e = cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
     for (int i = 0; i < 5; i++)
         if ((e = cudaEventCreateWithFlags(&h->lev[i], cudaEventDisableTiming)) != cudaSuccess) return fail(e);
@@ -743,8 +742,10 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
         if ((e = cudaMemsetAsync(h->lb_buf, 0, 2 * kMaxSpecies * sizeof(float), h->stream)) != cudaSuccess)
             return fail(e);
     }
-    if ((e = cudaMalloc(&h->st, sizeof(DevStatus))) != cudaSuccess) return fail(e);
-    if ((e = cudaMemsetAsync(h->st, 0, sizeof(DevStatus), h->stream)) != cudaSuccess) return fail(e);
+    // the time stamps of a step follow the status
+    const size_t st_bytes = sizeof(DevStatus) + kStamps * sizeof(unsigned long long);
+    if ((e = cudaMalloc(&h->st, st_bytes)) != cudaSuccess) return fail(e);
+    if ((e = cudaMemsetAsync(h->st, 0, st_bytes, h->stream)) != cudaSuccess) return fail(e);
     // pinned: the status, then the reductions
     if ((e = cudaMallocHost(&h->st_host, 256 + 8 * sizeof(double))) != cudaSuccess) return fail(e);
     static_assert(sizeof(DevStatus) <= 256, "the reductions start 256 bytes behind the status");
@@ -779,8 +780,6 @@ int pic_destroy(pic_handle *h) {
     double *diag[3] = {h->rho, h->gauss, h->gauss0};
     for (double *d : diag)
         if (d) cudaFree(d);
-    for (int i = 0; i < 6; i++)
-        if (h->ev[i]) cudaEventDestroy(h->ev[i]);
     for (int i = 0; i < 5; i++)
         if (h->lev[i]) cudaEventDestroy(h->lev[i]);
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
@@ -1151,38 +1150,38 @@ void energies_of(const pic_handle *h, double *out4) {
     out4[3] = out4[0] + out4[1] + out4[2];
 }
 
+unsigned long long *step_stamps(const pic_handle *h) { return (unsigned long long *)(h->st + 1); }
+
 // one step; energies (may be null) receives pic_energy's four numbers after it,
 // with the same wait
 int step_impl(pic_handle *h, double *energies) {
     int rc = set_device(h);
     if (rc) return rc;
     h->launches = 0;
-    cudaEventRecord(h->ev[0], h->stream);
+    unsigned long long *stamps = step_stamps(h);
     // the FP32 form forms the B half step inside the push's staged field tile
-    if (!h->mixed && (rc = do_b_half(h))) return rc;
-    cudaEventRecord(h->ev[1], h->stream);
-    if ((rc = do_push_deposit(h, h->mixed))) return rc;  // records ev[2], ev[3] around the kernel
+    if (!h->mixed && (rc = do_b_half(h, stamps))) return rc;
+    if ((rc = do_push_deposit(h, h->mixed, stamps))) return rc;
     StepParams p = make_params(h);
+    p.stamps = stamps;
     CK(launch_insert(p, h->stream), "insert");
-    cudaEventRecord(h->ev[4], h->stream);
     // (FP32 form: H in memory is still the full-step field, both half steps in one pass)
     if (h->mixed)
         fold_b_mixed(h->g, (float *const *)&h->f[PIC_EX], (float *const *)&h->f[PIC_HX], (double *const *)&h->f[PIC_JX],
-                     h->stream);
+                     h->stream, stamps);
     else
-        fold_b_plain(h->g, (double *const *)h->f, h->stream);
+        fold_b_plain(h->g, (double *const *)h->f, h->stream, stamps);
     CK(cudaGetLastError(), "fold and b_complete");
     h->launches += 2;
     if ((rc = do_e_update(h))) return rc;
-    if ((rc = do_e_ghosts(h, true))) return rc;
-    cudaEventRecord(h->ev[5], h->stream);
+    if ((rc = do_e_ghosts(h, stamps))) return rc;
     if (energies && (rc = enqueue_energy(h, true))) return rc;
     h->timed = h->timed ? 2 : 0;
     CK(cudaStreamSynchronize(h->stream), "sync");
     rc = handle_status(h);
     h->counters[3] = h->launches;
     if (!rc) {
-        h->timed = 1;  // pic_step_timings reads the events
+        h->timed = 1;  // pic_step_timings reads the stamps
         if (energies) energies_of(h, energies);
     }
     return rc;
@@ -1414,7 +1413,9 @@ int pic_step_timings(pic_handle *h, float *out5) {
     if (h->timed == 1) {
         cudaSetDevice(h->device);
         const int of[5][2] = {{0, 1}, {2, 3}, {3, 4}, {4, 5}, {0, 5}};
-        for (int i = 0; i < 5; i++) cudaEventElapsedTime(&h->timings[i], h->ev[of[i][0]], h->ev[of[i][1]]);
+        unsigned long long t[kStamps];
+        CK(cudaMemcpy(t, step_stamps(h), sizeof(t), cudaMemcpyDeviceToHost), "timings");
+        for (int i = 0; i < 5; i++) h->timings[i] = (float)((double)(t[of[i][1]] - t[of[i][0]]) * 1e-6);
         h->timed = 2;
     }
     for (int i = 0; i < 5; i++) out5[i] = h->timings[i];

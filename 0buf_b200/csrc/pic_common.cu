@@ -163,7 +163,9 @@ __global__ void k_gather_f(Grid g, int mixed, SpeciesView S, const int64_t *__re
 // while such entries are under way, so no slot is handed out twice and the
 // counts end at the capacity.
 template <class Out, bool MIXED>
-__global__ void k_insert(StepParams P) {
+__global__ void k_insert(const __grid_constant__ StepParams P) {
+    chain_enter();
+    stamp_entry(P.stamps, 3);
     unsigned n = P.st->out_count;
     if (n > P.out_cap) n = P.out_cap;
     Out *ob = (Out *)P.outbox;
@@ -269,7 +271,10 @@ __global__ void k_insert_left(Grid g, Out *ob, unsigned n, int species, SpeciesV
 // see begin_push: one launch in place of a memset per array (five of them at
 // 2 us each in a small step)
 __global__ void k_begin_push(double2 *J, size_t n2, unsigned *st, int nst, unsigned *lb, int nlb, unsigned *holes,
-                             int nholes) {
+                             int nholes, unsigned long long *stamps, int first) {
+    chain_enter();
+    if (first) stamp_entry(stamps, 0);
+    stamp_entry(stamps, 1);
     const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = i0; i < n2; i += stride) J[i] = make_double2(0.0, 0.0);
     for (size_t i = i0; i < (size_t)nholes; i += stride) holes[i] = 0u;
@@ -606,9 +611,7 @@ cudaError_t gather_from_bins_f(const Grid &g, int mixed, SpeciesView sv, const i
 
 cudaError_t launch_insert(const StepParams &p, cudaStream_t s) {
     int blocks = 148 * 4;
-    if (p.mixed) k_insert<OutMixed, true><<<blocks, 256, 0, s>>>(p);
-    else k_insert<OutPlain, false><<<blocks, 256, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_chained(p.mixed ? k_insert<OutMixed, true> : k_insert<OutPlain, false>, dim3(blocks), dim3(256), s, p);
 }
 
 cudaError_t cell_histogram(const StepParams &p, int *counts, cudaStream_t s) {
@@ -702,9 +705,8 @@ cudaError_t begin_push(const StepParams &p, size_t nodes, cudaStream_t s) {
     const int nholes = p.slices > 1 ? (p.nsp + 1) * p.g.ntiles : 0;
     const int nlb = p.lb_cur ? kMaxSpecies : 0;
     const int blocks = (int)std::min<size_t>((n2 + 255) / 256, 148 * 16);
-    k_begin_push<<<blocks, 256, 0, s>>>((double2 *)p.J[0], n2, (unsigned *)p.st, (int)(sizeof(DevStatus) / 4), p.lb_cur,
-                                        nlb, p.hole_count, nholes);
-    return cudaGetLastError();
+    return launch_chained(k_begin_push, dim3(blocks), dim3(256), s, (double2 *)p.J[0], n2, (unsigned *)p.st,
+                          (int)(sizeof(DevStatus) / 4), p.lb_cur, nlb, p.hole_count, nholes, p.stamps, p.b_half);
 }
 
 cudaError_t kinetic_energy(const StepParams &p, double *out, cudaStream_t s) {

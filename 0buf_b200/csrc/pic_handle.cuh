@@ -45,7 +45,6 @@ struct pic_handle {
     char err[256];
     int64_t counters[4];
     float timings[5];
-    cudaEvent_t ev[6];
     int64_t launches;  // kernels launched by the current/last step
     int timed;
     int kin_valid;  // st->kinetic holds the kinetic energy of the current momenta

@@ -94,6 +94,19 @@ __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Time stamps of a step's kernels (nanoseconds of the GPU's global timer), one
+// per phase boundary, in place of events between the launches: an event is work
+// of its own on the stream and keeps the next kernel from being launched ahead
+// (32x4x4 cells, FP64 72 -> 53 us per step, FP32 62 -> 46 without its six).
+constexpr int kStamps = 6;
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void stamp_entry(unsigned long long *stamps, int k) {
+    if (stamps && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) stamps[k] = global_ns();
+}
 template <typename... P, typename... A>
 inline cudaError_t launch_chained_smem(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                        A &&... args) {
@@ -316,6 +329,7 @@ struct StepParams {
     int *holes;
     unsigned *hole_count, *ticket;
     int prefetch;  // plain push: the next particle comes through shared memory (set by its launcher)
+    unsigned long long *stamps;  // kStamps of the step (null: a sub-step call)
 };
 
 // one 4- or 8-byte asynchronous copy from global to shared memory

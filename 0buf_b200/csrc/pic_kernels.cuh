@@ -6,18 +6,21 @@
 namespace pic {
 
 // plain form (pic_plain.cu, FP64, -fmad=false)
-void yee_b_half_plain(const Grid &g, double *const F[12], cudaStream_t s);
+// stamps (here and below, null: none): the step's time stamps
+void yee_b_half_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned long long *stamps = nullptr);
 void yee_b_complete_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void yee_e_update_plain(const Grid &g, double *const F[12], cudaStream_t s);
 void j_fold(const Grid &g, double *Jx, double *Jy, double *Jz, cudaStream_t s);
 // the J fold and the B completion in one launch
-void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s);
+void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned long long *stamps = nullptr);
 // st, out: device status and pinned host memory that receives it (null: none);
 // hist: three sums that receive E_c^2 over the nodes 1..N (null: none)
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr);
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr,
+                    unsigned long long *stamps = nullptr);
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr);
+                    const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr,
+                    unsigned long long *stamps = nullptr);
 // The differentiable run's step.  Before its push, in one launch: Ha = H + Q(E)
 // (the B half step, out of place, the bits of yee_b_half_*), J = 0 (three arrays
 // one after another) and, where keepE is given, a copy of E (three arrays).
@@ -41,7 +44,8 @@ cudaError_t place_particles_plain(const Grid &g, int64_t n, const double *x, con
 void yee_b_half_mixed(const Grid &g, float *const E[3], float *const H[3], cudaStream_t s);
 // the J fold, and both B half steps of a step in one pass, H = (H + Q(E)) + Q(E) (pic_step: the push forms the first
 // in shared memory), in one launch
-void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s);
+void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s,
+                  unsigned long long *stamps = nullptr);
 void yee_e_update_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s);
 size_t push_smem_mixed(const Grid &g);
 // dynamic + static shared memory of the mixed push kernel ((size_t)-1 if it cannot be queried)

@@ -99,8 +99,10 @@ __global__ void k_b_half_mixed(Grid g, const float *__restrict__ Ex, const float
 // the first `folds` blocks fold, the others step
 __global__ void k_fold_b_mixed(Grid g, int folds, int per_plane, double *Jx, double *Jy, double *Jz,
                                const float *__restrict__ Ex, const float *__restrict__ Ey, const float *__restrict__ Ez,
-                               float *Hx, float *Hy, float *Hz, float cx, float cy, float cz) {
+                               float *Hx, float *Hy, float *Hz, float cx, float cy, float cz,
+                               unsigned long long *stamps) {
     chain_enter();
+    stamp_entry(stamps, 4);
     if ((int)blockIdx.x < folds) {
         double *const J[3] = {Jx, Jy, Jz};
         const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -443,7 +445,9 @@ __host__ __device__ inline MixedSmem mixed_smem(int tx, int ty, int tz) {
 // memory offsets become immediates), 0 to take them from the grid
 // SPLIT: P.slices CTAs share a tile (see StepParams::slices)
 template <int TX, int TY, int TZ, bool SPLIT>
-__global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps maps, StepParams P) {
+__global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps maps, const __grid_constant__ StepParams P) {
+    chain_enter();
+    stamp_entry(P.stamps, 2);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long sBar;
     // hole-list counters in three sets by species (s mod 3), so that a species
@@ -995,12 +999,13 @@ void flat_begin_mixed(const Grid &g, const float *const E[3], const float *const
                    keepE, cx, cy, cz);
 }
 
-void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s) {
+void fold_b_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s,
+                  unsigned long long *stamps) {
     float cx = (float)(g.tau / g.hx), cy = (float)(g.tau / g.hy), cz = (float)(g.tau / g.hz);
     const int folds = (fold_orbits(g) + kPlaneThreads - 1) / kPlaneThreads;
     const dim3 plane = plane_grid(g);
     launch_chained(k_fold_b_mixed, dim3(folds + plane.x * plane.y), dim3(kPlaneThreads), s, g, folds, (int)plane.x, J[0],
-                   J[1], J[2], E[0], E[1], E[2], H[0], H[1], H[2], cx, cy, cz);
+                   J[1], J[2], E[0], E[1], E[2], H[0], H[1], H[2], cx, cy, cz, stamps);
 }
 
 void yee_e_update_mixed(const Grid &g, float *const E[3], float *const H[3], double *const J[3], cudaStream_t s) {
@@ -1075,8 +1080,7 @@ cudaError_t launch_push_mixed(const StepParams &p, const MixedMaps &maps, cudaSt
     size_t smem = push_smem_mixed(p.g);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fn<<<p.g.ntiles * (split ? p.slices : 1), kMixedThreads, smem, s>>>(maps, p);
-    return cudaGetLastError();
+    return launch_chained_smem(fn, dim3(p.g.ntiles * (split ? p.slices : 1)), dim3(kMixedThreads), smem, s, maps, p);
 }
 
 }  // namespace pic

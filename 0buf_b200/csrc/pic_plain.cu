@@ -24,8 +24,10 @@ namespace {
 //   Hz: i<=Nx, l<=Ny, k<=Nz+1   Q = 0.5*(tau/hy*(Ex[+y]-Ex) - tau/hx*(Ey[+x]-Ey))
 __global__ void k_b_half_plain(Grid g, const double *__restrict__ Ex, const double *__restrict__ Ey,
                                const double *__restrict__ Ez, double *Hx, double *Hy, double *Hz, double *Qx,
-                               double *Qy, double *Qz, double cx, double cy, double cz) {
+                               double *Qy, double *Qz, double cx, double cy, double cz,
+                               unsigned long long *stamps) {
     chain_enter();
+    stamp_entry(stamps, 0);
     // one thread per node of an x plane (l, k flattened: no idle z tail)
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= g.NY * g.NZ) return;
@@ -73,8 +75,9 @@ __global__ void k_b_complete_plain(Grid g, double *Hx, double *Hy, double *Hz, c
 // the first `folds` blocks fold, the others complete
 __global__ void k_fold_b_plain(Grid g, int folds, int per_plane, double *Jx, double *Jy, double *Jz, double *Hx,
                                double *Hy, double *Hz, const double *__restrict__ Qx, const double *__restrict__ Qy,
-                               const double *__restrict__ Qz) {
+                               const double *__restrict__ Qz, unsigned long long *stamps) {
     chain_enter();
+    stamp_entry(stamps, 4);
     if ((int)blockIdx.x < folds) {
         double *const J[3] = {Jx, Jy, Jz};
         const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -197,7 +200,8 @@ __device__ __forceinline__ Line line_of(const Grid &g, int dir, int a, int b) {
 }
 
 // periodicCurrentElement (kernels.cu:1124-1146) on all axes (pic_fold.cuh).  One
-// launch instead of one per axis: 32x4x4 cells 7.5 -> 2.5 us.
+// launch instead of one per axis (with the other launches saved, the field kernels
+// of a 32x4x4 step 21.4 -> 13.3 us).
 __global__ void k_j_fold(Grid g, double *Jx, double *Jy, double *Jz) {
     chain_enter();
     double *const J[3] = {Jx, Jy, Jz};
@@ -241,7 +245,8 @@ __device__ __forceinline__ size_t ghost_source(const Grid &g, const GhostPasses 
 constexpr int kHistRows = 4;
 template <typename T>
 __global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus *out, const T *__restrict__ Ex,
-                           const T *__restrict__ Ey, const T *__restrict__ Ez, double *hist) {
+                           const T *__restrict__ Ey, const T *__restrict__ Ez, double *hist,
+                           unsigned long long *stamps) {
     chain_enter();
     if (out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(DevStatus) / sizeof(unsigned))
         ((volatile unsigned *)out)[threadIdx.x] = ((const unsigned *)st)[threadIdx.x];
@@ -292,6 +297,8 @@ __global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus
     }
     E[L.base] = E[srcN];
     E[L.base + (size_t)(q.N + 1) * L.stride] = E[src1];
+    // the step's end: the latest of the blocks (larger than any earlier step's)
+    if (stamps && threadIdx.x == 0) atomicMax(&stamps[5], global_ns());
 }
 
 
@@ -370,7 +377,9 @@ static_assert(kPlainThreads == kPushThreads, "the slices of a tile are cut in bl
 #endif
 // SPLIT: P.slices CTAs share a tile (see StepParams::slices)
 template <bool LO32, bool SPLIT>
-__global__ void PIC_PLAIN_BOUNDS k_push_plain(StepParams P) {
+__global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams P) {
+    chain_enter();
+    stamp_entry(P.stamps, 2);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sNHoles, sNFront, sNMove;
     __shared__ double sRed[kPlainThreads / 32];
@@ -739,11 +748,11 @@ static inline dim3 plane_grid(const Grid &g) {
     return dim3((g.NY * g.NZ + kPlaneThreads - 1) / kPlaneThreads, g.NX);
 }
 
-void yee_b_half_plain(const Grid &g, double *const F[12], cudaStream_t s) {
+void yee_b_half_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned long long *stamps) {
     // getMagneticFieldTimeMeshFactors, gpu_plasma.h:512-522
     double cx = g.tau / (g.hx), cy = g.tau / (g.hy), cz = g.tau / g.hz;
     launch_chained(k_b_half_plain, plane_grid(g), dim3(kPlaneThreads), s, g, F[PIC_EX], F[PIC_EY], F[PIC_EZ], F[PIC_HX],
-                   F[PIC_HY], F[PIC_HZ], F[PIC_QX], F[PIC_QY], F[PIC_QZ], cx, cy, cz);
+                   F[PIC_HY], F[PIC_HZ], F[PIC_QX], F[PIC_QY], F[PIC_QZ], cx, cy, cz, stamps);
 }
 
 void yee_b_complete_plain(const Grid &g, double *const F[12], cudaStream_t s) {
@@ -762,11 +771,11 @@ void j_fold(const Grid &g, double *Jx, double *Jy, double *Jz, cudaStream_t s) {
     launch_chained(k_j_fold, dim3((fold_orbits(g) + 127) / 128), dim3(128), s, g, Jx, Jy, Jz);
 }
 
-void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s) {
+void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned long long *stamps) {
     const int folds = (fold_orbits(g) + kPlaneThreads - 1) / kPlaneThreads;
     const dim3 plane = plane_grid(g);
     launch_chained(k_fold_b_plain, dim3(folds + plane.x * plane.y), dim3(kPlaneThreads), s, g, folds, (int)plane.x,
-                   F[PIC_JX], F[PIC_JY], F[PIC_JZ], F[PIC_HX], F[PIC_HY], F[PIC_HZ], F[PIC_QX], F[PIC_QY], F[PIC_QZ]);
+                   F[PIC_JX], F[PIC_JY], F[PIC_JZ], F[PIC_HX], F[PIC_HY], F[PIC_HZ], F[PIC_QX], F[PIC_QY], F[PIC_QZ], stamps);
 }
 
 // ElectricFieldComponentEvaluatePeriodic for Ex, Ey, Ez (gpu_plasma.h:432-452,
@@ -791,7 +800,7 @@ void fold_b_twice_plain(const Grid &g, double *const F[12], cudaStream_t s) {
 
 template <typename T>
 static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                       DevStatus *out, double *hist) {
+                       DevStatus *out, double *hist, unsigned long long *stamps) {
     int Nx = g.nx, Ny = g.ny, Nz = g.nz;
     GhostPasses P{};
     int maxn = 0;
@@ -810,15 +819,15 @@ static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStr
     add(Ey, 2, 0, Nx + 1, 0, Ny, Nz);
     if (periodic) add(Ez, 1, 0, Nx + 1, 0, Nz, Ny);
     launch_chained(k_e_ghosts<T>, dim3((maxn + 127) / 128, P.n + (hist ? kHistRows : 0)), dim3(128), s, g, P, st, out, Ex, Ey,
-                   Ez, hist);
+                   Ez, hist, stamps);
 }
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st, DevStatus *out, double *hist) {
-    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out, hist);
+                    const DevStatus *st, DevStatus *out, double *hist, unsigned long long *stamps) {
+    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps);
 }
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                    DevStatus *out, double *hist) {
-    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out, hist);
+                    DevStatus *out, double *hist, unsigned long long *stamps) {
+    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps);
 }
 
 // shared memory of the next particle of every thread
@@ -846,8 +855,7 @@ cudaError_t launch_push_plain(const StepParams &in, bool lo32, cudaStream_t s) {
                       : (split ? k_push_plain<false, true> : k_push_plain<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<p.g.ntiles * (split ? p.slices : 1), kPlainThreads, smem, s>>>(p);
-    return cudaGetLastError();
+    return launch_chained_smem(kern, dim3(p.g.ntiles * (split ? p.slices : 1)), dim3(kPlainThreads), smem, s, p);
 }
 
 }  // namespace pic
