@@ -505,12 +505,11 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         sQ = ldexp(1.0, e2 - 62);
         sTileE = e2 - 62;  // tile quantum 2^(e2-62)
         sInvQ = (float)ldexp(1.0, 62 - e2);
+    }
+    if (threadIdx.x == 32) {  // beside the quantum
         mbar_init(&sBar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
         const unsigned e_bytes = (unsigned)((size_t)(SX + 1) * BY * BZ * sizeof(float));
         const unsigned h_bytes = (unsigned)((size_t)SX * BY * BZ * sizeof(float));
         mbar_arrive_expect_tx(&sBar, 3 * e_bytes + 3 * h_bytes);
@@ -518,6 +517,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         for (int f = 0; f < 6; f++) tma_load_3d(smem_raw + L.raw_of(f), &maps.m[f], &sBar, k0, l0, i0);
     }
     for (int idx = threadIdx.x; idx < 3 * nn; idx += blockDim.x) sJ[idx] = 0ull;
+    __syncthreads();  // the barrier is initialised
     bool staged = false;
     for (int it = 0; it < kTmaWaitLimit && !(staged = mbar_try_wait(&sBar, 0)); it++) {
     }
@@ -938,14 +938,11 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         atomicAdd(&P.st->kinetic, tot);
     }
     if (SPLIT && last_of_tile(P, t, &sNHoles[0])) {
-        for (int s = 0; s < P.nsp; s++) {
-            const SpeciesView &S = P.sp[s];
-            compact_listed(P, t, s, sFront, sHoles, bad, [&](int dst, int src) {
-                S.cell[dst] = __ldcg(&S.cell[src]);
-                S.ox[dst] = __ldcg(&S.ox[src]); S.oy[dst] = __ldcg(&S.oy[src]); S.oz[dst] = __ldcg(&S.oz[src]);
-                S.fx[dst] = __ldcg(&S.fx[src]); S.fy[dst] = __ldcg(&S.fy[src]); S.fz[dst] = __ldcg(&S.fz[src]);
-            });
-        }
+        compact_tile(P, t, sHoles, bad, [](const SpeciesView &S, int dst, int src) {
+            S.cell[dst] = __ldcg(&S.cell[src]);
+            S.ox[dst] = __ldcg(&S.ox[src]); S.oy[dst] = __ldcg(&S.oy[src]); S.oz[dst] = __ldcg(&S.oz[src]);
+            S.fx[dst] = __ldcg(&S.fx[src]); S.fy[dst] = __ldcg(&S.fy[src]); S.fz[dst] = __ldcg(&S.fz[src]);
+        });
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (moved) atomicAdd(&P.st->moved, moved);

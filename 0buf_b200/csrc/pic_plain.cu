@@ -724,15 +724,11 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
         atomicAdd(&P.st->kinetic, tot);
     }
     if (SPLIT && last_of_tile(P, t, &sNHoles)) {
-        int *ctr = sHoles;
-        for (int s = 0; s < P.nsp; s++) {
-            const SpeciesView &S = P.sp[s];
-            compact_listed(P, t, s, sFront, ctr, bad, [&](int dst, int src) {
-                S.cell[dst] = __ldcg(&S.cell[src]);
-                S.x[dst] = __ldcg(&S.x[src]); S.y[dst] = __ldcg(&S.y[src]); S.z[dst] = __ldcg(&S.z[src]);
-                S.px[dst] = __ldcg(&S.px[src]); S.py[dst] = __ldcg(&S.py[src]); S.pz[dst] = __ldcg(&S.pz[src]);
-            });
-        }
+        compact_tile(P, t, sHoles, bad, [](const SpeciesView &S, int dst, int src) {
+            S.cell[dst] = __ldcg(&S.cell[src]);
+            S.x[dst] = __ldcg(&S.x[src]); S.y[dst] = __ldcg(&S.y[src]); S.z[dst] = __ldcg(&S.z[src]);
+            S.px[dst] = __ldcg(&S.px[src]); S.py[dst] = __ldcg(&S.py[src]); S.pz[dst] = __ldcg(&S.pz[src]);
+        });
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (moved) atomicAdd(&P.st->moved, moved);
