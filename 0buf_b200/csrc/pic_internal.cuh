@@ -187,11 +187,6 @@ constexpr long long kFxMaxTileSlots = 1ll << 23;
 // nearest even, as rint): conversions between FP64 and integers run at a
 // quarter of the FP64 add rate.
 constexpr double kRound = 0x1.8p52;
-__device__ __forceinline__ double fx_split(double s, long long &ih) {
-    const double u = s + kRound;
-    ih = __double_as_longlong(u) - 0x4338000000000000ll;
-    return s - (u - kRound);  // the exact remainder
-}
 // a contribution rounded by u = s + kRound, into a node's low and high word
 __device__ __forceinline__ void shared_add_rounded(unsigned *plo, unsigned *phi, double u) {
     const unsigned lo = (unsigned)__double2loint(u);
@@ -200,11 +195,9 @@ __device__ __forceinline__ void shared_add_rounded(unsigned *plo, unsigned *phi,
     if (hi) atomicAdd(phi, hi);
 }
 __device__ __forceinline__ void fx_put2(unsigned long long *hi, unsigned long long *lo, double s) {
-    long long ih;
-    const double r = fx_split(s, ih);
-    const long long il = __double_as_longlong(fma(r, 1099511627776.0, kRound)) - 0x4338000000000000ll;  // 2^40
-    if (ih) shared_add64(hi, ih);
-    if (il) shared_add64(lo, il);
+    const double u = s + kRound, r = s - (u - kRound);  // the exact remainder
+    shared_add_rounded((unsigned *)hi, (unsigned *)hi + 1, u);
+    shared_add_rounded((unsigned *)lo, (unsigned *)lo + 1, fma(r, 1099511627776.0, kRound));  // 2^40
 }
 // The same split with an int32 second word (native 32-bit shared atomics: a
 // c2 FP64 push takes 22 ms less than with the 64-bit word).  The remainder
@@ -223,11 +216,9 @@ __device__ __forceinline__ int fx_lo32_bits(long long n) {
     return 31 - b;
 }
 __device__ __forceinline__ void fx_put_lo32(unsigned long long *hi, int *lo, double s, double lo_scale) {
-    long long ih;
-    const double r = fx_split(s, ih);
-    const int il = __double2loint(fma(r, lo_scale, kRound));  // lo_scale = 2^L: exact
-    if (ih) shared_add64(hi, ih);
-    if (il) atomicAdd(lo, il);
+    const double u = s + kRound, r = s - (u - kRound);
+    shared_add_rounded((unsigned *)hi, (unsigned *)hi + 1, u);
+    atomicAdd(lo, __double2loint(fma(r, lo_scale, kRound)));  // lo_scale = 2^L: exact
 }
 
 struct SpeciesView {
