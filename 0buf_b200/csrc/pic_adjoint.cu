@@ -26,6 +26,7 @@
 #include "pic_internal.cuh"
 #include "pic_kernels.cuh"
 #include "pic_handle.cuh"
+#include <type_traits>
 #include "pic_adjoint.cuh"
 #include "pic_plain_math.cuh"
 #include "pic_fold.cuh"
@@ -146,25 +147,20 @@ __device__ __forceinline__ constexpr bool node_axis(int c, int d) { return c < 3
 // (that component is then 0, as in k_push_plain)
 template <class V>
 __device__ __forceinline__ bool gather_fields(const V &A, const AxisTaps T[3], double F[6]) {
-    bool okn[3], okc[3], ok = true;
+    // every tap in 2..3; each of the six indices is some component's
+    if ((((T[0].tn ^ 2) | (T[0].tc ^ 2) | (T[1].tn ^ 2) | (T[1].tc ^ 2) | (T[2].tn ^ 2) | (T[2].tc ^ 2)) & ~1) != 0) {
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        okn[d] = T[d].tn >= 2 && T[d].tn <= 3;
-        okc[d] = T[d].tc >= 2 && T[d].tc <= 3;
+        for (int c = 0; c < 6; c++) F[c] = 0.0;
+        return false;
     }
 #pragma unroll
     for (int c = 0; c < 6; c++) {
         const bool nx = node_axis(c, 0), ny = node_axis(c, 1), nz = node_axis(c, 2);
-        if (!((nx ? okn[0] : okc[0]) && (ny ? okn[1] : okc[1]) && (nz ? okn[2] : okc[2]))) {
-            ok = false;
-            F[c] = 0.0;
-            continue;
-        }
         const int n = A.at(nx ? T[0].tn : T[0].tc, ny ? T[1].tn : T[1].tc, nz ? T[2].tn : T[2].tc);
         const double wx = nx ? T[0].wn : T[0].wc, wy = ny ? T[1].wn : T[1].wc, wz = nz ? T[2].wn : T[2].wc;
         F[c] = trilinear(A.base[c] + n, A.dx, A.dy, wx, 1. - wx, wy, 1. - wy, wz, 1. - wz);
     }
-    return ok;
+    return true;
 }
 
 // zigzag split of CurrentToMesh, cell.h:1306-1422
@@ -366,13 +362,15 @@ __device__ __forceinline__ int new_cell_plain(const Grid &g, int cell, int i, in
     return g.cell_of(rx, ry, rz);
 }
 
-// stages the window's nodes of `n` arrays src[c] into dst (n x w.nn doubles)
+// stages the window's nodes of N arrays src[c] into dst (cn doubles apart)
 template <int N, bool WRAP>
-__device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow<WRAP> &w, const double *const *src, double *dst) {
+__device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow<WRAP> &w, int cn, const double *const *src,
+                                             double *dst) {
     for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
-        const size_t n = w.grid_node(g, e);
+        size_t n;
+        if (!w.grid_node(g, e, n)) continue;
 #pragma unroll
-        for (int q = 0; q < N; q++) dst[q * w.nn + e] = src[q][n];
+        for (int q = 0; q < N; q++) dst[q * cn + e] = src[q][n];
     }
 }
 
@@ -406,7 +404,11 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     const FlatSp &S = P.sp[s];
     if ((int)threadIdx.x < count) next.start(S, ch.first + threadIdx.x);
     const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
-    const int nn = w.nn;
+    // (see AdjWindow: the strides at compile time where the window has them)
+    auto body = [&](auto fixed) {
+    constexpr bool FIX = decltype(fixed)::value;
+    const int SY = FIX ? kFixSY : w.SY, SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
+    const int cn = FIX ? kFlatWindow : nn;  // between the components
     if (threadIdx.x == 0) {
         // the quantum of k_push_plain's tile current, for this chunk
         int e2, e1;
@@ -417,11 +419,8 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
         sInvQ = ldexp(1.0, -eq);
     }
     const double *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window<6>(g, w, src, sF);
-    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
-        sJ[e] = 0ull;
-        ((int *)(sJ + 3 * nn))[e] = 0;
-    }
+    stage_window<6>(g, w, cn, src, sF);
+    for (int e = threadIdx.x; e < 9 * cn; e += blockDim.x) ((unsigned *)sJ)[e] = 0u;
     if (lane == 0) sQn[warp] = 0;
     __syncthreads();
     const double h3[3] = {g.hx, g.hy, g.hz}, r3[3] = {1.0 / g.hx, 1.0 / g.hy, 1.0 / g.hz};
@@ -450,7 +449,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
             int u3[3], n0;
-            const bool in = w.place(c3, u3, n0);
+            const bool in = w.place(c3, dX, dY, u3, n0);
             const double o3[3] = {(double)c3[0] * h3[0], (double)c3[1] * h3[1], (double)c3[2] * h3[2]};
             const unsigned long long rcode = BMODE == 2 ? P.branch[P.off[s] + j] : 0ull;
             AxisTaps T[3];
@@ -478,8 +477,8 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                 if (in) {
                     FieldView<true> A;
 #pragma unroll
-                    for (int c = 0; c < 6; c++) A.base[c] = sF + c * nn;
-                    A.n0 = n0; A.dx = w.SY * w.SZ; A.dy = w.SZ;
+                    for (int c = 0; c < 6; c++) A.base[c] = sF + c * cn;
+                    A.n0 = n0; A.dx = dX; A.dy = dY;
                     ok = gather_fields(A, T, F);
                 } else {
                     FieldView<false> A;
@@ -492,7 +491,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
             }
             double p2;
             const double ig = boris_move(tau1, F, p, p2);
-            if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) bad |= ST_NAN;
+            if (!isfinite(p2) && !(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) bad |= ST_NAN;
             Split SP;
             double x1[3];
             bool exact = true;
@@ -510,7 +509,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
 #pragma unroll
             for (int d = 0; d < 3; d++) sb[d] = cross ? SP.x2[d] : x1[d];
             if (in) {
-                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, u3[0] - 2, u3[1] - 2, u3[2] - 2, SP.i1,
+                pqr_plain<true>(sJ, lo_scale, cn, dX, dY, u3[0] - 2, u3[1] - 2, u3[2] - 2, SP.i1,
                                 x, sb, g.hx, g.hy, g.hz, rc, o3[0], o3[1], o3[2], bad);
                 if (cross) {
                     if (SP.i2[0] >= 2 && SP.i2[0] <= 3 && SP.i2[1] >= 2 && SP.i2[1] <= 3 && SP.i2[2] >= 2 &&
@@ -595,7 +594,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                     sa[q] = qd[q * kQueuePlain + e];
                     se[q] = qd[(3 + q) * kQueuePlain + e];
                 }
-                pqr_plain<true>(sJ, lo_scale, nn, w.SY, w.SZ, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
+                pqr_plain<true>(sJ, lo_scale, cn, dX, dY, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
                                 (double)w.at(0, a) * g.hx, (double)w.at(1, b) * g.hy, (double)w.at(2, c) * g.hz, bad);
             }
             qn -= d;
@@ -606,14 +605,18 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
-        const long long ih = (long long)sJ[e];
-        const int il = ((const int *)(sJ + 3 * nn))[e];
-        if (ih == 0 && il == 0) continue;
-        const int comp = e / nn, r = e - comp * nn;
-        atomicAdd(&P.J[comp][w.grid_node(g, r)], ((double)ih + (double)il / lo_scale) * sQ);
+        const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
+        const long long ih = (long long)sJ[a];
+        const int il = ((const int *)(sJ + 3 * cn))[a];
+        size_t n;
+        if ((ih == 0 && il == 0) || !w.grid_node(g, r, n)) continue;
+        atomicAdd(&P.J[comp][n], ((double)ih + (double)il / lo_scale) * sQ);
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (amb) atomicAdd(&P.st->ambiguous, amb);
+    };
+    if (w.fixed()) body(std::true_type{});
+    else body(std::false_type{});
 }
 
 // The taps in few registers: bit d tn - 2, bit 3 + d tc - 2, bit 6 + d cI - nI
@@ -864,8 +867,8 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
     double *sF = (double *)smem_raw, *sL = sF + 6 * nn;
     unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
     const double *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window<6>(g, w, src, sF);
-    stage_window<3>(g, w, A.LJ, sL);
+    stage_window<6>(g, w, nn, src, sF);
+    stage_window<3>(g, w, nn, A.LJ, sL);
     for (int e = threadIdx.x; e < 12 * nn; e += blockDim.x) sLo[e] = 0u;
     if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = 0u; sK = reverse_const(g, S); }
     __syncthreads();
@@ -882,7 +885,8 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
                 if (v == 0) continue;
                 if (again) sHi[e] = sLo[e] = 0u;
                 const int comp = e / nn, r = e - comp * nn;
-                        atomicAdd(&dst[comp][w.grid_node(g, r)], (double)v * q);
+                        size_t n;
+                        if (w.grid_node(g, r, n)) atomicAdd(&dst[comp][n], (double)v * q);
             }
         }
     };
@@ -906,7 +910,7 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
         if (near) {
             int u[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            if (!w.place(c3, u, n0)) {
+            if (!w.place(c3, dX, dY, u, n0)) {
                 near = false;
                 sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
             }

@@ -8,6 +8,7 @@
 #include "pic0buf.h"
 #include "pic_internal.cuh"
 #include "pic_handle.cuh"
+#include <type_traits>
 #include "pic_adjoint.cuh"
 
 namespace pic {
@@ -286,13 +287,14 @@ struct NextMix {
     }
 };
 
-// stages the window's nodes of N arrays src[c] into dst (N x w.nn floats)
+// stages the window's nodes of N arrays src[c] into dst (cn floats apart)
 template <int N, class T, bool WRAP>
-__device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WRAP> &w, const T *const *src, float *dst) {
+__device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WRAP> &w, int cn, const T *const *src, float *dst) {
     for (int e = threadIdx.x; e < w.nn; e += blockDim.x) {
-        const size_t n = w.grid_node(g, e);
+        size_t n;
+        if (!w.grid_node(g, e, n)) continue;
 #pragma unroll
-        for (int q = 0; q < N; q++) dst[q * w.nn + e] = (float)src[q][n];
+        for (int q = 0; q < N; q++) dst[q * cn + e] = (float)src[q][n];
     }
 }
 
@@ -323,9 +325,13 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
     const NextMix<6> next(sTail + (size_t)kW * 7 * kQueueMix * sizeof(float));
     if ((int)threadIdx.x < count) next.start(S, nullptr, ch.first + threadIdx.x);
     const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
-    const int nn = w.nn, dX = w.SY * w.SZ, dY = w.SZ;
-    unsigned *sLo = (unsigned *)smem_raw, *sHi = sLo + 3 * nn;
-    float *sF = (float *)(sHi + 3 * nn);
+    // (see AdjWindow: the strides at compile time where the window has them)
+    auto body = [&](auto fixed) {
+    constexpr bool FIX = decltype(fixed)::value;
+    const int SY = FIX ? kFixSY : w.SY, SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
+    const int cn = FIX ? kFlatWindowMix : nn;  // between the components
+    unsigned *sLo = (unsigned *)smem_raw, *sHi = sLo + 3 * cn;
+    float *sF = (float *)(sHi + 3 * cn);
     if (threadIdx.x == 0) {
         int e2, e1;
         frexp(2.5 * fabs(S.m) * (double)count, &e2);
@@ -336,8 +342,8 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         sK = mix_const(g, S);
     }
     const float *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window_m<6>(g, w, src, sF);
-    for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) sLo[e] = 0u;
+    stage_window_m<6>(g, w, cn, src, sF);
+    for (int e = threadIdx.x; e < 6 * cn; e += blockDim.x) sLo[e] = 0u;
     if (lane == 0) sQn[warp] = 0;
     __syncthreads();
     const MixConst &K = sK;
@@ -347,7 +353,7 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
     int qn = 0;
     auto put = [&](int n0) {
         return [=](int c, int a, int b, int k, float v) {
-            const int n = c * nn + n0 + a * dX + b * dY + k;
+            const int n = c * cn + n0 + a * dX + b * dY + k;
             const long long iv = __double_as_longlong(fma((double)v, inv_q, kRound)) - 0x4338000000000000ll;
             if (iv) shared_add64(sLo + n, sHi + n, iv);
         };
@@ -371,12 +377,12 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
             int u3[3], n0;
-            const bool in = w.place(c3, u3, n0);
+            const bool in = w.place(c3, dX, dY, u3, n0);
             float F[6];
             if (in) {
                 FieldViewM<true> V;
 #pragma unroll
-                for (int c = 0; c < 6; c++) V.base[c] = sF + c * nn + n0;
+                for (int c = 0; c < 6; c++) V.base[c] = sF + c * cn + n0;
                 V.dx = dX; V.dy = dY;
                 gather_fields_m(V, xs, F);
             } else {
@@ -456,12 +462,16 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
-        const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
-        if (v == 0) continue;
-        const int comp = e / nn, r = e - comp * nn;
-        atomicAdd(&P.J[comp][w.grid_node(g, r)], (double)v * sQ);
+        const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
+        const long long v = (long long)(((unsigned long long)sHi[a] << 32) | sLo[a]);
+        size_t n;
+        if (v == 0 || !w.grid_node(g, r, n)) continue;
+        atomicAdd(&P.J[comp][n], (double)v * sQ);
     }
     if (bad) atomicOr(&P.st->flags, bad);
+    };
+    if (w.fixed()) body(std::true_type{});
+    else body(std::false_type{});
 }
 
 // The reverse of one particle's step up to the adjoint of its interpolated
@@ -636,8 +646,8 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     float *sF = (float *)smem_raw, *sL = sF + 6 * nn;
     unsigned *sLo = (unsigned *)(sL + 3 * nn), *sHi = sLo + 6 * nn;
     const float *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window_m<6>(g, w, src, sF);
-    stage_window_m<3>(g, w, P.LJ, sL);
+    stage_window_m<6>(g, w, nn, src, sF);
+    stage_window_m<3>(g, w, nn, P.LJ, sL);
     for (int e = threadIdx.x; e < 12 * nn; e += blockDim.x) sLo[e] = 0u;
     if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = 0u; sK = mix_const(g, S); }
     __syncthreads();
@@ -653,7 +663,8 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
             if (v == 0) continue;
             if (again) sHi[e] = sLo[e] = 0u;
             const int comp = e / nn, r = e - comp * nn;
-                atomicAdd(&dst[comp][w.grid_node(g, r)], (double)v * q);
+                size_t n;
+                if (w.grid_node(g, r, n)) atomicAdd(&dst[comp][n], (double)v * q);
         }
     };
     for (int base = 0, it = 0; base < count; base += blockDim.x, it++) {
@@ -676,7 +687,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
         if (near) {
             int u[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            if (!w.place(c3, u, n0)) {
+            if (!w.place(c3, dX, dY, u, n0)) {
                 near = false;
                 sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
             }

@@ -598,7 +598,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
                     double sb[3];
 #pragma unroll
                     for (int d = 0; d < 3; d++) sb[d] = cross ? x2[d] : xn[d];
-                    pqr_plain<LO32>(sJ, lo_scale, nn, SY, SZ, bi, bl, bk, i1, xo, sb, hx, hy, hz, rc, x0, y0, z0, bad);
+                    pqr_plain<LO32>(sJ, lo_scale, nn, SY * SZ, SZ, bi, bl, bk, i1, xo, sb, hx, hy, hz, rc, x0, y0, z0, bad);
                     if (cross) {
                         if (i2[0] >= 2 && i2[0] <= 3 && i2[1] >= 2 && i2[1] <= 3 && i2[2] >= 2 && i2[2] <= 3) {
                             const int e = atomicAdd(&sQn[warp], 1);  // < 15 + 32: drained at 16
@@ -684,7 +684,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
                         sa[dd] = qd[dd * kQPlain + e];
                         sb[dd] = qd[(3 + dd) * kQPlain + e];
                     }
-                    pqr_plain<LO32>(sJ, lo_scale, nn, SY, SZ, a - 2, b - 2, c - 2, iv, sa, sb, hx, hy, hz, rc,
+                    pqr_plain<LO32>(sJ, lo_scale, nn, SY * SZ, SZ, a - 2, b - 2, c - 2, iv, sa, sb, hx, hy, hz, rc,
                                     (double)qi * hx, (double)ql * hy, (double)qk * hz, bad);
                 }
                 qn -= d;

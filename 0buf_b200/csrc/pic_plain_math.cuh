@@ -165,9 +165,9 @@ __device__ __forceinline__ int relay_point(const double xo[3], const double xn[3
 // inverse quantum, precomputed): the products feed only the current's
 // magnitude, never an index, and differ from the quotients by an ulp.  LO32
 // selects the int32 remainder word (fx_put_lo32; words at sJ + 3 nn as 3 nn
-// ints), else the 64-bit one (fx_put2; 3 nn words).
+// ints), else the 64-bit one (fx_put2; 3 nn words).  ex, ey: node strides.
 template <bool LO32>
-__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double lo_scale, int nn, int SY, int SZ,
+__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double lo_scale, int nn, int ex, int ey,
                                           int bi, int bl, int bk, const int iv[3], const double x[3],
                                           const double x1[3], double hx, double hy, double hz, const double rc[3],
                                           double x0, double y0, double z0, unsigned &bad) {
@@ -182,8 +182,7 @@ __device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, d
     sv = sv * rc[1];
     sw = sw * rc[2];
     if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) { bad |= ST_STENCIL; return; }
-    const int n = ((bi + iv[0]) * SY + (bl + iv[1])) * SZ + (bk + iv[2]);
-    const int ez = 1, ey = SZ, ex = SY * SZ;
+    const int n = (bi + iv[0]) * ex + (bl + iv[1]) * ey + (bk + iv[2]), ez = 1;
     int *lo32 = (int *)(sJ + 3 * nn);
     // component c, node offset o from n, contribution v in quanta
     auto add = [&](int c, int o, double v) {
