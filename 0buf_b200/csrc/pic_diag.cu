@@ -45,14 +45,17 @@ namespace {
 // `copies` boxes in turn, whose nodes lie 4 banks apart, and the next particle is
 // loaded before the current one is processed.  50.3M particles, 6x4x8 and 8x4x8
 // tiles: FP32 696 -> 399 us, FP64 752 -> 447 us (one box 714 and 712, two 637,
-// four 483 and 491; 16 boxes leave too few CTAs per SM); 805M FP32 9.95 -> 5.45 ms.
+// four 483 and 491; 16 boxes, which leave three CTAs per SM, 427 and 546); with
+// the tile's dimensions at compile time 386 and 408.  805M FP32 9.95 -> 5.26 ms.
 // With few tiles each is dealt out to several CTAs: the reference's default run
-// (13 tiles of 500k particles) 3546 -> 101 us FP64, 2118 -> 87 us FP32.
+// (13 tiles of 500k particles) 3546 -> 100 us FP64, 2118 -> 87 us FP32.
 // The copies: as many as five CTAs per SM leave room for.
 constexpr int kRhoCopies = 8, kRhoBytes = 40 * 1024;
 // words of a copy: nn low, nn high, and a pad
 __host__ __device__ inline int rho_stride(int nn) { return (2 * nn + 31) / 32 * 32 + 4; }
-template <bool MIXED>
+// TX, TY, TZ: the tile's cells per axis when fixed at compile time, 0 to take them
+// from the grid
+template <bool MIXED, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, int copies, double *rho) {
     using T = typename std::conditional<MIXED, float, double>::type;
     const Grid &g = P.g;
@@ -63,8 +66,9 @@ __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, int copies, d
     __shared__ int sMagic;
     const int t = blockIdx.x;
     const int tk = t % g.ntz, tl = (t / g.ntz) % g.nty, ti = t / (g.ntz * g.nty);
-    const int i0 = ti * g.tx, l0 = tl * g.ty, k0 = tk * g.tz;
-    const int SX = g.tx + 2, SY = g.ty + 2, SZ = g.tz + 2;
+    const int tx = TX ? TX : g.tx, ty = TY ? TY : g.ty, tz = TZ ? TZ : g.tz;
+    const int i0 = ti * tx, l0 = tl * ty, k0 = tk * tz;
+    const int SX = tx + 2, SY = ty + 2, SZ = tz + 2;
     const int nn = SX * SY * SZ, stride = rho_stride(nn);
     if (threadIdx.x == 0) {
         double bound = 0.0, one = 0.0;
@@ -272,7 +276,9 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
     int copies = kRhoCopies;
     while (copies > 1 && copies * box > (size_t)kRhoBytes) copies /= 2;
     const size_t smem = copies * box;
-    auto *k = p.mixed ? k_charge_tile<true> : k_charge_tile<false>;
+    // fixed dimensions for the automatic tiles of most grids, else runtime
+    auto *k = p.mixed ? (g.tx == 6 && g.ty == 4 && g.tz == 8 ? k_charge_tile<true, 6, 4, 8> : k_charge_tile<true, 0, 0, 0>)
+                      : (g.tx == 8 && g.ty == 4 && g.tz == 8 ? k_charge_tile<false, 8, 4, 8> : k_charge_tile<false, 0, 0, 0>);
     if (smem > 48 * 1024) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
