@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     __shared__ int sRed[15 * kW], sQn[kW];
     __shared__ double sQ, sInvQ;
     double *sF = (double *)smem_raw;
-    unsigned long long *sJ = (unsigned long long *)(sF + 6 * kFlatWindow);  // 3 nn words, then 3 nn ints
+    unsigned long long *sJ = (unsigned long long *)(sF + 6 * kFlatWindow);  // 9 words per node (pqr_plain)
     unsigned char *sTail = smem_raw + (size_t)kFlatWindow * (6 * sizeof(double) + 3 * 12);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double *qd = (double *)sTail + warp * 6 * kQueuePlain;
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
 #pragma unroll
             for (int d = 0; d < 3; d++) sb[d] = cross ? SP.x2[d] : x1[d];
             if (in) {
-                pqr_plain<true>(sJ, lo_scale, cn, dX, dY, u3[0] - 2, u3[1] - 2, u3[2] - 2, SP.i1,
+                pqr_plain<true>((unsigned *)sJ, lo_scale, cn, dX, dY, u3[0] - 2, u3[1] - 2, u3[2] - 2, SP.i1,
                                 x, sb, g.hx, g.hy, g.hz, rc, o3[0], o3[1], o3[2], bad);
                 if (cross) {
                     if (SP.i2[0] >= 2 && SP.i2[0] <= 3 && SP.i2[1] >= 2 && SP.i2[1] <= 3 && SP.i2[2] >= 2 &&
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
                     sa[q] = qd[q * kQueuePlain + e];
                     se[q] = qd[(3 + q) * kQueuePlain + e];
                 }
-                pqr_plain<true>(sJ, lo_scale, cn, dX, dY, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
+                pqr_plain<true>((unsigned *)sJ, lo_scale, cn, dX, dY, a - 2, b - 2, c - 2, iv, sa, se, g.hx, g.hy, g.hz, rc,
                                 (double)w.at(0, a) * g.hx, (double)w.at(1, b) * g.hy, (double)w.at(2, c) * g.hz, bad);
             }
             qn -= d;
@@ -606,8 +606,8 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     __syncthreads();
     for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
         const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
-        const long long ih = (long long)sJ[a];
-        const int il = ((const int *)(sJ + 3 * cn))[a];
+        long long ih, il;
+        fx_get<true>((const unsigned *)sJ + a, 3 * cn, ih, il);
         size_t n;
         if ((ih == 0 && il == 0) || !w.grid_node(g, r, n)) continue;
         atomicAdd(&P.J[comp][n], ((double)ih + (double)il / lo_scale) * sQ);

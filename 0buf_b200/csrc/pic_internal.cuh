@@ -194,10 +194,13 @@ __device__ __forceinline__ void shared_add_rounded(unsigned *plo, unsigned *phi,
     const unsigned hi = (unsigned)__double2hiint(u) - 0x43380000u + (old + lo < old ? 1u : 0u);
     if (hi) atomicAdd(phi, hi);
 }
-__device__ __forceinline__ void fx_put2(unsigned long long *hi, unsigned long long *lo, double s) {
+// (w: the node's low word; its high word and the remainder's low and high word
+// follow at distances of d: arrays of low and of high words use all banks, where
+// pairs of them put every low word on an even one)
+__device__ __forceinline__ void fx_put2(unsigned *w, int d, double s) {
     const double u = s + kRound, r = s - (u - kRound);  // the exact remainder
-    shared_add_rounded((unsigned *)hi, (unsigned *)hi + 1, u);
-    shared_add_rounded((unsigned *)lo, (unsigned *)lo + 1, fma(r, 1099511627776.0, kRound));  // 2^40
+    shared_add_rounded(w, w + d, u);
+    shared_add_rounded(w + 2 * d, w + 3 * d, fma(r, 1099511627776.0, kRound));  // 2^40
 }
 // The same split with an int32 second word (native 32-bit shared atomics: a
 // c2 FP64 push takes 22 ms less than with the 64-bit word).  The remainder
@@ -215,10 +218,16 @@ __device__ __forceinline__ int fx_lo32_bits(long long n) {
     while ((1ll << b) <= n) b++;
     return 31 - b;
 }
-__device__ __forceinline__ void fx_put_lo32(unsigned long long *hi, int *lo, double s, double lo_scale) {
+__device__ __forceinline__ void fx_put_lo32(unsigned *w, int d, double s, double lo_scale) {
     const double u = s + kRound, r = s - (u - kRound);
-    shared_add_rounded((unsigned *)hi, (unsigned *)hi + 1, u);
-    atomicAdd(lo, __double2loint(fma(r, lo_scale, kRound)));  // lo_scale = 2^L: exact
+    shared_add_rounded(w, w + d, u);
+    atomicAdd((int *)w + 2 * d, __double2loint(fma(r, lo_scale, kRound)));  // lo_scale = 2^L: exact
+}
+// the sums in the words of a node (LO32: with the int32 remainder)
+template <bool LO32>
+__device__ __forceinline__ void fx_get(const unsigned *w, int d, long long &ih, long long &il) {
+    ih = (long long)(((unsigned long long)w[d] << 32) | w[0]);
+    il = LO32 ? (long long)(int)w[2 * d] : (long long)(((unsigned long long)w[3 * d] << 32) | w[2 * d]);
 }
 
 struct SpeciesView {
@@ -320,6 +329,7 @@ struct StepParams {
     int *holes;
     unsigned *hole_count, *ticket;
     int prefetch;  // plain push: the next particle comes through shared memory (set by its launcher)
+    int jcopies;   // plain push: tile currents per CTA, 1 or 2 (set by its launcher)
     unsigned long long *stamps;  // kStamps of the step (null: a sub-step call)
 };
 

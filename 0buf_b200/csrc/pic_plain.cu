@@ -370,6 +370,9 @@ struct BinP {
 // ones; with the tile's dimensions fixed at compile time, one check of all taps,
 // deposits without tests for zero and uniform bin pointers 1394 -> 1137
 // instructions, and 128x64x64 cells, 50.3M particles, 3.22 -> 2.74 ms.
+// Then the shared-memory pipe was 76 % busy, half of it adds to one address taking
+// turns: a second tile current for the odd lanes and separate low and high words
+// 2.74 -> 2.63 ms (2.75 -> 2.65 with bins no longer in cell order).
 #ifndef PIC_PLAIN_THREADS
 #define PIC_PLAIN_THREADS 256
 #endif
@@ -410,10 +413,14 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
     const int SX = tx + 2, SY = ty + 2, SZ = tz + 2;
     const int nn = SX * SY * SZ;
     double *sF = (double *)smem_raw;  // Ex Ey Ez Hx Hy Hz
-    // fixed-point tile J: 3 nn high words, then the remainder words (3 nn
-    // 64-bit, or 3 nn int32 in the first half of that space)
+    // fixed-point tile J (pqr_plain): 3 nn low and 3 nn high words, then the
+    // remainder's (3 nn low, 3 nn high words, or 3 nn int32)
     unsigned long long *sJ = (unsigned long long *)(sF + 6 * nn);
-    int *sHoles = (int *)(sJ + 6 * nn);
+    // (lo32 with room for it: two currents, even lanes in one, odd lanes in the other)
+    const int jstride = (9 * nn + 1) / 2, jcopies = LO32 ? P.jcopies : 1;
+    const int jwords = jcopies == 2 ? 2 * jstride : 6 * nn;
+    unsigned *myJ = (unsigned *)(sJ + (LO32 ? (lane & (jcopies - 1)) * jstride : 0));
+    int *sHoles = (int *)(sJ + jwords);
     int *sFront = sHoles + kHoleMax;
     // this warp's segment queue: x2 and xn (6 x kQPlain doubles), and the
     // start cell (tile-local) with the segment's centre-cell bits
@@ -461,8 +468,8 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
         sF[3 * nn + idx] = in ? H[0][n] : 0.0;
         sF[4 * nn + idx] = in ? H[1][n] : 0.0;
         sF[5 * nn + idx] = in ? H[2][n] : 0.0;
-        for (int w = 0; w < 6; w++) sJ[w * nn + idx] = 0ull;
     }
+    for (int idx = threadIdx.x; idx < jwords; idx += blockDim.x) sJ[idx] = 0ull;
     __syncthreads();
 
     const double hx = g.hx, hy = g.hy, hz = g.hz, tau = g.tau;
@@ -598,7 +605,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
                     double sb[3];
 #pragma unroll
                     for (int d = 0; d < 3; d++) sb[d] = cross ? x2[d] : xn[d];
-                    pqr_plain<LO32>(sJ, lo_scale, nn, SY * SZ, SZ, bi, bl, bk, i1, xo, sb, hx, hy, hz, rc, x0, y0, z0, bad);
+                    pqr_plain<LO32>(myJ, lo_scale, nn, SY * SZ, SZ, bi, bl, bk, i1, xo, sb, hx, hy, hz, rc, x0, y0, z0, bad);
                     if (cross) {
                         if (i2[0] >= 2 && i2[0] <= 3 && i2[1] >= 2 && i2[1] <= 3 && i2[2] >= 2 && i2[2] <= 3) {
                             const int e = atomicAdd(&sQn[warp], 1);  // < 15 + 32: drained at 16
@@ -684,7 +691,7 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
                         sa[dd] = qd[dd * kQPlain + e];
                         sb[dd] = qd[(3 + dd) * kQPlain + e];
                     }
-                    pqr_plain<LO32>(sJ, lo_scale, nn, SY * SZ, SZ, a - 2, b - 2, c - 2, iv, sa, sb, hx, hy, hz, rc,
+                    pqr_plain<LO32>(myJ, lo_scale, nn, SY * SZ, SZ, a - 2, b - 2, c - 2, iv, sa, sb, hx, hy, hz, rc,
                                     (double)qi * hx, (double)ql * hy, (double)qk * hz, bad);
                 }
                 qn -= d;
@@ -724,8 +731,14 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
     if (SPLIT) __syncthreads();
     // ---- tile J -> global J (GPU_WriteAllCurrents, kernels.cu:83-112)
     for (int idx = threadIdx.x; idx < 3 * nn; idx += blockDim.x) {
-        const long long ih = (long long)sJ[idx];
-        const long long il = LO32 ? (long long)((const int *)(sJ + 3 * nn))[idx] : (long long)sJ[3 * nn + idx];
+        long long ih, il;
+        fx_get<LO32>((const unsigned *)sJ + idx, 3 * nn, ih, il);
+        if (jcopies == 2) {
+            long long ih2, il2;
+            fx_get<LO32>((const unsigned *)(sJ + jstride) + idx, 3 * nn, ih2, il2);
+            ih += ih2;
+            il += il2;
+        }
         if (ih != 0 || il != 0) {
             int comp = idx / nn, r = idx % nn;
             int c = r % SZ, b = (r / SZ) % SY, a = r / (SZ * SY);
@@ -879,6 +892,11 @@ cudaError_t launch_push_plain(const StepParams &in, bool lo32, cudaStream_t s) {
     auto fit = [&](size_t b) { return std::min<size_t>(PIC_PLAIN_MIN_BLOCKS, (size_t)per_sm / (b + 2048)); };
     p.prefetch = smem + kPlainPrefetch <= (size_t)per_block && fit(smem + kPlainPrefetch) >= fit(smem);
     if (p.prefetch) smem += kPlainPrefetch;
+    // a second tile current likewise
+    const size_t nn = (size_t)(p.g.tx + 2) * (p.g.ty + 2) * (p.g.tz + 2);
+    const size_t second = (2 * ((9 * nn + 1) / 2) - 6 * nn) * sizeof(unsigned long long);
+    p.jcopies = lo32 && smem + second <= (size_t)per_block && fit(smem + second) >= fit(smem) ? 2 : 1;
+    if (p.jcopies == 2) smem += second;
     const bool split = p.slices > 1;
     const PushPlainFn kern = push_plain_fn(p.g, lo32, split);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

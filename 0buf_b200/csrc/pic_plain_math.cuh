@@ -163,11 +163,11 @@ __device__ __forceinline__ int relay_point(const double xo[3], const double xn[3
 // reference's divisions by 12 and by tau*h*h are multiplications by their
 // reciprocals (rc[d] = 1 / (tau * h_e * h_f) times the charge weight and the
 // inverse quantum, precomputed): the products feed only the current's
-// magnitude, never an index, and differ from the quotients by an ulp.  LO32
-// selects the int32 remainder word (fx_put_lo32; words at sJ + 3 nn as 3 nn
-// ints), else the 64-bit one (fx_put2; 3 nn words).  ex, ey: node strides.
+// magnitude, never an index, and differ from the quotients by an ulp.  sJ: 3 nn
+// low words, 3 nn high words, then the remainders (LO32: 3 nn int32, fx_put_lo32;
+// else 3 nn low and 3 nn high words, fx_put2).  ex, ey: node strides.
 template <bool LO32>
-__device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, double lo_scale, int nn, int ex, int ey,
+__device__ __forceinline__ void pqr_plain(unsigned *__restrict__ sJ, double lo_scale, int nn, int ex, int ey,
                                           int bi, int bl, int bk, const int iv[3], const double x[3],
                                           const double x1[3], double hx, double hy, double hz, const double rc[3],
                                           double x0, double y0, double z0, unsigned &bad) {
@@ -183,12 +183,11 @@ __device__ __forceinline__ void pqr_plain(unsigned long long *__restrict__ sJ, d
     sw = sw * rc[2];
     if (iv[0] < 2 || iv[0] > 3 || iv[1] < 2 || iv[1] > 3 || iv[2] < 2 || iv[2] > 3) { bad |= ST_STENCIL; return; }
     const int n = (bi + iv[0]) * ex + (bl + iv[1]) * ey + (bk + iv[2]), ez = 1;
-    int *lo32 = (int *)(sJ + 3 * nn);
     // component c, node offset o from n, contribution v in quanta
     auto add = [&](int c, int o, double v) {
-        const int w = c * nn + n + o;
-        if (LO32) fx_put_lo32(&sJ[w], &lo32[w], v, lo_scale);
-        else fx_put2(&sJ[w], &sJ[3 * nn + w], v);
+        unsigned *w = sJ + c * nn + n + o;
+        if (LO32) fx_put_lo32(w, 3 * nn, v, lo_scale);
+        else fx_put2(w, 3 * nn, v);
     };
     add(0, 0, su * fma(dy1, dz1, s1));
     add(0, ez, su * fma(dy1, dz, -s1));
