@@ -48,9 +48,9 @@ BYTES_PER_CELL_UPDATE = {"fp32": 72, "fp64": 120}
 # profiles/push_plain_128x64x64_ncu.md (5.267 GB)
 NCU_TRAFFIC_PER_PARTICLE = {"fp32": 2.830e9 / 50331648, "fp64": 5.267e9 / 50331648}
 KERNELS_PER_STEP_NOTE = {
-    "fp32": "push (forms the B half step of its staged tile), insert, clamp, j_fold x3, b_half twice in one pass, "
-            "e_update, e_ghosts (both rounds in one launch); plus k_contribution_bound once per species after a load",
-    "fp64": "b_half, push, insert, clamp, j_fold x3, b_complete, e_update, e_ghosts"}
+    "fp32": "begin (clears J and the status), push (forms the B half step of its staged tile), insert, J fold with both "
+            "b_half steps, e_update, e_ghosts; plus k_contribution_bound once per species after a load",
+    "fp64": "b_half, begin, push, insert, J fold with b_complete, e_update, e_ghosts"}
 
 
 def peaks():

@@ -251,8 +251,9 @@ int pic_momentum(pic_handle *h, double *out);
  * with respect to the initial momenta of one species, and through
  * p0 = drift + vth * xi to that species' drift and thermal spread.
  * Particle order of the gradient = pic_get_particles order at the call to
- * pic_forward.  The buffers stay allocated until pic_adjoint_free, the next
- * pic_forward or pic_destroy.  Both forms are supported: the plain form
+ * pic_forward.  The buffers stay allocated until pic_adjoint_free or
+ * pic_destroy; the next pic_forward takes over those of about its own size and
+ * frees the others.  Both forms are supported: the plain form
  * differentiates in FP64, the mixed form in FP32 (particles) with FP64 field
  * adjoints. */
 typedef struct pic_loss {
