@@ -303,8 +303,9 @@ __device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WR
 // k_flat_push_plain; the FP32 contributions are summed in 64-bit fixed point
 // (quantum 2^-50 of the light-speed bound of the chunk, or 2^-51 of one
 // particle's) and added to the FP64 global J once.
-// Bound: instruction issue (1104 instructions per 32 particles, issue slots 70 %
-// busy).  128x32x32 cells, 12.6M particles: 0.916 -> 0.635 ms per step (before:
+// Bound: instruction issue (1059 instructions per 32 particles, issue slots 65 %
+// busy).  128x32x32 cells, 12.6M particles: 0.916 -> 0.635 ms per step, with the
+// window's strides at compile time and chained launches 0.587 (before:
 // taps gathered from and currents added to global memory; four CTAs per SM at
 // 64 registers: 0.688; lanes spread over 4 or 8 places: 0.625, 0.660, and slower
 // at 3M particles).
@@ -622,7 +623,8 @@ __device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j)
 // global arrays once.  A contribution fits an int32, so its add touches the high
 // word only when the low one carries or borrows.
 // Bound: instruction issue and the shared-memory pipe.  128x32x32 cells: 1.90 ->
-// 1.37 ms per reverse step (two CTAs per SM at 128 registers: 1.46; before: two
+// 1.37 ms per reverse step, with windows past the grid's ends 1.32 (two CTAs per
+// SM at 128 registers: 1.46; before: two
 // kernels that gathered from global memory).
 __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_constant__ MixParams P) {
     chain_enter();

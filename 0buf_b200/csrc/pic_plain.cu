@@ -361,7 +361,7 @@ struct BinP {
 // threads win: 71.1 ms against 72.7 (384: 75.0, 448: 76.0).
 //
 // Bound: dependent FP64 operations (4 warps per scheduler at 128 registers;
-// `wait` is the top stall, FP64 pipe 35 %, shared-memory pipe 55 %, DRAM 15 %).
+// `wait` is the top stall, FP64 pipe 47 %, shared-memory pipe 65 %, DRAM 24 %).
 // What shortened the chains, 256x64x64 cells, 201M particles: 17.1 ms; exact
 // cheaper quotients, truncations and roundings and fused multiply-adds
 // (pic_plain_math.cuh; 1648 -> 1367 instructions per 32 particles) 14.0 ms; the
