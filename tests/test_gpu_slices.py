@@ -63,10 +63,11 @@ def test_sliced_push_matches_oracle(pkg, oracle_mod, cells, ppc, empty, precisio
             assert sim.counters()[0] > 0
 
 
-# FP64 push with and without the shared-memory copy of the next particle: the
+# FP64 push with and without the shared-memory copy of the next particle and the
+# second tile current (8x8x8 has room for it, the others have not): the
 # copy is left out where it would cost a CTA per SM (8x6x8 cells) or does not
 # fit (16x9x8), kept otherwise (16x8x8, one CTA per SM)
-@pytest.mark.parametrize("tile", [(8, 6, 8), (16, 9, 8), (16, 8, 8)])
+@pytest.mark.parametrize("tile", [(8, 6, 8), (16, 9, 8), (16, 8, 8), (8, 8, 8)])
 def test_plain_push_tiles_of_every_staging(pkg, oracle_mod, tile):
     cells, ppc = (20, 13, 17), 6
     L = tuple(c * H for c in cells)
