@@ -258,6 +258,15 @@ __device__ __forceinline__ AdjWindow<WRAP> chunk_window(const Grid &g, const int
     __syncthreads();
     return *out;
 }
+// The block-wide maximum that the adjoint kernels take of every batch of 256
+// particles lies in one of three slots of shared memory: batch `it` collects into
+// max_slot(it), one barrier follows, every thread reads the slot, and thread 0
+// clears max_cleared(it), where batch it + 2 will collect.  Between two barriers
+// the threads then read slot it, clear slot it + 2 and collect into slot it + 1,
+// in any order: with two slots a late clear wiped out the next batch's maximum.
+constexpr int kMaxSlots = 3;
+__host__ __device__ __forceinline__ int max_slot(int it) { return it % kMaxSlots; }
+__host__ __device__ __forceinline__ int max_cleared(int it) { return (it + 2) % kMaxSlots; }
 // e with 2^(e-1) <= x < 2^e for a positive normal float, at least -120
 __device__ __forceinline__ int adj_exponent(float x) {
     const int e = x > 0.f ? (int)((__float_as_uint(x) >> 23) & 0xff) - 126 : -120;

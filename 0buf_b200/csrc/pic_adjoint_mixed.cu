@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow<true> sWin;
     __shared__ int sRed[15 * kW], sFar;
-    __shared__ unsigned sMax[2];
+    __shared__ unsigned sMax[kMaxSlots];
     __shared__ MixConst sK;
     const Grid &g = P.g;
     const AdjChunk ch = P.chunks[blockIdx.x];
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     stage_window_m<6>(g, w, nn, src, sF);
     stage_window_m<3>(g, w, nn, P.LJ, sL);
     for (int e = threadIdx.x; e < 12 * nn; e += blockDim.x) sLo[e] = 0u;
-    if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = 0u; sK = mix_const(g, S); }
+    if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = sMax[2] = 0u; sK = mix_const(g, S); }
     __syncthreads();
     const MixConst &K = sK;
     int E = -1000;  // contributions below 2^E = 2^30 quanta; none yet
@@ -706,10 +706,10 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
         }
         // the block's largest |lambda_F| against the quantum in use
         const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
-        if (lane == 0 && wm) atomicMax(&sMax[it & 1], wm);
+        if (lane == 0 && wm) atomicMax(&sMax[max_slot(it)], wm);
         __syncthreads();
-        const float bm = __uint_as_float(sMax[it & 1]);
-        if (threadIdx.x == 0) sMax[(it & 1) ^ 1] = 0u;
+        const float bm = __uint_as_float(sMax[max_slot(it)]);
+        if (threadIdx.x == 0) sMax[max_cleared(it)] = 0u;
         if (bm >= limit && bm > 0.f) {  // block-uniform
             flush(true);
             E = max(adj_exponent(bm), -90) + 2;
