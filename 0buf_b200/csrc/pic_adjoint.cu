@@ -875,10 +875,10 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
     __syncthreads();
     const ReverseConst &K = sK;
     // contributions below 2^50 quanta, at most kAdjChunk per node and component: sums below 2^61
-    int E = -1000;  // none yet
-    double limit = 0.0, inv_q = 0.0;
+    int E = kNoQuantum;
+    double inv_q = 0.0;
     auto flush = [&](bool again) {
-        if (E > -1000) {
+        if (E != kNoQuantum) {
             const double q = pow2_d(E - 50);
             double *const dst[6] = {A.LE[0], A.LE[1], A.LE[2], A.LH[0], A.LH[1], A.LH[2]};
             for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
@@ -919,33 +919,32 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
         PackedTaps T;
         double gx[3], lu[3], lF[6], gi[3] = {0.0, 0.0, 0.0};
         bool seen = false;
-        float amax = 0.f;
+        unsigned amax = 0u;  // high word of the largest |lambda_F|
         if (near) {
             FieldView<true> V;
 #pragma unroll
             for (int c = 0; c < 6; c++) V.base[c] = sF + c * nn;
             V.n0 = n0; V.dx = dX; V.dy = dY;
             seen = reverse_particle(g, K, V, sL, sL + nn, sL + 2 * nn, n0, dX, dY, c3, x, p, gn, lP, T, gx, lu, lF);
-            double am = 0.0;
+            if (seen) {
 #pragma unroll
-            for (int c = 0; c < 6; c++) am = fmax(am, fabs(lF[c]));
-            if (seen) amax = (float)am;
+                for (int c = 0; c < 6; c++) amax = max(amax, (unsigned)__double2hiint(lF[c]) & 0x7fffffffu);
+            }
         }
         // the block's largest |lambda_F| against the quantum in use
-        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+        const unsigned wm = __reduce_max_sync(0xffffffffu, amax);
         if (lane == 0 && wm) atomicMax(&sMax[max_slot(it)], wm);
         __syncthreads();
-        const float bm = __uint_as_float(sMax[max_slot(it)]);
+        const unsigned bm = sMax[max_slot(it)];
         if (threadIdx.x == 0) sMax[max_cleared(it)] = 0u;
-        if ((double)bm >= limit && bm > 0.f) {  // block-uniform
+        const int En = bm ? quantum_for(E, exponent_hi(bm), kLeastPlain) : E;
+        if (En != E) {  // block-uniform
             flush(true);
-            E = adj_exponent(bm) + 2;
-            // a float rounded down from a larger double stays below 2^E
-            limit = pow2_d(E - 1);
+            E = En;
             inv_q = pow2_d(50 - E);
             __syncthreads();
         }
-        if (near && seen && amax > 0.f) {
+        if (near && amax) {
             auto put = [&](int c) {
                 const double lam = lF[c] * inv_q;
                 unsigned *lo = sLo + c * nn + n0;

@@ -267,11 +267,21 @@ __device__ __forceinline__ AdjWindow<WRAP> chunk_window(const Grid &g, const int
 constexpr int kMaxSlots = 3;
 __host__ __device__ __forceinline__ int max_slot(int it) { return it % kMaxSlots; }
 __host__ __device__ __forceinline__ int max_cleared(int it) { return (it + 2) % kMaxSlots; }
-// e with 2^(e-1) <= x < 2^e for a positive normal float, at least -120
-__device__ __forceinline__ int adj_exponent(float x) {
-    const int e = x > 0.f ? (int)((__float_as_uint(x) >> 23) & 0xff) - 126 : -120;
-    return max(e, -120);
+// The quantum of the sums in a window: contributions up to 2^E, E from the largest
+// |lambda of a field value| of the batch at hand (its bits, which order as the
+// values do), two powers of two above it at first.
+constexpr int kNoQuantum = -2000;  // none yet
+// e with 2^(e-1) <= x < 2^e, from the high word of a non-negative normal double
+__host__ __device__ __forceinline__ int exponent_hi(unsigned hi) { return (int)(hi >> 20) - 1022; }
+// the same from the bits of a non-negative normal float
+__host__ __device__ __forceinline__ int exponent_f(unsigned bits) { return (int)(bits >> 23) - 126; }
+// E for a batch of exponent e when E0 is in use, at least `least`; E0 if that does
+__host__ __device__ __forceinline__ int quantum_for(int E0, int e, int least) {
+    if (e < least - 2) e = least - 2;
+    return e > E0 ? e + 2 : E0;
 }
+// least E: 2^(E - 50) and its inverse are normal doubles, 2^(30 - E) a normal float
+constexpr int kLeastPlain = -900, kLeastMix = -93;
 
 // 2^e as a double from its exponent bits (|e| < 1000)
 __device__ __forceinline__ double pow2_d(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }

@@ -654,10 +654,10 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     if (threadIdx.x == 0) { sFar = 0; sMax[0] = sMax[1] = sMax[2] = 0u; sK = mix_const(g, S); }
     __syncthreads();
     const MixConst &K = sK;
-    int E = -1000;  // contributions below 2^E = 2^30 quanta; none yet
-    float limit = 0.f, inv_q = 0.f;
+    int E = kNoQuantum;  // contributions below 2^E = 2^30 quanta
+    float inv_q = 0.f;
     auto flush = [&](bool again) {
-        if (E == -1000) return;
+        if (E == kNoQuantum) return;
         const double q = pow2_d(E - 30);
         double *const dst[6] = {P.LE[0], P.LE[1], P.LE[2], P.LH[0], P.LH[1], P.LH[2]};
         for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
@@ -708,12 +708,12 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
         const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
         if (lane == 0 && wm) atomicMax(&sMax[max_slot(it)], wm);
         __syncthreads();
-        const float bm = __uint_as_float(sMax[max_slot(it)]);
+        const unsigned bm = sMax[max_slot(it)];
         if (threadIdx.x == 0) sMax[max_cleared(it)] = 0u;
-        if (bm >= limit && bm > 0.f) {  // block-uniform
+        const int En = bm ? quantum_for(E, exponent_f(bm), kLeastMix) : E;
+        if (En != E) {  // block-uniform
             flush(true);
-            E = max(adj_exponent(bm), -90) + 2;
-            limit = __uint_as_float((unsigned)(E + 127) << 23);
+            E = En;
             inv_q = __uint_as_float((unsigned)(30 - E + 127) << 23);
             __syncthreads();
         }
