@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
     double inv_q = 0.0;
     auto flush = [&](bool again) {
         if (E != kNoQuantum) {
-            const double q = pow2_d(E - 50);
+            const double q = pow2_d(E - kBitsPlain);
             double *const dst[6] = {A.LE[0], A.LE[1], A.LE[2], A.LH[0], A.LH[1], A.LH[2]};
             for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
                 const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
@@ -937,11 +937,11 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
         __syncthreads();
         const unsigned bm = sMax[max_slot(it)];
         if (threadIdx.x == 0) sMax[max_cleared(it)] = 0u;
-        const int En = bm ? quantum_for(E, exponent_hi(bm), kLeastPlain) : E;
+        const int En = bm ? quantum_for(E, exponent_hi(bm), kKeepPlain, kLeastPlain) : E;
         if (En != E) {  // block-uniform
             flush(true);
             E = En;
-            inv_q = pow2_d(50 - E);
+            inv_q = pow2_d(kBitsPlain - E);
             __syncthreads();
         }
         if (near && amax) {

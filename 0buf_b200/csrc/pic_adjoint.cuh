@@ -269,18 +269,26 @@ __host__ __device__ __forceinline__ int max_slot(int it) { return it % kMaxSlots
 __host__ __device__ __forceinline__ int max_cleared(int it) { return (it + 2) % kMaxSlots; }
 // The quantum of the sums in a window: contributions up to 2^E, E from the largest
 // |lambda of a field value| of the batch at hand (its bits, which order as the
-// values do), two powers of two above it at first.
+// values do), two powers of two above it at first.  Where a batch's largest is
+// past 2^E, or more than `keep` powers of two below it, the sums so far go to the
+// global arrays and the window starts again at the batch's own quantum: a chunk's
+// particles are not rounded in the units of a strongly amplified one among them.
+// keep: no contribution is rounded more coarsely than by 2^-45 (FP64) or 2^-23
+// (FP32) of its batch's largest.
 constexpr int kNoQuantum = -2000;  // none yet
 // e with 2^(e-1) <= x < 2^e, from the high word of a non-negative normal double
 __host__ __device__ __forceinline__ int exponent_hi(unsigned hi) { return (int)(hi >> 20) - 1022; }
 // the same from the bits of a non-negative normal float
 __host__ __device__ __forceinline__ int exponent_f(unsigned bits) { return (int)(bits >> 23) - 126; }
 // E for a batch of exponent e when E0 is in use, at least `least`; E0 if that does
-__host__ __device__ __forceinline__ int quantum_for(int E0, int e, int least) {
-    if (e < least - 2) e = least - 2;
-    return e > E0 ? e + 2 : E0;
+__host__ __device__ __forceinline__ int quantum_for(int E0, int e, int keep, int least) {
+    const int own = e + 2 < least ? least : e + 2;
+    return e > E0 || (e + keep < E0 && own < E0) ? own : E0;
 }
-// least E: 2^(E - 50) and its inverse are normal doubles, 2^(30 - E) a normal float
+// quanta below 2^E, as powers of two; least E: 2^(E - 50) and its inverse are
+// normal doubles, 2^(30 - E) a normal float
+constexpr int kBitsPlain = 50, kBitsMix = 30;
+constexpr int kKeepPlain = kBitsPlain - 44, kKeepMix = kBitsMix - 22;
 constexpr int kLeastPlain = -900, kLeastMix = -93;
 
 // 2^e as a double from its exponent bits (|e| < 1000)

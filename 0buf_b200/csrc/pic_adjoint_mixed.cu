@@ -619,8 +619,8 @@ __device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j)
 // ---- adjoint of the particle part of one step (k_adj_particles_plain in FP32):
 // one CTA per chunk with its window of E, H and lambda_J staged; lambda_E and
 // lambda_H are summed there in 64-bit words in units of 2^-30 of the largest
-// |lambda of a field value| (at most 4 times the block's) and added to the FP64
-// global arrays once.  A contribution fits an int32, so its add touches the high
+// |lambda of a field value| of a batch of 256 particles (quantum_for) and added
+// to the FP64 global arrays at the end.  A contribution fits an int32, so its add touches the high
 // word only when the low one carries or borrows.
 // Bound: instruction issue and the shared-memory pipe.  128x32x32 cells: 1.90 ->
 // 1.37 ms per reverse step, with windows past the grid's ends 1.32 (two CTAs per
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
     float inv_q = 0.f;
     auto flush = [&](bool again) {
         if (E == kNoQuantum) return;
-        const double q = pow2_d(E - 30);
+        const double q = pow2_d(E - kBitsMix);
         double *const dst[6] = {P.LE[0], P.LE[1], P.LE[2], P.LH[0], P.LH[1], P.LH[2]};
         for (int e = threadIdx.x; e < 6 * nn; e += blockDim.x) {
             const long long v = (long long)(((unsigned long long)sHi[e] << 32) | sLo[e]);
@@ -710,11 +710,11 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
         __syncthreads();
         const unsigned bm = sMax[max_slot(it)];
         if (threadIdx.x == 0) sMax[max_cleared(it)] = 0u;
-        const int En = bm ? quantum_for(E, exponent_f(bm), kLeastMix) : E;
+        const int En = bm ? quantum_for(E, exponent_f(bm), kKeepMix, kLeastMix) : E;
         if (En != E) {  // block-uniform
             flush(true);
             E = En;
-            inv_q = __uint_as_float((unsigned)(30 - E + 127) << 23);
+            inv_q = __uint_as_float((unsigned)(kBitsMix - E + 127) << 23);
             __syncthreads();
         }
         if (near && amax > 0.f) {

@@ -6,4 +6,11 @@ extern "C" {
 int dm_max_slots() { return pic::kMaxSlots; }
 int dm_max_slot(int it) { return pic::max_slot(it); }
 int dm_max_cleared(int it) { return pic::max_cleared(it); }
+int dm_no_quantum() { return pic::kNoQuantum; }
+int dm_quantum_plain(int E, unsigned hi) {
+    return pic::quantum_for(E, pic::exponent_hi(hi), pic::kKeepPlain, pic::kLeastPlain);
+}
+int dm_quantum_mixed(int E, unsigned bits) {
+    return pic::quantum_for(E, pic::exponent_f(bits), pic::kKeepMix, pic::kLeastMix);
+}
 }

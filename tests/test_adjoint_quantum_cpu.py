@@ -1,8 +1,9 @@
 """The block-wide maximum of the adjoint kernels, whose slots are shared by
-batches that only one barrier separates: the code of the kernels' header, run on
-the host."""
+batches that only one barrier separates, and the quantum that follows it: the code
+of the kernels' header, run on the host."""
 import itertools
 
+import numpy as np
 import pytest
 
 from device_math_build import load
@@ -43,3 +44,23 @@ def test_two_slots_lose_a_maximum():
     thread 0, while another warp already collects the next batch there"""
     got = maxima(2, lambda it: it & 1, lambda it: (it & 1) ^ 1, ("read", "collect", "clear"), VALUES)
     assert got != VALUES
+
+
+@pytest.mark.parametrize("form,bits,coarsest,least", [("plain", 50, 44, -900), ("mixed", 30, 22, -93)])
+def test_quantum_holds_a_batch_and_rounds_it_no_coarser(dm, form, bits, coarsest, least):
+    """Over batches whose largest value jumps by any power of two: every contribution
+    is below 2^bits quanta, and the quantum is at most 2^-coarsest of the power of two
+    above the batch's largest (except below the least quantum)."""
+    rng = np.random.default_rng(3)
+    plain = form == "plain"
+    quantum = dm.dm_quantum_plain if plain else dm.dm_quantum_mixed
+    lo, hi = (-1000, 1000) if plain else (-126, 126)
+    E = dm.dm_no_quantum()
+    for e in np.concatenate([rng.integers(lo, hi, 2000), np.cumsum(rng.integers(-4, 5, 2000)).clip(lo, hi), [hi, lo, hi]]):
+        v = rng.uniform(1.0, 2.0) * 2.0 ** float(e)
+        word = int(np.float64(v).view(np.uint64) >> np.uint64(32)) if plain else int(np.float32(v).view(np.uint32))
+        E = quantum(E, word)
+        top = int(e) + 1  # v < 2^top
+        assert top <= E and E >= least
+        assert E - bits <= top - coarsest or E == least
+        assert quantum(E, word) == E
