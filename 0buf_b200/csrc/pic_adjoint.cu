@@ -832,7 +832,8 @@ __device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
 // particle and step).  The quantum follows the largest |lambda of a field
 // value| of the 256 particles at hand: where that outgrows the quantum in use,
 // the sums so far are added to the global arrays and start again at one that
-// leaves 2^-48 of it.
+// leaves 2^-48 of it.  A particle whose adjoints are not finite goes the same way
+// as those outside: the FP64 sums in global memory then show it.
 // Bound: latency at 16 warps per SM (128 registers, some spills) and the shared
 // memory pipe (64 %: 91 shared atomics and 110 loads per particle).  128x32x32
 // cells: 3.3 -> 2.3 ms per reverse step (before: two kernels, lambda of the
@@ -929,6 +930,11 @@ __global__ void __launch_bounds__(kT, 2) k_adj_particles_plain(const __grid_cons
             if (seen) {
 #pragma unroll
                 for (int c = 0; c < 6; c++) amax = max(amax, (unsigned)__double2hiint(lF[c]) & 0x7fffffffu);
+                if (amax >= 0x7ff00000u) {  // no fixed point for an infinity or a NaN
+                    near = false;
+                    amax = 0u;
+                    sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
+                }
             }
         }
         // the block's largest |lambda_F| against the quantum in use

@@ -694,7 +694,8 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
                 sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
             }
         }
-        float gx[3], lu[3], lF[6], gi[3] = {0.f, 0.f, 0.f}, amax = 0.f;
+        float gx[3], lu[3], lF[6], gi[3] = {0.f, 0.f, 0.f};
+        unsigned amax = 0u;  // bits of the largest |lambda_F|
         if (near) {
             FieldViewM<true> V;
 #pragma unroll
@@ -702,10 +703,15 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
             V.dx = dX; V.dy = dY;
             reverse_particle_m(K, V, sL + n0, sL + nn + n0, sL + 2 * nn + n0, dX, dY, xs, p, gn, lP, gx, lu, lF);
 #pragma unroll
-            for (int c = 0; c < 6; c++) amax = fmaxf(amax, fabsf(lF[c]));
+            for (int c = 0; c < 6; c++) amax = max(amax, __float_as_uint(lF[c]) & 0x7fffffffu);
+            if (amax >= 0x7f800000u) {  // no fixed point for an infinity or a NaN
+                near = false;
+                amax = 0u;
+                sList[atomicAdd(&sFar, 1)] = (unsigned short)jc;
+            }
         }
         // the block's largest |lambda_F| against the quantum in use
-        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+        const unsigned wm = __reduce_max_sync(0xffffffffu, amax);
         if (lane == 0 && wm) atomicMax(&sMax[max_slot(it)], wm);
         __syncthreads();
         const unsigned bm = sMax[max_slot(it)];
@@ -717,7 +723,7 @@ __global__ void __launch_bounds__(kT, 3) k_adj_particles_mixed(const __grid_cons
             inv_q = __uint_as_float((unsigned)(kBitsMix - E + 127) << 23);
             __syncthreads();
         }
-        if (near && amax > 0.f) {
+        if (near && amax) {
             auto put = [&](int c) {
                 unsigned *lo = sLo + c * nn + n0;
                 return [=](int a, int b, int k, float v, float wz, float vz) {

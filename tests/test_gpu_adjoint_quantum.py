@@ -80,3 +80,20 @@ def test_large_adjoints_beside_small_ones(pkg, precision, tx, first):
     assert away.sum() > 100 and np.abs(alone[near]).max() > 1e5 * np.abs(alone[away]).max() > 0
     err = np.linalg.norm(rows[away] - alone[away]) / np.linalg.norm(alone[away])
     assert err < (1e-10 if precision == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("precision,tx,top", [("fp64", 8, 1024), ("fp32", 6, 128)])
+def test_adjoints_that_overflow_do_not_come_out_finite(pkg, precision, tx, top):
+    """Scaled so that products of the large adjoints with the fields (2^-3k) overflow
+    and the others' do not: a particle's gradient is either not finite or the
+    unscaled run's, scaled (1e-9 and 1e-4 of the largest)."""
+    spike = (tx, 4, 8)
+    base, x = spiked(pkg, precision, spike)
+    k = -int(np.ceil((top + 10 - np.log2(np.abs(base).max())) / 3))
+    with np.errstate(all="ignore"):
+        got, y = spiked(pkg, precision, spike, k=k)
+        assert np.array_equal(x, y)
+        ok = np.isfinite(got).all(1)
+        assert 0.9 < ok.mean() < 1.0
+        err = np.abs(got[ok] * 2.0 ** (2 * k) - base[ok]).max()
+    assert err < (1e-9 if precision == "fp64" else 1e-4) * np.abs(base).max()
