@@ -177,12 +177,19 @@ __global__ void k_rho_fold(Grid g, double *rho, int dir) {
 // copy; reductions into red[0] max |G - G0|, red[1] max |rho|, red[2] sum (G - G0)^2,
 // red[3] max |G0| (non-negative doubles compared through their bit patterns)
 // (a block walks over many nodes and reduces once: one atomic per warp on the
-// same four addresses took 1.65 ms of a 512x128x128 call, this takes 0.27)
+// same four addresses took 1.65 ms of a 512x128x128 call, this takes 0.27).  The
+// maxima are taken of the bit patterns: a NaN is above every number and stays.
+__device__ __forceinline__ unsigned long long max_bits(unsigned long long m, unsigned long long v) { return v > m ? v : m; }
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
 template <typename T>
 __global__ void k_gauss(Grid g, const T *__restrict__ Ex, const T *__restrict__ Ey, const T *__restrict__ Ez,
                         const double *__restrict__ rho, double *G, double *G0, int set_baseline, double *red) {
-    __shared__ double part[4][8];
-    double dmax = 0.0, rmax = 0.0, d2 = 0.0, g0max = 0.0;
+    __shared__ unsigned long long part[3][8];
+    __shared__ double part2[8];
+    unsigned long long m[3] = {0ull, 0ull, 0ull};  // |G - G0|, |rho|, |G0|
+    double d2 = 0.0;
     const size_t sx = (size_t)g.NY * g.pz, sy = g.pz;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rows = g.NX * g.NY, stride = gridDim.x * (blockDim.x >> 5);
@@ -195,30 +202,36 @@ __global__ void k_gauss(Grid g, const T *__restrict__ Ex, const T *__restrict__ 
             if (inner && k >= 1 && k <= g.nz) {
                 v = ((double)Ex[n] - (double)Ex[n - sx]) / g.hx + ((double)Ey[n] - (double)Ey[n - sy]) / g.hy +
                     ((double)Ez[n] - (double)Ez[n - 1]) / g.hz - rho[n];
-                rmax = fmax(rmax, fabs(rho[n]));
+                m[1] = max_bits(m[1], abs_bits(rho[n]));
             }
             if (G) G[n] = v;
             if (set_baseline) G0[n] = v;
             const double base = set_baseline ? v : G0[n];
-            dmax = fmax(dmax, fabs(v - base));
+            m[0] = max_bits(m[0], abs_bits(v - base));
             d2 += (v - base) * (v - base);
-            g0max = fmax(g0max, fabs(base));
+            m[2] = max_bits(m[2], abs_bits(base));
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
-        dmax = fmax(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
-        rmax = fmax(rmax, __shfl_down_sync(0xffffffffu, rmax, o));
+#pragma unroll
+        for (int q = 0; q < 3; q++) m[q] = max_bits(m[q], __shfl_down_sync(0xffffffffu, m[q], o));
         d2 += __shfl_down_sync(0xffffffffu, d2, o);
-        g0max = fmax(g0max, __shfl_down_sync(0xffffffffu, g0max, o));
     }
-    if (lane == 0) { part[0][warp] = dmax; part[1][warp] = rmax; part[2][warp] = d2; part[3][warp] = g0max; }
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) part[q][warp] = m[q];
+        part2[warp] = d2;
+    }
     __syncthreads();
-    if (threadIdx.x < 4) {
+    const int nw = blockDim.x >> 5;
+    if (threadIdx.x < 3) {
+        unsigned long long v = 0ull;
+        for (int w = 0; w < nw; w++) v = max_bits(v, part[threadIdx.x][w]);
+        atomicMax((unsigned long long *)&red[threadIdx.x == 2 ? 3 : threadIdx.x], v);
+    } else if (threadIdx.x == 3) {
         double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-            v = threadIdx.x == 2 ? v + part[2][w] : fmax(v, part[threadIdx.x][w]);
-        if (threadIdx.x == 2) atomicAdd(&red[2], v);
-        else atomicMax((unsigned long long *)&red[threadIdx.x], (unsigned long long)__double_as_longlong(v));
+        for (int w = 0; w < nw; w++) v += part2[w];
+        atomicAdd(&red[2], v);
     }
 }
 
