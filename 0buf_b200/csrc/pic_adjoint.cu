@@ -1787,22 +1787,16 @@ int pic_perturb_momenta(pic_handle *h, int species, int64_t n, const double *dp,
     d0[g.ntiles] = acc;
     if (acc != n) return set_err(h, PIC_ERR_ARG, "pic_perturb_momenta: n is not the species' particle count");
     if (n == 0) return PIC_OK;
+    ScratchGuard guard(h);
     int64_t *dd = nullptr;
     double *dv = nullptr;
-    CK(cudaMalloc(&dd, (g.ntiles + 1) * sizeof(int64_t)), "alloc");
-    cudaError_t e = cudaMalloc(&dv, (size_t)n * 3 * sizeof(double));
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dd, d0.data(), (g.ntiles + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dv, dp, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) {
-        k_perturb_momenta<<<g.ntiles, 256, 0, h->stream>>>(h->sp[species].v, h->mixed, dd, dv, eps);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dd);
-    if (dv) cudaFree(dv);
-    CK(e, "perturb momenta");
+    CK(guard.alloc(&dd, g.ntiles + 1), "alloc");
+    CK(guard.alloc(&dv, (size_t)n * 3), "alloc");
+    CK(cudaMemcpyAsync(dd, d0.data(), (g.ntiles + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream), "H2D");
+    CK(cudaMemcpyAsync(dv, dp, (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->stream), "H2D");
+    k_perturb_momenta<<<g.ntiles, 256, 0, h->stream>>>(h->sp[species].v, h->mixed, dd, dv, eps);
+    CK(cudaGetLastError(), "perturb momenta");
+    CK(cudaStreamSynchronize(h->stream), "perturb momenta");
     h->kin_valid = 0;
     return PIC_OK;
 }

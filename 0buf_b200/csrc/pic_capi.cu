@@ -49,12 +49,11 @@ static void release_spare(pic_handle *h) {
 cudaError_t dev_alloc(pic_handle *h, void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes > 0 ? bytes : 16);
     if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
         const bool spare = h->spare != nullptr;
         release_spare(h);
-        if (adj_reclaim(h) || spare) {
-            cudaGetLastError();
-            e = cudaMalloc(p, bytes > 0 ? bytes : 16);
-        }
+        if (adj_reclaim(h) || spare) e = cudaMalloc(p, bytes > 0 ? bytes : 16);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // not the next launch's error
     }
     return e;
 }
@@ -1046,8 +1045,9 @@ int pic_init_species_profile(pic_handle *h, int species, const pic_profile *prof
                 first[c] = start[t] + fill[t];
                 fill[t] += cnt[c];
             }
+    ScratchGuard guard(h);
     int *d = nullptr;
-    CK(cudaMalloc(&d, 2 * (size_t)nc * sizeof(int)), "alloc counts");
+    CK(guard.alloc(&d, 2 * (size_t)nc), "alloc counts");
     cudaError_t e = cudaMemcpyAsync(d, cnt.data(), (size_t)nc * sizeof(int), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d + nc, first.data(), (size_t)nc * sizeof(int), cudaMemcpyHostToDevice, h->stream);
@@ -1058,7 +1058,6 @@ int pic_init_species_profile(pic_handle *h, int species, const pic_profile *prof
         e = init_cells(g, h->mixed, h->sp[species].v, species, d, d + nc, drift_x, drift_y, drift_z, vth, seed,
                        h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d);
     CK(e, "init species (profile)");
     h->kin_valid = 0;
     return ensure_outbox(h);
@@ -1318,9 +1317,10 @@ int pic_get_particles(pic_handle *h, int species, int64_t cap, double *x, double
     int *dcell = nullptr;
     int64_t *dd = nullptr;
     size_t N = (size_t)acc;
-    CK(cudaMalloc(&buf, N * 6 * sizeof(double)), "alloc");
-    CK(cudaMalloc(&dcell, N * sizeof(int)), "alloc");
-    CK(cudaMalloc(&dd, (g.ntiles + 1) * sizeof(int64_t)), "alloc");
+    ScratchGuard guard(h);
+    CK(guard.alloc(&buf, N * 6), "alloc");
+    CK(guard.alloc(&dcell, N), "alloc");
+    CK(guard.alloc(&dd, g.ntiles + 1), "alloc");
     CK(cudaMemcpyAsync(dd, dstart.data(), (g.ntiles + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream), "H2D");
     CK(gather_from_bins(g, h->mixed, v, dd, buf, buf + N, buf + 2 * N, buf + 3 * N, buf + 4 * N, buf + 5 * N, dcell,
                         h->stream), "gather");
@@ -1330,9 +1330,6 @@ int pic_get_particles(pic_handle *h, int species, int64_t cap, double *x, double
     std::vector<int> hc(N);
     CK(cudaMemcpyAsync(hc.data(), dcell, N * sizeof(int), cudaMemcpyDeviceToHost, h->stream), "D2H");
     CK(cudaStreamSynchronize(h->stream), "sync");
-    cudaFree(buf);
-    cudaFree(dcell);
-    cudaFree(dd);
     if (cell) {
         for (size_t j = 0; j < N; j++) {
             int c = hc[j];

@@ -326,11 +326,17 @@ using namespace pic_host;
 namespace {
 int ensure_diag(pic_handle *h) {
     const size_t bytes = h->g.nodes_pitched() * sizeof(double);
-    if (!h->rho) {
-        CK(cudaMalloc(&h->rho, bytes), "alloc rho");
-        CK(cudaMalloc(&h->gauss, bytes), "alloc residual");
-        CK(cudaMalloc(&h->gauss0, bytes), "alloc residual baseline");
-        CK(cudaMemsetAsync(h->gauss0, 0, bytes, h->stream), "memset");
+    if (!h->rho) {  // all three or none
+        double *d[3] = {nullptr, nullptr, nullptr};
+        cudaError_t e = cudaSuccess;
+        for (int a = 0; a < 3 && e == cudaSuccess; a++) e = dev_alloc(h, (void **)&d[a], bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(d[2], 0, bytes, h->stream);
+        if (e != cudaSuccess) {
+            for (double *p : d)
+                if (p) dev_free(h, p);
+            return cuda_err(h, e, "alloc the charge diagnostic");
+        }
+        h->rho = d[0]; h->gauss = d[1]; h->gauss0 = d[2];
         h->gauss_has_base = 0;
     }
     return PIC_OK;
