@@ -1838,7 +1838,7 @@ int pic_backward(pic_handle *h, const pic_loss *loss, pic_grads *grads) {
     const size_t N = g.nodes_pitched();
     const size_t fbytes = N * (h->mixed ? sizeof(float) : sizeof(double));
     int64_t np = total_particles(A);
-    if (!A.segp) {
+    if (!A.rf) {  // the last of them: after a failure the next call gets the rest
         if ((rc = adj_alloc(h, kAdjSegp, (void **)&A.segp, A.pbytes * (size_t)(A.K2 + 1), "the segment states"))) return rc;
         if ((rc = adj_alloc(h, kAdjSegf, (void **)&A.segf, fbytes * 6 * (size_t)A.K2, "the segment fields"))) return rc;
         if (A.K2 < A.K) {

@@ -65,3 +65,25 @@ def test_kept_adjoint_buffers_are_given_back(pkg, name):
         with device_filled(MB):
             got = call(sim, name)
     assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)  # FP64 sums in any order
+
+
+def test_backward_after_one_that_found_no_memory(pkg):
+    """The first pic_backward gets the segment states and not the particle adjoints;
+    the next, with memory, gives the gradient of a fresh handle (1e-9, the order of
+    FP64 sums)."""
+    loss = dict(field="Ex", window=2, species=0)
+
+    def run(fill):
+        with make(pkg) as sim:
+            order = np.lexsort([sim.particles(0)[k] for k in ("px", "y", "x")])
+            sim.forward(4, 4)
+            if fill:
+                n = sim.num_particles(0)
+                with device_filled(5 * 52 * n + 64 * MB + 24 * n):  # states and fields, half of the adjoints
+                    with pytest.raises(pkg.PicError, match="particle adjoints|field"):
+                        sim.backward(**loss)
+            return sim.backward(**loss)["d_p0"][order]
+
+    want, got = run(False), run(True)
+    assert np.linalg.norm(want) > 0
+    assert np.linalg.norm(got - want) < 1e-9 * np.linalg.norm(want)
