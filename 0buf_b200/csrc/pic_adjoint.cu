@@ -1336,7 +1336,7 @@ int check_adj_status(pic_handle *h, AdjState &A, const char *where) {
 int adj_alloc(pic_handle *h, AdjSlot slot, void **p, size_t bytes, const char *what) {
     AdjState::Buf &b = h->adj->pool[slot];
     if (bytes == 0) bytes = 256;
-    if (b.p && (b.cap < bytes || b.cap > 2 * bytes + (1 << 20))) {
+    if (b.p && !kept_serves(b.cap, bytes)) {
         cudaFree(b.p);
         b.p = nullptr;
     }

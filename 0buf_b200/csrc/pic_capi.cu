@@ -151,10 +151,10 @@ int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> 
 
 // A species' arrays for `slots` slots, carved from one allocation (a driver
 // call per array costs a rebin of a small run more than its copies).  *arena of
-// `have` bytes is used again when it is large enough and at most twice what is
-// needed (a program that loads its species anew for every run then allocates
-// nothing), and is freed otherwise.
-cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **arena, size_t *have) {
+// `have` bytes is used again when it is large enough and not much too large
+// (kept_serves; a rebin's spare, whose successor grows again: up to twice what is
+// needed, with kKeepSlack), and is freed otherwise.
+cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **arena, size_t *have, bool spare = false) {
     const size_t n = (size_t)slots, el = h->mixed ? sizeof(float) : sizeof(double);
     size_t o = 0;
     auto room = [&](size_t bytes) { size_t a = o; o += (bytes + 255) / 256 * 256; return a; };
@@ -163,7 +163,8 @@ cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **a
     for (size_t &a : val) a = room(n * el);
     const size_t st = room(((size_t)h->g.ntiles + 1) * sizeof(int)), ct = room((size_t)h->g.ntiles * sizeof(int));
     const size_t sp = room(n / (kHoleSpill / 2) * sizeof(int));
-    if (*arena && (*have < o || *have > 2 * o + (1 << 20))) {
+    const bool twice = spare && *have >= o && *have - o <= std::min(o, kKeepSlack) + ((size_t)1 << 20);
+    if (*arena && !twice && !kept_serves(*have, o)) {
         dev_free(h, *arena);
         *arena = nullptr;
     }
@@ -360,7 +361,7 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     h->spare = nullptr;
     h->spare_bytes = 0;
     cudaError_t e = cudaErrorMemoryAllocation;
-    if (!layout_bins(h, counts, start, &sp.h_start)) e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
+    if (!layout_bins(h, counts, start, &sp.h_start)) e = carve_species(h, start[g.ntiles], v, &arena, &bytes, true);
     if (e == cudaErrorMemoryAllocation) {  // no room for kept capacities
         cudaGetLastError();
         const int rc = layout_bins(h, counts, start);
@@ -368,7 +369,7 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
             if (arena) dev_free(h, arena);
             return rc;
         }
-        e = carve_species(h, start[g.ntiles], v, &arena, &bytes);
+        e = carve_species(h, start[g.ntiles], v, &arena, &bytes, true);
     }
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 #include <vector>
 #include "pic0buf.h"
 #include "pic_internal.cuh"
@@ -29,7 +30,7 @@ struct pic_handle {
         int loaded;
         std::vector<int> h_start;
         // FP32 form: the bound of its contributions is known from a push
-        // (cleared whenever the bins are rebuilt)
+        // (cleared when the species is loaded; a rebin keeps the particles)
         int lb_known;
     } sp[pic::kMaxSpecies];
     void *outbox;
@@ -96,6 +97,14 @@ int need_particles(pic_handle *h);
 // c2 species' bins, against 0.16 s for the whole load with cudaMalloc)
 cudaError_t dev_alloc(pic_handle *h, void **p, size_t bytes);
 void dev_free(pic_handle *h, void *p);
+// whether a kept buffer of `have` bytes serves for `need`: what it holds too much
+// can't be taken back while it is in use, so that is kept below 65 MB (1 MB in a
+// small run).  A program that repeats a run with other random numbers, whose bins
+// differ by per cents, still allocates nothing.
+constexpr size_t kKeepSlack = (size_t)64 << 20;
+inline bool kept_serves(size_t have, size_t need) {
+    return have >= need && have - need <= std::min(need / 16, kKeepSlack) + ((size_t)1 << 20);
+}
 template <class T>
 cudaError_t dev_alloc_n(pic_handle *h, T **p, size_t n) {
     return dev_alloc(h, (void **)p, n * sizeof(T));

@@ -87,3 +87,29 @@ def test_backward_after_one_that_found_no_memory(pkg):
     want, got = run(False), run(True)
     assert np.linalg.norm(want) > 0
     assert np.linalg.norm(got - want) < 1e-9 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("kind", ["species", "adjoint"])
+def test_a_smaller_run_holds_no_more_than_a_fresh_one(pkg, kind):
+    """After a run 1.8 times as large: at most 65 MB more per kept buffer of hundreds of
+    MB (one species' arrays; the adjoint's state, checkpoints, segment states and
+    adjoints), where up to twice the need was held."""
+    import torch
+
+    def used(first):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        with make(pkg, 20 if kind == "species" else PPC) as sim:
+            if kind == "species":
+                if first:
+                    sim.init_species(0, 36, vth=0.05, seed=5)
+                sim.init_species(0, 20, vth=0.05, seed=5)
+            else:
+                if first:
+                    sim.forward(9, 1)
+                sim.forward(5, 1)
+            return before - torch.cuda.mem_get_info()[0]
+
+    used(True)  # what the process keeps anyway
+    fresh, after = used(False), used(True)
+    assert after - fresh <= (1 if kind == "species" else 4) * 65 * MB + 4 * MB
