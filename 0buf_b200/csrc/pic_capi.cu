@@ -122,8 +122,10 @@ void free_species(pic_handle *h, int s, bool give_back) {
 //     what its count asks for (particles that slosh between tiles).
 // 256x64x64 cells, stress configuration: 15 -> 9 rebuilds in 240 steps.
 constexpr double kKeepCapacity = 1.5;
-int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> &start,
-                const std::vector<int> *old = nullptr) {
+// Null, or why there can be no such bins (the caller's to report: it may do without
+// old).
+const char *layout_bins(const pic_handle *h, const std::vector<int> &counts, std::vector<int> &start,
+                        const std::vector<int> *old = nullptr) {
     const Grid &g = h->g;
     double slack = h->cfg.capacity_slack > 0 ? h->cfg.capacity_slack : 0.25;
     start.resize(g.ntiles + 1);
@@ -141,12 +143,12 @@ int layout_bins(pic_handle *h, const std::vector<int> &counts, std::vector<int> 
         // the plain form's two-word tile J stays exact up to kFxMaxTileSlots
         // particles in a tile over all species
         if (!h->mixed && cap > kFxMaxTileSlots / h->cfg.nspecies)
-            return set_err(h, PIC_ERR_ARG, "too many particles in one tile for the FP64 tile current");
+            return "too many particles in one tile for the FP64 tile current";
         acc += cap;
-        if (acc > 0x7fffff00LL) return set_err(h, PIC_ERR_ARG, "species capacity exceeds 2^31 slots");
+        if (acc > 0x7fffff00LL) return "species capacity exceeds 2^31 slots";
     }
     start[g.ntiles] = (int)acc;
-    return PIC_OK;
+    return nullptr;
 }
 
 // A species' arrays for `slots` slots, carved from one allocation (a driver
@@ -192,8 +194,7 @@ cudaError_t carve_species(pic_handle *h, int64_t slots, SpeciesView &v, void **a
 int alloc_species(pic_handle *h, int s, const std::vector<int> &counts) {
     const Grid &g = h->g;
     std::vector<int> start;
-    int rc = layout_bins(h, counts, start);
-    if (rc) return rc;
+    if (const char *why = layout_bins(h, counts, start)) return set_err(h, PIC_ERR_ARG, why);
     free_species(h, s, false);
     SpeciesView &v = h->sp[s].v;
     const int64_t acc = start[g.ntiles];
@@ -364,10 +365,9 @@ int rebin_species(pic_handle *h, int s, unsigned n_out, bool dead) {
     if (!layout_bins(h, counts, start, &sp.h_start)) e = carve_species(h, start[g.ntiles], v, &arena, &bytes, true);
     if (e == cudaErrorMemoryAllocation) {  // no room for kept capacities
         cudaGetLastError();
-        const int rc = layout_bins(h, counts, start);
-        if (rc) {
+        if (const char *why = layout_bins(h, counts, start)) {
             if (arena) dev_free(h, arena);
-            return rc;
+            return set_err(h, PIC_ERR_ARG, why);
         }
         e = carve_species(h, start[g.ntiles], v, &arena, &bytes, true);
     }
