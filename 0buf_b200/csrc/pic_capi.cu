@@ -742,8 +742,8 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
         if ((e = cudaMemsetAsync(h->lb_buf, 0, 2 * kMaxSpecies * sizeof(float), h->stream)) != cudaSuccess)
             return fail(e);
     }
-    // the time stamps of a step follow the status
-    const size_t st_bytes = sizeof(DevStatus) + kStamps * sizeof(unsigned long long);
+    // the time stamps of the last step that succeeded, and of one under way, follow the status
+    const size_t st_bytes = sizeof(DevStatus) + 2 * kStamps * sizeof(unsigned long long);
     if ((e = cudaMalloc(&h->st, st_bytes)) != cudaSuccess) return fail(e);
     if ((e = cudaMemsetAsync(h->st, 0, st_bytes, h->stream)) != cudaSuccess) return fail(e);
     // pinned: the status, then the reductions
@@ -1150,7 +1150,10 @@ void energies_of(const pic_handle *h, double *out4) {
     out4[3] = out4[0] + out4[1] + out4[2];
 }
 
-unsigned long long *step_stamps(const pic_handle *h) { return (unsigned long long *)(h->st + 1); }
+// stamps of the last step that succeeded (next: of the step under way)
+unsigned long long *step_stamps(const pic_handle *h, bool next = false) {
+    return (unsigned long long *)(h->st + 1) + (h->stamp_half ^ (int)next) * kStamps;
+}
 
 // one step; energies (may be null) receives pic_energy's four numbers after it,
 // with the same wait
@@ -1158,7 +1161,7 @@ int step_impl(pic_handle *h, double *energies) {
     int rc = set_device(h);
     if (rc) return rc;
     h->launches = 0;
-    unsigned long long *stamps = step_stamps(h);
+    unsigned long long *stamps = step_stamps(h, true);
     // the FP32 form forms the B half step inside the push's staged field tile
     if (!h->mixed && (rc = do_b_half(h, stamps))) return rc;
     if ((rc = do_push_deposit(h, h->mixed, stamps))) return rc;
@@ -1176,11 +1179,11 @@ int step_impl(pic_handle *h, double *energies) {
     if ((rc = do_e_update(h))) return rc;
     if ((rc = do_e_ghosts(h, stamps))) return rc;
     if (energies && (rc = enqueue_energy(h, true))) return rc;
-    h->timed = h->timed ? 2 : 0;
     CK(cudaStreamSynchronize(h->stream), "sync");
     rc = handle_status(h);
     h->counters[3] = h->launches;
     if (!rc) {
+        h->stamp_half ^= 1;
         h->timed = 1;  // pic_step_timings reads the stamps
         if (energies) energies_of(h, energies);
     }

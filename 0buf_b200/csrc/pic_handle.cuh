@@ -47,7 +47,8 @@ struct pic_handle {
     int64_t counters[4];
     float timings[5];
     int64_t launches;  // kernels launched by the current/last step
-    int timed;
+    int timed;       // 0: no step yet; 1: stamps not read yet; 2: in timings
+    int stamp_half;  // which half of the stamps holds the last step that succeeded
     int kin_valid;  // st->kinetic holds the kinetic energy of the current momenta
     pic::AdjState *adj;
     // charge-conservation diagnostic (pic_diag.cu), allocated on first use:

@@ -430,7 +430,7 @@ const char *pic_error_string(int status);
  * [1] particles no cell accepted (dropped), [2] particles two or more cells
  * accepted (duplicated), [3] kernel launches of the step. */
 int pic_step_counters(pic_handle *h, int64_t *out4);
-/* Timings of the last pic_step in milliseconds (time stamps that the step's
+/* Timings of the last pic_step that succeeded, in milliseconds (time stamps that the step's
  * kernels take on the GPU): [0] B half step, [1] the push/deposit kernel alone, [2] migration
  * arrivals, [3] J fold + B completion + E update + E ghosts, [4] whole step. */
 int pic_step_timings(pic_handle *h, float *out5);
