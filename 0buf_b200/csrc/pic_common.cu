@@ -175,7 +175,7 @@ __global__ void k_insert(const __grid_constant__ StepParams P) {
     const Grid &g = P.g;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         Out o;
-        if (MIXED) {  // entries are 32 bytes from an allocation's start
+        if constexpr (MIXED) {
             ((float4 *)&o)[0] = ((const float4 *)(ob + e))[0];
             ((float4 *)&o)[1] = ((const float4 *)(ob + e))[1];
         } else {

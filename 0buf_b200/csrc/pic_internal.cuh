@@ -271,11 +271,12 @@ struct OutPlain {
     double x, y, z, px, py, pz;
     int cell, species;
 };
-// one migrating particle (mixed form): 32 bytes
-struct OutMixed {
+// one migrating particle (mixed form): 32 bytes, read and written in halves of 16
+struct __align__(16) OutMixed {
     float ox, oy, oz, px, py, pz;
     int cell, species;
 };
+static_assert(sizeof(OutMixed) == 32 && alignof(OutMixed) == 16, "two 128-bit accesses");
 
 // Momenta of the live particles among slots start + {j, j + B, j + 2B, j + 3B}
 // (B = blockDim.x) below start + jend, zeros for the others.  All loads are

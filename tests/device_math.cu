@@ -3,6 +3,8 @@
 #include "pic_adjoint.cuh"
 
 extern "C" {
+int dm_out_mixed_align() { return (int)alignof(pic::OutMixed); }
+int dm_out_mixed_size() { return (int)sizeof(pic::OutMixed); }
 int dm_max_slots() { return pic::kMaxSlots; }
 int dm_max_slot(int it) { return pic::max_slot(it); }
 int dm_max_cleared(int it) { return pic::max_cleared(it); }
