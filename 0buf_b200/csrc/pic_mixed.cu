@@ -740,13 +740,22 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
             {
                 // |round(v/q_s)| <= lb/q_s + 1/2 per contribution, one contribution
                 // per node and lane.  The sum stays below 2^25, where floats are 2
-                // apart: rounded to nearest, it never counts less than that.
+                // apart: rounded to nearest, it never counts less than that.  A
+                // contribution past cmax goes another way and need not count: it is
+                // left out where it alone would flush (a plasma set in motion within
+                // one step has every particle past cmax: a flush per particle, push
+                // 3.39 -> 1.08 ms at 128x64x64 cells, 25M particles).
                 const float add = fmaf(lb, inv_qs, 1.f);
-                if (__any_sync(FULL, run + add > kRunLimit)) {
-                    flush_current();
-                    run = 0.f;
+                float next = run + add;
+                if (__builtin_expect(__any_sync(FULL, next > kRunLimit), 0)) {
+                    const bool counts = lb <= cmax;
+                    if (!counts) next = run;
+                    if (__any_sync(FULL, next > kRunLimit)) {
+                        flush_current();
+                        next = counts ? add : 0.f;
+                    }
                 }
-                run += add;
+                run = next;
             }
             // the second zigzag segment exists only where a cell-centre plane is crossed
             const bool cross = dep && (crs[0] || crs[1] || crs[2]);
