@@ -1,8 +1,9 @@
 // Differentiable run of the FP32 mixed form: the fixed-order push and the
 // adjoint particle kernels.  Same arithmetic as k_push_mixed (cell units,
-// FP32 offsets and momenta, rsqrtf), with the current added straight into the
-// FP64 global J; the adjoint runs in FP32 per particle and adds into FP64
-// field adjoints.  Field transposes and the host sequence: pic_adjoint.cu.
+// FP32 offsets and momenta, rsqrtf).  A CTA's current is summed in its window in
+// 64-bit fixed point and added to the FP64 global J; the adjoint runs in FP32 per
+// particle, and its field adjoints are summed likewise.  Field transposes and the
+// host sequence: pic_adjoint.cu.
 #include <cuda_runtime.h>
 #include <math.h>
 #include "pic0buf.h"
@@ -42,7 +43,7 @@ __device__ __forceinline__ void comp_taps_m(const MTaps &T, int c, int t[3], flo
         w[d] = nd ? T.wn[d] : T.wc[d];
     }
 }
-// interp_mixed's expression order; the eight taps at A, A + dx, ...
+// trilinear interpolation of the eight taps at A, A + dx, ...
 __device__ __forceinline__ float interp_gm(const float *__restrict__ A, int dx, int dy, const float w[3]) {
     const int dz = 1;
     float sx = w[0], sy = w[1], sz = w[2];
@@ -139,7 +140,7 @@ __device__ __forceinline__ bool stencil_ok(const int iv[3]) {
 }
 
 // pqr_mixed (pic_mixed.cu): add(component, x, y, z node offset from the
-// particle's cell, FP32 contribution); false when the segment has no length
+// particle's cell, FP32 contribution); nothing where the segment has no length
 template <class Add>
 __device__ __forceinline__ void seg_mixed(const int iv[3], const float xs[3], const float xe[3], float wx, float wy,
                                           float wz, Add add) {
@@ -301,8 +302,9 @@ __device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WR
 // ---- fixed-order push of the FP32 form.  One CTA per chunk of consecutive
 // particles with the chunk's window staged in shared memory, as
 // k_flat_push_plain; the FP32 contributions are summed in 64-bit fixed point
-// (quantum 2^-50 of the light-speed bound of the chunk, or 2^-51 of one
-// particle's) and added to the FP64 global J once.
+// (quantum 2^-62 of the light-speed bound of the chunk, but at least 2^-51 of one
+// particle's: 2^-52 |m| of rounding beside the 2^-25 |m| h / tau that an offset's own
+// FP32 rounding makes) and added to the FP64 global J once.
 // Bound: instruction issue (1059 instructions per 32 particles, issue slots 65 %
 // busy).  128x32x32 cells, 12.6M particles: 0.916 -> 0.635 ms per step, with the
 // window's strides at compile time and chained launches 0.587 (before:

@@ -704,7 +704,7 @@ int pic_create(const pic_config *cfg, pic_handle **out) {
     int rc = set_device(h);
     if (rc) { delete h; return rc; }
     size_t smem = h->mixed ? push_smem_total_mixed(g) : push_smem_plain(g);
-    h->sms = 148;
+    h->sms = kSMs;
     cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);

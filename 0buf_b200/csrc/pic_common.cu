@@ -618,7 +618,7 @@ cudaError_t gather_from_bins_f(const Grid &g, int mixed, SpeciesView sv, const i
 }
 
 cudaError_t launch_insert(const StepParams &p, cudaStream_t s) {
-    int blocks = 148 * 8;
+    int blocks = 8 * kSMs;
     return launch_chained(p.mixed ? k_insert<OutMixed, true> : k_insert<OutPlain, false>, dim3(blocks), dim3(256), s, p);
 }
 
@@ -712,14 +712,14 @@ cudaError_t begin_push(const StepParams &p, size_t nodes, cudaStream_t s) {
     const size_t n2 = 3 * nodes / 2;  // a multiple of four nodes per row
     const int nholes = p.slices > 1 ? (p.nsp + 1) * p.g.ntiles : 0;
     const int nlb = p.lb_cur ? kMaxSpecies : 0;
-    const int blocks = (int)std::min<size_t>((n2 + 255) / 256, 148 * 16);
+    const int blocks = (int)std::min<size_t>((n2 + 255) / 256, 16 * kSMs);
     return launch_chained(k_begin_push, dim3(blocks), dim3(256), s, (double2 *)p.J[0], n2, (unsigned *)p.st,
                           (int)(sizeof(DevStatus) / 4), p.lb_cur, nlb, p.hole_count, nholes, p.stamps, p.b_half);
 }
 
 cudaError_t kinetic_energy(const StepParams &p, double *out, cudaStream_t s) {
     const int shares = tile_shares(p.g.ntiles);
-    k_kinetic<<<dim3(std::min(p.g.ntiles * shares, 148 * 8), p.nsp), 256, 0, s>>>(p, shares, out);
+    k_kinetic<<<dim3(std::min(p.g.ntiles * shares, 8 * kSMs), p.nsp), 256, 0, s>>>(p, shares, out);
     return cudaGetLastError();
 }
 

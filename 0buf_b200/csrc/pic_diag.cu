@@ -277,7 +277,7 @@ cudaError_t momentum(const StepParams &p, double *out, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(out, 0, 3 * p.nsp * sizeof(double), s);
     if (e != cudaSuccess) return e;
     const int shares = tile_shares(p.g.ntiles);
-    k_momentum<<<dim3(std::min(p.g.ntiles * shares, 148 * 8), p.nsp), 256, 0, s>>>(p, shares, out);
+    k_momentum<<<dim3(std::min(p.g.ntiles * shares, 8 * kSMs), p.nsp), 256, 0, s>>>(p, shares, out);
     return cudaGetLastError();
 }
 
@@ -307,7 +307,7 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
 
 cudaError_t gauss_residual(const Grid &g, int mixed, const void *const E[3], const double *rho, double *G, double *G0,
                            int set_baseline, double *red, cudaStream_t s) {
-    const int bx = 256, grid = std::min((g.NX * g.NY + 7) / 8, 148 * 8);
+    const int bx = 256, grid = std::min((g.NX * g.NY + 7) / 8, 8 * kSMs);
     if (mixed)
         k_gauss<float><<<grid, bx, 0, s>>>(g, (const float *)E[0], (const float *)E[1], (const float *)E[2], rho, G,
                                            G0, set_baseline, red);

@@ -25,6 +25,7 @@
 namespace pic {
 
 constexpr int kMaxSpecies = PIC_MAX_SPECIES;
+constexpr int kSMs = 148;               // of a B200: the grids of walks over nodes, particles and tiles
 constexpr int kHoleMax = 1024;          // departures per tile per species listed before the spill list
 constexpr int kHoleSpill = 16;          // one spill entry per this many slots of the bin
 constexpr int kPushThreads = 256;       // threads of a push CTA: particles per block of a slice
@@ -161,10 +162,6 @@ __device__ __forceinline__ void shared_add64_small(unsigned *plo, unsigned *phi,
     const unsigned old = atomicAdd(plo, lo);
     const unsigned hi = (unsigned)(v >> 31) + (old + lo < old ? 1u : 0u);
     if (hi) atomicAdd(phi, hi);
-}
-__device__ __forceinline__ void fx_add(unsigned long long *a, double v, double inv_q) {
-    long long iv = __double2ll_rn(v * inv_q);
-    if (iv) shared_add64(a, iv);
 }
 __device__ __forceinline__ void fx_addf(unsigned long long *a, float v, float inv_q) {
     long long iv = __float2ll_rn(v * inv_q);
@@ -345,7 +342,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Shares that a reduction over the bins deals a tile out in: enough blocks for
 // eight per SM where the tiles alone are too few.
-inline int tile_shares(int ntiles) { return ntiles >= 148 * 8 ? 1 : (148 * 8 + ntiles - 1) / ntiles; }
+inline int tile_shares(int ntiles) { return ntiles >= 8 * kSMs ? 1 : (8 * kSMs + ntiles - 1) / ntiles; }
 
 // The particles of one species that slice q of P.slices of tile t handles:
 // [jbeg, jend) of the bin.  The bins of all species, cut into blocks of

@@ -5,7 +5,7 @@
 // size of the box: a particle is (int32 cell, FP32 offset in [0,1) per axis,
 // FP32 momentum).  Push, deposit and Yee run in FP32; the deposit
 // pre-reduces each tile's current in shared memory (64-bit fixed point, see
-// fx_add) and adds the tile into the global J in FP64.
+// fx_addf) and adds the tile into the global J in FP64.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -491,7 +491,7 @@ __global__ void PIC_MIXED_BOUNDS k_push_mixed(const __grid_constant__ MixedMaps 
         return;
     }
     if (threadIdx.x == 0) {
-        // quantum of the fixed-point tile J (see fx_add): |contribution| < 1.0834 |m| per segment
+        // quantum of the fixed-point tile J (see fx_addf): |contribution| < 1.0834 |m| per segment
         double bound = 0.0;
         for (int s = 0, first = 0; s < P.nsp; s++) {
             const int count = P.sp[s].tile_count[t];
@@ -981,7 +981,7 @@ cudaError_t contribution_bound_mixed(const Grid &g, const SpeciesView &S, int64_
     if (cap <= 0) return cudaSuccess;
     const float ctx = (float)(g.tau / g.hx), cty = (float)(g.tau / g.hy), ctz = (float)(g.tau / g.hz);
     const float wx = (float)(S.m * g.hx / g.tau), wy = (float)(S.m * g.hy / g.tau), wz = (float)(S.m * g.hz / g.tau);
-    const int blocks = (int)std::min<int64_t>((cap + 255) / 256, 148 * 8);
+    const int blocks = (int)std::min<int64_t>((cap + 255) / 256, 8 * kSMs);
     k_contribution_bound<<<blocks, 256, 0, s>>>(S, (int)cap, wx, wy, wz, ctx, cty, ctz, out);
     return cudaGetLastError();
 }

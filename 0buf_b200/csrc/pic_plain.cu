@@ -1,10 +1,12 @@
 // Plain form (FP64, reference arithmetic) kernels of the B200 PIC step.
 //
-// Compiled with -fmad=false: every FP64 expression below is the reference's
-// expression in the reference's order (citations per function), evaluated as
-// separate IEEE multiplies and adds like the host build of the reference, so
-// that fields match the CPU oracle bit for bit and particles match except
-// where the order of the current sums differs (shared/global atomics).
+// Compiled with -fmad=false.  The field kernels evaluate the reference's FP64
+// expressions in the reference's order (citations per function) as separate IEEE
+// multiplies and adds like its host build: given the same current, the fields match
+// the CPU oracle bit for bit.  The push takes every index, crossing and wrap from its
+// positions as the reference does, bit for bit; its continuous values
+// (interpolation, rotation, weights) are fused and rounded once where the reference
+// rounds twice (pic_plain_math.cuh), and the current is summed in fixed point.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <algorithm>
@@ -303,8 +305,6 @@ __global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus
 
 
 // ------------------------------------------------------- particle push --
-enum : int { kCE = 5 };  // CellExtent, cell.h:23
-
 // Interpolate3D, cell.h:1054-1153, on the staged field tile.  (bi,bl,bk) is
 // the tile-local node of reference tile index (0,0,0) of the particle's cell,
 // i.e. cell_local - 2; the reference tile index (i,l,k) must stay in 2..3 so
@@ -357,8 +357,8 @@ struct BinP {
 // spills.  While 64-bit shared atomics were compare-and-swap loops, 512-thread
 // CTAs at 64 registers (32 warps, ~240 B of spills) hid their round trips
 // better (c2 push 208.7 ms against 246.5 at 256 threads); with the split
-// 64-bit add (shared_add64) the atomics cost nothing measurable and 256
-// threads win: 71.1 ms against 72.7 (384: 75.0, 448: 76.0).
+// 64-bit add (shared_add64) 256 threads win: 71.1 ms against 72.7 (384: 75.0,
+// 448: 76.0).
 //
 // Bound: dependent FP64 operations (4 warps per scheduler at 128 registers;
 // `wait` is the top stall, FP64 pipe 47 %, shared-memory pipe 65 %, DRAM 24 %).
@@ -443,7 +443,11 @@ __global__ void PIC_PLAIN_BOUNDS k_push_plain(const __grid_constant__ StepParams
             ntile += jend - jbeg;
         }
         // a quantum that holds every sum of the tile below 2^62 and every single
-        // contribution below 2^51 (fx_split)
+        // contribution below 2^51 (fx_put2).  The second alone decides in tiles of
+        // fewer than about 800 particles: with the remainder word a contribution is
+        // rounded at 2^-71 |m| or below, where the rounding of its end point x1
+        // (2^-54 x1 / tau, and x1 > tau 2^-17 but for a few particles at a box face)
+        // is 2^-71 |m| at least and mostly 2^-54 |m|
         int e2, e1;
         frexp(bound, &e2);  // bound < 2^e2
         frexp(one, &e1);
@@ -807,10 +811,6 @@ void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned l
                    F[PIC_JX], F[PIC_JY], F[PIC_JZ], F[PIC_HX], F[PIC_HY], F[PIC_HZ], F[PIC_QX], F[PIC_QY], F[PIC_QZ], stamps);
 }
 
-// ElectricFieldComponentEvaluatePeriodic for Ex, Ey, Ez (gpu_plasma.h:432-452,
-// arguments gpu_plasma.h:486-505).  Reference mode skips the y pass of Ex and
-// Ez; periodic mode performs it.  Round A holds the first pass of each
-// component, round B the second; both run in one launch (GhostPasses).
 void flat_begin_plain(const Grid &g, const double *const E[3], const double *const H[3], double *Ha, double *J,
                       double *keepE, cudaStream_t s) {
     const double cx = g.tau / g.hx, cy = g.tau / g.hy, cz = g.tau / g.hz;
@@ -827,6 +827,10 @@ void fold_b_twice_plain(const Grid &g, double *const F[12], cudaStream_t s) {
                    F[PIC_QX], F[PIC_QY], F[PIC_QZ], cx, cy, cz);
 }
 
+// ElectricFieldComponentEvaluatePeriodic for Ex, Ey, Ez (gpu_plasma.h:432-452,
+// arguments gpu_plasma.h:486-505).  Reference mode skips the y pass of Ex and
+// Ez; periodic mode performs it.  Round A holds the first pass of each
+// component, round B the second; both run in one launch (GhostPasses).
 template <typename T>
 static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStream_t s, const DevStatus *st,
                        DevStatus *out, double *hist, unsigned long long *stamps) {

@@ -7,7 +7,8 @@
 //   - sums of products whose value is continuous (the interpolation, the Boris
 //     rotation, the deposit's weights) use fused multiply-adds, one rounding
 //     where the reference has two;
-//   - 1 / sqrt(v) is rsqrt(v), within an ulp like the two operations.
+//   - 1 / sqrt(v) is rsqrt(v): measured on a B200 within 0.51 ulp for v in [1, 1e12],
+//     where the two operations are within 1.5.
 // Both translation units are compiled with -fmad=false: a product and a sum
 // are fused only where fma() is written.
 #pragma once
@@ -30,8 +31,10 @@ __device__ __forceinline__ double div_by(double a, double h, double rh) {
 
 // (int)t and t rounded down for 0 <= t < 2^32: adding 2^52 rounded down leaves
 // the integer part in the low word.  Conversions between FP64 and integers run
-// at a quarter of the FP64 add rate.  For t < 0 (or t >= 2^32, or NaN) exact
-// is false and i is not in any index range that its caller then uses.
+// at a quarter of the FP64 add rate.  For t < 0, t >= 2^32 or NaN trunc_checked's
+// exact is false and i no index.  floor_pos does not tell: the taps it serves come
+// from a particle that lies in its box, u + 1 below 2^32, and a negative t gives a
+// negative index, which the callers' range checks report.
 __device__ __forceinline__ double floor_pos(double t, int &i) {
     const double m = __dadd_rd(t, 0x1p52);
     i = __double2loint(m);
