@@ -65,6 +65,7 @@ struct FlatParams {
     // bmode 1 records them, 2 replays them (see branch_code)
     unsigned long long *branch;
     int bmode;
+    int *far;  // counts the particles outside their chunk's window (null: not)
 };
 // adjoint of one species: lambda_x (3) and lambda_p (3), same order
 struct LamSp {
@@ -79,6 +80,7 @@ struct AdjParams {
 };
 
 constexpr int kW = kT / 32;        // warps per CTA
+constexpr int kDirectBlocks = 3, kDirectAdjBlocks = 2;  // CTAs per SM of the kernels without a window
 constexpr int kQueuePlain = 48;    // queued second segments per warp, as in k_push_plain
 constexpr int kFlatWindow = 900;   // nodes of the forward's window: 109 KB of shared memory, two CTAs per SM
 constexpr int kAdjWindow = 704;    // nodes of the adjoint's: 112 KB
@@ -381,16 +383,17 @@ __device__ __forceinline__ void stage_window(const Grid &g, const AdjWindow<WRAP
 // the nodes around its cells -- is staged into shared memory, and its current
 // is summed there in the exact fixed point of k_push_plain and added to the
 // global J once; a particle outside the window gathers from and adds to
-// global memory.  Bound: dependent FP64 operations, as k_push_plain.  128x32x32
+// global memory.  DIRECT: no window, all particles as those outside it (see
+// AdjState::direct_from).  Bound: dependent FP64 operations, as k_push_plain.  128x32x32
 // cells, 12.6M particles: 1.58 -> 1.12 ms per step (before: taps gathered from
 // and currents added to global memory, one particle per thread); with the
 // deposit's tests gone and the window's strides at compile time 0.98.
-template <int BMODE>
-__global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
+template <int BMODE, bool DIRECT>
+__global__ void __launch_bounds__(kT, DIRECT ? kDirectBlocks : 2) k_flat_push_plain(FlatParams P) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow<false> sWin;
-    __shared__ int sRed[15 * kW], sQn[kW];
+    __shared__ int sRed[15 * kW], sQn[kW], sFar;
     __shared__ double sQ, sInvQ;
     double *sF = (double *)smem_raw;
     unsigned long long *sJ = (unsigned long long *)(sF + 6 * kFlatWindow);  // 9 words per node (pqr_plain)
@@ -403,33 +406,39 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
     const AdjChunk ch = P.chunks[blockIdx.x];
     const int s = ch.species, count = ch.count;
     const FlatSp &S = P.sp[s];
-    if ((int)threadIdx.x < count) next.start(S, ch.first + threadIdx.x);
-    const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
+    AdjWindow<false> w{};
+    if (!DIRECT) {
+        if ((int)threadIdx.x < count) next.start(S, ch.first + threadIdx.x);
+        w = chunk_window(g, S.cell + ch.first, count, kFlatWindow, sRed, &sWin);
+    }
     // (see AdjWindow: the strides at compile time where the window has them)
     auto body = [&](auto fixed) {
     constexpr bool FIX = decltype(fixed)::value;
-    const int SY = FIX ? kFixSY : w.SY, SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
+    const int SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
     const int cn = FIX ? kFlatWindow : nn;  // between the components
-    if (threadIdx.x == 0) {
-        // the quantum of k_push_plain's tile current, for this chunk
-        int e2, e1;
-        frexp(2.5 * fabs(S.m) * (double)count, &e2);
-        frexp(1.0834 * fabs(S.m), &e1);
-        const int eq = max(e2 - 62, e1 - 51);
-        sQ = ldexp(1.0, eq);
-        sInvQ = ldexp(1.0, -eq);
-    }
     const double *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window<6>(g, w, cn, src, sF);
-    for (int e = threadIdx.x; e < 9 * cn; e += blockDim.x) ((unsigned *)sJ)[e] = 0u;
-    if (lane == 0) sQn[warp] = 0;
-    __syncthreads();
+    if (!DIRECT) {
+        if (threadIdx.x == 0) {
+            sFar = 0;
+            // the quantum of k_push_plain's tile current, for this chunk
+            int e2, e1;
+            frexp(2.5 * fabs(S.m) * (double)count, &e2);
+            frexp(1.0834 * fabs(S.m), &e1);
+            const int eq = max(e2 - 62, e1 - 51);
+            sQ = ldexp(1.0, eq);
+            sInvQ = ldexp(1.0, -eq);
+        }
+        stage_window<6>(g, w, cn, src, sF);
+        for (int e = threadIdx.x; e < 9 * cn; e += blockDim.x) ((unsigned *)sJ)[e] = 0u;
+        if (lane == 0) sQn[warp] = 0;
+        __syncthreads();
+    }
     const double h3[3] = {g.hx, g.hy, g.hz}, r3[3] = {1.0 / g.hx, 1.0 / g.hy, 1.0 / g.hz};
     const double tau = g.tau, tau1 = S.q_m * tau * 0.5;
     const double lo_scale = ldexp(1.0, fx_lo32_bits(count));
     // the charge weight over pqr's tau*h*h divisors, and in quanta
     const double rg[3] = {S.m / (tau * g.hy * g.hz), S.m / (tau * g.hx * g.hz), S.m / (tau * g.hx * g.hy)};
-    const double rc[3] = {rg[0] * sInvQ, rg[1] * sInvQ, rg[2] * sInvQ};
+    const double inv_q = DIRECT ? 1.0 : sInvQ, rc[3] = {rg[0] * inv_q, rg[1] * inv_q, rg[2] * inv_q};
     const double L3[3] = {g.lx, g.ly, g.lz};
     const int n3[3] = {g.nx, g.ny, g.nz};
     unsigned bad = 0;
@@ -442,15 +451,24 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
         const int64_t j = ch.first + jc;
         int cell = -1;
         double x[3] = {0.0, 0.0, 0.0}, p[3] = {0.0, 0.0, 0.0};
-        cp_async_wait_all();
-        if (jc < count) cell = next.take(x, p);
-        __syncwarp();  // the reads come before the next copies into the same place
-        if (jc + (int)blockDim.x < count) next.start(S, j + blockDim.x);
+        if (DIRECT) {
+            if (jc < count) {
+                cell = S.cell[j];
+#pragma unroll
+                for (int d = 0; d < 3; d++) { x[d] = S.v[d][j]; p[d] = S.v[3 + d][j]; }
+            }
+        } else {
+            cp_async_wait_all();
+            if (jc < count) cell = next.take(x, p);
+            __syncwarp();  // the reads come before the next copies into the same place
+            if (jc + (int)blockDim.x < count) next.start(S, j + blockDim.x);
+        }
         if (cell >= 0) {
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            int u3[3], n0;
-            const bool in = w.place(c3, dX, dY, u3, n0);
+            int u3[3] = {0, 0, 0}, n0 = 0;
+            const bool in = !DIRECT && w.place(c3, dX, dY, u3, n0);
+            if (!DIRECT && !in) atomicAdd(&sFar, 1);
             const double o3[3] = {(double)c3[0] * h3[0], (double)c3[1] * h3[1], (double)c3[2] * h3[2]};
             const unsigned long long rcode = BMODE == 2 ? P.branch[P.off[s] + j] : 0ull;
             AxisTaps T[3];
@@ -580,6 +598,7 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
             O.v[0][j] = xr[0]; O.v[1][j] = xr[1]; O.v[2][j] = xr[2];
             O.v[3][j] = p[0]; O.v[4][j] = p[1]; O.v[5][j] = p[2];
         }
+        if (DIRECT) continue;
         // ---- the warp's queued second segments, one per lane
         __syncwarp();
         qn = sQn[warp];
@@ -604,19 +623,22 @@ __global__ void __launch_bounds__(kT, 2) k_flat_push_plain(FlatParams P) {
         }
         __syncwarp();
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
-        const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
-        long long ih, il;
-        fx_get<true>((const unsigned *)sJ + a, 3 * cn, ih, il);
-        size_t n;
-        if ((ih == 0 && il == 0) || !w.grid_node(g, r, n)) continue;
-        atomicAdd(&P.J[comp][n], ((double)ih + (double)il / lo_scale) * sQ);
+    if (!DIRECT) {
+        __syncthreads();
+        if (threadIdx.x == 0 && P.far && sFar) atomicAdd(P.far, sFar);
+        for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
+            const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
+            long long ih, il;
+            fx_get<true>((const unsigned *)sJ + a, 3 * cn, ih, il);
+            size_t n;
+            if ((ih == 0 && il == 0) || !w.grid_node(g, r, n)) continue;
+            atomicAdd(&P.J[comp][n], ((double)ih + (double)il / lo_scale) * sQ);
+        }
     }
     if (bad) atomicOr(&P.st->flags, bad);
     if (amb) atomicAdd(&P.st->ambiguous, amb);
     };
-    if (w.fixed()) body(std::true_type{});
+    if (!DIRECT && w.fixed()) body(std::true_type{});
     else body(std::false_type{});
 }
 
@@ -782,7 +804,7 @@ __device__ __forceinline__ void reverse_component(const double *V, int dX, int d
 }
 
 // a particle outside its chunk's window: everything through global memory
-__device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
+__device__ __forceinline__ void reverse_global(const AdjParams &A, int s, int64_t j) {
     const FlatParams &P = A.f;
     const Grid &g = P.g;
     const FlatSp &S = P.sp[s];
@@ -819,6 +841,15 @@ __device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) {
         Lm.v[d][j] = fma(gi[d], K.r3[d], gx[d]);
         Lm.v[3 + d][j] = lu[d];
     }
+}
+
+__device__ __noinline__ void reverse_far(const AdjParams &A, int s, int64_t j) { reverse_global(A, s, j); }
+// all particles of a step that way
+__global__ void __launch_bounds__(kT, kDirectAdjBlocks) k_adj_direct_plain(const __grid_constant__ AdjParams A) {
+    chain_enter();
+    const AdjChunk ch = A.f.chunks[blockIdx.x];
+    const int lane = threadIdx.x & 31, mine = (lane >> 3) * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
+    for (int e = mine; e < ch.count; e += blockDim.x) reverse_global(A, ch.species, ch.first + e);
 }
 
 // ---- adjoint of the particle part of one step: recompute the push, transpose
@@ -1264,17 +1295,28 @@ int64_t total_particles(const AdjState &A) {
     return t;
 }
 
+constexpr int kFarPoll = 8;  // (see far_passed)
+FarPost far_post(pic_handle *h, const AdjState &A, const double *hist, int n) {
+    FarPost p;
+    if (hist && n % kFarPoll == kFarPoll - 1 && n < A.direct_from) {
+        p.far = A.far + n;
+        p.host = (unsigned long long *)(h->hred + 7);
+        p.step = n;
+    }
+    return p;
+}
+
 // one forward step of the flat state on the field set F (plain): particles read
 // from `state`, written to `out` (the same buffer when out is null).  keep: E and
 // the half-step H of the step go there (six arrays; null: the half-step H to A.ha).
-// hist: receives the sums of E_c^2 after the step (null: none).
+// hist: receives the sums of E_c^2 after the step (null: none, a recompute); n: the step.
 // Five chained launches (before: eight operations, one after the other, and a
 // copy of the fields in a recompute); the reverse of a step is six (before:
 // eight).  Small runs wait on them: 16x8x8 cells, 24.6k particles, FP64 forward
 // 33.0 -> 26.1 us per step, backward 93.8 -> 70.7; 64x32x32 cells, 3.1M FP32
 // 201 -> 187 and 662 -> 630.
 int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, char *keep,
-                    double *hist) {
+                    double *hist, int n) {
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
     const size_t N = g.nodes_pitched();
@@ -1283,8 +1325,14 @@ int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_F
                      (double *)keep, s);  // J: the three arrays lie one after another
     FlatParams P = flat_params(h, A, state, F, out);
     for (int c = 0; c < 3; c++) P.H[c] = Ha + c * N;
-    if (A.nchunks > 0) {
-        auto *kern = P.bmode == 0 ? k_flat_push_plain<0> : (P.bmode == 1 ? k_flat_push_plain<1> : k_flat_push_plain<2>);
+    P.far = hist ? A.far + n : nullptr;
+    if (A.nchunks > 0 && n >= A.direct_from) {
+        auto *kern = P.bmode == 0 ? k_flat_push_plain<0, true>
+                                  : (P.bmode == 1 ? k_flat_push_plain<1, true> : k_flat_push_plain<2, true>);
+        CK(launch_chained(kern, dim3(A.nchunks), dim3(kT), s, P), "flat push");
+    } else if (A.nchunks > 0) {
+        auto *kern = P.bmode == 0 ? k_flat_push_plain<0, false>
+                                  : (P.bmode == 1 ? k_flat_push_plain<1, false> : k_flat_push_plain<2, false>);
         const size_t smem = (size_t)kFlatWindow * (6 * sizeof(double) + 3 * 12) + (size_t)kW * kQueuePlain * 52 + kNextBytes;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "flat push");
         CK(launch_chained_smem(kern, dim3(A.nchunks), dim3(kT), smem, s, P), "flat push");
@@ -1292,7 +1340,7 @@ int flat_step_plain(pic_handle *h, AdjState &A, char *state, void *const F[PIC_F
     fold_b_twice_plain(g, (double *const *)F, s);
     yee_e_update_plain(g, (double *const *)F, s);
     e_ghosts_plain(g, (double *)F[PIC_EX], (double *)F[PIC_EY], (double *)F[PIC_EZ],
-                   h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist);
+                   h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist, nullptr, far_post(h, A, hist, n));
     CK(cudaGetLastError(), "flat step fields");
     return PIC_OK;
 }
@@ -1435,8 +1483,8 @@ MixParams mix_params(pic_handle *h, AdjState &A, char *state, void *const F[PIC_
 
 // one forward step of the fixed-order state on the field set F (see flat_step_plain)
 int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_COUNT], char *out, char *keep,
-              double *hist) {
-    if (!h->mixed) return flat_step_plain(h, A, state, F, out, keep, hist);
+              double *hist, int n) {
+    if (!h->mixed) return flat_step_plain(h, A, state, F, out, keep, hist, n);
     const Grid &g = h->g;
     cudaStream_t s = h->stream;
     float *const *E = (float *const *)&F[PIC_EX];
@@ -1446,20 +1494,72 @@ int flat_step(pic_handle *h, AdjState &A, char *state, void *const F[PIC_FIELD_C
     flat_begin_mixed(g, (const float *const *)E, (const float *const *)H, Ha, (double *)F[PIC_JX], (float *)keep, s);
     MixParams P = mix_params(h, A, state, F, out);
     for (int c = 0; c < 3; c++) P.H[c] = Ha + c * N;
-    CK(launch_flat_push_mixed(P, A.nchunks, s), "flat push");
+    P.far = hist ? A.far + n : nullptr;
+    CK(launch_flat_push_mixed(P, A.nchunks, n >= A.direct_from, s), "flat push");
     fold_b_mixed(g, E, H, (double *const *)&F[PIC_JX], s);
     yee_e_update_mixed(g, E, H, (double *const *)&F[PIC_JX], s);
-    e_ghosts_mixed(g, E[0], E[1], E[2], h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist);
+    e_ghosts_mixed(g, E[0], E[1], E[2], h->cfg.ghosts == PIC_GHOSTS_PERIODIC, s, nullptr, nullptr, hist, nullptr,
+                   far_post(h, A, hist, n));
     CK(cudaGetLastError(), "flat step fields");
     return PIC_OK;
+}
+
+// Steps without windows.  A chunk's particles share a window while they stay near
+// each other; in a hot or long run they spread, and those outside the window go
+// through global memory in kernels whose shared memory leaves no L1: with half of
+// them outside the reverse step took 3 times as long as kernels without windows.  A
+// run whose fraction outside passes far_limit therefore goes on without.  far[n] is
+// that fraction's numerator of step n.  limit: where the two were equally fast
+// (64x32x32 cells, vth .2, steps of half a cell at light speed; particles per cell and
+// species p, fraction: FP64 forward 16 0, 64 .02, 250 .06, reverse 16 .02, 64 .03,
+// 250 .13; FP32 forward 16 .02, 64 .5, 250 .65, reverse 16 .09, 64 .12, 250 .27).
+// With vth .3 for 100 steps: FP64 960 and 5140 us per step forward and backward ->
+// 610 and 2040, FP32 618 and 4250 -> 485 and 1720.
+double far_limit(bool mixed, bool reverse, double p) {
+    if (!mixed) return reverse ? .005 + p / 2000 : p / 4000;
+    return reverse ? .08 + p / 1300 : std::min(.65, std::max(0.0, (p - 12) / 110));
+}
+// the first reverse step without windows: from the forward's counts, which end where
+// it went on without windows itself; from there they grow as in the last 8 steps
+int reverse_direct_from(const std::vector<int> &far, int known, double particles, double limit) {
+    const int steps = (int)far.size();
+    for (int n = 0; n < known; n++)
+        if (far[n] > limit * particles) return n;
+    if (known >= steps || known < 9) return known < steps ? known : steps;
+    const double last = far[known - 1], slope = std::max(0.0, (last - far[known - 9]) / 8);
+    for (int n = known; n < steps; n++)
+        if (last + slope * (n - known + 1) > limit * particles) return n;
+    return steps;
+}
+
+// The forward learns of far[n] from the kernels themselves: every kFarPoll steps the
+// last kernel of a step writes the count and the step to pinned memory, and the host,
+// which enqueues ahead, waits there for the count of kFarPoll + 1 steps ago.  The
+// device still has kFarPoll steps to do then.
+bool far_passed(pic_handle *h, int n, double limit) {
+    const volatile unsigned long long *slot = (const volatile unsigned long long *)(h->hred + 7);
+    for (long long spin = 1;; spin++) {
+        const unsigned long long v = *slot;
+        if ((int)(v >> 32) >= n + 1) return (double)(unsigned)v > limit;
+        // finished, or failed: the run's end reports it
+        if (spin % 4096 == 0) {
+            if (cudaStreamQuery(h->stream) != cudaErrorNotReady) return false;
+            cudaGetLastError();  // not the next launch's
+        }
+    }
 }
 
 int forward_run(pic_handle *h, AdjState &A) {
     const Grid &g = h->g;
     cudaStream_t st = h->stream;
     const size_t fbytes = field_bytes(h);
+    const double particles = (double)total_particles(A);
+    const double limit = particles * far_limit(h->mixed, false, particles / ((double)A.nsp * g.ncells()));
+    *(volatile unsigned long long *)(h->hred + 7) = 0ull;
     CK(cudaEventRecord(A.e0, st), "event");
     for (int n = 0; n < A.steps; n++) {
+        if (n >= 2 * kFarPoll && n % kFarPoll == 0 && A.direct_from == A.steps && far_passed(h, n - kFarPoll - 1, limit))
+            A.direct_from = n;
         if (n % A.K == 0) {
             int c = n / A.K;
             CK(cudaMemcpyAsync(A.ckp + (size_t)c * A.pbytes, A.cur, A.pbytes, cudaMemcpyDeviceToDevice, st), "ckpt");
@@ -1475,7 +1575,7 @@ int forward_run(pic_handle *h, AdjState &A) {
             A.step_branch = const_cast<unsigned long long *>(A.branch_src) + (size_t)n * np_all;
             A.step_bmode = 2;
         }
-        int rc = flat_step(h, A, A.cur, h->f, nullptr, nullptr, A.hist + 3 * n);
+        int rc = flat_step(h, A, A.cur, h->f, nullptr, nullptr, A.hist + 3 * n, n);
         A.step_branch = nullptr;
         A.step_bmode = 0;
         if (rc) return rc;
@@ -1536,7 +1636,9 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
             o += 6 * (size_t)A.n[s];
         }
         for (int c = 0; c < 3; c++) { P.LJ[c] = LJ[c]; P.LE[c] = LE[c]; P.LH[c] = LH[c]; }
-        if (A.nchunks > 0) {
+        if (A.nchunks > 0 && n >= A.direct_adj_from) {
+            CK(launch_chained(k_adj_direct_plain, dim3(A.nchunks), dim3(kT), st, P), "adjoint particles");
+        } else if (A.nchunks > 0) {
             const size_t smem = (size_t)kAdjWindow * 120 + kNextBytes + kNextLamBytes + kAdjChunk * sizeof(unsigned short);
             CK(cudaFuncSetAttribute(k_adj_particles_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "adjoint particles");
@@ -1550,7 +1652,7 @@ int reverse_step(pic_handle *h, AdjState &A, const pic_loss &L, int n, char *sta
             o += 6 * (size_t)A.n[s];
         }
         for (int c = 0; c < 3; c++) { P.LJ[c] = LJ[c]; P.LE[c] = LE[c]; P.LH[c] = LH[c]; }
-        CK(launch_adj_particles_mixed(P, A.nchunks, st), "adjoint particles");
+        CK(launch_adj_particles_mixed(P, A.nchunks, n >= A.direct_adj_from, st), "adjoint particles");
         launch_chained(k_adj_b_half<float>, plane_blocks(g), dim3(kT), st, FA, (const float *)inject, L.field, w2);
     }
     CK(cudaGetLastError(), "reverse step");
@@ -1586,7 +1688,7 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
                        "sub-checkpoint fields");
                     if (q == nsub - 1) break;  // the last sub-segment starts here
                 }
-                int rc = flat_step(h, A, A.segp, RF, nullptr, nullptr, nullptr);
+                int rc = flat_step(h, A, A.segp, RF, nullptr, nullptr, nullptr, start + j);
                 if (rc) return rc;
             }
         }
@@ -1598,7 +1700,7 @@ int backward_run(pic_handle *h, AdjState &A, const pic_loss &L) {
             CK(cudaMemcpyAsync(A.rf, sf, ehb, cudaMemcpyDeviceToDevice, st), "restore fields");
             for (int j = 0; j < slen; j++) {
                 int rc = flat_step(h, A, A.segp + (size_t)j * A.pbytes, RF, A.segp + (size_t)(j + 1) * A.pbytes,
-                                   A.segf + (size_t)j * ehb, nullptr);
+                                   A.segf + (size_t)j * ehb, nullptr, s0 + j);
                 if (rc) return rc;
             }
             for (int j = slen - 1; j >= 0; j--) {
@@ -1699,7 +1801,7 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     if ((rc = adj_alloc(h, kAdjCur, (void **)&A.cur, A.pbytes, "the particle state"))) return rc;
     if ((rc = adj_alloc(h, kAdjCkp, (void **)&A.ckp, A.pbytes * A.nseg, "the particle checkpoints"))) return rc;
     if ((rc = adj_alloc(h, kAdjCkf, (void **)&A.ckf, fbytes * 6 * A.nseg, "the field checkpoints"))) return rc;
-    if ((rc = adj_alloc(h, kAdjHist, (void **)&A.hist, sizeof(double) * 3 * steps, "the history"))) return rc;
+    if ((rc = adj_alloc(h, kAdjHist, (void **)&A.hist, sizeof(double) * 4 * steps, "the history"))) return rc;
     if ((rc = adj_alloc(h, kAdjSt, (void **)&A.st, sizeof(AdjStatus), "the status"))) return rc;
     if ((rc = adj_alloc(h, kAdjRed, (void **)&A.red, sizeof(double) * 8, "the reduction scratch"))) return rc;
     if ((rc = adj_alloc(h, kAdjHa, (void **)&A.ha, fbytes * 3, "the half-step B"))) return rc;
@@ -1712,7 +1814,9 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     if (A.K2 == A.K)
         for (int q : {kAdjSubp, kAdjSubf})
             if (A.pool[q].p) { cudaFree(A.pool[q].p); A.pool[q].p = nullptr; }
-    CK(cudaMemsetAsync(A.hist, 0, sizeof(double) * 3 * steps, h->stream), "zero history");
+    CK(cudaMemsetAsync(A.hist, 0, sizeof(double) * 4 * steps, h->stream), "zero history");
+    A.far = (int *)(A.hist + 3 * steps);
+    A.direct_from = A.direct_adj_from = steps;
     CK(cudaMemsetAsync(A.st, 0, sizeof(AdjStatus), h->stream), "zero status");
     // bins -> flat order
     int *cell[kMaxSpecies];
@@ -1744,6 +1848,10 @@ static int forward_impl(pic_handle *h, int steps, int ckpt_every, int sub_every,
     CK(cudaMemcpy(A.hhist.data(), A.hist, sizeof(double) * 3 * steps, cudaMemcpyDeviceToHost), "history");
     const double w = g.hx * g.hy * g.hz;
     for (double &x : A.hhist) x *= w;
+    std::vector<int> far(steps);
+    CK(cudaMemcpy(far.data(), A.far, sizeof(int) * steps, cudaMemcpyDeviceToHost), "particles outside the windows");
+    A.direct_adj_from = reverse_direct_from(far, A.direct_from, (double)total_particles(A),
+                                            far_limit(h->mixed, true, (double)total_particles(A) / ((double)A.nsp * g.ncells())));
     // the handle continues from the final state: flat order -> bins
     for (int s = 0; s < A.nsp; s++) {
         if (!h->mixed)

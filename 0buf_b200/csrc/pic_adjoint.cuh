@@ -67,6 +67,9 @@ struct AdjState {
     AdjChunk *chunks;  // nchunks of them, device
     int nchunks;
     double *hist;      // steps x 3: sum over nodes 1..N of E_c^2 after each step
+    int *far;          // steps: particles outside their chunk's window, as far as windows were used
+    // the first steps, forward and in reverse, whose particle kernels use no windows
+    int direct_from, direct_adj_from;
     // frozen branches (plain form): mode 1 records every step's discrete
     // choices into branch (steps x particles codes), mode 2 replays those of
     // branch_src; step_branch / step_bmode are what the next flat push uses
@@ -318,13 +321,14 @@ struct MixParams {
     const float *H[3];          // push: H after the half step
     double *J[3];
     AdjStatus *st;
+    int *far;                   // push: counts the particles outside their chunk's window (null: not)
     // adjoint
     float *lam[kMaxSpecies][6]; // lambda_x (cell units), lambda_p
     const double *LJ[3];
     double *LE[3], *LH[3];
 };
-cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, cudaStream_t s);
-cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStream_t s);
+cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, bool direct, cudaStream_t s);
+cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, bool direct, cudaStream_t s);
 void adj_gather_mixed(const Grid &g, const SpeciesView &S, const int64_t *d0, int *cell, void *const v[6],
                       cudaStream_t s);
 // lambda_p (3 FP32 arrays of n) and p0 (3 FP32 arrays) -> 6 FP64 arrays of n

@@ -261,6 +261,7 @@ __device__ __forceinline__ MixConst mix_const(const Grid &g, const MixSp &S) {
 }
 
 constexpr int kW = kT / 32;          // warps per CTA
+constexpr int kDirectBlocks = 4, kDirectAdjBlocks = 3;  // CTAs per SM of the kernels without a window
 constexpr int kQueueMix = 48;        // queued second segments per warp: drained at 16, at most 15 + 32
 constexpr int kFlatWindowMix = 800;  // nodes of the forward's window: 56 KB of shared memory, three CTAs per SM (80 registers)
 constexpr int kAdjWindowMix = 672;   // nodes of the adjoint's: 73 KB, three
@@ -304,18 +305,20 @@ __device__ __forceinline__ void stage_window_m(const Grid &g, const AdjWindow<WR
 // k_flat_push_plain; the FP32 contributions are summed in 64-bit fixed point
 // (quantum 2^-62 of the light-speed bound of the chunk, but at least 2^-51 of one
 // particle's: 2^-52 |m| of rounding beside the 2^-25 |m| h / tau that an offset's own
-// FP32 rounding makes) and added to the FP64 global J once.
+// FP32 rounding makes) and added to the FP64 global J once.  DIRECT: no window (see
+// AdjState::direct_from).
 // Bound: instruction issue (1059 instructions per 32 particles, issue slots 65 %
 // busy).  128x32x32 cells, 12.6M particles: 0.916 -> 0.635 ms per step, with the
 // window's strides at compile time and chained launches 0.587 (before:
 // taps gathered from and currents added to global memory; four CTAs per SM at
 // 64 registers: 0.688; lanes spread over 4 or 8 places: 0.625, 0.660, and slower
 // at 3M particles).
-__global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant__ MixParams P) {
+template <bool DIRECT>
+__global__ void __launch_bounds__(kT, DIRECT ? kDirectBlocks : 3) k_flat_push_mixed(const __grid_constant__ MixParams P) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ AdjWindow<false> sWin;
-    __shared__ int sRed[15 * kW], sQn[kW];
+    __shared__ int sRed[15 * kW], sQn[kW], sFar;
     __shared__ double sQ, sInvQ;
     __shared__ MixConst sK;
     const Grid &g = P.g;
@@ -326,12 +329,15 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *qd = (float *)sTail + warp * 7 * kQueueMix;  // x2, xe, then the cell and class code
     const NextMix<6> next(sTail + (size_t)kW * 7 * kQueueMix * sizeof(float));
-    if ((int)threadIdx.x < count) next.start(S, nullptr, ch.first + threadIdx.x);
-    const AdjWindow<false> w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
+    AdjWindow<false> w{};
+    if (!DIRECT) {
+        if ((int)threadIdx.x < count) next.start(S, nullptr, ch.first + threadIdx.x);
+        w = chunk_window(g, S.cell + ch.first, count, kFlatWindowMix, sRed, &sWin);
+    }
     // (see AdjWindow: the strides at compile time where the window has them)
     auto body = [&](auto fixed) {
     constexpr bool FIX = decltype(fixed)::value;
-    const int SY = FIX ? kFixSY : w.SY, SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
+    const int SZ = FIX ? kFixSZ : w.SZ, dX = FIX ? kFixSX : w.SX, dY = SZ, nn = w.nn;
     const int cn = FIX ? kFlatWindowMix : nn;  // between the components
     unsigned *sLo = (unsigned *)smem_raw, *sHi = sLo + 3 * cn;
     float *sF = (float *)(sHi + 3 * cn);
@@ -343,11 +349,14 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         sQ = ldexp(1.0, eq);
         sInvQ = ldexp(1.0, -eq);
         sK = mix_const(g, S);
+        sFar = 0;
     }
     const float *src[6] = {P.E[0], P.E[1], P.E[2], P.H[0], P.H[1], P.H[2]};
-    stage_window_m<6>(g, w, cn, src, sF);
-    for (int e = threadIdx.x; e < 6 * cn; e += blockDim.x) sLo[e] = 0u;
-    if (lane == 0) sQn[warp] = 0;
+    if (!DIRECT) {
+        stage_window_m<6>(g, w, cn, src, sF);
+        for (int e = threadIdx.x; e < 6 * cn; e += blockDim.x) sLo[e] = 0u;
+        if (lane == 0) sQn[warp] = 0;
+    }
     __syncthreads();
     const MixConst &K = sK;
     const double inv_q = sInvQ;
@@ -368,19 +377,28 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         const int64_t j = ch.first + jc;
         int cell = -1;
         float xs[3], p[3];
-        cp_async_wait_all();
-        if (jc < count) {
-            cell = next.cell();
-            next.take3(0, xs);
-            next.take3(3, p);
+        if (DIRECT) {
+            if (jc < count) {
+                cell = S.cell[j];
+#pragma unroll
+                for (int d = 0; d < 3; d++) { xs[d] = S.v[d][j]; p[d] = S.v[3 + d][j]; }
+            }
+        } else {
+            cp_async_wait_all();
+            if (jc < count) {
+                cell = next.cell();
+                next.take3(0, xs);
+                next.take3(3, p);
+            }
+            __syncwarp();  // the reads come before the next copies into the same place
+            if (jc + (int)blockDim.x < count) next.start(S, nullptr, j + blockDim.x);
         }
-        __syncwarp();  // the reads come before the next copies into the same place
-        if (jc + (int)blockDim.x < count) next.start(S, nullptr, j + blockDim.x);
         if (cell >= 0) {
             int c3[3];
             g.cell_ijk(cell, c3[0], c3[1], c3[2]);
-            int u3[3], n0;
-            const bool in = w.place(c3, dX, dY, u3, n0);
+            int u3[3], n0 = 0;
+            const bool in = !DIRECT && w.place(c3, dX, dY, u3, n0);
+            if (!DIRECT && !in) atomicAdd(&sFar, 1);
             float F[6];
             if (in) {
                 FieldViewM<true> V;
@@ -441,6 +459,7 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
             O.v[0][j] = xe[0]; O.v[1][j] = xe[1]; O.v[2][j] = xe[2];
             O.v[3][j] = B.pp[0]; O.v[4][j] = B.pp[1]; O.v[5][j] = B.pp[2];
         }
+        if (DIRECT) continue;
         // ---- the warp's queued second segments, one per lane
         __syncwarp();
         qn = sQn[warp];
@@ -463,17 +482,20 @@ __global__ void __launch_bounds__(kT, 3) k_flat_push_mixed(const __grid_constant
         }
         __syncwarp();
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
-        const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
-        const long long v = (long long)(((unsigned long long)sHi[a] << 32) | sLo[a]);
-        size_t n;
-        if (v == 0 || !w.grid_node(g, r, n)) continue;
-        atomicAdd(&P.J[comp][n], (double)v * sQ);
+    if (!DIRECT) {
+        __syncthreads();
+        if (threadIdx.x == 0 && P.far && sFar) atomicAdd(P.far, sFar);
+        for (int e = threadIdx.x; e < 3 * nn; e += blockDim.x) {
+            const int comp = e / nn, r = e - comp * nn, a = comp * cn + r;
+            const long long v = (long long)(((unsigned long long)sHi[a] << 32) | sLo[a]);
+            size_t n;
+            if (v == 0 || !w.grid_node(g, r, n)) continue;
+            atomicAdd(&P.J[comp][n], (double)v * sQ);
+        }
     }
     if (bad) atomicOr(&P.st->flags, bad);
     };
-    if (w.fixed()) body(std::true_type{});
+    if (!DIRECT && w.fixed()) body(std::true_type{});
     else body(std::false_type{});
 }
 
@@ -582,7 +604,7 @@ __device__ __forceinline__ void reverse_component_m(const float *V, int dX, int 
 }
 
 // a particle outside its chunk's window: everything through global memory
-__device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j) {
+__device__ __forceinline__ void reverse_global_m(const MixParams &P, int s, int64_t j) {
     const Grid &g = P.g;
     const MixSp &S = P.sp[s];
     float *const *Lm = P.lam[s];
@@ -616,6 +638,15 @@ __device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j)
         Lm[d][j] = gx[d] + gi[d];
         Lm[3 + d][j] = lu[d];
     }
+}
+
+__device__ __noinline__ void reverse_far_m(const MixParams &P, int s, int64_t j) { reverse_global_m(P, s, j); }
+// all particles of a step that way
+__global__ void __launch_bounds__(kT, kDirectAdjBlocks) k_adj_direct_mixed(const __grid_constant__ MixParams P) {
+    chain_enter();
+    const AdjChunk ch = P.chunks[blockIdx.x];
+    const int lane = threadIdx.x & 31, mine = (lane >> 3) * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
+    for (int e = mine; e < ch.count; e += blockDim.x) reverse_global_m(P, ch.species, ch.first + e);
 }
 
 // ---- adjoint of the particle part of one step (k_adj_particles_plain in FP32):
@@ -783,16 +814,18 @@ __global__ void k_widen(const float *__restrict__ lp, const float *__restrict__ 
 
 }  // namespace
 
-cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, cudaStream_t s) {
+cudaError_t launch_flat_push_mixed(const MixParams &P, int nchunks, bool direct, cudaStream_t s) {
     if (nchunks <= 0) return cudaSuccess;
+    if (direct) return launch_chained(k_flat_push_mixed<true>, dim3(nchunks), dim3(kT), s, P);
     const size_t smem = (size_t)kFlatWindowMix * 48 + (size_t)kW * 7 * kQueueMix * sizeof(float) + NextMix<6>::bytes;
-    cudaError_t e = cudaFuncSetAttribute(k_flat_push_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_flat_push_mixed<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_chained_smem(k_flat_push_mixed, dim3(nchunks), dim3(kT), smem, s, P);
+    return launch_chained_smem(k_flat_push_mixed<false>, dim3(nchunks), dim3(kT), smem, s, P);
 }
 
-cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, cudaStream_t s) {
+cudaError_t launch_adj_particles_mixed(const MixParams &P, int nchunks, bool direct, cudaStream_t s) {
     if (nchunks <= 0) return cudaSuccess;
+    if (direct) return launch_chained(k_adj_direct_mixed, dim3(nchunks), dim3(kT), s, P);
     const size_t smem = (size_t)kAdjWindowMix * 84 + NextMix<12>::bytes + kAdjChunk * sizeof(unsigned short);
     cudaError_t e = cudaFuncSetAttribute(k_adj_particles_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

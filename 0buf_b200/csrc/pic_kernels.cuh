@@ -15,12 +15,18 @@ void j_fold(const Grid &g, double *Jx, double *Jy, double *Jz, cudaStream_t s);
 void fold_b_plain(const Grid &g, double *const F[12], cudaStream_t s, unsigned long long *stamps = nullptr);
 // st, out: device status and pinned host memory that receives it (null: none);
 // hist: three sums that receive E_c^2 over the nodes 1..N (null: none)
+// post: a count that goes to pinned host memory with the step, (step + 1) << 32 | count
+struct FarPost {
+    const int *far = nullptr;
+    unsigned long long *host = nullptr;
+    int step = 0;
+};
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
                     const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr,
-                    unsigned long long *stamps = nullptr);
+                    unsigned long long *stamps = nullptr, FarPost post = {});
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s,
                     const DevStatus *st = nullptr, DevStatus *out = nullptr, double *hist = nullptr,
-                    unsigned long long *stamps = nullptr);
+                    unsigned long long *stamps = nullptr, FarPost post = {});
 // The differentiable run's step.  Before its push, in one launch: Ha = H + Q(E)
 // (the B half step, out of place, the bits of yee_b_half_*), J = 0 (three arrays
 // one after another) and, where keepE is given, a copy of E (three arrays).

@@ -248,8 +248,10 @@ constexpr int kHistRows = 4;
 template <typename T>
 __global__ void k_e_ghosts(Grid g, GhostPasses P, const DevStatus *st, DevStatus *out, const T *__restrict__ Ex,
                            const T *__restrict__ Ey, const T *__restrict__ Ez, double *hist,
-                           unsigned long long *stamps) {
+                           unsigned long long *stamps, FarPost post) {
     chain_enter();
+    if (post.host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        *(volatile unsigned long long *)post.host = (unsigned long long)(post.step + 1) << 32 | (unsigned)*post.far;
     if (out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < sizeof(DevStatus) / sizeof(unsigned))
         ((volatile unsigned *)out)[threadIdx.x] = ((const unsigned *)st)[threadIdx.x];
     if ((int)blockIdx.y >= P.n) {
@@ -833,7 +835,7 @@ void fold_b_twice_plain(const Grid &g, double *const F[12], cudaStream_t s) {
 // component, round B the second; both run in one launch (GhostPasses).
 template <typename T>
 static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                       DevStatus *out, double *hist, unsigned long long *stamps) {
+                       DevStatus *out, double *hist, unsigned long long *stamps, FarPost post) {
     int Nx = g.nx, Ny = g.ny, Nz = g.nz;
     GhostPasses P{};
     int maxn = 0;
@@ -852,15 +854,15 @@ static void e_ghosts_t(const Grid &g, T *Ex, T *Ey, T *Ez, int periodic, cudaStr
     add(Ey, 2, 0, Nx + 1, 0, Ny, Nz);
     if (periodic) add(Ez, 1, 0, Nx + 1, 0, Nz, Ny);
     launch_chained(k_e_ghosts<T>, dim3((maxn + 127) / 128, P.n + (hist ? kHistRows : 0)), dim3(128), s, g, P, st, out, Ex, Ey,
-                   Ez, hist, stamps);
+                   Ez, hist, stamps, post);
 }
 void e_ghosts_plain(const Grid &g, double *Ex, double *Ey, double *Ez, int periodic, cudaStream_t s,
-                    const DevStatus *st, DevStatus *out, double *hist, unsigned long long *stamps) {
-    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps);
+                    const DevStatus *st, DevStatus *out, double *hist, unsigned long long *stamps, FarPost post) {
+    e_ghosts_t<double>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps, post);
 }
 void e_ghosts_mixed(const Grid &g, float *Ex, float *Ey, float *Ez, int periodic, cudaStream_t s, const DevStatus *st,
-                    DevStatus *out, double *hist, unsigned long long *stamps) {
-    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps);
+                    DevStatus *out, double *hist, unsigned long long *stamps, FarPost post) {
+    e_ghosts_t<float>(g, Ex, Ey, Ez, periodic, s, st, out, hist, stamps, post);
 }
 
 // shared memory of the next particle of every thread
