@@ -78,7 +78,11 @@ StepParams make_params(pic_handle *h) {
     p.g = h->g;
     p.nsp = h->cfg.nspecies;
     p.mixed = h->mixed;
-    for (int s = 0; s < p.nsp; s++) p.sp[s] = h->sp[s].v;
+    p.slots = 0;
+    for (int s = 0; s < p.nsp; s++) {
+        p.sp[s] = h->sp[s].v;
+        p.slots = std::max<long long>(p.slots, h->sp[s].cap_total);
+    }
     for (int c = 0; c < 3; c++) {
         p.E[c] = h->f[PIC_EX + c];
         p.H[c] = h->f[PIC_HX + c];
@@ -1135,12 +1139,12 @@ int pic_e_ghosts(pic_handle *h) { return h ? (set_device(h) ? h->status : do_e_g
 
 namespace {
 
-// enqueues the field energies, and the kinetic energy of the last push where it
-// is current, into hred
-int enqueue_energy(pic_handle *h, bool kinetic) {
+// enqueues the field energies, and the kinetic energy at `kinetic` (device; null:
+// none), into hred
+int enqueue_energy(pic_handle *h, const double *kinetic) {
     const void *E[3] = {h->f[PIC_EX], h->f[PIC_EY], h->f[PIC_EZ]};
     const void *H[3] = {h->f[PIC_HX], h->f[PIC_HY], h->f[PIC_HZ]};
-    CK(field_energy(h->g, h->mixed, E, H, kinetic ? h->st : nullptr, h->dred, h->hred, h->stream), "field energy");
+    CK(field_energy(h->g, h->mixed, E, H, kinetic, h->dred, h->hred, h->stream), "field energy");
     return PIC_OK;
 }
 void energies_of(const pic_handle *h, double *out4) {
@@ -1178,7 +1182,7 @@ int step_impl(pic_handle *h, double *energies) {
     h->launches += 2;
     if ((rc = do_e_update(h))) return rc;
     if ((rc = do_e_ghosts(h, stamps))) return rc;
-    if (energies && (rc = enqueue_energy(h, true))) return rc;
+    if (energies && (rc = enqueue_energy(h, &h->st->kinetic))) return rc;
     CK(cudaStreamSynchronize(h->stream), "sync");
     rc = handle_status(h);
     h->counters[3] = h->launches;
@@ -1352,14 +1356,15 @@ int pic_energy(pic_handle *h, double *out4) {
     if (rc) return rc;
     rc = need_particles(h);
     if (rc) return rc;
-    if ((rc = enqueue_energy(h, h->kin_valid))) return rc;
+    const double *kinetic = &h->st->kinetic;  // of the last push, where it is current
     if (!h->kin_valid) {
         double *kin = h->dred + 4;
         CK(cudaMemsetAsync(kin, 0, sizeof(double), h->stream), "memset");
         StepParams p = make_params(h);
         CK(kinetic_energy(p, kin, h->stream), "kinetic");
-        CK(cudaMemcpyAsync(h->hred + 3, kin, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "D2H");
+        kinetic = kin;
     }
+    if ((rc = enqueue_energy(h, kinetic))) return rc;
     CK(cudaStreamSynchronize(h->stream), "sync");
     energies_of(h, out4);
     return PIC_OK;
@@ -1369,7 +1374,7 @@ int pic_energy_reference(pic_handle *h, double *out) {
     if (!h || !out) return set_err(h, PIC_ERR_ARG, "bad argument");
     int rc = set_device(h);
     if (rc) return rc;
-    if ((rc = enqueue_energy(h, false))) return rc;
+    if ((rc = enqueue_energy(h, nullptr))) return rc;
     CK(cudaStreamSynchronize(h->stream), "sync");
     *out = h->hred[2];
     return PIC_OK;

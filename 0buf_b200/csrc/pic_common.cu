@@ -478,7 +478,7 @@ __device__ __forceinline__ void load4(const double *p, double v[4]) {
 template <typename T>
 __global__ void k_field_energy(Grid g, const T *__restrict__ Ex, const T *__restrict__ Ey, const T *__restrict__ Ez,
                                const T *__restrict__ Hx, const T *__restrict__ Hy, const T *__restrict__ Hz,
-                               const DevStatus *st, double *scratch, double *host) {
+                               const double *kinetic, double *scratch, double *host) {
     chain_enter();
     __shared__ double red[32];
     __shared__ int last;
@@ -526,7 +526,7 @@ __global__ void k_field_energy(Grid g, const T *__restrict__ Ex, const T *__rest
         if (threadIdx.x == 0) ((volatile double *)host)[q] = t;
     }
     if (threadIdx.x == 0) {
-        if (st) ((volatile double *)host)[3] = st->kinetic;
+        if (kinetic) ((volatile double *)host)[3] = *kinetic;
         *ticket = 0u;  // for the next call
     }
 }
@@ -536,11 +536,15 @@ __global__ void k_kinetic(StepParams P, int shares, double *out) {
     __shared__ double red[32];
     const SpeciesView &S = P.sp[blockIdx.y];
     double M = S.m / S.q_m, acc = 0.0;
+    bool any = false;
     for (int u = blockIdx.x; u < P.g.ntiles * shares; u += gridDim.x) {
         const int t = u / shares, q = u - t * shares;
         const long long n = S.tile_count[t];
-        const int start = S.tile_start[t], jend = (int)(n * (q + 1) / shares);
-        for (int j = (int)(n * q / shares) + threadIdx.x; j < jend; j += 4 * blockDim.x) {
+        const int filled = shares_filled(n, shares);
+        if (q >= filled) continue;
+        any = true;
+        const int start = S.tile_start[t], jend = (int)(n * (q + 1) / filled);
+        for (int j = (int)(n * q / filled) + threadIdx.x; j < jend; j += 4 * blockDim.x) {
             double p[4][3];
             load_momenta4(P.mixed, S, start, j, jend, p);
 #pragma unroll
@@ -550,6 +554,7 @@ __global__ void k_kinetic(StepParams P, int shares, double *out) {
             }
         }
     }
+    if (!any) return;  // the whole block
     double tot = block_sum(acc, red);
     if (threadIdx.x == 0) atomicAdd(out, tot);
 }
@@ -694,17 +699,17 @@ cudaError_t init_cells(const Grid &g, int mixed, SpeciesView sv, int species_ind
     return cudaGetLastError();
 }
 
-cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], const DevStatus *st,
-                         double *scratch, double *host, cudaStream_t s) {
+cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3],
+                         const double *kinetic, double *scratch, double *host, cudaStream_t s) {
     const int bx = 256;
     const int64_t quads = (int64_t)g.NX * g.NY * (g.pz / 4);
     const dim3 grid((unsigned)std::min<int64_t>((quads + bx - 1) / bx, kEnergyBlocks));
     if (mixed)
         return launch_chained(k_field_energy<float>, grid, dim3(bx), s, g, (const float *)E[0], (const float *)E[1],
-                              (const float *)E[2], (const float *)H[0], (const float *)H[1], (const float *)H[2], st,
+                              (const float *)E[2], (const float *)H[0], (const float *)H[1], (const float *)H[2], kinetic,
                               scratch, host);
     return launch_chained(k_field_energy<double>, grid, dim3(bx), s, g, (const double *)E[0], (const double *)E[1],
-                          (const double *)E[2], (const double *)H[0], (const double *)H[1], (const double *)H[2], st,
+                          (const double *)E[2], (const double *)H[0], (const double *)H[1], (const double *)H[2], kinetic,
                           scratch, host);
 }
 
@@ -718,7 +723,7 @@ cudaError_t begin_push(const StepParams &p, size_t nodes, cudaStream_t s) {
 }
 
 cudaError_t kinetic_energy(const StepParams &p, double *out, cudaStream_t s) {
-    const int shares = tile_shares(p.g.ntiles);
+    const int shares = tile_shares(p, p.nsp);
     k_kinetic<<<dim3(std::min(p.g.ntiles * shares, 8 * kSMs), p.nsp), 256, 0, s>>>(p, shares, out);
     return cudaGetLastError();
 }

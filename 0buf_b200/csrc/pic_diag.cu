@@ -33,7 +33,7 @@ namespace pic {
 namespace {
 
 // The particles of every species in a share of a tile (blockIdx.y of
-// gridDim.y) add their eight weights into shared (tx+2)(ty+2)(tz+2) node boxes
+// shares_filled) add their eight weights into shared (tx+2)(ty+2)(tz+2) node boxes
 // in 64-bit fixed point (exact and order-independent: q = 2^(E-62) with 2^E >
 // sum |m| over the tile's particles, each node receives at most that much), and
 // the boxes are added into the global rho.  A contribution below 2^51 quanta
@@ -70,6 +70,10 @@ __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, int copies, d
     const int i0 = ti * tx, l0 = tl * ty, k0 = tk * tz;
     const int SX = tx + 2, SY = ty + 2, SZ = tz + 2;
     const int nn = SX * SY * SZ, stride = rho_stride(nn);
+    long long inside = 0;
+    for (int s = 0; s < nsp; s++) inside += sp[s].tile_count[t];
+    const int filled = shares_filled(inside, gridDim.y);
+    if ((int)blockIdx.y >= filled) return;  // the whole block
     if (threadIdx.x == 0) {
         double bound = 0.0, one = 0.0;
         for (int s = 0; s < nsp; s++) {
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__(256) k_charge_tile(StepParams P, int copies, d
         const SpeciesView &S = sp[s];
         const int start = S.tile_start[t];
         const long long all = S.tile_count[t];
-        const unsigned jbeg = (unsigned)(all * blockIdx.y / gridDim.y), jend = (unsigned)(all * (blockIdx.y + 1) / gridDim.y);
+        const unsigned jbeg = (unsigned)(all * blockIdx.y / filled), jend = (unsigned)(all * (blockIdx.y + 1) / filled);
         const double mq = S.m * inv_q;  // exact: inv_q is a power of two
         const int *cell = S.cell + start;
         const T *px = MIXED ? (const T *)(S.ox + start) : (const T *)(S.x + start);
@@ -244,11 +248,15 @@ __global__ void k_momentum(StepParams P, int shares, double *out) {
     const SpeciesView &S = P.sp[blockIdx.y];
     const double M = S.m / S.q_m;
     double acc[3] = {0.0, 0.0, 0.0};
+    bool any = false;
     for (int u = blockIdx.x; u < P.g.ntiles * shares; u += gridDim.x) {
         const int t = u / shares, q = u - t * shares;
         const long long n = S.tile_count[t];
-        const int start = S.tile_start[t], jend = (int)(n * (q + 1) / shares);
-        for (int j = (int)(n * q / shares) + threadIdx.x; j < jend; j += 4 * blockDim.x) {
+        const int filled = shares_filled(n, shares);
+        if (q >= filled) continue;
+        any = true;
+        const int start = S.tile_start[t], jend = (int)(n * (q + 1) / filled);
+        for (int j = (int)(n * q / filled) + threadIdx.x; j < jend; j += 4 * blockDim.x) {
             double p[4][3];
             load_momenta4(P.mixed, S, start, j, jend, p);
 #pragma unroll
@@ -257,6 +265,7 @@ __global__ void k_momentum(StepParams P, int shares, double *out) {
             }
         }
     }
+    if (!any) return;  // the whole block
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int a = 0; a < 3; a++) {
         double v = acc[a];
@@ -276,7 +285,7 @@ __global__ void k_momentum(StepParams P, int shares, double *out) {
 cudaError_t momentum(const StepParams &p, double *out, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(out, 0, 3 * p.nsp * sizeof(double), s);
     if (e != cudaSuccess) return e;
-    const int shares = tile_shares(p.g.ntiles);
+    const int shares = tile_shares(p, p.nsp);
     k_momentum<<<dim3(std::min(p.g.ntiles * shares, 8 * kSMs), p.nsp), 256, 0, s>>>(p, shares, out);
     return cudaGetLastError();
 }
@@ -296,7 +305,7 @@ cudaError_t charge_density(const StepParams &p, double *rho, cudaStream_t s) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<dim3(g.ntiles, tile_shares(g.ntiles)), 256, smem, s>>>(p, copies, rho);
+    k<<<dim3(g.ntiles, tile_shares(p, 1)), 256, smem, s>>>(p, copies, rho);
     for (int dir = 0; dir < 3; dir++) {
         const int A = dir == 0 ? g.NY : g.NX;
         const int B = dir == 2 ? g.NY : g.NZ;

@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 #include <utility>
 #include "pic0buf.h"
 
@@ -302,6 +303,7 @@ struct StepParams {
     int nsp;
     int mixed;
     SpeciesView sp[kMaxSpecies];
+    long long slots;  // of the species with the most
     // plain: double fields; mixed: float E/H, double J
     const void *E[3];
     const void *H[3];
@@ -340,9 +342,22 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Shares that a reduction over the bins deals a tile out in: enough blocks for
-// eight per SM where the tiles alone are too few.
-inline int tile_shares(int ntiles) { return ntiles >= 8 * kSMs ? 1 : (8 * kSMs + ntiles - 1) / ntiles; }
+// Shares that a reduction over the bins deals a tile out in, by `rows` rows of blocks
+// (one per species, or one for all): enough blocks for eight per SM where the tiles
+// alone are too few, but none of fewer than kShareLeast particles.  A momentum call on
+// 8x8x8 cells of 4 particles took 37 us with 3552 blocks of one or two particles each,
+// takes 25; 64x32x32 cells, eight species of 8, 62 and 47.
+constexpr int kShareLeast = 1024;
+inline int tile_shares(const StepParams &p, int rows) {
+    const int most = 8 * kSMs, tiles = p.g.ntiles * rows;
+    return (int)std::min<long long>((most + tiles - 1) / tiles, 1 + p.nsp / rows * p.slots / kShareLeast);
+}
+// those of them that a tile of n particles fills, one at least; blocks without a
+// share add nothing
+__device__ __forceinline__ int shares_filled(long long n, int shares) {
+    const long long s = (n + kShareLeast - 1) / kShareLeast;
+    return s < 1 ? 1 : (s < shares ? (int)s : shares);
+}
 
 // The particles of one species that slice q of P.slices of tile t handles:
 // [jbeg, jend) of the bin.  The bins of all species, cut into blocks of

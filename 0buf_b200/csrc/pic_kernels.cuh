@@ -107,11 +107,11 @@ cudaError_t init_species_bins(const Grid &g, int mixed, SpeciesView sv, int spec
 cudaError_t init_cells(const Grid &g, int mixed, SpeciesView sv, int species_index, const int *count,
                        const int *first, double dx, double dy, double dz, double vth, uint64_t seed, cudaStream_t s);
 // FP64 reductions: host[0] sum E^2, host[1] sum H^2 over nodes 1..N, host[2] sum E^2 all nodes (reference), host[3]
-// st->kinetic (st null: left alone).  host: pinned memory, written by the kernel; scratch: kEnergyScratch doubles,
+// *kinetic (null: left alone).  host: pinned memory, written by the kernel; scratch: kEnergyScratch doubles,
 // the first zero before the first call
 constexpr int kEnergyBlocks = 8 * kSMs, kEnergyScratch = 8 + 3 * kEnergyBlocks;
-cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3], const DevStatus *st,
-                         double *scratch, double *host, cudaStream_t s);
+cudaError_t field_energy(const Grid &g, int mixed, const void *const E[3], const void *const H[3],
+                         const double *kinetic, double *scratch, double *host, cudaStream_t s);
 cudaError_t kinetic_energy(const StepParams &p, double *out, cudaStream_t s);
 // charge-conservation diagnostic (pic_diag.cu, FP64): rho on the cell-centre
 // nodes, folded; G = div E - rho on interior nodes with reductions
