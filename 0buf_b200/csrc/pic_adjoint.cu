@@ -1295,12 +1295,15 @@ int64_t total_particles(const AdjState &A) {
     return t;
 }
 
-constexpr int kFarPoll = 8;  // (see far_passed)
+// (see far_passed) two words in turn: the host has read one before the step that
+// writes there again is enqueued
+constexpr int kFarPoll = 8;
+unsigned long long *far_slot(pic_handle *h, int n) { return (unsigned long long *)(h->hred + 6 + (n / kFarPoll & 1)); }
 FarPost far_post(pic_handle *h, const AdjState &A, const double *hist, int n) {
     FarPost p;
     if (hist && n % kFarPoll == kFarPoll - 1 && n < A.direct_from) {
         p.far = A.far + n;
-        p.host = (unsigned long long *)(h->hred + 7);
+        p.host = far_slot(h, n);
         p.step = n;
     }
     return p;
@@ -1537,7 +1540,7 @@ int reverse_direct_from(const std::vector<int> &far, int known, double particles
 // which enqueues ahead, waits there for the count of kFarPoll + 1 steps ago.  The
 // device still has kFarPoll steps to do then.
 bool far_passed(pic_handle *h, int n, double limit) {
-    const volatile unsigned long long *slot = (const volatile unsigned long long *)(h->hred + 7);
+    const volatile unsigned long long *slot = far_slot(h, n);
     for (long long spin = 1;; spin++) {
         const unsigned long long v = *slot;
         if ((int)(v >> 32) >= n + 1) return (double)(unsigned)v > limit;
@@ -1555,7 +1558,7 @@ int forward_run(pic_handle *h, AdjState &A) {
     const size_t fbytes = field_bytes(h);
     const double particles = (double)total_particles(A);
     const double limit = particles * far_limit(h->mixed, false, particles / ((double)A.nsp * g.ncells()));
-    *(volatile unsigned long long *)(h->hred + 7) = 0ull;
+    for (int q = 0; q < 2; q++) *(volatile unsigned long long *)far_slot(h, q * kFarPoll) = 0ull;
     CK(cudaEventRecord(A.e0, st), "event");
     for (int n = 0; n < A.steps; n++) {
         if (n >= 2 * kFarPoll && n % kFarPoll == 0 && A.direct_from == A.steps && far_passed(h, n - kFarPoll - 1, limit))
